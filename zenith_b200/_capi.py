@@ -6,9 +6,12 @@ this package fails.  Build it with ``python -m zenith_b200.build``.
 from __future__ import annotations
 
 import ctypes as C
+from importlib.machinery import ExtensionFileLoader
+from importlib.util import module_from_spec, spec_from_file_location
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libzenith_b200.so"
+NATIVE_PATH = LIB_PATH.parent / "_native.so"
 
 OK, ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_LAUNCH, ERR_TIMEOUT, ERR_DRIVER, ERR_TOO_LARGE = range(7)
 DT_S32, DT_F32, DT_F16, DT_S8 = range(4)
@@ -115,6 +118,23 @@ def lib() -> C.CDLL:
             fn.restype = _RESTYPES.get(name, C.c_int)
         _lib = handle
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The native host path of the operators (``csrc/host/native_ops.cpp``), loaded once."""
+    global _native
+    if _native is None:
+        if not NATIVE_PATH.exists():
+            raise RuntimeError(f"{NATIVE_PATH} is missing: build the extension with `python -m zenith_b200.build`")
+        spec = spec_from_file_location("zenith_b200._native", NATIVE_PATH,
+                                       loader=ExtensionFileLoader("zenith_b200._native", str(NATIVE_PATH)))
+        module = module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def status_string(status: int) -> str:

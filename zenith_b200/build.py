@@ -1,4 +1,5 @@
-"""Builds ``zenith_b200/lib/libzenith_b200.so`` from ``zenith_b200/csrc/*.cu`` with nvcc for sm_100a.
+"""Builds ``zenith_b200/lib/libzenith_b200.so`` from ``zenith_b200/csrc/*.cu`` with nvcc for sm_100a, and
+``zenith_b200/lib/_native.so`` (the native host path of the operators, against torch's headers) with g++.
 
 The library links against the static CUDA runtime only, so it loads on a machine without a
 driver (compute entry points then return an error status).  Objects are rebuilt only when a
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -21,6 +23,8 @@ INCLUDE = PKG.parent / "include"
 LIB_DIR = PKG / "lib"
 OBJ_DIR = LIB_DIR / "obj"
 LIB_PATH = LIB_DIR / "libzenith_b200.so"
+NATIVE_SRC = CSRC / "host" / "native_ops.cpp"
+NATIVE_PATH = LIB_DIR / "_native.so"
 
 NVCC_FLAGS = [
     "-std=c++17",
@@ -78,7 +82,29 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_native(force)
     return LIB_PATH
+
+
+def _build_native(force: bool) -> None:
+    """The Python module: linked against the library beside it (found through ``$ORIGIN``) and torch's libraries, which
+    the interpreter has loaded by the time it imports this one."""
+    newest = max(p.stat().st_mtime for p in (NATIVE_SRC, INCLUDE / "zenith_b200.h", Path(__file__)))
+    if not force and NATIVE_PATH.exists() and NATIVE_PATH.stat().st_mtime > newest:
+        return
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
+           cuda / "include"]
+    cmd = ["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden", "-DUSE_CUDA",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in inc], str(NATIVE_SRC),
+           f"-L{LIB_DIR}", "-lzenith_b200", "-Wl,-rpath,$ORIGIN", f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cuda",
+           "-ltorch_cpu", "-lc10_cuda", "-lc10", "-o", str(NATIVE_PATH)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {NATIVE_SRC.name}:\n{r.stdout}\n{r.stderr}")
 
 
 if __name__ == "__main__":
