@@ -101,7 +101,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * FA_BQ;  // 0: the grid has one query tile
   const int h = blockIdx.y;
@@ -151,7 +151,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0 && any_keys) {
+    if (any_keys && elect_one()) {
       mbar_arrive_expect_tx(qk_full, 2 * TILE_BYTES);
 #pragma unroll
       for (int dc = 0; dc < DC; ++dc) {
@@ -164,7 +164,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && any_keys) {
+    if (any_keys && elect_one()) {
       bool ok = mbar_wait(qk_full, 0, abort_flag);
       if (ok) {
         tc_fence_after_sync();

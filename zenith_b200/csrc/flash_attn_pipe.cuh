@@ -68,7 +68,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * 256;
   const int h = blockIdx.y;
@@ -139,7 +139,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0 && n_blocks > 0) {
+    if (n_blocks > 0 && elect_one()) {
       bool ok = true;
       mbar_arrive_expect_tx(q_full, 2 * TILE_BYTES);
 #pragma unroll
@@ -167,7 +167,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_blocks > 0) {
+    if (n_blocks > 0 && elect_one()) {
       auto issue_qk = [&](int g, int j) {
         const uint32_t qa = smem_u32(sQ + g * TILE_BYTES);
         const uint32_t ka = smem_u32(sK + (j % KV_STAGES) * TILE_BYTES);

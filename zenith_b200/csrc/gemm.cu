@@ -131,18 +131,24 @@ static int run_gemm(const void* A, int64_t lda, const void* B, int64_t ldb, Gemm
   else st = encode_tmap_2d(&tb, tmap_dtype<KIND>(), B, uint64_t(p.N), uint64_t(p.K), uint64_t(ldb) * ELEM, BK, BK);
   if (st != ZEN_OK) return st;
   p.num_k_blocks = (p.K + BK - 1) / BK;
-  // fp16 / int8 outputs with 16-byte aligned rows leave through shared memory and TMA stores of
-  // 32-row x 64-column blocks; anything else is stored by the epilogue threads directly
+  // Outputs with 16-byte aligned rows leave through shared memory: fp16 / int8 by TMA stores of 32-row blocks, one slab
+  // wide, 4-byte types as row pieces; anything else is stored by the epilogue threads directly
   CUtensorMap tc = ta;
   p.staged_store = 0;
   const int oelem = p.out_dtype == ZEN_DT_S8 ? 1 : p.out_dtype == ZEN_DT_F16 ? 2 : 4;
-  if ((p.out_dtype == ZEN_DT_F16 || p.out_dtype == ZEN_DT_S8) && reinterpret_cast<uintptr_t>(p.out) % 16 == 0 &&
-      (p.ldo * oelem) % 16 == 0) {
-    st = encode_tmap_2d(&tc, p.out_dtype == ZEN_DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8,
-                        p.out, uint64_t(p.N), uint64_t(p.M), uint64_t(p.ldo) * oelem, 64, 32,
-                        p.out_dtype == ZEN_DT_F16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
-    if (st != ZEN_OK) return st;
+  if (reinterpret_cast<uintptr_t>(p.out) % 16 == 0 && (p.ldo * oelem) % 16 == 0) {
     p.staged_store = 1;
+    if (oelem < 4) {
+      constexpr int SLAB = gemm_slab_cols<BN>();
+      const int row_bytes = SLAB * oelem;
+      st = encode_tmap_2d(&tc, p.out_dtype == ZEN_DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8,
+                          p.out, uint64_t(p.N), uint64_t(p.M), uint64_t(p.ldo) * oelem, SLAB, 32,
+                          row_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                          : row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                          : row_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                            : CU_TENSOR_MAP_SWIZZLE_NONE);
+      if (st != ZEN_OK) return st;
+    }
   }
   if constexpr (PAIR) return launch_gemm_pair<KIND, BN, STAGES>(ta, tb, tc, p, stream);
   else return launch_gemm<KIND, BN, STAGES, B_MN>(ta, tb, tc, p, stream);

@@ -102,7 +102,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* epi_rows = reinterpret_cast<float*>(ctrl + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int cluster_id = blockIdx.x / LN_CLUSTER;
@@ -141,10 +141,9 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
   const uint32_t tmem_base = *tmem_slot;
   grid_launch_dependents();
   // constant weights: request the first weight tiles while the previous kernel may still be running
-  // (see gemm_tc_kernel); `pre` lives in the producer thread
-  int pre = 0;
-  if (threadIdx.x == 0 && p.early_b && cluster_id < p.tiles_m) {
-    pre = nkb < STAGES ? nkb : STAGES;
+  // (see gemm_tc_kernel)
+  const int pre = p.early_b && cluster_id < p.tiles_m ? (nkb < STAGES ? nkb : STAGES) : 0;
+  if (warp == 0 && elect_one()) {
     for (int kb = 0; kb < pre; ++kb) {
       mbar_arrive_expect_tx(&full_bar[kb], STAGE_BYTES);
       tma_load_2d(smem + size_t(kb) * STAGE_BYTES + A_BYTES, &tmap_b, &full_bar[kb], kb * BK, n_base);
@@ -154,7 +153,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -189,7 +188,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;

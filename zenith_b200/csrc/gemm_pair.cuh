@@ -23,7 +23,7 @@ template <int BN, int STAGES>
 __host__ __device__ constexpr size_t gemm_pair_smem_bytes() {
   // ring (A 16 KB + B BN/2 x 128 B per stage) + output staging (4 KB per active epilogue warp) + barriers / flags
   // (256 B) + per-epilogue-warp scale and bias entries + alignment slack
-  return size_t(STAGES) * (GEMM_BM * 128 + (BN / 2) * 128) + size_t((BN + 63) / 64) * 4 * 4096 + 256 +
+  return size_t(STAGES) * (GEMM_BM * 128 + (BN / 2) * 128) + size_t(gemm_stage_total<BN>()) + 256 +
          size_t(GEMM_EPI_WARPS) * 3 * 64 * 4 + 1024;
 }
 
@@ -53,9 +53,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  constexpr int SLABS = (BN + 63) / 64;
-  uint8_t* out_stage = smem + size_t(STAGES) * STAGE_BYTES;  // [SLABS][4 quadrants][4 KB], 1024-byte aligned
-  uint8_t* ctrl = out_stage + size_t(SLABS) * 4 * 4096;
+  uint8_t* out_stage = smem + size_t(STAGES) * STAGE_BYTES;  // one staging block per epilogue warp, 1024-byte aligned
+  uint8_t* ctrl = out_stage + gemm_stage_total<BN>();
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);  // used in the leader only
   uint64_t* empty_bar = full_bar + STAGES;                  // one set per CTA, signalled by the leader's commits
   uint64_t* tfull_bar = empty_bar + STAGES;                 // one set per CTA, signalled by the leader's commits
@@ -64,7 +63,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* epi_rows = reinterpret_cast<float*>(ctrl + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0: leader
   const bool leader = rank == 0;
@@ -76,7 +75,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (p.staged_store) tma_prefetch_desc(&tmap_c);
+    tma_prefetch_desc(&tmap_c);
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
@@ -108,10 +107,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   grid_launch_dependents();
   // Constant weights: the B tiles of the first tile's first k-blocks are requested before the dependency wait
   // (see gemm_tc_kernel); the leader announces the bytes of the whole stage (both CTAs, A and B).
-  int pre = 0;
-  if (threadIdx.x == 0 && p.early_b && pair < num_tiles) {
+  const int pre = p.early_b && pair < num_tiles ? (nkb < STAGES ? nkb : STAGES) : 0;
+  if (warp == 0 && elect_one()) {
     const int n0 = (pair / p.tiles_m) * BN + int(rank) * HALF_N;
-    pre = nkb < STAGES ? nkb : STAGES;
     for (int kb = 0; kb < pre; ++kb) {
       if (leader) mbar_arrive_expect_tx(&full_bar[kb], 2 * STAGE_BYTES);
       tma_load_2d_pair(smem + size_t(kb) * STAGE_BYTES + A_BYTES, &tmap_b, full_bar_leader + uint32_t(kb) * 8u, kb * BK, n0);
@@ -121,7 +119,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (each CTA: its own halves)
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -156,7 +154,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;

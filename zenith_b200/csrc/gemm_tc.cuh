@@ -4,11 +4,11 @@
 //
 //   warp 0      : TMA producer  — 128-byte-swizzled tiles of A and B into a STAGES-deep ring
 //   warp 1      : allocates TMEM, issues tcgen05.mma (one lane), commits stage / accumulator barriers
-//   warps 2..17 : epilogue — four warps per 32-lane TMEM quadrant, each owning one 64-column slab of the
-//                 tile: tcgen05.ld in 16-column steps, dequant / bias / activation / requant, then the
-//                 32 x 64 block is staged in swizzled shared memory and written by one TMA store
-//                 (full 128-byte lines; edges clipped by the tensor map).  fp32 / int32 outputs and
-//                 unaligned outputs use per-thread 16-byte global stores instead.
+//   warps 2..17 : epilogue — four warps per 32-lane TMEM quadrant, each owning one slab (64 columns, a quarter
+//                 of a narrow tile) of the tile: tcgen05.ld in 16-column steps, dequant / bias / activation / requant, then the
+//                 32-row block is staged in swizzled shared memory and written by one TMA store
+//                 (full 128-byte lines; edges clipped by the tensor map).  fp32 / int32 outputs leave as
+//                 row pieces from the same staging memory, unaligned outputs straight from the threads.
 //
 // TMEM holds two accumulators (2 x BN columns) so the epilogue of tile i overlaps the MMAs of
 // tile i+1.  CTAs are persistent: tile t = blockIdx.x + i * gridDim.x, M-fastest.
@@ -36,7 +36,7 @@ struct GemmParams {
   float out_scale;
   const float* w_scale;
   const float* bias;
-  int staged_store;  // 1: fp16 / int8 output leaves through shared memory and TMA stores
+  int staged_store;  // 1: the output leaves through shared memory (fp16 / int8: TMA stores; 4-byte types: transposed row pieces)
   // L2 prefetch hint: read-only ranges (16-byte aligned, sizes multiples of 16) that later kernels will
   // read, e.g. the next GEMMs' weights; every CTA asks for its slice while it waits for its own operands
   const uint8_t* pf_ptr[2];
@@ -80,6 +80,24 @@ constexpr int GEMM_BM = 128;
 constexpr int GEMM_EPI_WARPS = 16;
 constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
 
+// Columns of the tile that one epilogue warp works on: narrow tiles are spread over all 16 warps too (with 64-column slabs a
+// 128 x 64 tile kept 4 of them busy and its epilogue, exposed when a CTA has one tile, took four times as long).
+template <int BN>
+__host__ __device__ constexpr int gemm_slab_cols() { return BN <= 128 ? BN / 4 : 64; }
+
+// Staging block of one epilogue warp: 32 rows of its slab in fp16, and at least one 16-column step of 4-byte outputs.
+template <int BN>
+__host__ __device__ constexpr int gemm_stage_bytes() { return 64 * gemm_slab_cols<BN>() > 2048 ? 64 * gemm_slab_cols<BN>() : 2048; }
+template <int BN>
+__host__ __device__ constexpr int gemm_stage_total() { return BN / gemm_slab_cols<BN>() * 4 * gemm_stage_bytes<BN>(); }
+
+// 16-byte unit `u` of row `r` in a staging block with rows of ROW_BYTES: the swizzle of the output tensor map.
+template <int ROW_BYTES>
+__device__ __forceinline__ int stage_unit(int u, int r) {
+  static_assert(ROW_BYTES == 128 || ROW_BYTES == 64 || ROW_BYTES == 32 || ROW_BYTES == 16, "row");
+  return ROW_BYTES == 128 ? u ^ (r & 7) : ROW_BYTES == 64 ? u ^ ((r >> 1) & 3) : ROW_BYTES == 32 ? u ^ ((r >> 2) & 1) : u;
+}
+
 template <int BN>
 __host__ __device__ constexpr uint32_t gemm_tmem_cols() {
   return 2 * BN <= 32 ? 32u : 2 * BN <= 64 ? 64u : 2 * BN <= 128 ? 128u : 2 * BN <= 256 ? 256u : 512u;
@@ -87,9 +105,9 @@ __host__ __device__ constexpr uint32_t gemm_tmem_cols() {
 
 template <int BN, int STAGES>
 __host__ __device__ constexpr size_t gemm_smem_bytes() {
-  // ring + output staging (4 KB per active epilogue warp) + barriers/flags (256 B) + per-epilogue-warp
+  // ring + output staging of the active epilogue warps + barriers/flags (256 B) + per-epilogue-warp
   // scale and bias entries + alignment slack
-  return size_t(STAGES) * (GEMM_BM * 128 + BN * 128) + size_t((BN + 63) / 64) * 4 * 4096 + 256 +
+  return size_t(STAGES) * (GEMM_BM * 128 + BN * 128) + size_t(gemm_stage_total<BN>()) + 256 +
          size_t(GEMM_EPI_WARPS) * 3 * 64 * 4 + 1024;
 }
 
@@ -177,19 +195,49 @@ __device__ __forceinline__ void pack_q(const int (&q)[GEMM_CW], uint32_t (&packe
                 ((uint32_t(q[4 * j + 2]) & 0xffu) << 16) | ((uint32_t(q[4 * j + 3]) & 0xffu) << 24);
 }
 
+// 16 four-byte columns of 32 rows (lane = row) to global memory through the warp's 2 KB staging block: each lane then stores
+// 16-byte pieces so that four lanes cover the 64 contiguous bytes of a row.  Stored straight from the lanes, every
+// instruction touched 32 rows with half-used sectors (a 4096 x 768 fp32 output: 10.4 us, this way 7.1).  Warp-collective.
+__device__ __forceinline__ void store_rows_4byte(const uint32_t (&w)[GEMM_CW], uint8_t* stage, int lane, const GemmParams& p, int row0,
+                                                 int col0) {
+  __syncwarp();  // the previous step's pieces have been read
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    *reinterpret_cast<uint4*>(stage + lane * 64 + (stage_unit<64>(u, lane) << 4)) = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
+  __syncwarp();
+  const int u = lane & 3, col = col0 + 4 * u;
+  uint32_t* out = static_cast<uint32_t*>(p.out);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = 8 * k + (lane >> 2);
+    const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 64 + (stage_unit<64>(u, r) << 4));
+    if (row0 + r >= p.M) continue;
+    uint32_t* o = out + int64_t(row0 + r) * p.ldo + col;
+    if (col + 4 <= p.N) *reinterpret_cast<uint4*>(o) = v;
+    else {
+      if (col < p.N) o[0] = v.x;
+      if (col + 1 < p.N) o[1] = v.y;
+      if (col + 2 < p.N) o[2] = v.z;
+    }
+  }
+}
+
 // One GEMM_CW-column step of one accumulator row: dequant / bias / activation / conversion / store.
 // OUT and ACT are compile-time so that the independent element chains carry no branches and the
 // compiler can interleave them.
-// `stage` != nullptr: this lane's row of the warp's staging block (fp16: 128-byte rows, 128B swizzle;
-// int8: 64-byte rows, 64B swizzle — the layouts the output tensor map expects); `istep` is the
-// position of the step inside the 64-column slab.
-template <int KIND, int OUT, int ACT>
+// `stage` != nullptr: the warp's staging block of 32 rows of SLAB columns, swizzled as the output tensor map expects;
+// `istep` is the position of the step inside the slab.
+template <int KIND, int OUT, int ACT, int SLAB>
 __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], const float* sc, const float* bi,
                                                const GemmParams& p, int row, int col0, bool full, float inv_scale,
                                                uint8_t* stage, int lane, int istep) {
   constexpr int CW = GEMM_CW;
   const int nvalid = p.N - col0;  // >= 1
   if constexpr (OUT == ZEN_DT_S32) {
+    if (stage != nullptr) {
+      store_rows_4byte(r, stage, lane, p, row - lane, col0);
+      return;
+    }
     int32_t* o = static_cast<int32_t*>(p.out) + int64_t(row) * p.ldo + col0;
     if (full) store_words<CW>(o, r);
     else {
@@ -247,7 +295,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], con
       }
       pack_q(q, w);
       if (stage != nullptr) {
-        *reinterpret_cast<uint4*>(stage + lane * 64 + ((istep ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(stage + lane * SLAB + (stage_unit<SLAB>(istep, lane) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         return;
       }
       int8_t* o = static_cast<int8_t*>(p.out) + int64_t(row) * p.ldo + col0;
@@ -266,6 +314,10 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], con
         if constexpr (ACT == ZEN_ACT_RELU) y[j] = y[j] > 0.0f ? y[j] : 0.0f;
       }
       if constexpr (OUT == ZEN_DT_F32) {
+        if (stage != nullptr) {
+          store_rows_4byte(reinterpret_cast<const uint32_t(&)[CW]>(y), stage, lane, p, row - lane, col0);
+          return;
+        }
         float* o = static_cast<float*>(p.out) + int64_t(row) * p.ldo + col0;
         if (full) store_words<CW>(o, reinterpret_cast<const uint32_t*>(y));
         else {
@@ -282,9 +334,9 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], con
           w[j] = *reinterpret_cast<const uint32_t*>(&h);
         }
         if (stage != nullptr) {
-          uint8_t* srow = stage + lane * 128;
-          *reinterpret_cast<uint4*>(srow + (((2 * istep) ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-          *reinterpret_cast<uint4*>(srow + (((2 * istep + 1) ^ (lane & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+          uint8_t* srow = stage + lane * (2 * SLAB);
+          *reinterpret_cast<uint4*>(srow + (stage_unit<2 * SLAB>(2 * istep, lane) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(srow + (stage_unit<2 * SLAB>(2 * istep + 1, lane) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
           return;
         }
         if (full) store_words<CW / 2>(o, w);
@@ -395,7 +447,7 @@ __device__ __noinline__ void requant_i8_fixup(uint32_t taddr, const float* sc, c
 }
 
 // One step of the int8 -> int8 nearest-even epilogue (all 32 lanes must call it).
-template <int ACT>
+template <int ACT, int SLAB>
 __device__ __forceinline__ void epilogue_step_s8(const uint32_t (&r)[GEMM_CW], uint32_t taddr, const float* sc,
                                                  const float* bi, const float* fold, float risk_thr, const GemmParams& p,
                                                  int row, int col0, bool row_ok, bool vec_ok, float inv_scale,
@@ -406,7 +458,7 @@ __device__ __forceinline__ void epilogue_step_s8(const uint32_t (&r)[GEMM_CW], u
   int8_t* dst;
   bool live;
   if (stage != nullptr) {
-    dst = reinterpret_cast<int8_t*>(stage + lane * 64 + ((istep ^ ((lane >> 1) & 3)) << 4));
+    dst = reinterpret_cast<int8_t*>(stage + lane * SLAB + (stage_unit<SLAB>(istep, lane) << 4));
     live = true;
     *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
   } else {
@@ -427,16 +479,16 @@ __device__ __forceinline__ void epilogue_step_s8(const uint32_t (&r)[GEMM_CW], u
   if (any != 0) requant_i8_fixup<ACT>(taddr, sc, bi, p.x_scale, p.out_scale, any, redo, dst);
 }
 
-template <int KIND, int OUT>
+template <int KIND, int OUT, int SLAB>
 __device__ __forceinline__ void epilogue_chunk_act(const uint32_t (&r)[GEMM_CW], const float* sc, const float* bi,
                                                    const GemmParams& p, int row, int col0, bool full, float inv_scale,
                                                    uint8_t* stage, int lane, int istep) {
   if (p.act == ZEN_ACT_GELU)
-    epilogue_chunk<KIND, OUT, ZEN_ACT_GELU>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_GELU, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
   else if (p.act == ZEN_ACT_RELU)
-    epilogue_chunk<KIND, OUT, ZEN_ACT_RELU>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_RELU, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
   else
-    epilogue_chunk<KIND, OUT, ZEN_ACT_NONE>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_NONE, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -470,27 +522,29 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
                                                    int lane, int first_tile, int tile_step, int num_tiles, int row_off) {
   constexpr int TILE_M = PAIR ? 2 * GEMM_BM : GEMM_BM;
   const int quad = warp & 3;        // TMEM lane quadrant this warp may read: rows quad*32 .. +31 of the CTA's 128
-  const int sub = (warp - 2) >> 2;  // 64-column slab of the tile owned by this warp
-  constexpr int STEPS = 64 / GEMM_CW;
-  if (sub * 64 < BN) {
+  const int sub = (warp - 2) >> 2;  // slab of the tile owned by this warp
+  constexpr int SLAB = gemm_slab_cols<BN>();
+  constexpr int STEPS = SLAB / GEMM_CW;
+  if (sub * SLAB < BN) {
     float* s_scale = epi_rows + (warp - 2) * 3 * 64;
     float* s_bias = s_scale + 64;
     float* s_fold = s_bias + 64;  // fl(x_scale * w_scale[n]): the one-multiply form of the int8 -> int8 fast path
-    const int slab_cols = (BN - sub * 64) < 64 ? (BN - sub * 64) : 64;
     const int elem = p.out_dtype == ZEN_DT_S8 ? 1 : p.out_dtype == ZEN_DT_F16 ? 2 : 4;
     const bool vec_ok = (reinterpret_cast<uintptr_t>(p.out) % 16 == 0) && ((p.ldo * elem) % 16 == 0);
     const bool staged = p.staged_store != 0;
-    uint8_t* stage = staged ? out_stage + size_t(sub * 4 + quad) * 4096 : nullptr;
+    const bool tma_out = staged && elem != 4;
+    uint8_t* stage = staged ? out_stage + size_t(sub * 4 + quad) * gemm_stage_bytes<BN>() : nullptr;
     const float inv_scale = ZEN_DIV(1.0f, p.out_scale);
     int acc = 0;
     uint32_t acc_phase = 0;
     // Per-column scale and bias of the slab: lane l holds columns l and l + 32.  The values of the
     // next tile are fetched while the current tile's steps run, so that no tile starts on a global load.
     auto fetch_cols = [&](int tile, float (&sv)[2], float (&bv)[2]) {
-      const int nn = (tile / p.tiles_m) * BN + sub * 64;
+      const int nn = (tile / p.tiles_m) * BN + sub * SLAB;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int col = nn + lane + 32 * u;
+        if (32 * u >= SLAB) break;
         // predicated loads with no dependent instruction behind them: the warp issues in order and
         // would otherwise sit on the load until it returns
         sv[u] = 1.0f;
@@ -503,7 +557,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
     if (first_tile < num_tiles) fetch_cols(first_tile, sv, bv);
     for (int tile = first_tile; tile < num_tiles; tile += tile_step) {
       const int m0 = (tile % p.tiles_m) * TILE_M + row_off;
-      const int n0 = (tile / p.tiles_m) * BN + sub * 64;
+      const int n0 = (tile / p.tiles_m) * BN + sub * SLAB;
       __syncwarp();
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
@@ -516,7 +570,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
       const float bmax = __int_as_float(__reduce_max_sync(0xffffffffu, max(__float_as_int(fabsf(bv[0])), __float_as_int(fabsf(bv[1])))));
       const float risk_thr = 0.5f - 2e-6f - inv_scale * fmaf(4.2e-7f, bmax, 1.6e-7f);
       if (tile + tile_step < num_tiles) fetch_cols(tile + tile_step, sv, bv);
-      if (staged) {
+      if (tma_out) {
         if (lane == 0) tma_store_wait_read();  // the previous tile's store has finished reading the block
       }
       __syncwarp();
@@ -524,13 +578,12 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
       tc_fence_after_sync();
       const int row = m0 + quad * 32 + lane;
       const bool row_ok = row < p.M;
-      const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(acc * BN + sub * 64);
+      const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(acc * BN + sub * SLAB);
       // The loop is kept rolled: the step body (above all the GELU + requant one) is large, and
       // unrolling it made instruction fetch the bottleneck.  (Requesting the columns of step i + 1
       // before working on step i was tried twice and lost both times: 16 more live registers.)
 #pragma unroll 1
       for (int i = 0; i < STEPS; ++i) {
-        if (i * GEMM_CW >= slab_cols) break;
         uint32_t r[GEMM_CW];
         __syncwarp();
         tmem_ld_32x16(tacc + uint32_t(i * GEMM_CW), r);
@@ -543,11 +596,11 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
             const float* fo = s_fold + i * GEMM_CW;
             const uint32_t ta = tacc + uint32_t(i * GEMM_CW);
             if (p.act == ZEN_ACT_GELU)
-              epilogue_step_s8<ZEN_ACT_GELU>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
+              epilogue_step_s8<ZEN_ACT_GELU, SLAB>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
             else if (p.act == ZEN_ACT_RELU)
-              epilogue_step_s8<ZEN_ACT_RELU>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
+              epilogue_step_s8<ZEN_ACT_RELU, SLAB>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
             else
-              epilogue_step_s8<ZEN_ACT_NONE>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
+              epilogue_step_s8<ZEN_ACT_NONE, SLAB>(r, ta, sc, bi, fo, risk_thr, p, row, col0, row_ok, vec_ok, inv_scale, stage, lane, i);
             continue;
           }
         }
@@ -558,23 +611,23 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
         if constexpr (KIND == KIND_I8) {
           switch (p.out_dtype) {
             case ZEN_DT_S32:
-              epilogue_chunk<KIND, ZEN_DT_S32, ZEN_ACT_NONE>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+              epilogue_chunk<KIND, ZEN_DT_S32, ZEN_ACT_NONE, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
               break;
-            case ZEN_DT_F32: epilogue_chunk_act<KIND, ZEN_DT_F32>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
-            case ZEN_DT_F16: epilogue_chunk_act<KIND, ZEN_DT_F16>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
-            default: epilogue_chunk_act<KIND, ZEN_DT_S8>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
+            case ZEN_DT_F32: epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
+            case ZEN_DT_F16: epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
+            default: epilogue_chunk_act<KIND, ZEN_DT_S8, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
           }
         } else {
           if (p.out_dtype == ZEN_DT_F32)
-            epilogue_chunk_act<KIND, ZEN_DT_F32>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+            epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
           else
-            epilogue_chunk_act<KIND, ZEN_DT_F16>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+            epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
         }
       }
       __syncwarp();
       tc_fence_before_sync();
       release_accumulator<PAIR>(tempty, acc, lane);  // the accumulator is free as soon as it has been read
-      if (staged) {
+      if (tma_out) {
         fence_proxy_async_smem();  // this lane's writes to the block -> visible to the TMA engine
         __syncwarp();
         if (lane == 0 && n0 < p.N && m0 + quad * 32 < p.M) {
@@ -585,7 +638,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
-    if (staged && lane == 0) tma_store_wait_all();
+    if (tma_out && lane == 0) tma_store_wait_all();
   } else {
     // no slab for this warp at this tile width: it still owes its arrivals on the accumulator barriers
     int acc = 0;
@@ -621,9 +674,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  constexpr int SLABS = (BN + 63) / 64;  // 64-column slabs of the tile, one per epilogue warp of a quadrant
-  uint8_t* out_stage = smem + size_t(STAGES) * STAGE_BYTES;  // [SLABS][4 quadrants][4 KB], 1024-byte aligned
-  uint8_t* ctrl = out_stage + size_t(SLABS) * 4 * 4096;
+  uint8_t* out_stage = smem + size_t(STAGES) * STAGE_BYTES;  // one staging block per epilogue warp, 1024-byte aligned
+  uint8_t* ctrl = out_stage + gemm_stage_total<BN>();
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;
@@ -632,7 +684,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* epi_rows = reinterpret_cast<float*>(ctrl + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int nkb = p.num_k_blocks;
@@ -640,7 +692,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (p.staged_store) tma_prefetch_desc(&tmap_c);
+    tma_prefetch_desc(&tmap_c);
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
@@ -669,12 +721,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   grid_launch_dependents();
   // Constant weights: the B tiles of the first tile's first k-blocks are requested now, while the previous
   // kernel may still be running (this CTA became resident when that kernel's CTA left the SM); only the A
-  // tiles, which the previous kernel may be writing, wait.  `pre` lives in the producer thread.
+  // tiles, which the previous kernel may be writing, wait.
   int pre = 0;
   if constexpr (!B_MN) {
-    if (threadIdx.x == 0 && p.early_b && int(blockIdx.x) < num_tiles) {
+    if (p.early_b && int(blockIdx.x) < num_tiles) pre = nkb < STAGES ? nkb : STAGES;
+    if (warp == 0 && elect_one()) {
       const int n0 = (int(blockIdx.x) / p.tiles_m) * BN;
-      pre = nkb < STAGES ? nkb : STAGES;
       for (int kb = 0; kb < pre; ++kb) {
         mbar_arrive_expect_tx(&full_bar[kb], STAGE_BYTES);
         tma_load_2d(smem + size_t(kb) * STAGE_BYTES + A_BYTES, &tmap_b, &full_bar[kb], kb * BK, n0);
@@ -685,7 +737,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -730,7 +782,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;

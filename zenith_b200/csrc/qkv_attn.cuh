@@ -106,7 +106,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pair_bar + 24);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int items = p.B * p.heads;
   const int nkb = p.num_k_blocks;
@@ -167,10 +167,9 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
   grid_launch_dependents();
   // constant weights: the weight tiles of the first item's first k-blocks are requested before the dependency wait
-  int pre = 0;
-  if (threadIdx.x == 0 && p.early_b && n_mine > 0) {
+  const int pre = p.early_b && n_mine > 0 ? (nkb < QA_STAGES ? nkb : QA_STAGES) : 0;
+  if (warp == 0 && elect_one()) {
     const int h = int(blockIdx.x) % p.heads;
-    pre = nkb < QA_STAGES ? nkb : QA_STAGES;
     for (int kb = 0; kb < pre; ++kb) {
       mbar_arrive_expect_tx(&full_bar[kb], QA_STAGE_BYTES);
       uint8_t* sb = smem + size_t(kb) * QA_STAGE_BYTES + A_BYTES;
@@ -182,7 +181,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -221,7 +220,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ projection MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -254,7 +253,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   } else if (warp < 4) {
     // ------------------------------------------------------------------ attention MMA issuer of one buffer set
-    if (lane == 0) {
+    if (elect_one()) {
       const int set = warp - 2;
       const uint32_t region = tmem_base + uint32_t(set * QA_BN);
       const uint32_t qa = smem_u32(sets + size_t(set) * QA_SET_BYTES);
