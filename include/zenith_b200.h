@@ -134,11 +134,23 @@ int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const void* w, int6
  *                           a tuning hook for benchmarks.  Not accepted by the *_add_layernorm_ex forms.
  *   ZEN_GEMM_PAIR / _NO_PAIR force or forbid the CTA-pair kernel, which the library otherwise chooses by shape;
  *                           results are identical either way.  Tuning / test hook.
+ *   ZEN_GEMM_SPLIT_K(n)     run the product on the small-product kernel with its K split n ways (1, 2, 4, 8), 15 = never on
+ *                           that kernel; otherwise the library chooses by shape.  int8 results do not depend on it; with
+ *                           fp16 operands the fp32 partial sums are added in another order.
+ *                           *_add_layernorm_ws forms: 15 = one kernel, 14 = two launches with the large-tile GEMM.
+ *   ZEN_GEMM_NARROW         with ZEN_GEMM_SPLIT_K: its 32-column tile (K split at most 4 ways) instead of 64 columns.
  * None of this has a counterpart in the reference. */
 #define ZEN_GEMM_CONST_WEIGHTS 0x1u
 #define ZEN_GEMM_NO_PAIR 0x2u /* never run this GEMM on CTA pairs (one CTA per 128-row tile) */
 #define ZEN_GEMM_PAIR 0x4u    /* always run it on CTA pairs (two CTAs per 256-row tile, tcgen05 cta_group::2) */
 #define ZEN_GEMM_TILE_N(bn) ((unsigned)(bn) << 8)
+#define ZEN_GEMM_SPLIT_K(n) ((unsigned)(n) << 20)
+#define ZEN_GEMM_NARROW 0x1000000u
+
+/* The ZEN_GEMM_SPLIT_K / ZEN_GEMM_NARROW flags the library would choose for a product of `rows` rows (elem_bytes 1, 2 or 4;
+ * layernorm != 0: for the *_add_layernorm_ws forms).  A caller that runs the same rows in batches of another size (a packed
+ * batch has fewer rows than its padded form) passes the flags of one size everywhere: every row then keeps its bits. */
+unsigned zen_gemm_plan(int elem_bytes, int rows, int N, int K, int layernorm);
 
 /* zen_linear_i8_prefetch with per-call options. */
 int zen_linear_i8_ex(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ldw, int M, int N, int K, float x_scale,
@@ -155,6 +167,20 @@ int zen_linear_f16_add_layernorm_ex(const void* x, int64_t ldx, const void* w, i
                                     const float* bias, const void* residual, int64_t ldr, const void* gamma,
                                     const void* beta, float eps, void* y, int8_t* yq, float out_scale, int round_mode,
                                     unsigned flags, void* stream);
+
+/* The same with a caller-provided workspace of M * N floats (16-byte aligned, scratch; NULL = the forms above): where the
+ * four-CTA clusters of the one-kernel form would leave the chip idle (few rows) or run in more than one round, the call
+ * becomes two launches, the projection with bias in fp32 into the workspace, then residual add and LayerNorm of its rows.
+ * Same results bit for bit (with fp16 operands: for the same K split). */
+int zen_linear_i8_add_layernorm_ws(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ldw, int M, int N, int K,
+                                   float x_scale, const float* w_scale, const float* bias, const void* residual,
+                                   int64_t ldr, const void* gamma, const void* beta, float eps, void* y, int8_t* yq,
+                                   float out_scale, int round_mode, void* workspace, size_t workspace_bytes,
+                                   unsigned flags, void* stream);
+int zen_linear_f16_add_layernorm_ws(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K,
+                                    const float* bias, const void* residual, int64_t ldr, const void* gamma,
+                                    const void* beta, float eps, void* y, int8_t* yq, float out_scale, int round_mode,
+                                    void* workspace, size_t workspace_bytes, unsigned flags, void* stream);
 
 /* FP16 Linear: y = x[M,K] . w[N,K]^T (+ bias[n], fp32) ; act ; out F16 or F32.  fp32 accumulate,
  * tcgen05 kind::f16.  K, ldx, ldw multiples of 8.

@@ -1,0 +1,79 @@
+"""The small-product GEMM (32 / 64-column tiles, K split over a cluster) and the two-launch LayerNorm form, forced through the
+call flags at the edges of their tiles, against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from zenith_b200 import _capi
+from zenith_b200._capi import ACT_GELU, ACT_NONE, DT_F16, DT_F32, DT_S8, DT_S32, GEMM_NARROW, gemm_split_k
+
+pytestmark = pytest.mark.gpu
+FORMS = [gemm_split_k(k) for k in (1, 2, 4, 8)] + [gemm_split_k(k) | GEMM_NARROW for k in (1, 2, 4)]
+
+
+def rng(seed):
+    return np.random.default_rng(seed)
+
+
+def dev(a, cuda):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+
+def call(fn, *args):
+    _capi.call(fn, *[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args], torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("flags", FORMS)
+@pytest.mark.parametrize("M,N,K", [(1, 32, 1024), (24, 768, 768), (129, 72, 1040), (200, 130, 2048)])
+def test_int8_bit_exact_in_every_form(cuda, M, N, K, flags):
+    x = rng(M).integers(-128, 128, (M, K), dtype=np.int8)
+    w = rng(N).integers(-128, 128, (N, K), dtype=np.int8)
+    ws = ((rng(1).random(N) + 0.5) * 3e-4).astype(np.float32)
+    b = (rng(2).standard_normal(N) * 0.1).astype(np.float32)
+    for dt, td, name, act in ((DT_S32, torch.int32, "s32", ACT_NONE), (DT_F32, torch.float32, "f32", ACT_NONE),
+                              (DT_F16, torch.float16, "f16", ACT_NONE), (DT_S8, torch.int8, "s8", ACT_GELU)):
+        out = torch.zeros((M, N), dtype=td, device=cuda)
+        call("zen_linear_i8_ex", dev(x, cuda), K, dev(w, cuda), K, M, N, K, 0.02, dev(ws, cuda), dev(b, cuda), act, dt, 0.03, 0, out, N,
+             None, 0, None, 0, flags)
+        if dt == DT_S32:
+            want = O.gemm_s8(x, w)
+        else:
+            want = O.linear_int8(x, w, 0.02, ws, b, "gelu" if act else "none", name, 0.03)
+        assert np.array_equal(out.cpu().numpy(), want), name
+    assert _capi.device_status() == 0
+
+
+@pytest.mark.parametrize("flags", FORMS)
+def test_fp16_in_every_form(cuda, flags):
+    M, N, K = 130, 200, 1536
+    x = rng(1).standard_normal((M, K)).astype(np.float16)
+    w = (rng(2).standard_normal((N, K)) * 0.05).astype(np.float16)
+    out = torch.zeros((M, N), dtype=torch.float32, device=cuda)
+    call("zen_linear_f16_ex", dev(x, cuda), K, dev(w, cuda), K, M, N, K, None, ACT_NONE, DT_F32, out, N, flags)
+    want = O.gemm_f32_nt(x.astype(np.float32), w.astype(np.float32))
+    assert np.max(np.abs(out.cpu().numpy() - want)) < 1e-3 * np.abs(want).max()
+    assert _capi.device_status() == 0
+
+
+@pytest.mark.parametrize("flags", [gemm_split_k(k) | GEMM_NARROW for k in (2, 4)] + [gemm_split_k(14), gemm_split_k(15), 0])
+@pytest.mark.parametrize("M,N,K", [(1, 768, 768), (129, 768, 1536), (300, 1024, 4096), (1025, 768, 128)])
+def test_layernorm_forms(cuda, M, N, K, flags):
+    x = rng(M).integers(-128, 128, (M, K), dtype=np.int8)
+    w = rng(K).integers(-128, 128, (N, K), dtype=np.int8)
+    ws = ((rng(1).random(N) + 0.5) * 2e-4).astype(np.float32)
+    b = (rng(2).standard_normal(N) * 0.1).astype(np.float32)
+    res = rng(3).standard_normal((M, N)).astype(np.float16)
+    g = (1 + 0.1 * rng(4).standard_normal(N)).astype(np.float16)
+    be = (0.1 * rng(5).standard_normal(N)).astype(np.float16)
+    y = torch.zeros((M, N), dtype=torch.float16, device=cuda)
+    yq = torch.zeros((M, N), dtype=torch.int8, device=cuda)
+    scratch = torch.empty((M, N), dtype=torch.float32, device=cuda)
+    call("zen_linear_i8_add_layernorm_ws", dev(x, cuda), K, dev(w, cuda), K, M, N, K, 0.02, dev(ws, cuda), dev(b, cuda), dev(res, cuda), N,
+         dev(g, cuda), dev(be, cuda), 1e-12, y, yq, 0.03, 0, scratch, scratch.numel() * 4, flags)
+    t = O.linear_int8(x, w, 0.02, ws, b, "none", "f32") + res.astype(np.float32)
+    want = O.layernorm(t, g.astype(np.float32), be.astype(np.float32), 1e-12)
+    got = y.float().cpu().numpy()
+    assert np.max(np.abs(got - want)) < 4e-3
+    assert np.array_equal(yq.cpu().numpy(), O.quantize(got, 0.03))
+    assert _capi.device_status() == 0

@@ -17,12 +17,18 @@ OK, ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_LAUNCH, ERR_TIMEOUT, ERR_DRIVER, ERR_T
 DT_S32, DT_F32, DT_F16, DT_S8 = range(4)
 ACT_NONE, ACT_GELU, ACT_RELU = range(3)
 ROUND_NEAREST_EVEN, ROUND_TRUNC = range(2)
-GEMM_CONST_WEIGHTS, GEMM_NO_PAIR, GEMM_PAIR = 0x1, 0x2, 0x4
+GEMM_CONST_WEIGHTS, GEMM_NO_PAIR, GEMM_PAIR, GEMM_NARROW = 0x1, 0x2, 0x4, 0x1000000
 
 
 def gemm_tile_n(bn: int) -> int:
     """``ZEN_GEMM_TILE_N(bn)``: the flag bits that force a GEMM tile width (0 = automatic)."""
     return int(bn) << 8
+
+
+def gemm_split_k(n: int) -> int:
+    """``ZEN_GEMM_SPLIT_K(n)``: the flag bits that send a product to the small-product kernel with K split n ways."""
+    return int(n) << 20
+
 
 _p, _i, _f, _i64, _u = C.c_void_p, C.c_int, C.c_float, C.c_int64, C.c_uint
 
@@ -30,6 +36,7 @@ _p, _i, _f, _i64, _u = C.c_void_p, C.c_int, C.c_float, C.c_int64, C.c_uint
 SIGNATURES = {
     "zen_version": [],
     "zen_status_string": [_i],
+    "zen_gemm_plan": [_i, _i, _i, _i, _i],
     "zen_device_status_read": [C.POINTER(C.c_int)],
     "zen_device_status_clear": [],
     "zen_selftest_wait_limit": [_p, _p],
@@ -42,6 +49,10 @@ SIGNATURES = {
     "zen_linear_i8_add_layernorm_ex": [_p, _i64, _p, _i64, _i, _i, _i, _f, _p, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _u,
                                        _p],
     "zen_linear_f16_add_layernorm_ex": [_p, _i64, _p, _i64, _i, _i, _i, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _u, _p],
+    "zen_linear_i8_add_layernorm_ws": [_p, _i64, _p, _i64, _i, _i, _i, _f, _p, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _p,
+                                       C.c_size_t, _u, _p],
+    "zen_linear_f16_add_layernorm_ws": [_p, _i64, _p, _i64, _i, _i, _i, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _p, C.c_size_t,
+                                        _u, _p],
     "zen_linear_f16_ex": [_p, _i64, _p, _i64, _i, _i, _i, _p, _i, _i, _p, _i64, _u, _p],
     "zen_linear_i8_add_layernorm": [_p, _i64, _p, _i64, _i, _i, _i, _f, _p, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _p],
     "zen_linear_f16_add_layernorm": [_p, _i64, _p, _i64, _i, _i, _i, _p, _p, _i64, _p, _p, _f, _p, _p, _f, _i, _p],
@@ -89,7 +100,7 @@ SIGNATURES = {
     "zen_unpad_rows_f16": [_p, _p, _i, _i, _i, _i, _p, _p],
 }
 _RESTYPES = {"zen_status_string": C.c_char_p, "zen_matmul_f32_workspace_bytes": C.c_size_t,
-             "zen_minmax_workspace_bytes": C.c_size_t}
+             "zen_minmax_workspace_bytes": C.c_size_t, "zen_gemm_plan": C.c_uint}
 
 _lib = None
 

@@ -1,6 +1,7 @@
 // Host side of the tcgen05 GEMMs: tile selection, tensor maps, launches, C ABI.
 #include "gemm_tc.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_small.h"
 #include "tma_host.cuh"
 #include <map>
 #include <mutex>
@@ -188,6 +189,15 @@ static int pick_bn_pair(int M, int N, unsigned flags) {
   return best;
 }
 
+// Whether (and with what tile and K split) a product runs on the small-product kernel: by shape, or as the flags say.  A
+// forced tile width or pair choice is about the large-tile kernels.
+static SmallChoice use_small(int kind, int M, int N, int K, unsigned flags) {
+  const int f = forced_split(flags);
+  if (f != 0) return {forced_small_bn(flags), f == 15 ? 0 : f};
+  if (flags & (ZEN_GEMM_PAIR | ZEN_GEMM_NO_PAIR | (0x3ffu << 8))) return {64, 0};
+  return small_rule(kind == KIND_F16 ? 2 : kind == KIND_TF32 ? 4 : 1, M, N, K, false);
+}
+
 // out[c, r] = in[r, c] for a row-major [rows, cols] fp32 matrix, 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256) transpose_f32_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                             int rows, int cols) {
@@ -212,6 +222,40 @@ static int launch_transpose_f32(const float* in, float* out, int rows, int cols,
   return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
 }
 
+// int8 or fp16 operands, B K-major: the small-product kernel, CTA pairs or the one-CTA kernel by shape (or by `flags`).
+int run_gemm_auto(int kind, const void* A, int64_t lda, const void* B, int64_t ldb, const GemmParams& p, unsigned flags, cudaStream_t s) {
+  static const int allowed[] = {64, 128, 192, 256};
+  if (const SmallChoice c = use_small(kind, p.M, p.N, p.K, flags); c.ks > 0) return launch_gemm_small(kind, c.bn, c.ks, false, A, lda, B, ldb, p, s);
+  if (kind == KIND_I8) {
+    if (use_pair(p.M, p.N, p.K, p.out_dtype == ZEN_DT_S8 && p.act == ZEN_ACT_GELU, flags)) {
+      switch (pick_bn_pair(p.M, p.N, flags)) {
+        case 128: return run_gemm<KIND_I8, 128, 6, false, true>(A, lda, B, ldb, p, s);
+        case 192: return run_gemm<KIND_I8, 192, 5, false, true>(A, lda, B, ldb, p, s);
+        default: return run_gemm<KIND_I8, 256, 4, false, true>(A, lda, B, ldb, p, s);
+      }
+    }
+    switch (pick_bn(p.M, p.N, allowed, 4, flags)) {
+      case 64: return run_gemm<KIND_I8, 64, 7, false>(A, lda, B, ldb, p, s);
+      case 128: return run_gemm<KIND_I8, 128, 5, false>(A, lda, B, ldb, p, s);
+      case 192: return run_gemm<KIND_I8, 192, 4, false>(A, lda, B, ldb, p, s);
+      default: return run_gemm<KIND_I8, 256, 3, false>(A, lda, B, ldb, p, s);
+    }
+  }
+  if (use_pair(p.M, p.N, 2 * p.K /* fp16 operands: twice the bytes per element */, false, flags)) {
+    switch (pick_bn_pair(p.M, p.N, flags)) {
+      case 128: return run_gemm<KIND_F16, 128, 6, false, true>(A, lda, B, ldb, p, s);
+      case 192: return run_gemm<KIND_F16, 192, 5, false, true>(A, lda, B, ldb, p, s);
+      default: return run_gemm<KIND_F16, 256, 4, false, true>(A, lda, B, ldb, p, s);
+    }
+  }
+  switch (pick_bn(p.M, p.N, allowed, 4, flags)) {
+    case 64: return run_gemm<KIND_F16, 64, 7, false>(A, lda, B, ldb, p, s);
+    case 128: return run_gemm<KIND_F16, 128, 5, false>(A, lda, B, ldb, p, s);
+    case 192: return run_gemm<KIND_F16, 192, 4, false>(A, lda, B, ldb, p, s);
+    default: return run_gemm<KIND_F16, 256, 3, false>(A, lda, B, ldb, p, s);
+  }
+}
+
 }  // namespace zen
 
 using namespace zen;
@@ -221,6 +265,12 @@ ZEN_DEFINE_TU_STATUS(gemm)
 extern "C" {
 
 int zen_version(void) { return ZEN_VERSION; }
+
+unsigned zen_gemm_plan(int elem_bytes, int rows, int N, int K, int layernorm) {
+  if ((elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4) || rows <= 0 || N <= 0 || K <= 0) return 0u;
+  const SmallChoice c = layernorm ? layernorm_rule(elem_bytes, rows, N, K) : small_rule(elem_bytes, rows, N, K, false);
+  return ZEN_GEMM_SPLIT_K(c.ks > 0 ? c.ks : 15) | (c.bn == 32 ? ZEN_GEMM_NARROW : 0u);
+}
 
 const char* zen_status_string(int s) {
   switch (s) {
@@ -237,7 +287,9 @@ const char* zen_status_string(int s) {
 
 static bool flags_ok(unsigned flags) {
   const unsigned bn = (flags >> 8) & 0x3ffu;
-  if (flags & ~(ZEN_GEMM_CONST_WEIGHTS | ZEN_GEMM_PAIR | ZEN_GEMM_NO_PAIR | (0x3ffu << 8))) return false;
+  if (flags & ~(ZEN_GEMM_CONST_WEIGHTS | ZEN_GEMM_PAIR | ZEN_GEMM_NO_PAIR | ZEN_GEMM_NARROW | (0x3ffu << 8) | (0xfu << 20))) return false;
+  const int ks = forced_split(flags);
+  if (ks != 0 && ks != 1 && ks != 2 && ks != 4 && ks != 8 && ks != 15) return false;
   if ((flags & ZEN_GEMM_PAIR) && (flags & ZEN_GEMM_NO_PAIR)) return false;
   return bn == 0 || bn == 64 || bn == 128 || bn == 192 || bn == 256;
 }
@@ -284,21 +336,7 @@ int zen_linear_i8_ex(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ld
       p.pf_bytes[i] = uint64_t(hi - lo);
     }
   }
-  static const int allowed[] = {64, 128, 192, 256};
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (use_pair(M, N, K, out_dtype == ZEN_DT_S8 && act == ZEN_ACT_GELU, flags)) {
-    switch (pick_bn_pair(M, N, flags)) {
-      case 128: return run_gemm<KIND_I8, 128, 6, false, true>(xq, ldx, wq, ldw, p, s);
-      case 192: return run_gemm<KIND_I8, 192, 5, false, true>(xq, ldx, wq, ldw, p, s);
-      default: return run_gemm<KIND_I8, 256, 4, false, true>(xq, ldx, wq, ldw, p, s);
-    }
-  }
-  switch (pick_bn(M, N, allowed, 4, flags)) {
-    case 64: return run_gemm<KIND_I8, 64, 7, false>(xq, ldx, wq, ldw, p, s);
-    case 128: return run_gemm<KIND_I8, 128, 5, false>(xq, ldx, wq, ldw, p, s);
-    case 192: return run_gemm<KIND_I8, 192, 4, false>(xq, ldx, wq, ldw, p, s);
-    default: return run_gemm<KIND_I8, 256, 3, false>(xq, ldx, wq, ldw, p, s);
-  }
+  return run_gemm_auto(KIND_I8, xq, ldx, wq, ldw, p, flags, static_cast<cudaStream_t>(stream));
 }
 
 int zen_linear_f16(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K, const float* bias,
@@ -317,21 +355,7 @@ int zen_linear_f16_ex(const void* x, int64_t ldx, const void* w, int64_t ldw, in
   p.out = out; p.ldo = ldo; p.out_dtype = out_dtype; p.act = act;
   p.x_scale = 1.0f; p.out_scale = 1.0f; p.w_scale = nullptr; p.bias = bias;
   p.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
-  static const int allowed[] = {64, 128, 192, 256};
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (use_pair(M, N, 2 * K /* fp16 operands: twice the bytes per element */, false, flags)) {
-    switch (pick_bn_pair(M, N, flags)) {
-      case 128: return run_gemm<KIND_F16, 128, 6, false, true>(x, ldx, w, ldw, p, s);
-      case 192: return run_gemm<KIND_F16, 192, 5, false, true>(x, ldx, w, ldw, p, s);
-      default: return run_gemm<KIND_F16, 256, 4, false, true>(x, ldx, w, ldw, p, s);
-    }
-  }
-  switch (pick_bn(M, N, allowed, 4, flags)) {
-    case 64: return run_gemm<KIND_F16, 64, 7, false>(x, ldx, w, ldw, p, s);
-    case 128: return run_gemm<KIND_F16, 128, 5, false>(x, ldx, w, ldw, p, s);
-    case 192: return run_gemm<KIND_F16, 192, 4, false>(x, ldx, w, ldw, p, s);
-    default: return run_gemm<KIND_F16, 256, 3, false>(x, ldx, w, ldw, p, s);
-  }
+  return run_gemm_auto(KIND_F16, x, ldx, w, ldw, p, flags, static_cast<cudaStream_t>(stream));
 }
 
 int zen_linear_f8(const uint8_t* xq, int64_t ldx, const uint8_t* wq, int64_t ldw, int M, int N, int K, float x_scale,
@@ -349,6 +373,7 @@ int zen_linear_f8(const uint8_t* xq, int64_t ldx, const uint8_t* wq, int64_t ldw
   p.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
   static const int allowed[] = {64, 128, 192, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const SmallChoice c = use_small(KIND_F8, M, N, K, flags); c.ks > 0) return launch_gemm_small(KIND_F8, c.bn, c.ks, false, xq, ldx, wq, ldw, p, s);
   switch (pick_bn(M, N, allowed, 4, flags)) {
     case 64: return run_gemm<KIND_F8, 64, 7, false>(xq, ldx, wq, ldw, p, s);
     case 128: return run_gemm<KIND_F8, 128, 5, false>(xq, ldx, wq, ldw, p, s);
@@ -368,6 +393,7 @@ int zen_linear_f32(const float* x, int64_t ldx, const float* w, int64_t ldw, int
   p.x_scale = 1.0f; p.out_scale = 1.0f; p.w_scale = nullptr; p.bias = bias;
   static const int allowed[] = {64, 128, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const SmallChoice c = use_small(KIND_TF32, M, N, K, 0u); c.ks > 0) return launch_gemm_small(KIND_TF32, c.bn, c.ks, false, x, ldx, w, ldw, p, s);
   switch (pick_bn(M, N, allowed, 3, 0u)) {
     case 64: return run_gemm<KIND_TF32, 64, 7, false>(x, ldx, w, ldw, p, s);
     case 128: return run_gemm<KIND_TF32, 128, 5, false>(x, ldx, w, ldw, p, s);
@@ -384,6 +410,7 @@ int zen_wmma_matmul_f16(const void* A, const void* B, float* C, int M, int N, in
   p.x_scale = 1.0f; p.out_scale = 1.0f;
   static const int allowed[] = {64, 128, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const SmallChoice c = use_small(KIND_F16, M, N, K, 0u); c.ks > 0) return launch_gemm_small(KIND_F16, c.bn, c.ks, true, A, K, B, N, p, s);
   switch (pick_bn(M, N, allowed, 3, 0u)) {
     case 64: return run_gemm<KIND_F16, 64, 7, true>(A, K, B, N, p, s);
     case 128: return run_gemm<KIND_F16, 128, 5, true>(A, K, B, N, p, s);

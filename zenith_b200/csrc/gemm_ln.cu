@@ -20,7 +20,7 @@
 // is complete the epilogue is bound by instruction issue (about 14 instructions per output at 0.45 per clock and
 // scheduler: dequantise + residual + statistics 1.0 us, normalise + requantise 2.8 us, stores 1.3 us), not by the
 // second trip through tensor memory, which overlaps that arithmetic here.
-#include "gemm_tc.cuh"
+#include "gemm_small.h"
 #include "tma_host.cuh"
 
 namespace zen {
@@ -41,6 +41,7 @@ struct GemmLnParams {
 };
 
 constexpr int LN_CLUSTER = 4;
+constexpr int LN_ROWS_WIDE_MAX = 1024;  // rows up to which ln_rows_kernel spreads a row over H / 128 warps
 
 __device__ __forceinline__ void st_cluster_f32x2(uint32_t cluster_addr, float a, float b) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
@@ -466,6 +467,122 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   gemm_ln_body<KIND_F16, BN, STAGES>(tmap_a, tmap_b, tmap_y, tmap_q, tmap_r, p);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Residual add and LayerNorm of fp32 rows (projection + bias, from the GEMM's fp32 output) -> fp16 (+ int8 copy): the second
+// launch of the two-kernel form.  With few rows the row's latency is what counts: it is spread over H / 128 warps with one
+// 16-byte unit per lane.  With many, one warp owns a row (no block barrier) and holds it in registers.
+// ---------------------------------------------------------------------------------------------
+struct LnRowsParams {
+  const float* t;          // [rows, H]: projection + bias
+  const __half* residual;  // row stride ldr
+  int64_t ldr;
+  const __half* gamma;
+  const __half* beta;
+  __half* y;
+  int8_t* yq;
+  float out_scale, eps;
+  int round_mode;
+  int rows;
+};
+
+template <int H, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? H / 4 : 128) ln_rows_kernel(const LnRowsParams p) {
+  constexpr int VPL = WIDE ? 1 : H / 128;  // float4 units per lane
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = WIDE ? int(blockIdx.x) : int(blockIdx.x) * 4 + warp;
+  const int c0 = WIDE ? warp * 128 + lane * 4 : lane * 4;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (row >= p.rows) return;  // whole rows only: every warp of a row meets the block barriers below
+  const float* t = p.t + int64_t(row) * H + c0;
+  const __half* res = p.residual + int64_t(row) * p.ldr + c0;
+  float2 v[VPL][2];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const float4 f = *reinterpret_cast<const float4*>(t + i * 128);
+    const uint2 u = *reinterpret_cast<const uint2*>(res + i * 128);
+    const __half2* rh = reinterpret_cast<const __half2*>(&u);
+    v[i][0] = f2add(make_float2(f.x, f.y), __half22float2(rh[0]));
+    v[i][1] = f2add(make_float2(f.z, f.w), __half22float2(rh[1]));
+  }
+  uint2 gb[VPL], bb[VPL];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    gb[i] = *reinterpret_cast<const uint2*>(p.gamma + c0 + i * 128);
+    bb[i] = *reinterpret_cast<const uint2*>(p.beta + c0 + i * 128);
+  }
+  __shared__ float red[2][H / 128];
+  auto row_sum = [&](float2 s2, int use) -> float {
+    float s = s2.x + s2.y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if constexpr (WIDE) {
+      if (lane == 0) red[use][warp] = s;
+      __syncthreads();
+      s = 0.f;
+#pragma unroll
+      for (int w = 0; w < H / 128; ++w) s += red[use][w];
+    }
+    return s;
+  };
+  float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) s2 = f2add(s2, f2add(v[i][0], v[i][1]));
+  const float mean = row_sum(s2, 0) * (1.0f / float(H));
+  const float2 nmu = make_float2(-mean, -mean);
+  float2 q2 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < VPL; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      v[i][h] = f2add(v[i][h], nmu);
+      q2 = f2fma(v[i][h], v[i][h], q2);
+    }
+  const float rstd = rsqrtf(fmaf(row_sum(q2, 1), 1.0f / float(H), p.eps));
+  const float2 rstd2 = make_float2(rstd, rstd);
+  const float inv_q = ZEN_DIV(1.0f, p.out_scale);
+  const int64_t off = int64_t(row) * H + c0;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const __half2* g = reinterpret_cast<const __half2*>(&gb[i]);
+    const __half2* b = reinterpret_cast<const __half2*>(&bb[i]);
+    uint2 w;
+    float2 of[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 o = f2fma(f2mul(v[i][h], rstd2), __half22float2(g[h]), __half22float2(b[h]));
+      const __half2 hv = __floats2half2_rn(o.x, o.y);
+      (h ? w.y : w.x) = *reinterpret_cast<const uint32_t*>(&hv);
+      of[h] = __half22float2(hv);
+    }
+    *reinterpret_cast<uint2*>(p.y + off + i * 128) = w;
+    if (p.yq) {
+      uint32_t qw[1];
+      if (p.round_mode == 0) {
+        const uint32_t risky = quantize_pairs_rn<4>(of, inv_q, qw);
+        if (risky) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (risky & (1u << j)) patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), 0));
+        }
+      } else {
+        qw[0] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), p.round_mode));
+      }
+      *reinterpret_cast<uint32_t*>(p.yq + off + i * 128) = qw[0];
+    }
+  }
+}
+
+template <int H>
+static int launch_ln_rows(const LnRowsParams& p, cudaStream_t s) {
+  if (p.rows <= LN_ROWS_WIDE_MAX)
+    return launch_pdl(PDL_GEMM, ln_rows_kernel<H, true>, dim3(unsigned(p.rows)), dim3(H / 4), 0, s, p);
+  return launch_pdl(PDL_GEMM, ln_rows_kernel<H, false>, dim3(unsigned((p.rows + 3) / 4)), dim3(128), 0, s, p);
+}
+
 template <int KIND, int BN, int STAGES>
 static int launch_gemm_ln(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ty, const CUtensorMap& tq,
                           const CUtensorMap& tr, const GemmLnParams& p, cudaStream_t stream) {
@@ -505,18 +622,43 @@ template <int KIND>
 static int run_linear_add_layernorm(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K, float x_scale,
                                     const float* w_scale, const float* bias, const void* residual, int64_t ldr,
                                     const void* gamma, const void* beta, float eps, void* y, int8_t* yq, float out_scale,
-                                    int round_mode, unsigned flags, void* stream) {
+                                    int round_mode, void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
   constexpr int ELEM = GemmKind<KIND>::ELEM;  // bytes per operand element
   constexpr int KA = 16 / ELEM;               // elements per 16 bytes: the unit K and the row strides must be a multiple of
   if (!x || !w || !residual || !gamma || !beta || !y || M <= 0 || N <= 0 || K <= 0) return ZEN_ERR_INVALID_ARG;
   if (round_mode != ZEN_ROUND_NEAREST_EVEN && round_mode != ZEN_ROUND_TRUNC) return ZEN_ERR_INVALID_ARG;
-  if (flags & ~unsigned(ZEN_GEMM_CONST_WEIGHTS)) return ZEN_ERR_INVALID_ARG;
+  if (flags & ~(unsigned(ZEN_GEMM_CONST_WEIGHTS) | ZEN_GEMM_NARROW | (0xfu << 20))) return ZEN_ERR_INVALID_ARG;
   if (yq && !(out_scale > 0.0f)) return ZEN_ERR_INVALID_ARG;
   if (N != 768 && N != 1024) return ZEN_ERR_UNSUPPORTED;  // four CTAs x 192 (or 256) columns hold one row
   if (K % KA || ldx % KA || ldw % KA || ldx < K || ldw < K || ldr % 8 || ldr < N) return ZEN_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(y) % 16 || reinterpret_cast<uintptr_t>(yq) % 16 ||
       reinterpret_cast<uintptr_t>(residual) % 16)
     return ZEN_ERR_UNSUPPORTED;
+  int form = 15;
+  unsigned narrow = 0;
+  if (workspace != nullptr) {
+    if (workspace_bytes < size_t(M) * size_t(N) * 4 || reinterpret_cast<uintptr_t>(workspace) % 16) return ZEN_ERR_INVALID_ARG;
+    form = forced_split(flags);
+    narrow = flags & ZEN_GEMM_NARROW;
+    if (form == 0) {
+      const SmallChoice c = layernorm_rule(ELEM, M, N, K);
+      form = c.ks;
+      narrow = c.bn == 32 ? ZEN_GEMM_NARROW : 0u;
+    }
+    if (form != 1 && form != 2 && form != 4 && form != 8 && form != 14 && form != 15) return ZEN_ERR_INVALID_ARG;
+  }
+  if (form != 15) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    GemmParams g{};
+    g.M = M; g.N = N; g.K = K;
+    g.out = workspace; g.ldo = N; g.out_dtype = ZEN_DT_F32; g.act = ZEN_ACT_NONE; g.fold = 1;
+    g.x_scale = x_scale; g.out_scale = 1.0f; g.w_scale = w_scale; g.bias = bias;
+    g.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
+    if (int st = run_gemm_auto(KIND, x, ldx, w, ldw, g, ZEN_GEMM_SPLIT_K(form == 14 ? 15 : form) | narrow, s); st != ZEN_OK) return st;
+    const LnRowsParams lp{static_cast<const float*>(workspace), static_cast<const __half*>(residual), ldr, static_cast<const __half*>(gamma),
+                          static_cast<const __half*>(beta), static_cast<__half*>(y), yq, yq ? out_scale : 1.0f, eps, round_mode, M};
+    return N == 768 ? launch_ln_rows<768>(lp, s) : launch_ln_rows<1024>(lp, s);
+  }
   const int BN = N / LN_CLUSTER;
   constexpr int BK = 128 / ELEM;
   GemmLnParams p{};
@@ -554,7 +696,7 @@ extern "C" int zen_linear_i8_add_layernorm_ex(const int8_t* xq, int64_t ldx, con
                                               float eps, void* y, int8_t* yq, float out_scale, int round_mode,
                                               unsigned flags, void* stream) {
   return run_linear_add_layernorm<KIND_I8>(xq, ldx, wq, ldw, M, N, K, x_scale, w_scale, bias, residual, ldr, gamma, beta, eps,
-                                           y, yq, out_scale, round_mode, flags, stream);
+                                           y, yq, out_scale, round_mode, nullptr, 0, flags, stream);
 }
 
 extern "C" int zen_linear_i8_add_layernorm(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ldw, int M, int N,
@@ -563,7 +705,7 @@ extern "C" int zen_linear_i8_add_layernorm(const int8_t* xq, int64_t ldx, const 
                                            float eps, void* y, int8_t* yq, float out_scale, int round_mode,
                                            void* stream) {
   return run_linear_add_layernorm<KIND_I8>(xq, ldx, wq, ldw, M, N, K, x_scale, w_scale, bias, residual, ldr, gamma, beta, eps,
-                                           y, yq, out_scale, round_mode, 0u, stream);
+                                           y, yq, out_scale, round_mode, nullptr, 0, 0u, stream);
 }
 
 extern "C" int zen_linear_f16_add_layernorm_ex(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K,
@@ -571,7 +713,7 @@ extern "C" int zen_linear_f16_add_layernorm_ex(const void* x, int64_t ldx, const
                                                const void* beta, float eps, void* y, int8_t* yq, float out_scale,
                                                int round_mode, unsigned flags, void* stream) {
   return run_linear_add_layernorm<KIND_F16>(x, ldx, w, ldw, M, N, K, 1.0f, nullptr, bias, residual, ldr, gamma, beta, eps, y,
-                                            yq, out_scale, round_mode, flags, stream);
+                                            yq, out_scale, round_mode, nullptr, 0, flags, stream);
 }
 
 extern "C" int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K,
@@ -579,5 +721,22 @@ extern "C" int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const vo
                                             const void* beta, float eps, void* y, int8_t* yq, float out_scale,
                                             int round_mode, void* stream) {
   return run_linear_add_layernorm<KIND_F16>(x, ldx, w, ldw, M, N, K, 1.0f, nullptr, bias, residual, ldr, gamma, beta, eps, y,
-                                            yq, out_scale, round_mode, 0u, stream);
+                                            yq, out_scale, round_mode, nullptr, 0, 0u, stream);
+}
+
+extern "C" int zen_linear_i8_add_layernorm_ws(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ldw, int M, int N, int K,
+                                              float x_scale, const float* w_scale, const float* bias, const void* residual,
+                                              int64_t ldr, const void* gamma, const void* beta, float eps, void* y, int8_t* yq,
+                                              float out_scale, int round_mode, void* workspace, size_t workspace_bytes,
+                                              unsigned flags, void* stream) {
+  return run_linear_add_layernorm<KIND_I8>(xq, ldx, wq, ldw, M, N, K, x_scale, w_scale, bias, residual, ldr, gamma, beta, eps, y, yq,
+                                           out_scale, round_mode, workspace, workspace_bytes, flags, stream);
+}
+
+extern "C" int zen_linear_f16_add_layernorm_ws(const void* x, int64_t ldx, const void* w, int64_t ldw, int M, int N, int K,
+                                               const float* bias, const void* residual, int64_t ldr, const void* gamma,
+                                               const void* beta, float eps, void* y, int8_t* yq, float out_scale, int round_mode,
+                                               void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
+  return run_linear_add_layernorm<KIND_F16>(x, ldx, w, ldw, M, N, K, 1.0f, nullptr, bias, residual, ldr, gamma, beta, eps, y, yq,
+                                            out_scale, round_mode, workspace, workspace_bytes, flags, stream);
 }

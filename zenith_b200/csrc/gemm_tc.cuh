@@ -37,6 +37,8 @@ struct GemmParams {
   const float* w_scale;
   const float* bias;
   int staged_store;  // 1: the output leaves through shared memory (fp16 / int8: TMA stores; 4-byte types: transposed row pieces)
+  int fold;          // fp32 output of an int8 product: y = acc * (x_scale * w_scale[n]) + bias[n] in one multiply-add (the sum
+                     // that a LayerNorm follows: a tolerance path), instead of the bit-exact three roundings
   // L2 prefetch hint: read-only ranges (16-byte aligned, sizes multiples of 16) that later kernels will
   // read, e.g. the next GEMMs' weights; every CTA asks for its slice while it waits for its own operands
   const uint8_t* pf_ptr[2];
@@ -229,8 +231,8 @@ __device__ __forceinline__ void store_rows_4byte(const uint32_t (&w)[GEMM_CW], u
 // `istep` is the position of the step inside the slab.
 template <int KIND, int OUT, int ACT, int SLAB>
 __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], const float* sc, const float* bi,
-                                               const GemmParams& p, int row, int col0, bool full, float inv_scale,
-                                               uint8_t* stage, int lane, int istep) {
+                                               const float* fo, const GemmParams& p, int row, int col0, bool full,
+                                               float inv_scale, uint8_t* stage, int lane, int istep) {
   constexpr int CW = GEMM_CW;
   const int nvalid = p.N - col0;  // >= 1
   if constexpr (OUT == ZEN_DT_S32) {
@@ -261,8 +263,11 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], con
         for (int h = 0; h < 2; ++h) {
           const int j = 4 * j4 + 2 * h;
           const float2 a = make_float2(float(int32_t(r[j])), float(int32_t(r[j + 1])));
-          const float2 v = f2mul_then_add(f2mul(a, xs2), make_float2(ss[2 * h], ss[2 * h + 1]),
-                                          make_float2(bb[2 * h], bb[2 * h + 1]));
+          float2 v;
+          if (OUT == ZEN_DT_F32 && ACT == ZEN_ACT_NONE && p.fold)
+            v = f2fma(a, make_float2(fo[j], fo[j + 1]), make_float2(bb[2 * h], bb[2 * h + 1]));
+          else
+            v = f2mul_then_add(f2mul(a, xs2), make_float2(ss[2 * h], ss[2 * h + 1]), make_float2(bb[2 * h], bb[2 * h + 1]));
           y[j] = v.x;
           y[j + 1] = v.y;
         }
@@ -377,9 +382,9 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[GEMM_CW], con
 //   too small.
 // Flagged elements are recomputed with the definition itself (requant_i8_fixup).
 //
-template <int ACT>
-__device__ __forceinline__ uint32_t requant_i8_step(const uint32_t (&r)[GEMM_CW], const float* fold, const float* bi,
-                                                    float risk_thr, float inv_scale, uint32_t (&w)[GEMM_CW / 4]) {
+template <int ACT, int CW>
+__device__ __forceinline__ uint32_t requant_i8_step(const uint32_t (&r)[CW], const float* fold, const float* bi,
+                                                    float risk_thr, float inv_scale, uint32_t (&w)[CW / 4]) {
   constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23
   const float2 neg_magic = make_float2(-MAGIC, -MAGIC);
   const float2 pos_magic = make_float2(MAGIC, MAGIC);
@@ -387,7 +392,7 @@ __device__ __forceinline__ uint32_t requant_i8_step(const uint32_t (&r)[GEMM_CW]
   uint32_t span = 0;
   uint32_t risky = 0;
 #pragma unroll
-  for (int j4 = 0; j4 < GEMM_CW / 4; ++j4) {
+  for (int j4 = 0; j4 < CW / 4; ++j4) {
     const float4 s4 = reinterpret_cast<const float4*>(fold)[j4];
     const float4 b4 = reinterpret_cast<const float4*>(bi)[j4];
     uint32_t mb[4];
@@ -423,7 +428,7 @@ __device__ __forceinline__ uint32_t requant_i8_step(const uint32_t (&r)[GEMM_CW]
     }
     w[j4] = pack_sat_s8x4(mb[0], mb[1], mb[2], mb[3]);
   }
-  return span >= 0x00800000u ? (1u << GEMM_CW) - 1u : risky;
+  return span >= 0x00800000u ? (1u << CW) - 1u : risky;
 }
 
 // The exact definition for the columns flagged in `any` (the union of the lanes' masks), one column
@@ -481,14 +486,14 @@ __device__ __forceinline__ void epilogue_step_s8(const uint32_t (&r)[GEMM_CW], u
 
 template <int KIND, int OUT, int SLAB>
 __device__ __forceinline__ void epilogue_chunk_act(const uint32_t (&r)[GEMM_CW], const float* sc, const float* bi,
-                                                   const GemmParams& p, int row, int col0, bool full, float inv_scale,
-                                                   uint8_t* stage, int lane, int istep) {
+                                                   const float* fo, const GemmParams& p, int row, int col0, bool full,
+                                                   float inv_scale, uint8_t* stage, int lane, int istep) {
   if (p.act == ZEN_ACT_GELU)
-    epilogue_chunk<KIND, OUT, ZEN_ACT_GELU, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_GELU, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, istep);
   else if (p.act == ZEN_ACT_RELU)
-    epilogue_chunk<KIND, OUT, ZEN_ACT_RELU, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_RELU, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, istep);
   else
-    epilogue_chunk<KIND, OUT, ZEN_ACT_NONE, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, istep);
+    epilogue_chunk<KIND, OUT, ZEN_ACT_NONE, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, istep);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -608,20 +613,21 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
         const bool full = vec_ok && (col0 + GEMM_CW <= p.N);
         const float* sc = s_scale + i * GEMM_CW;
         const float* bi = s_bias + i * GEMM_CW;
+        const float* fo = s_fold + i * GEMM_CW;
         if constexpr (KIND == KIND_I8) {
           switch (p.out_dtype) {
             case ZEN_DT_S32:
-              epilogue_chunk<KIND, ZEN_DT_S32, ZEN_ACT_NONE, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+              epilogue_chunk<KIND, ZEN_DT_S32, ZEN_ACT_NONE, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i);
               break;
-            case ZEN_DT_F32: epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
-            case ZEN_DT_F16: epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
-            default: epilogue_chunk_act<KIND, ZEN_DT_S8, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i); break;
+            case ZEN_DT_F32: epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i); break;
+            case ZEN_DT_F16: epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i); break;
+            default: epilogue_chunk_act<KIND, ZEN_DT_S8, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i); break;
           }
         } else {
           if (p.out_dtype == ZEN_DT_F32)
-            epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+            epilogue_chunk_act<KIND, ZEN_DT_F32, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i);
           else
-            epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, p, row, col0, full, inv_scale, stage, lane, i);
+            epilogue_chunk_act<KIND, ZEN_DT_F16, SLAB>(r, sc, bi, fo, p, row, col0, full, inv_scale, stage, lane, i);
         }
       }
       __syncwarp();

@@ -156,6 +156,23 @@ class _EncoderBase:
         self.launches_per_forward = len(self._launches)
         self._streams = [torch.cuda.Stream(device=d) for _ in range(len(self._micro) - 1)]
 
+    def _plan(self, elem_bytes: int, N: int, K: int, layernorm: bool = False) -> int:
+        """Kernel-choice flags of a GEMM of this pass, chosen for the rows of the whole padded batch: the packed form and
+        micro-batches then run every row on the same kernels and keep its bits."""
+        return _capi.lib().zen_gemm_plan(elem_bytes, self._shape[0] * self._shape[1], N, K, int(layernorm))
+
+    def _fused_layernorm(self) -> bool:
+        """Whether attention-output and FFN2 of the prepared shape run as one ``*_add_layernorm_ws`` call each.  Not asked
+        for, hidden 1024 does so up to 2048 rows, where the call's two launches with fp32 rows in between beat the separate
+        kernels (9.9 against 12.4 us for FFN2 at 512 rows); with more, the fp32 rows cost more than they save."""
+        if self.fuse_layernorm or self.cfg.hidden != 1024 or self._ln_asked is not None:
+            return self.fuse_layernorm
+        return self._shape[0] * self._shape[1] <= 2048
+
+    def _workspace(self, T: int) -> torch.Tensor:
+        """fp32 rows of a projection on its way to a LayerNorm (scratch of one launch pair)."""
+        return torch.empty((T, self.cfg.hidden), dtype=torch.float32, device=self.device)
+
     def _add(self, fn: str, *args) -> None:
         self._launches.append((getattr(_capi.lib(), fn), fn, args))
 
@@ -305,6 +322,7 @@ class Fp16Encoder(_EncoderBase):
         """``fuse_layernorm``: attention-output and FFN2 as one GEMM + residual + LayerNorm kernel each (5 launches
         per layer instead of 7); possible for hidden 768 and 1024, on by default for 768."""
         super().__init__(cfg, params, device, micro_batches, gemm_pair)
+        self._ln_asked = fuse_layernorm
         self.fuse_layernorm = (cfg.hidden == 768) if fuse_layernorm is None else bool(fuse_layernorm)
         if self.fuse_layernorm and cfg.hidden not in (768, 1024):
             raise RuntimeError("the fused GEMM + LayerNorm kernel needs hidden == 768 or 1024")
@@ -331,6 +349,7 @@ class Fp16Encoder(_EncoderBase):
         self.h1 = torch.empty((T, H), **f16)
         self.g = torch.empty((T, F), **f16)
         self.o = torch.empty((T, H), **f16)
+        self.ln_ws = self._workspace(T) if self._fused_layernorm() else None
         self.out = self.x[len(self.layers) & 1]
 
     def _build(self, b0: int, B: int, S: int) -> None:
@@ -343,7 +362,12 @@ class Fp16Encoder(_EncoderBase):
         # the weights of this object are written once, in __init__: every GEMM of the launch list carries the
         # constant-weights promise for its own call (nothing process-wide is switched)
         CW = GEMM_CONST_WEIGHTS
-        GF = self.gemm_flags  # the plain GEMMs also carry the kernel choice
+        # the plain GEMMs also carry the kernel choice
+        GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(2, n, k))
+              for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
+        fused_ln = self._fused_layernorm()
+        self.launches_per_layer = 5 if fused_ln else 7
+        ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
         self.lead_launches = 2 if packed else 1
         if packed:
             self._add("zen_pack_tokens_i32", self.ids.data_ptr(), None, self.kv_lens.data_ptr(), B, S, T,
@@ -362,7 +386,7 @@ class Fp16Encoder(_EncoderBase):
         for L in self.layers:
             x, xn = self.x[cur], self.x[cur ^ 1]
             self._add("zen_linear_f16_ex", P(x), H, L["wqkv"].data_ptr(), H, T, 3 * H, H, L["bqkv"].data_ptr(),
-                      ACT_NONE, DT_F16, P(self.qkv), 3 * H, GF)
+                      ACT_NONE, DT_F16, P(self.qkv), 3 * H, GF[3 * H, H])
             if packed:
                 self._add("zen_flash_attention_unpadded_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H,
                           P(self.ctx), None, 1.0, B, nh, S, hd, T, 3 * H, hd, 3 * H, hd, 3 * H, hd, H, hd,
@@ -370,24 +394,24 @@ class Fp16Encoder(_EncoderBase):
             else:
                 self._add("zen_flash_attention_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H, P(self.ctx), None,
                           1.0, B, nh, S, hd, *qs, *qs, *qs, *os_, kv, 0, 1.0 / math.sqrt(hd))
-            if self.fuse_layernorm:
-                self._add("zen_linear_f16_add_layernorm_ex", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H,
+            if fused_ln:
+                self._add("zen_linear_f16_add_layernorm_ws", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H,
                           L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(), cfg.eps, P(self.h1),
-                          None, 1.0, ROUND_NEAREST_EVEN, CW)
+                          None, 1.0, ROUND_NEAREST_EVEN, *ws, CW | self._plan(2, H, H, True))
             else:
                 self._add("zen_linear_f16_ex", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H, L["bo"].data_ptr(),
-                          ACT_NONE, DT_F16, P(self.ao), H, GF)
+                          ACT_NONE, DT_F16, P(self.ao), H, GF[H, H])
                 self._add("zen_add_layernorm_f16", P(self.ao), P(x), L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(),
                           P(self.h1), None, 1.0, ROUND_NEAREST_EVEN, T, H, cfg.eps)
             self._add("zen_linear_f16_ex", P(self.h1), H, L["w1"].data_ptr(), H, T, F, H, L["b1"].data_ptr(),
-                      ACT_GELU, DT_F16, P(self.g), F, GF)
-            if self.fuse_layernorm:
-                self._add("zen_linear_f16_add_layernorm_ex", P(self.g), F, L["w2"].data_ptr(), F, T, H, F,
+                      ACT_GELU, DT_F16, P(self.g), F, GF[F, H])
+            if fused_ln:
+                self._add("zen_linear_f16_add_layernorm_ws", P(self.g), F, L["w2"].data_ptr(), F, T, H, F,
                           L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(), L["ln2_b"].data_ptr(), cfg.eps, P(xn),
-                          None, 1.0, ROUND_NEAREST_EVEN, CW)
+                          None, 1.0, ROUND_NEAREST_EVEN, *ws, CW | self._plan(2, H, F, True))
             else:
                 self._add("zen_linear_f16_ex", P(self.g), F, L["w2"].data_ptr(), F, T, H, F, L["b2"].data_ptr(),
-                          ACT_NONE, DT_F16, P(self.o), H, GF)
+                          ACT_NONE, DT_F16, P(self.o), H, GF[H, F])
                 self._add("zen_add_layernorm_f16", P(self.o), P(self.h1), L["ln2_g"].data_ptr(), L["ln2_b"].data_ptr(),
                           P(xn), None, 1.0, ROUND_NEAREST_EVEN, T, H, cfg.eps)
             cur ^= 1
@@ -480,6 +504,7 @@ class Int8Encoder(_EncoderBase):
         super().__init__(cfg, params, device, micro_batches, gemm_pair)
         self.fuse_attention = fuse_attention
         self.keep_qkv = bool(keep_qkv)
+        self._ln_asked = fuse_layernorm
         self.fuse_layernorm = (cfg.hidden == 768) if fuse_layernorm is None else bool(fuse_layernorm)
         if self.fuse_layernorm and cfg.hidden not in (768, 1024):
             raise RuntimeError("the fused GEMM + LayerNorm kernel needs hidden == 768 or 1024")
@@ -517,6 +542,7 @@ class Int8Encoder(_EncoderBase):
         self.h1q = torch.empty((T, H), **s8)
         self.gq = torch.empty((T, F), **s8)
         self.o = torch.empty((T, H), **f16)
+        self.ln_ws = self._workspace(T) if self._fused_layernorm() else None
         self.out = self.x[len(self.layers) & 1]
 
     def _build(self, b0: int, B: int, S: int) -> None:
@@ -529,13 +555,17 @@ class Int8Encoder(_EncoderBase):
         # the weights of this object are written once, in __init__: every GEMM of the launch list carries the
         # constant-weights promise for its own call (nothing process-wide is switched)
         CW = GEMM_CONST_WEIGHTS
-        GF = self.gemm_flags  # the plain GEMMs also carry the kernel choice
+        # the plain GEMMs also carry the kernel choice
+        GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(1, n, k))
+              for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
+        fused_ln = self._fused_layernorm()
+        ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
         sc = self.act_scales
         can_fuse = S <= 128 and hd == 64
         if self.fuse_attention and not can_fuse:
             raise RuntimeError("the fused QKV + attention kernel needs seq <= 128 and head_dim == 64")
         fused_attn = can_fuse if self.fuse_attention is None else bool(self.fuse_attention)
-        self.launches_per_layer = (5 if self.fuse_layernorm else 7) - (1 if fused_attn else 0)
+        self.launches_per_layer = (5 if fused_ln else 7) - (1 if fused_attn else 0)
         self.lead_launches = 2 if packed else 1
         if packed:
             self._add("zen_pack_tokens_i32", self.ids.data_ptr(), None, self.kv_lens.data_ptr(), B, S, T,
@@ -564,7 +594,7 @@ class Int8Encoder(_EncoderBase):
                 # longer sequences (or head size 128): projection, then attention on the packed rows from the offsets
                 self._add("zen_linear_i8_ex", P(xq), H, L["wqkv"].data_ptr(), H, T, 3 * H, H, a["x"],
                           L["wqkv_s"].data_ptr(), L["bqkv"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
-                          P(self.qkv), 3 * H, *pf(L["wo"], L["w1"]), GF)
+                          P(self.qkv), 3 * H, *pf(L["wo"], L["w1"]), GF[3 * H, H])
                 self._add("zen_flash_attention_unpadded_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H,
                           P(self.ctx), P(self.ctxq), a["ctx"], B, nh, S, hd, T, 3 * H, hd, 3 * H, hd, 3 * H, hd, H, hd,
                           self.cu_seqlens.data_ptr(), 0, 1.0 / math.sqrt(hd))
@@ -580,31 +610,31 @@ class Int8Encoder(_EncoderBase):
             else:
                 self._add("zen_linear_i8_ex", P(xq), H, L["wqkv"].data_ptr(), H, T, 3 * H, H, a["x"],
                           L["wqkv_s"].data_ptr(), L["bqkv"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
-                          P(self.qkv), 3 * H, *pf(L["wo"], L["w1"]), GF)
+                          P(self.qkv), 3 * H, *pf(L["wo"], L["w1"]), GF[3 * H, H])
                 self._add("zen_flash_attention_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H, P(self.ctx),
                           P(self.ctxq), a["ctx"], B, nh, S, hd, *qs, *qs, *qs, *os_, kv, 0, 1.0 / math.sqrt(hd))
-            if self.fuse_layernorm:
-                self._add("zen_linear_i8_add_layernorm_ex", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
+            if fused_ln:
+                self._add("zen_linear_i8_add_layernorm_ws", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(),
-                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, CW)
+                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, *ws, CW | self._plan(1, H, H, True))
             else:
                 self._add("zen_linear_i8_ex", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
-                          P(self.ao), H, None, 0, None, 0, GF)
+                          P(self.ao), H, None, 0, None, 0, GF[H, H])
                 self._add("zen_add_layernorm_f16", P(self.ao), P(x), L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(),
                           P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, T, H, cfg.eps)
             self._add("zen_linear_i8_ex", P(self.h1q), H, L["w1"].data_ptr(), H, T, F, H, a["h1"],
                       L["w1_s"].data_ptr(), L["b1"].data_ptr(), ACT_GELU, DT_S8, a["gelu"], ROUND_NEAREST_EVEN,
-                      P(self.gq), F, *pf(L["w2"], None if last else self.layers[li + 1]["wqkv"]), GF)
-            if self.fuse_layernorm:
-                self._add("zen_linear_i8_add_layernorm_ex", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
+                      P(self.gq), F, *pf(L["w2"], None if last else self.layers[li + 1]["wqkv"]), GF[F, H])
+            if fused_ln:
+                self._add("zen_linear_i8_add_layernorm_ws", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(),
                           L["ln2_b"].data_ptr(), cfg.eps, P(xn), None if last else P(xqn),
-                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, CW)
+                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, *ws, CW | self._plan(1, H, F, True))
             else:
                 self._add("zen_linear_i8_ex", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
-                          P(self.o), H, None, 0, None, 0, GF)
+                          P(self.o), H, None, 0, None, 0, GF[H, F])
                 self._add("zen_add_layernorm_f16", P(self.o), P(self.h1), L["ln2_g"].data_ptr(), L["ln2_b"].data_ptr(),
                           P(xn), None if last else P(xqn), 1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, T, H,
                           cfg.eps)

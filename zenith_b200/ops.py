@@ -135,9 +135,17 @@ def linear_int8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", 
     return out
 
 
+def _layernorm_workspace(elem_bytes: int, M: int, N: int, K: int, device):
+    """fp32 scratch of a ``*_add_layernorm_ws`` call, or None where the call runs as one kernel; with its size in bytes."""
+    if N not in (768, 1024) or (_capi.lib().zen_gemm_plan(elem_bytes, M, N, K, 1) >> 20) & 0xf == 15:
+        return None, 0
+    return torch.empty((M, N), dtype=torch.float32, device=device), M * N * 4
+
+
 def linear_int8_add_layernorm(xq, wq, x_scale: float, w_scale, bias, residual, gamma, beta, eps: float, *,
                               out_scale: float | None = None, round="nearest_even", constant_weights=False):
-    """``LayerNorm(dequant(xq @ wq.T) + bias + residual) * gamma + beta`` in one kernel (hidden size 768).
+    """``LayerNorm(dequant(xq @ wq.T) + bias + residual) * gamma + beta`` (hidden size 768 or 1024): one kernel, or
+    two launches with fp32 rows in between where that is faster (few rows, or more than one round of the one kernel).
 
     Returns fp16 ``y`` and, with ``out_scale``, also the int8 copy ``quantize(y, out_scale)``.
     """
@@ -157,16 +165,19 @@ def linear_int8_add_layernorm(xq, wq, x_scale: float, w_scale, bias, residual, g
     y = torch.empty((M, N), dtype=torch.float16, device=xq.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=xq.device) if out_scale is not None else None
     if M:
-        _call("zen_linear_i8_add_layernorm_ex", xq.data_ptr(), K, wq.data_ptr(), K, M, N, K, float(x_scale), _ptr(w_scale),
+        ws, ws_bytes = _layernorm_workspace(1, M, N, K, xq.device)
+        _call("zen_linear_i8_add_layernorm_ws", xq.data_ptr(), K, wq.data_ptr(), K, M, N, K, float(x_scale), _ptr(w_scale),
               _ptr(bias), residual.data_ptr(), N, gamma.data_ptr(), beta.data_ptr(), float(eps), y.data_ptr(), _ptr(yq),
-              float(out_scale or 1.0), _ROUND[round], _capi.GEMM_CONST_WEIGHTS if constant_weights else 0, _stream())
+              float(out_scale or 1.0), _ROUND[round], _ptr(ws), ws_bytes, _capi.GEMM_CONST_WEIGHTS if constant_weights else 0,
+              _stream())
+        launch_count_add(0 if ws is None else 1)
     return y if yq is None else (y, yq)
 
 
 def linear_fp16_add_layernorm(x, w, bias, residual, gamma, beta, eps: float, *, out_scale: float | None = None,
                               round="nearest_even", constant_weights=False):
-    """``LayerNorm(x @ w.T + bias + residual) * gamma + beta`` with fp16 operands in one kernel (hidden 768 or
-    1024).  Returns fp16 ``y`` and, with ``out_scale``, also ``quantize(y, out_scale)``."""
+    """``LayerNorm(x @ w.T + bias + residual) * gamma + beta`` with fp16 operands (hidden 768 or 1024), as
+    ``linear_int8_add_layernorm``.  Returns fp16 ``y`` and, with ``out_scale``, also ``quantize(y, out_scale)``."""
     _require(x, "x", torch.float16, 2)
     _require(w, "w", torch.float16, 2)
     _require(residual, "residual", torch.float16, 2)
@@ -181,9 +192,11 @@ def linear_fp16_add_layernorm(x, w, bias, residual, gamma, beta, eps: float, *, 
     y = torch.empty((M, N), dtype=torch.float16, device=x.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=x.device) if out_scale is not None else None
     if M:
-        _call("zen_linear_f16_add_layernorm_ex", x.data_ptr(), K, w.data_ptr(), K, M, N, K, _ptr(bias), residual.data_ptr(), N,
+        ws, ws_bytes = _layernorm_workspace(2, M, N, K, x.device)
+        _call("zen_linear_f16_add_layernorm_ws", x.data_ptr(), K, w.data_ptr(), K, M, N, K, _ptr(bias), residual.data_ptr(), N,
               gamma.data_ptr(), beta.data_ptr(), float(eps), y.data_ptr(), _ptr(yq), float(out_scale or 1.0), _ROUND[round],
-              _capi.GEMM_CONST_WEIGHTS if constant_weights else 0, _stream())
+              _ptr(ws), ws_bytes, _capi.GEMM_CONST_WEIGHTS if constant_weights else 0, _stream())
+        launch_count_add(0 if ws is None else 1)
     return y if yq is None else (y, yq)
 
 
