@@ -37,6 +37,23 @@ def test_attention_fp16(cuda, B, H, S, D, causal, lens):
     assert np.mean(np.abs(got - want)) < 2e-4
 
 
+@pytest.mark.parametrize("S,D", [(129, 64), (255, 128), (257, 64), (383, 128), (385, 128), (640, 64), (2048, 64), (2049, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_at_tile_edges(cuda, S, D, causal):
+    """Ends of query tiles and key blocks, a tile without keys of its own, both tile counts per CTA (the line lies at 2048
+    tokens for head size 64), key lengths at and next to a block's end; the last query rows against the oracle."""
+    lens = [S, max(1, S - 127), 128, 0] if S < 1000 else [S, S - 1, 1025, 128]
+    r = rng(S + D)
+    q, k, v = (r.standard_normal((4, 2, S, D)).astype(np.float16) for _ in range(3))
+    kl = np.array(lens, np.int32)
+    o = ops.flash_attention(*(torch.from_numpy(a).to(cuda) for a in (q, k, v)), causal=causal, kv_lens=torch.from_numpy(kl).to(cuda))
+    got = o.float().cpu().numpy()
+    assert not np.isnan(got).any()
+    rows = np.unique(np.clip([0, 1, 127, 128, S // 2, S - 129, S - 128, S - 1], 0, S - 1))
+    want = O.attention_rows(q.astype(np.float32), k.astype(np.float32), v.astype(np.float32), rows, kl, causal)
+    assert np.max(np.abs(got[:, :, rows] - want)) < 1e-2
+
+
 def test_fully_masked_batch_yields_zeros(cuda):
     o, want = run(cuda, 2, 2, 200, 64, lens=[0, 77])
     assert torch.all(o[0] == 0) and np.all(want[0] == 0)

@@ -41,7 +41,6 @@ struct GemmLnParams {
 };
 
 constexpr int LN_CLUSTER = 4;
-constexpr int LN_ROWS_WIDE_MAX = 1024;  // rows up to which ln_rows_kernel spreads a row over H / 128 warps
 
 __device__ __forceinline__ void st_cluster_f32x2(uint32_t cluster_addr, float a, float b) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
@@ -53,8 +52,16 @@ __device__ __forceinline__ void chan_merge(float& n_a, float& mean_a, float& m2_
   const float delta = mean_b - mean_a;
   const float f = n_b / n;
   mean_a = fmaf(delta, f, mean_a);
-  m2_a = m2_a + m2_b + delta * delta * n_a * f;
+  m2_a = fmaf(__fmul_rn(__fmul_rn(delta, delta), n_a), f, __fadd_rn(m2_a, m2_b));
   n_a = n;
+}
+
+// (mean, m2) of 16-column group i of a slab <- merge of groups 0 .. i - 1 (pmean, pm2) with it: n_a = 16 i, n_b = 16
+__device__ __forceinline__ void slab_merge(int i, float pmean, float pm2, float& mean, float& m2) {
+  const float f = i == 1 ? 0.5f : i == 2 ? (1.0f / 3.0f) : i == 3 ? 0.25f : 1.0f / float(i + 1);
+  const float delta = __fsub_rn(mean, pmean);
+  mean = fmaf(delta, f, pmean);
+  m2 = fmaf(__fmul_rn(delta, delta), __fmul_rn(float(GEMM_CW * i), f), __fadd_rn(pm2, m2));
 }
 
 template <int BN, int STAGES>
@@ -314,16 +321,10 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
             q22 = f2fma(d, d, q22);
           }
           const float q2 = q22.x + q22.y;
-          if (i == 0) {
-            mean = mu;
-            m2 = q2;
-          } else {
-            // pairwise update with n_a = 16 i, n_b = 16: n_b / n = 1 / (i + 1)
-            const float f = i == 1 ? 0.5f : i == 2 ? (1.0f / 3.0f) : i == 3 ? 0.25f : 1.0f / float(i + 1);
-            const float delta = mu - mean;
-            mean = fmaf(delta, f, mean);
-            m2 = m2 + q2 + delta * delta * (float(GEMM_CW * i) * f);
-          }
+          float gm = mu, gq = q2;
+          if (i > 0) slab_merge(i, mean, m2, gm, gq);
+          mean = gm;
+          m2 = gq;
         }
         tmem_wait_st();
         pstats[sub * 128 + r] = make_float2(mean, m2);
@@ -363,7 +364,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
             chan_merge(c, mu, q2, float(BN), o.x, o.y);
           }
         }
-        const float rstd = rsqrtf(q2 * inv_n + p.eps);
+        const float rstd = rsqrtf(fmaf(q2, inv_n, p.eps));
 
         // ---- pass B: normalise y (read back from tensor memory), stage fp16 (+ int8), TMA stores
 #pragma unroll 1
@@ -469,8 +470,12 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 
 // ---------------------------------------------------------------------------------------------
 // Residual add and LayerNorm of fp32 rows (projection + bias, from the GEMM's fp32 output) -> fp16 (+ int8 copy): the second
-// launch of the two-kernel form.  With few rows the row's latency is what counts: it is spread over H / 128 warps with one
-// 16-byte unit per lane.  With many, one warp owns a row (no block barrier) and holds it in registers.
+// launch of the two-kernel form.  A row is spread over H / 128 warps, one 16-byte unit per lane: what counts with few rows
+// is one row's latency (1.6 us per launch at 24 .. 128 rows; a warp per row 2.9), and with many the warps of ten rows hide it.
+//
+// The arithmetic is that of the fused kernel, operation for operation, so that a row's result has the same bits in either
+// form: 16-column groups summed pair by pair (here the running sums hop over the four lanes that hold a group), groups
+// merged one after the other to 64-column slabs, slabs to quarters, quarters to the row.
 // ---------------------------------------------------------------------------------------------
 struct LnRowsParams {
   const float* t;          // [rows, H]: projection + bias
@@ -482,105 +487,99 @@ struct LnRowsParams {
   int8_t* yq;
   float out_scale, eps;
   int round_mode;
-  int rows;
 };
 
-template <int H, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? H / 4 : 128) ln_rows_kernel(const LnRowsParams p) {
-  constexpr int VPL = WIDE ? 1 : H / 128;  // float4 units per lane
+template <int H>
+__global__ void __launch_bounds__(H / 4) ln_rows_kernel(const LnRowsParams p) {
+  constexpr int SLABS = H / 64;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row = WIDE ? int(blockIdx.x) : int(blockIdx.x) * 4 + warp;
-  const int c0 = WIDE ? warp * 128 + lane * 4 : lane * 4;
+  const int64_t row = blockIdx.x;
+  const int c0 = int(threadIdx.x) * 4;
   grid_launch_dependents();
   grid_dependency_wait();
-  if (row >= p.rows) return;  // whole rows only: every warp of a row meets the block barriers below
-  const float* t = p.t + int64_t(row) * H + c0;
-  const __half* res = p.residual + int64_t(row) * p.ldr + c0;
-  float2 v[VPL][2];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const float4 f = *reinterpret_cast<const float4*>(t + i * 128);
-    const uint2 u = *reinterpret_cast<const uint2*>(res + i * 128);
-    const __half2* rh = reinterpret_cast<const __half2*>(&u);
-    v[i][0] = f2add(make_float2(f.x, f.y), __half22float2(rh[0]));
-    v[i][1] = f2add(make_float2(f.z, f.w), __half22float2(rh[1]));
-  }
-  uint2 gb[VPL], bb[VPL];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    gb[i] = *reinterpret_cast<const uint2*>(p.gamma + c0 + i * 128);
-    bb[i] = *reinterpret_cast<const uint2*>(p.beta + c0 + i * 128);
-  }
-  __shared__ float red[2][H / 128];
-  auto row_sum = [&](float2 s2, int use) -> float {
-    float s = s2.x + s2.y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if constexpr (WIDE) {
-      if (lane == 0) red[use][warp] = s;
-      __syncthreads();
-      s = 0.f;
-#pragma unroll
-      for (int w = 0; w < H / 128; ++w) s += red[use][w];
-    }
-    return s;
-  };
+  const float4 f = *reinterpret_cast<const float4*>(p.t + row * H + c0);
+  const uint2 u = *reinterpret_cast<const uint2*>(p.residual + row * p.ldr + c0);
+  const uint2 gb = *reinterpret_cast<const uint2*>(p.gamma + c0);
+  const uint2 bb = *reinterpret_cast<const uint2*>(p.beta + c0);
+  const __half2* rh = reinterpret_cast<const __half2*>(&u);
+  const float2 y[2] = {f2add(make_float2(f.x, f.y), __half22float2(rh[0])), f2add(make_float2(f.z, f.w), __half22float2(rh[1]))};
+  const int sub = lane & 3, group = (lane >> 2) & 3;  // lane of the 16-column group, group of the 64-column slab
+  // sum of the group: lane 0 starts, each lane adds its two pairs to what the lane before it has
   float2 s2 = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) s2 = f2add(s2, f2add(v[i][0], v[i][1]));
-  const float mean = row_sum(s2, 0) * (1.0f / float(H));
-  const float2 nmu = make_float2(-mean, -mean);
-  float2 q2 = make_float2(0.f, 0.f);
+  for (int k = 0; k < 4; ++k) {
+    const float2 in = make_float2(__shfl_up_sync(0xffffffffu, s2.x, 1), __shfl_up_sync(0xffffffffu, s2.y, 1));
+    if (sub == k) s2 = f2add(f2add(k == 0 ? make_float2(0.f, 0.f) : in, y[0]), y[1]);
+  }
+  float mean = __shfl_sync(0xffffffffu, (s2.x + s2.y) * (1.0f / GEMM_CW), lane | 3);
+  const float2 gmu = make_float2(-mean, -mean);
+  const float2 d0 = f2add(y[0], gmu), d1 = f2add(y[1], gmu);
+  float2 q22 = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < VPL; ++i)
+  for (int k = 0; k < 4; ++k) {
+    const float2 in = make_float2(__shfl_up_sync(0xffffffffu, q22.x, 1), __shfl_up_sync(0xffffffffu, q22.y, 1));
+    if (sub == k) q22 = f2fma(d1, d1, f2fma(d0, d0, k == 0 ? make_float2(0.f, 0.f) : in));
+  }
+  float m2 = q22.x + q22.y;  // lane 3 of the group
+  // groups of the slab in turn: the running (mean, M2) hop from one group's lane 3 to the next one's
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      v[i][h] = f2add(v[i][h], nmu);
-      q2 = f2fma(v[i][h], v[i][h], q2);
+  for (int i = 1; i < 4; ++i) {
+    const float pm = __shfl_up_sync(0xffffffffu, mean, 4), pq = __shfl_up_sync(0xffffffffu, m2, 4);
+    if (group == i) slab_merge(i, pm, pq, mean, m2);
+  }
+  __shared__ float2 slab[SLABS];
+  if ((lane & 15) == 15) slab[2 * warp + (lane >> 4)] = make_float2(mean, m2);
+  __syncthreads();
+  float c = float(H / 4), mu = 0.f, q2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float cc = 64.f, m = slab[k * (SLABS / 4)].x, q = slab[k * (SLABS / 4)].y;
+#pragma unroll
+    for (int s = 1; s < SLABS / 4; ++s) chan_merge(cc, m, q, 64.f, slab[k * (SLABS / 4) + s].x, slab[k * (SLABS / 4) + s].y);
+    if (k == 0) {
+      mu = m;
+      q2 = q;
+    } else {
+      chan_merge(c, mu, q2, float(H / 4), m, q);
     }
-  const float rstd = rsqrtf(fmaf(row_sum(q2, 1), 1.0f / float(H), p.eps));
-  const float2 rstd2 = make_float2(rstd, rstd);
-  const float inv_q = ZEN_DIV(1.0f, p.out_scale);
-  const int64_t off = int64_t(row) * H + c0;
+  }
+  const float rstd = rsqrtf(fmaf(q2, 1.0f / float(H), p.eps));
+  const float2 nmu = make_float2(-mu, -mu), rstd2 = make_float2(rstd, rstd);
+  const int64_t off = row * H + c0;
+  const __half2* g = reinterpret_cast<const __half2*>(&gb);
+  const __half2* b = reinterpret_cast<const __half2*>(&bb);
+  uint2 w;
+  float2 of[2];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const __half2* g = reinterpret_cast<const __half2*>(&gb[i]);
-    const __half2* b = reinterpret_cast<const __half2*>(&bb[i]);
-    uint2 w;
-    float2 of[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float2 o = f2fma(f2mul(v[i][h], rstd2), __half22float2(g[h]), __half22float2(b[h]));
-      const __half2 hv = __floats2half2_rn(o.x, o.y);
-      (h ? w.y : w.x) = *reinterpret_cast<const uint32_t*>(&hv);
-      of[h] = __half22float2(hv);
-    }
-    *reinterpret_cast<uint2*>(p.y + off + i * 128) = w;
-    if (p.yq) {
-      uint32_t qw[1];
-      if (p.round_mode == 0) {
-        const uint32_t risky = quantize_pairs_rn<4>(of, inv_q, qw);
-        if (risky) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (risky & (1u << j)) patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), 0));
-        }
-      } else {
-        qw[0] = 0;
+  for (int h = 0; h < 2; ++h) {
+    const float2 o = f2fma(f2mul(f2add(y[h], nmu), rstd2), __half22float2(g[h]), __half22float2(b[h]));
+    const __half2 hv = __floats2half2_rn(o.x, o.y);
+    (h ? w.y : w.x) = *reinterpret_cast<const uint32_t*>(&hv);
+    of[h] = __half22float2(hv);
+  }
+  *reinterpret_cast<uint2*>(p.y + off) = w;
+  if (p.yq) {
+    uint32_t qw[1];
+    if (p.round_mode == 0) {
+      const uint32_t risky = quantize_pairs_rn<4>(of, ZEN_DIV(1.0f, p.out_scale), qw);
+      if (risky) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), p.round_mode));
+          if (risky & (1u << j)) patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), 0));
       }
-      *reinterpret_cast<uint32_t*>(p.yq + off + i * 128) = qw[0];
+    } else {
+      qw[0] = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), p.round_mode));
     }
+    *reinterpret_cast<uint32_t*>(p.yq + off) = qw[0];
   }
 }
 
 template <int H>
-static int launch_ln_rows(const LnRowsParams& p, cudaStream_t s) {
-  if (p.rows <= LN_ROWS_WIDE_MAX)
-    return launch_pdl(PDL_GEMM, ln_rows_kernel<H, true>, dim3(unsigned(p.rows)), dim3(H / 4), 0, s, p);
-  return launch_pdl(PDL_GEMM, ln_rows_kernel<H, false>, dim3(unsigned((p.rows + 3) / 4)), dim3(128), 0, s, p);
+static int launch_ln_rows(const LnRowsParams& p, int rows, cudaStream_t s) {
+  return launch_pdl(PDL_GEMM, ln_rows_kernel<H>, dim3(unsigned(rows)), dim3(H / 4), 0, s, p);
 }
 
 template <int KIND, int BN, int STAGES>
@@ -656,8 +655,8 @@ static int run_linear_add_layernorm(const void* x, int64_t ldx, const void* w, i
     g.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
     if (int st = run_gemm_auto(KIND, x, ldx, w, ldw, g, ZEN_GEMM_SPLIT_K(form == 14 ? 15 : form) | narrow, s); st != ZEN_OK) return st;
     const LnRowsParams lp{static_cast<const float*>(workspace), static_cast<const __half*>(residual), ldr, static_cast<const __half*>(gamma),
-                          static_cast<const __half*>(beta), static_cast<__half*>(y), yq, yq ? out_scale : 1.0f, eps, round_mode, M};
-    return N == 768 ? launch_ln_rows<768>(lp, s) : launch_ln_rows<1024>(lp, s);
+                          static_cast<const __half*>(beta), static_cast<__half*>(y), yq, yq ? out_scale : 1.0f, eps, round_mode};
+    return N == 768 ? launch_ln_rows<768>(lp, M, s) : launch_ln_rows<1024>(lp, M, s);
   }
   const int BN = N / LN_CLUSTER;
   constexpr int BK = 128 / ELEM;

@@ -161,14 +161,6 @@ class _EncoderBase:
         micro-batches then run every row on the same kernels and keep its bits."""
         return _capi.lib().zen_gemm_plan(elem_bytes, self._shape[0] * self._shape[1], N, K, int(layernorm))
 
-    def _fused_layernorm(self) -> bool:
-        """Whether attention-output and FFN2 of the prepared shape run as one ``*_add_layernorm_ws`` call each.  Not asked
-        for, hidden 1024 does so up to 2048 rows, where the call's two launches with fp32 rows in between beat the separate
-        kernels (9.9 against 12.4 us for FFN2 at 512 rows); with more, the fp32 rows cost more than they save."""
-        if self.fuse_layernorm or self.cfg.hidden != 1024 or self._ln_asked is not None:
-            return self.fuse_layernorm
-        return self._shape[0] * self._shape[1] <= 2048
-
     def _workspace(self, T: int) -> torch.Tensor:
         """fp32 rows of a projection on its way to a LayerNorm (scratch of one launch pair)."""
         return torch.empty((T, self.cfg.hidden), dtype=torch.float32, device=self.device)
@@ -322,7 +314,6 @@ class Fp16Encoder(_EncoderBase):
         """``fuse_layernorm``: attention-output and FFN2 as one GEMM + residual + LayerNorm kernel each (5 launches
         per layer instead of 7); possible for hidden 768 and 1024, on by default for 768."""
         super().__init__(cfg, params, device, micro_batches, gemm_pair)
-        self._ln_asked = fuse_layernorm
         self.fuse_layernorm = (cfg.hidden == 768) if fuse_layernorm is None else bool(fuse_layernorm)
         if self.fuse_layernorm and cfg.hidden not in (768, 1024):
             raise RuntimeError("the fused GEMM + LayerNorm kernel needs hidden == 768 or 1024")
@@ -344,12 +335,14 @@ class Fp16Encoder(_EncoderBase):
             self.out_padded = torch.empty((B * S, H), **f16)
         self.x = [torch.empty((T, H), **f16) for _ in range(2)]
         self.qkv = torch.empty((T, 3 * H), **f16)
-        self.ctx = torch.empty((T, H), **f16)
+        # rows of no sequence (beyond a packed batch's total) are never written: zeros, so that nothing non-finite can reach
+        # the values of the last sequence's key tile
+        self.ctx = torch.zeros((T, H), **f16)
         self.ao = torch.empty((T, H), **f16)
         self.h1 = torch.empty((T, H), **f16)
         self.g = torch.empty((T, F), **f16)
         self.o = torch.empty((T, H), **f16)
-        self.ln_ws = self._workspace(T) if self._fused_layernorm() else None
+        self.ln_ws = self._workspace(T) if self.fuse_layernorm else None
         self.out = self.x[len(self.layers) & 1]
 
     def _build(self, b0: int, B: int, S: int) -> None:
@@ -365,7 +358,7 @@ class Fp16Encoder(_EncoderBase):
         # the plain GEMMs also carry the kernel choice
         GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(2, n, k))
               for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
-        fused_ln = self._fused_layernorm()
+        fused_ln = self.fuse_layernorm
         self.launches_per_layer = 5 if fused_ln else 7
         ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
         self.lead_launches = 2 if packed else 1
@@ -504,7 +497,6 @@ class Int8Encoder(_EncoderBase):
         super().__init__(cfg, params, device, micro_batches, gemm_pair)
         self.fuse_attention = fuse_attention
         self.keep_qkv = bool(keep_qkv)
-        self._ln_asked = fuse_layernorm
         self.fuse_layernorm = (cfg.hidden == 768) if fuse_layernorm is None else bool(fuse_layernorm)
         if self.fuse_layernorm and cfg.hidden not in (768, 1024):
             raise RuntimeError("the fused GEMM + LayerNorm kernel needs hidden == 768 or 1024")
@@ -535,14 +527,16 @@ class Int8Encoder(_EncoderBase):
         self.x = [torch.empty((T, H), **f16) for _ in range(2)]
         self.xq = [torch.empty((T, H), **s8) for _ in range(2)]
         self.qkv = torch.empty((T, 3 * H), **f16)
-        self.ctx = torch.empty((T, H), **f16)
-        self.ctxq = torch.empty((T, H), **s8)
+        # rows of no sequence (beyond a packed batch's total) are never written: zeros, so that nothing non-finite can reach
+        # the values of the last sequence's key tile
+        self.ctx = torch.zeros((T, H), **f16)
+        self.ctxq = torch.zeros((T, H), **s8)
         self.ao = torch.empty((T, H), **f16)
         self.h1 = torch.empty((T, H), **f16)
         self.h1q = torch.empty((T, H), **s8)
         self.gq = torch.empty((T, F), **s8)
         self.o = torch.empty((T, H), **f16)
-        self.ln_ws = self._workspace(T) if self._fused_layernorm() else None
+        self.ln_ws = self._workspace(T) if self.fuse_layernorm else None
         self.out = self.x[len(self.layers) & 1]
 
     def _build(self, b0: int, B: int, S: int) -> None:
@@ -558,7 +552,7 @@ class Int8Encoder(_EncoderBase):
         # the plain GEMMs also carry the kernel choice
         GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(1, n, k))
               for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
-        fused_ln = self._fused_layernorm()
+        fused_ln = self.fuse_layernorm
         ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
         sc = self.act_scales
         can_fuse = S <= 128 and hd == 64
