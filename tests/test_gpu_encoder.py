@@ -237,3 +237,31 @@ def test_fp16_encoder_with_fused_layernorm_kernels(cuda):
     assert torch.equal(enc.replay(), eager)
     taps = enc.forward_with_taps(*tdev(ids, lens, cuda))
     assert len(taps["h1"]) == cfg.layers and all(lo < hi for lo, hi in taps["h1"])
+
+
+@pytest.mark.parametrize("micro_batches", [1, 2])
+def test_repeated_plain_calls_equal_the_first(cuda, params, micro_batches):
+    """From its third call for a shape on ``forward`` replays a recorded graph: same bits as the launches it recorded, for
+    new inputs, after a change of shape, on another stream, and inside a caller's own capture."""
+    enc, ref = (Fp16Encoder(CFG, params, cuda, micro_batches=micro_batches) for _ in range(2))
+    mk = lambda s, B, S: tdev(rng(s).integers(0, CFG.vocab, (B, S)), (S - rng(s).integers(0, S // 2, B)).astype(np.int32), cuda)
+    for B, S in ((3, 40), (2, 64), (3, 40)):
+        for i in range(5):
+            ids, lens = mk(10 * B + i, B, S)
+            ref._plain_calls = 0  # the reference never records
+            assert torch.equal(enc.forward(ids, lens), ref.forward(ids, lens)), (B, S, i)
+        assert enc._pass_graph is not None and ref._pass_graph is None
+    ids, lens = mk(77, 3, 40)
+    want = ref.forward(ids, lens).clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = enc.forward(ids, lens).clone()
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(got, want)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = enc.forward(ids, lens)
+    out.zero_()
+    g.replay()
+    assert torch.equal(out, want)

@@ -29,16 +29,19 @@ inline SmallChoice small_rule(int elem_bytes, int M, int N, int K, bool layernor
 }
 
 // Form of a projection + residual + LayerNorm: the value of the ZEN_GEMM_SPLIT_K field, 15 = one kernel (four-CTA clusters),
-// 14 = large-tile GEMM with fp32 output and a LayerNorm of its rows, else the small-product kernel and that LayerNorm.  One
-// round of the clusters (37 row blocks) takes 9.5 - 10.4 us (K 768) or 16.4 (K 3072) whatever the rows; the two launches
-// take 7.4 / 10.5 us at 1024 rows, 10.3 / 14.1 at 2048, 11.9 / 17.3 at 4096, and 14.6 / 22.3 against the clusters' second
-// round of 19.6 / 30.9 at 4864.  At hidden 1024 a cluster holds 256 columns per CTA in a two-stage ring: never better.
+// 14 = large-tile GEMM with fp32 output and a LayerNorm of its rows, else the small-product kernel and that LayerNorm.  A
+// round of the clusters (37 row blocks) takes 9.5 - 10.4 us (K 768) or 16.4 (K 3072) whatever it holds; the two launches
+// take 7.4 / 10.5 us at 1024 rows, 10.3 / 14.1 at 2048, 12 / 17 at 4096, 18 / 25 at 4864 against 19.6 / 30.9, 25 / 32 at
+// 7680 against 20 / 31: they win in a first round that is not full and where a further round would hold little.  At hidden
+// 1024 a cluster CTA holds 256 columns in a two-stage ring and never wins.
 inline SmallChoice layernorm_rule(int elem_bytes, int M, int N, int K) {
   const SmallChoice c = small_rule(elem_bytes, M, N, K, true);
   if (c.ks > 0) return c;
-  const long kb = (long(K) * elem_bytes + 127) / 128;
-  if (N != 768 || M <= (kb >= 16 ? 3072 : 1536) || M > 37 * GEMM_BM) return {64, 14};
-  return {64, 15};
+  const bool deep = (long(K) * elem_bytes + 127) / 128 >= 16;
+  const int blocks = (M + GEMM_BM - 1) / GEMM_BM;
+  const int last = (blocks - 1) % 37 + 1;  // row blocks of the last round
+  const bool two = blocks <= 37 ? last <= (deep ? 24 : 12) : last <= (deep ? 18 : 5);
+  return {64, N != 768 || two ? 14 : 15};
 }
 
 // kind: KIND_*; bn: 64 or 32; ks: 1, 2, 4 or (bn 64) 8; b_mn: B is [K, N] (fp16 only, bn 64).  num_k_blocks is filled in here.

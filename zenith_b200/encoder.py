@@ -113,6 +113,8 @@ class _EncoderBase:
         self._packed_rows = None  # row capacity of the packed (unpadded) form, None in the padded form
         self._launches: list = []
         self._graph = None
+        self._pass_graph = None
+        self._plain_calls = 0
         self.launches_per_forward = 0
 
     # -- per-shape state --------------------------------------------------------------------
@@ -129,6 +131,8 @@ class _EncoderBase:
         self._shape = (B, S, packed_rows)
         self._packed_rows = packed_rows
         self._graph = None
+        self._pass_graph = None  # graph of the plain call, recorded once a shape has come a third time
+        self._plain_calls = 0
         d = self.device
         # token ids and key lengths share one allocation, so that a host can feed both with one copy
         self.inputs = torch.zeros(B * S + B, dtype=torch.int32, device=d)
@@ -190,6 +194,31 @@ class _EncoderBase:
                 main.wait_stream(s)
         ops.launch_count += len(self._launches)
 
+    def _run_plain(self) -> None:
+        """One pass for ``forward`` / ``forward_unpadded``.  Issuing 49 and more launches one by one costs the host 340 us,
+        more than a short batch takes on the device (BERT-base W8A8, one 24-token sequence: 300 us), so from the third call
+        for a shape on the pass is one graph of the same launches (recorded without running anything or waiting for the
+        device).  Inside a caller's own stream capture the launches are issued as they are."""
+        if torch.cuda.is_current_stream_capturing():
+            self._run()
+            return
+        if self._pass_graph is None:
+            self._plain_calls += 1
+            if self._plain_calls < 3:
+                self._run()
+                return
+            side = torch.cuda.Stream(device=self.device)
+            side.wait_stream(torch.cuda.current_stream())
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.stream(side):
+                graph.capture_begin(capture_error_mode="thread_local")
+                self._run()
+                graph.capture_end()
+            ops.launch_count -= len(self._launches)  # recorded, not launched
+            self._pass_graph = graph
+        self._pass_graph.replay()
+        ops.launch_count += len(self._launches)
+
     # -- public ------------------------------------------------------------------------------
     def set_inputs(self, ids, kv_lens=None) -> None:
         """Copy token ids ([B,S] integer tensor, any device) and key lengths into the static buffers."""
@@ -213,7 +242,7 @@ class _EncoderBase:
         """Hidden states ``[B*S, hidden]`` fp16 (a static buffer, overwritten by the next call)."""
         self._prepare(*ids.shape, None)
         self.set_inputs(ids, kv_lens)
-        self._run()
+        self._run_plain()
         return self.out
 
     # Unpadded form: the valid tokens of the batch are packed back to back (sequence b in rows cu_seqlens[b] ..),
@@ -234,7 +263,7 @@ class _EncoderBase:
         cap = min(B * S, self.unpadded_capacity(kv_lens.tolist(), S) if capacity is None else int(capacity))
         self._prepare(B, S, cap)
         self.set_inputs(ids, kv_lens)
-        self._run()
+        self._run_plain()
         return self.out_padded
 
     def capture_unpadded(self, B: int, S: int, capacity: int, slots: int = 1) -> None:
