@@ -327,7 +327,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
             for (int e = 0; e < 16; ++e)
               if (risky & (1u << e))
-                patch_q_byte(qw, e, zen_det_round_clamp_i8(ZEN_DIV((e & 1) ? val[e >> 1].y : val[e >> 1].x, p.o_scale), 0));
+                patch_q_byte(qw, e, exact_q8((e & 1) ? val[e >> 1].y : val[e >> 1].x, p.o_scale, 0));
           }
           // 16 values = 16-byte unit g % 4 of the row's 64-byte chunk g / 4
           *reinterpret_cast<uint4*>(stq + (g / 4) * (4 * 2048) + lane * 64 + (((g % 4) ^ ((lane >> 1) & 3)) << 4)) =

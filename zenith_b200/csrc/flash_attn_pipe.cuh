@@ -453,7 +453,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               if (risky & (1u << e))
-                patch_q_byte(qw, e, zen_det_round_clamp_i8(ZEN_DIV((e & 1) ? val[e >> 1].y : val[e >> 1].x, p.o_scale), 0));
+                patch_q_byte(qw, e, exact_q8((e & 1) ? val[e >> 1].y : val[e >> 1].x, p.o_scale, 0));
           }
           *reinterpret_cast<uint2*>(p.oq + off) = make_uint2(qw[0], qw[1]);
         }

@@ -404,13 +404,13 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
 #pragma unroll
                 for (int j = 0; j < GEMM_CW; ++j)
                   if (risky & (1u << j))
-                    patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), 0));
+                    patch_q_byte(qw, j, exact_q8((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale, 0));
               }
             } else {
               int q[GEMM_CW];
 #pragma unroll
               for (int j = 0; j < GEMM_CW; ++j)
-                q[j] = zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), p.round_mode);
+                q[j] = exact_q8((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale, p.round_mode);
               pack_q(q, qw);
             }
             *reinterpret_cast<uint4*>(stq + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = make_uint4(qw[0], qw[1], qw[2], qw[3]);
@@ -565,13 +565,13 @@ __global__ void __launch_bounds__(H / 4) ln_rows_kernel(const LnRowsParams p) {
       if (risky) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (risky & (1u << j)) patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), 0));
+          if (risky & (1u << j)) patch_q_byte(qw, j, exact_q8((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale, 0));
       }
     } else {
       qw[0] = 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        patch_q_byte(qw, j, zen_det_round_clamp_i8(ZEN_DIV((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale), p.round_mode));
+        patch_q_byte(qw, j, exact_q8((j & 1) ? of[j >> 1].y : of[j >> 1].x, p.out_scale, p.round_mode));
     }
     *reinterpret_cast<uint32_t*>(p.yq + off) = qw[0];
   }

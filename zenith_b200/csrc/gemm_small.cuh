@@ -76,6 +76,12 @@ __device__ __forceinline__ void gs_store(void* out, int64_t off, const uint32_t*
   }
 }
 
+// The requantised value by the definition (out of line: rare, and long when inlined for every column).
+template <int ACT>
+__device__ __noinline__ int gs_exact_requant(int acc, float x_scale, float scale, float bias, float out_scale, int round_mode) {
+  return zen_det_round_clamp_i8(ZEN_DIV(zen_det_act(zen_det_dequant(acc, x_scale, scale, bias), ACT), out_scale), round_mode);
+}
+
 // Epilogue of W columns of one row: the arithmetic of epilogue_chunk / epilogue_step_s8, from registers to global memory.
 template <int KIND, int ACT, int W>
 __device__ __forceinline__ void gs_epilogue(const uint32_t (&a)[W], const float* sc, const float* bi, const float* fo, float risk_thr,
@@ -96,14 +102,14 @@ __device__ __forceinline__ void gs_epilogue(const uint32_t (&a)[W], const float*
 #pragma unroll
           for (int j = 0; j < W; ++j)
             if (redo & (1u << j))
-              patch_q_byte(w, j, zen_det_round_clamp_i8(ZEN_DIV(zen_det_act(zen_det_dequant(int32_t(a[j]), p.x_scale, sc[j], bi[j]), ACT), p.out_scale), 0));
+              patch_q_byte(w, j, gs_exact_requant<ACT>(int32_t(a[j]), p.x_scale, sc[j], bi[j], p.out_scale, 0));
         }
       } else {
 #pragma unroll
         for (int j4 = 0; j4 < W / 4; ++j4) w[j4] = 0;
 #pragma unroll
         for (int j = 0; j < W; ++j)
-          patch_q_byte(w, j, zen_det_round_clamp_i8(ZEN_DIV(zen_det_act(zen_det_dequant(int32_t(a[j]), p.x_scale, sc[j], bi[j]), ACT), p.out_scale), p.round_mode));
+          patch_q_byte(w, j, gs_exact_requant<ACT>(int32_t(a[j]), p.x_scale, sc[j], bi[j], p.out_scale, p.round_mode));
       }
       gs_store<int8_t, W>(p.out, off, w, nvalid, vec_ok);
       return;
