@@ -320,6 +320,14 @@ int zen_qkv_attention_i8(const int8_t* xq, int64_t ldx, const int8_t* wqkv, int6
  *   valid row's result equals, bit for bit, the padded call's result for that token.
  * zen_unpad_rows_f16: padded[b * S + s] = packed[cu_seqlens[b] + s] for valid positions, zeros for padding.
  * No counterpart in the reference (its roadmap lists variable-length batching as future work). */
+/* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
+ * computed in fp16 with fp32 softmax and accumulation.  Two launches: the operands to fp16 in `workspace`
+ * (zen_flash_attention_f32_workspace_bytes, 16-byte aligned), attention with fp32 stores. */
+size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D);
+int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
+                            const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,
+                            void* stream);
+
 /* zen_flash_attention_unpadded_f16: zen_flash_attention_f16 on packed tensors: token t of Q sits at q + t*q_st + h*q_sh + d
  * (likewise K, V, O), sequence b owns tokens cu_seqlens[b] .. cu_seqlens[b + 1] - 1 (cut at `rows`; at most max_seqlen
  * each: a longer one is cut to its first max_seqlen tokens), causal counts positions within the sequence.  Any

@@ -139,3 +139,16 @@ def test_properties_at_encoder_size(cuda):
     # the truncated call has 77 query rows as well (the binding wants equal shapes); compare those rows
     ref = ops.flash_attention(q[:, :, :77].contiguous(), k[:, :, :77].contiguous(), v[:, :, :77].contiguous())
     assert (cut[:, :, :77].float() - ref.float()).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("S,D,causal", [(1, 64, False), (128, 128, True), (129, 64, True), (300, 64, False)])
+def test_fp32_binding_rounds_like_the_fp16_call(cuda, S, D, causal):
+    q, k, v = (torch.from_numpy(rng(S + i).standard_normal((2, 3, S, D)).astype(np.float32)).to(cuda) for i in range(3))
+    lens = torch.tensor([S, max(1, S // 2)], dtype=torch.int32, device=cuda)
+    got = ops.flash_attention(q, k, v, causal=causal, kv_lens=lens)
+    want = ops.flash_attention(q.half(), k.half(), v.half(), causal=causal, kv_lens=lens).float()
+    assert got.dtype == torch.float32
+    if S > 128:
+        assert torch.equal(got, want)  # the same kernel
+    else:
+        assert (got - want).abs().max().item() < 2e-3

@@ -127,3 +127,15 @@ def test_embed_layernorm(cuda):
     e = f(word)[ids] + np.tile(f(pos)[:S], (B, 1)) + f(typ)[tids]
     assert np.max(np.abs(y.float().cpu().numpy() - O.layernorm(e, f(g), f(b), 1e-12))) < 1e-2
     assert np.array_equal(yq.cpu().numpy(), O.quantize(y.float().cpu().numpy(), 0.04))
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4099, 300001])
+@pytest.mark.parametrize("dtype", [np.float32, np.float16])
+def test_quantize_vector_and_tail(cuda, n, dtype):
+    """Sixteen values per step, the ragged end, views that are not 16-byte aligned, values on and off rounding boundaries."""
+    x = (rng(n).standard_normal(n + 1) * 2).astype(dtype)
+    x[: n // 3] = (np.round(x[: n // 3].astype(np.float32) / 0.03125) * 0.03125 + 0.015625).astype(dtype)
+    t = dev(x, cuda)
+    for v in (t[:n].contiguous(), t[1:]):
+        got = ops.quantize(v, 0.03125).cpu().numpy()
+        assert np.array_equal(got, O.quantize(v.float().cpu().numpy(), 0.03125))

@@ -17,6 +17,7 @@
 #include "zen_common.cuh"
 #include "det_math.h"
 #include "tma_host.cuh"
+#include <initializer_list>
 
 namespace zen {
 
@@ -26,6 +27,7 @@ constexpr int FA_THREADS = 192;
 
 struct FaParams {
   void* o;
+  int o_f32;  // long-sequence kernel: the fp16 results are stored as fp32 (the fp32 binding)
   int8_t* oq;
   float o_scale;
   int B, H, S;
@@ -460,6 +462,38 @@ extern "C" int zen_flash_attention_f16(const void* q, const void* k, const void*
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (S <= FA_BKV) return D == 64 ? launch_fa<64>(tq, tk, tv, p, s) : launch_fa<128>(tq, tk, tv, p, s);
   return launch_fa_long(D, tq, tk, tv, p, s);
+}
+
+extern "C" int zen_convert3_f32_to_f16(const float* a, const float* b, const float* c, void* y, int64_t n, void* stream);
+
+extern "C" size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D) {
+  if (B <= 0 || H <= 0 || S <= 0 || D <= 0) return 0;
+  return size_t(3) * size_t(B) * size_t(H) * size_t(S) * size_t(D) * 2;
+}
+
+extern "C" int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
+                                       const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,
+                                       void* stream) {
+  if (!q || !k || !v || !o || !workspace || B <= 0 || H <= 0 || S <= 0) return ZEN_ERR_INVALID_ARG;
+  if (D != 64 && D != 128) return ZEN_ERR_UNSUPPORTED;
+  if (H > 65535 || B > 65535) return ZEN_ERR_UNSUPPORTED;
+  if (workspace_bytes < zen_flash_attention_f32_workspace_bytes(B, H, S, D)) return ZEN_ERR_INVALID_ARG;
+  for (const void* t : {static_cast<const void*>(q), static_cast<const void*>(k), static_cast<const void*>(v), static_cast<const void*>(o),
+                        static_cast<const void*>(workspace)})
+    if (reinterpret_cast<uintptr_t>(t) % 16) return ZEN_ERR_UNSUPPORTED;
+  const int64_t n = int64_t(B) * H * S * D;
+  if (int st = zen_convert3_f32_to_f16(q, k, v, workspace, n, stream); st != ZEN_OK) return st;
+  const __half* w = static_cast<const __half*>(workspace);
+  FaParams p{};
+  p.o = o; p.o_f32 = 1; p.B = B; p.H = H; p.S = S;
+  p.o_sb = int64_t(H) * S * D; p.o_sh = int64_t(S) * D; p.o_ss = D; p.kv_lens = kv_lens; p.causal = causal ? 1 : 0;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  CUtensorMap tq, tk, tv;
+  int st = encode_qkv_map(&tq, w, B, H, S, D, p.o_sb, p.o_sh, D, p.q_perm);
+  if (st == ZEN_OK) st = encode_qkv_map(&tk, w + n, B, H, S, D, p.o_sb, p.o_sh, D, p.k_perm);
+  if (st == ZEN_OK) st = encode_qkv_map(&tv, w + 2 * n, B, H, S, D, p.o_sb, p.o_sh, D, p.v_perm);
+  if (st != ZEN_OK) return st;
+  return launch_fa_long(D, tq, tk, tv, p, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale,

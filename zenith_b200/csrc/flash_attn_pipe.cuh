@@ -439,6 +439,14 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         if (qr >= q_len) continue;
         const uint4 v = *reinterpret_cast<const uint4*>(stage + dc * CHUNK_BYTES + rr * 128 + ((u ^ (rr & 7)) << 4));
         const int64_t off = base + int64_t(qr) * p.o_ss + dc * 64 + u * 8;
+        if (p.o_f32) {
+          const __half2* hp = reinterpret_cast<const __half2*>(&v);
+          const float2 a0 = __half22float2(hp[0]), a1 = __half22float2(hp[1]), a2 = __half22float2(hp[2]), a3 = __half22float2(hp[3]);
+          float4* of = reinterpret_cast<float4*>(static_cast<float*>(p.o) + off);
+          of[0] = make_float4(a0.x, a0.y, a1.x, a1.y);
+          of[1] = make_float4(a2.x, a2.y, a3.x, a3.y);
+          continue;
+        }
         *reinterpret_cast<uint4*>(static_cast<__half*>(p.o) + off) = v;
         if (p.oq) {
           // the int8 copy quantizes the fp16 values that were stored (branch-free rounding, exact division only next to a

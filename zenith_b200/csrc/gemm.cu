@@ -201,6 +201,7 @@ static SmallChoice use_small(int kind, int M, int N, int K, unsigned flags) {
 // out[c, r] = in[r, c] for a row-major [rows, cols] fp32 matrix, 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256) transpose_f32_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                             int rows, int cols) {
+  grid_launch_dependents();  // the GEMM behind this kernel sets itself up meanwhile
   __shared__ float tile[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;

@@ -349,7 +349,7 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!f32 && !plain(q, dev, at::kHalf, 4)) Py_RETURN_NONE;
   const ScalarType st = q->scalar_type();
   if (!plain(k, dev, st, 4) || !plain(v, dev, st, 4) || k->sizes() != q->sizes() || v->sizes() != q->sizes()) Py_RETURN_NONE;
-  const int64_t B = q->size(0), H = q->size(1), S = q->size(2), D = q->size(3), n = q->numel();
+  const int64_t B = q->size(0), H = q->size(1), S = q->size(2), D = q->size(3);
   const int32_t* lens = nullptr;
   if (a[4] != Py_None) {
     const at::Tensor* t = tensor_of(a[4]);
@@ -364,18 +364,15 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int64_t sb = H * S * D, sh = S * D;
   return serve<1>([&](at::Tensor* o) {
     void* s = stream_of(dev);
-    auto run = [&](const void* qp, const void* kp, const void* vp, void* op) {
-      return zen_flash_attention_f16(qp, kp, vp, op, nullptr, 1.0f, int(B), int(H), int(S), int(D), sb, sh, D, sb, sh, D, sb, sh, D, sb, sh, D,
-                                     lens, causal, float(scale), s) == ZEN_OK;
-    };
     o[0] = empty(q->sizes(), st, dev);
-    if (!f32) return run(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), o[0].data_ptr());
-    at::Tensor h = empty({4, n}, at::kHalf, dev);
-    uint8_t* hp = static_cast<uint8_t*>(h.data_ptr());
-    const at::Tensor* in[3] = {q, k, v};
-    for (int i = 0; i < 3; ++i)
-      if (zen_convert_f32_to_f16(static_cast<const float*>(in[i]->const_data_ptr()), hp + 2 * n * i, n, s) != ZEN_OK) return false;
-    return run(hp, hp + 2 * n, hp + 4 * n, hp + 6 * n) && zen_convert_f16_to_f32(hp + 6 * n, static_cast<float*>(o[0].data_ptr()), n, s) == ZEN_OK;
+    if (!f32)
+      return zen_flash_attention_f16(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), o[0].data_ptr(), nullptr, 1.0f, int(B), int(H),
+                                     int(S), int(D), sb, sh, D, sb, sh, D, sb, sh, D, sb, sh, D, lens, causal, float(scale), s) == ZEN_OK;
+    const size_t bytes = zen_flash_attention_f32_workspace_bytes(int(B), int(H), int(S), int(D));
+    at::Tensor ws = empty({int64_t(bytes)}, at::kByte, dev);
+    return zen_flash_attention_f32(static_cast<const float*>(q->const_data_ptr()), static_cast<const float*>(k->const_data_ptr()),
+                                   static_cast<const float*>(v->const_data_ptr()), static_cast<float*>(o[0].data_ptr()), int(B), int(H), int(S),
+                                   int(D), lens, causal, float(scale), ws.data_ptr(), bytes, s) == ZEN_OK;
   });
 }
 

@@ -419,6 +419,7 @@ template <> struct EwWord<16> { using type = uint4; };
 // alignment of the element type.
 template <int OP, typename TI, typename TO, int VEC>
 __global__ void __launch_bounds__(256) ew_kernel(const EwParams p) {
+  grid_launch_dependents();  // a GEMM behind this kernel sets itself up meanwhile (it waits for the data at its own pace)
   const TI* x = static_cast<const TI*>(p.x);
   TO* y = static_cast<TO*>(p.y);
   const int64_t nvec = p.n / VEC;
@@ -445,6 +446,38 @@ __global__ void __launch_bounds__(256) ew_kernel(const EwParams p) {
   }
 }
 
+// int8 quantisation, nearest-even, zero point 0 (the path of every Linear): 16 values per thread and step, the rounding of
+// quantize_pairs_rn (exact, a division only next to a boundary) and one 16-byte store.  With a true division for every
+// value the kernel was bound by instruction issue: 3.2 TB/s on 8 M fp32 values.
+template <typename TI>
+__global__ void __launch_bounds__(256) quantize_kernel(const EwParams p) {
+  grid_launch_dependents();
+  constexpr int V = 16 * int(sizeof(TI)) / 16;  // 16-byte loads per step
+  const int64_t steps = p.n / 16, stride = int64_t(gridDim.x) * blockDim.x;
+  const float inv = ZEN_DIV(1.0f, p.scale);
+  const uint4* x = static_cast<const uint4*>(p.x);
+  uint4* y = static_cast<uint4*>(p.y);
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < steps; i += stride) {
+    uint4 raw[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) raw[k] = x[i * V + k];
+    constexpr int P = 8 / V;  // pairs per load
+    float2 v[8];
+#pragma unroll
+    for (int k = 0; k < V; ++k) Vec16<TI>::unpack2(raw[k], reinterpret_cast<float2(&)[P]>(v[k * P]));
+    uint32_t w[4];
+    const uint32_t risky = quantize_pairs_rn<16>(v, inv, w);
+    if (risky) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (risky & (1u << j)) patch_q_byte(w, j, exact_q8((j & 1) ? v[j >> 1].y : v[j >> 1].x, p.scale, 0));
+    }
+    y[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  for (int64_t i = steps * 16 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < p.n; i += stride)
+    static_cast<int8_t*>(p.y)[i] = int8_t(exact_q8(float(static_cast<const TI*>(p.x)[i]), p.scale, 0));
+}
+
 template <int OP, typename TI, typename TO>
 static int launch_ew(const EwParams& p, cudaStream_t s) {
   if (p.n <= 0) return ZEN_OK;
@@ -460,6 +493,32 @@ static int launch_ew(const EwParams& p, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
 }
 
+template <typename TI>
+static int launch_quantize(const EwParams& p, cudaStream_t s) {
+  if (p.zero_point != 0 || p.round_mode != 0 || reinterpret_cast<uintptr_t>(p.x) % 16 || reinterpret_cast<uintptr_t>(p.y) % 16)
+    return launch_ew<EW_QUANT, TI, int8_t>(p, s);
+  if (p.n <= 0) return ZEN_OK;
+  int64_t blocks = (p.n / 16 + 255) / 256;
+  const int64_t cap = int64_t(num_sms()) * 8;
+  blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
+  quantize_kernel<TI><<<int(blocks), 256, 0, s>>>(p);
+  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+}
+
+// Three fp32 tensors of n values to fp16, back to back in y (the operands of the fp32 attention binding): one launch.
+__global__ void __launch_bounds__(256) convert3_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
+                                                       __half* __restrict__ y, int64_t n) {
+  grid_launch_dependents();
+  const float* x = blockIdx.y == 0 ? a : blockIdx.y == 1 ? b : c;
+  __half* o = y + int64_t(blockIdx.y) * n;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) {
+    float v[8];
+    Vec16<float>::load(x + 8 * i, reinterpret_cast<float(&)[4]>(v[0]));
+    Vec16<float>::load(x + 8 * i + 4, reinterpret_cast<float(&)[4]>(v[4]));
+    Vec16<__half>::store(o + 8 * i, v);
+  }
+}
 
 // ------------------------------------------------------------------------------------------
 // Unpadded batches: the valid tokens of a padded [B, S] batch packed back to back
@@ -560,13 +619,13 @@ int zen_quantize_f32(const float* x, int8_t* q, int64_t n, float scale, int zero
   if (n < 0 || (n > 0 && (!x || !q)) || !(scale > 0.f) || (round_mode != 0 && round_mode != 1))
     return ZEN_ERR_INVALID_ARG;
   EwParams p{x, q, nullptr, n, 1, scale, zero_point, round_mode};
-  return launch_ew<EW_QUANT, float, int8_t>(p, static_cast<cudaStream_t>(stream));
+  return launch_quantize<float>(p, static_cast<cudaStream_t>(stream));
 }
 int zen_quantize_f16(const void* x, int8_t* q, int64_t n, float scale, int zero_point, int round_mode, void* stream) {
   if (n < 0 || (n > 0 && (!x || !q)) || !(scale > 0.f) || (round_mode != 0 && round_mode != 1))
     return ZEN_ERR_INVALID_ARG;
   EwParams p{x, q, nullptr, n, 1, scale, zero_point, round_mode};
-  return launch_ew<EW_QUANT, __half, int8_t>(p, static_cast<cudaStream_t>(stream));
+  return launch_quantize<__half>(p, static_cast<cudaStream_t>(stream));
 }
 int zen_quantize_e4m3_f32(const float* x, uint8_t* q, int64_t n, float scale, void* stream) {
   if (n < 0 || (n > 0 && (!x || !q)) || !(scale > 0.f)) return ZEN_ERR_INVALID_ARG;
@@ -587,6 +646,14 @@ int zen_convert_f32_to_f16(const float* x, void* y, int64_t n, void* stream) {
   if (n < 0 || (n > 0 && (!x || !y))) return ZEN_ERR_INVALID_ARG;
   EwParams p{x, y, nullptr, n, 1, 1.f, 0, 0};
   return launch_ew<EW_CONVERT, float, __half>(p, static_cast<cudaStream_t>(stream));
+}
+// (internal to the library: used by zen_flash_attention_f32)
+__attribute__((visibility("hidden"))) int zen_convert3_f32_to_f16(const float* a, const float* b, const float* c, void* y, int64_t n, void* stream) {
+  int64_t blocks = (n / 8 + 255) / 256;
+  const int64_t cap = int64_t(num_sms()) * 3;
+  blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
+  convert3_kernel<<<dim3(unsigned(blocks), 3), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
+  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
 }
 int zen_convert_f16_to_f32(const void* x, float* y, int64_t n, void* stream) {
   if (n < 0 || (n > 0 && (!x || !y))) return ZEN_ERR_INVALID_ARG;

@@ -552,14 +552,14 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
     """``softmax(scale * Q K^T) V`` for ``[batch, heads, seq, dim]`` tensors.
 
     fp16 inputs run directly; fp32 inputs (the reference binding's dtype,
-    core/bindings/cuda_bindings.cpp:90-106) are converted to fp16 on the device, run on the
-    tensor cores with fp32 softmax and accumulation, and returned as fp32.
+    core/bindings/cuda_bindings.cpp:90-106) are converted to fp16 on the device (one launch), run on the
+    tensor cores with fp32 softmax and accumulation, and returned as fp32 (written by the kernel).
     ``kv_lens[b]`` masks keys at positions >= kv_lens[b]; a row with no valid key yields zeros.
     """
     global launch_count
     out = native.flash_attention(q, k, v, causal, kv_lens, scale)
     if out is not None:
-        launch_count += 1 if out.dtype == torch.float16 else 5
+        launch_count += 1 if out.dtype == torch.float16 else 2
         return out
     if not q.is_cuda:
         raise RuntimeError("Q must be CUDA tensor")
@@ -569,9 +569,18 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
         raise RuntimeError("K and V must have the shape of Q")
     B, H, S, D = q.shape
     if q.dtype == torch.float32:
-        qh, kh, vh = (to_fp16(t.contiguous()) for t in (q, k, v))
-        oh = flash_attention(qh, kh, vh, causal=causal, kv_lens=kv_lens, scale=scale)
-        return to_fp32(oh)
+        q, k, v = (t.contiguous() for t in (q, k, v))
+        for name, t in (("Q", q), ("K", k), ("V", v)):
+            _require(t, name, torch.float32, 4)
+        if kv_lens is not None:
+            _require(kv_lens, "kv_lens", torch.int32, 1)
+        out = torch.empty_like(q)
+        nbytes = _capi.lib().zen_flash_attention_f32_workspace_bytes(B, H, S, D)
+        workspace = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        _call("zen_flash_attention_f32", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, S, D, _ptr(kv_lens),
+              1 if causal else 0, float(1.0 / math.sqrt(D) if scale is None else scale), workspace.data_ptr(), nbytes, _stream())
+        launch_count_add(1)
+        return out
     for name, t in (("Q", q), ("K", k), ("V", v)):
         _require(t, name, torch.float16, 4)
     out = torch.empty_like(q)
