@@ -152,3 +152,13 @@ def test_fp32_binding_rounds_like_the_fp16_call(cuda, S, D, causal):
         assert torch.equal(got, want)  # the same kernel
     else:
         assert (got - want).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("B,H,S,D,causal", [(110, 9, 33, 64, False), (50, 9, 128, 64, True), (37, 9, 100, 128, False)])
+def test_single_block_kernel_many_items(cuda, B, H, S, D, causal):
+    """More (head, batch) items than the SMs take at a time: tiles, columns and barriers are used again, empty sequences
+    between full ones."""
+    o, want = run(cuda, B, H, S, D, causal, [(7 * b) % (S + 1) for b in range(B)], seed=3)
+    got = o.float().cpu().numpy()
+    assert not np.isnan(got).any()
+    assert np.max(np.abs(got - want)) < 1e-2 * max(1.0, np.abs(want).max())

@@ -81,9 +81,8 @@ __device__ __forceinline__ bool elect_one() {
 // Kernel families launched with the programmatic-stream-serialization attribute: a build-time constant.
 enum { PDL_GEMM = 1, PDL_ATTENTION = 2, PDL_ROW = 4 };
 #ifndef ZEN_PDL_FAMILIES
-#define ZEN_PDL_FAMILIES 1
+#define ZEN_PDL_FAMILIES 3
 #endif
-constexpr bool kAttentionLaunchesEarly = (ZEN_PDL_FAMILIES & PDL_ATTENTION) != 0;
 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
