@@ -265,3 +265,15 @@ def test_repeated_plain_calls_equal_the_first(cuda, params, micro_batches):
     out.zero_()
     g.replay()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("B,S,launches", [(1, 48, 5), (1, 49, 4), (112, 6, 5), (112, 16, 4), (150, 8, 5)])
+def test_int8_encoder_attention_form_by_size(cuda, params, B, S, launches):
+    """Few rows, or many rounds of mostly empty tiles: projection and attention as two launches, with the same bits."""
+    scales = Int8Scales(act=[dict(x=0.03, ctx=0.01, h1=0.03, gelu=0.02)] * CFG.layers, weights=quantize_weights(params))
+    ids, lens = tdev(rng(B).integers(0, CFG.vocab, (B, S)), rng(S).integers(1, S + 1, B).astype(np.int32), cuda)
+    mk = lambda f: Int8Encoder(CFG, params, scales, cuda, fuse_layernorm=False, fuse_attention=f)
+    enc = mk(None)
+    out = enc.forward(ids, lens)
+    assert enc.launches_per_layer == launches + 2  # LayerNorms not fused
+    assert torch.equal(out, mk(True).forward(ids, lens)) and torch.equal(out, mk(False).forward(ids, lens))

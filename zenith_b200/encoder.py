@@ -521,7 +521,8 @@ class Int8Encoder(_EncoderBase):
         BERT-large's 12k-token shards the separate kernels measured faster: 8.98 vs 10.26 ms per pass).  In the
         fused form the projection output is not rounded to fp16 before the residual add.
         ``fuse_attention``: QKV projection and attention as ONE kernel (``zen_qkv_attention_i8``), possible for
-        sequences of at most 128 tokens with head size 64 and on by default there; same results bit for bit.
+        sequences of at most 128 tokens with head size 64 and by default used where it is the faster form
+        (``_attention_fuses``); same results bit for bit.
         ``keep_qkv``: the fused kernel also writes the fp16 projection to ``self.qkv`` (tests, inspection)."""
         super().__init__(cfg, params, device, micro_batches, gemm_pair)
         self.fuse_attention = fuse_attention
@@ -587,7 +588,7 @@ class Int8Encoder(_EncoderBase):
         can_fuse = S <= 128 and hd == 64
         if self.fuse_attention and not can_fuse:
             raise RuntimeError("the fused QKV + attention kernel needs seq <= 128 and head_dim == 64")
-        fused_attn = can_fuse if self.fuse_attention is None else bool(self.fuse_attention)
+        fused_attn = (can_fuse and self._attention_fuses(packed)) if self.fuse_attention is None else bool(self.fuse_attention)
         self.launches_per_layer = (5 if fused_ln else 7) - (1 if fused_attn else 0)
         self.lead_launches = 2 if packed else 1
         if packed:
@@ -665,6 +666,22 @@ class Int8Encoder(_EncoderBase):
         if packed:
             self._add("zen_unpad_rows_f16", self.x[cur].data_ptr(), self.cu_seqlens.data_ptr(), B, S, H, T,
                       self.out_padded.data_ptr())
+
+    def _attention_fuses(self, packed: bool) -> bool:
+        """Whether the fused projection + attention kernel is the faster form (the results are the same bits).
+
+        It gives every (sequence, head) a tile of 128 rows whatever the sequence's length, one per SM at a time: with r
+        rounds of those, two launches on the real rows are faster up to about 80 r^2 rows, and for a handful of rows, where
+        the projection is one narrow product.  Measured on the 12- and 24-layer encoders, the two launches against the
+        fused kernel: 1 x 24 -2.5 %, 100 x 8 -23 %, 64 x 16 -12 %, 128 x 24 -14 %, 64 x 48 -2.5 %, 128 x 64 -0.6 %, but
+        2 x 40 +0.3 %, 48 x 32 +0.8 %, 24 x 40 +3.6 %, 128 x 80 +1.4 %, 8 x 128 +11 %.  Packed rows keep the fused kernel,
+        whose tiles they share."""
+        if packed:
+            return True
+        B, S = self._shape[:2]
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        rounds = -(-B * self.cfg.heads // sms)
+        return B * S > 48 and (rounds < 3 or B * S > 80 * rounds * rounds)
 
     def forward_layerwise(self, ids, kv_lens=None):
         """Generator for tests: runs the pass one layer at a time and yields ``(layer, buffers)`` after
