@@ -336,6 +336,8 @@ int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v
                                      int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh, int64_t k_st,
                                      int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st, int64_t o_sh,
                                      const int32_t* cu_seqlens, int causal, float scale, void* stream);
+/* inputs[0 .. B*S) = ids, inputs[B*S .. B*S + B) = kv_lens (NULL: S each): the two copies of a batch as one launch. */
+int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S, int32_t* inputs, void* stream);
 int zen_pack_tokens_i32(const int32_t* ids, const int32_t* type_ids, const int32_t* kv_lens, int B, int S, int capacity,
                         int32_t* cu_seqlens, int32_t* ids_packed, int32_t* pos_packed, int32_t* type_packed, void* stream);
 int zen_embed_layernorm_unpadded_f16(const int32_t* ids_packed, const int32_t* pos_packed, const int32_t* type_packed,

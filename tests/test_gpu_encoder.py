@@ -277,3 +277,16 @@ def test_int8_encoder_attention_form_by_size(cuda, params, B, S, launches):
     out = enc.forward(ids, lens)
     assert enc.launches_per_layer == launches + 2  # LayerNorms not fused
     assert torch.equal(out, mk(True).forward(ids, lens)) and torch.equal(out, mk(False).forward(ids, lens))
+
+
+@pytest.mark.parametrize("B,S", [(1, 1), (3, 85), (5, 120)])
+def test_inputs_reach_the_static_buffers(cuda, params, B, S):
+    """int32 ids and lengths on the device (one launch), other types and the host (copies), no lengths."""
+    enc = Fp16Encoder(CFG, params, cuda)
+    ids, lens = tdev(rng(S).integers(0, CFG.vocab, (B, S)).astype(np.int32), rng(B).integers(0, S + 1, B).astype(np.int32), cuda)
+    full = torch.full_like(lens, S)
+    for a, l, want in ((ids, lens, lens), (ids.long(), lens.long(), lens), (ids.cpu(), lens, lens), (ids.T.contiguous().T, lens, lens),
+                       (ids, None, full)):
+        enc.set_inputs(a, l)
+        assert torch.equal(enc.ids.view(B, S), ids) and torch.equal(enc.kv_lens, want)
+        enc.inputs.zero_()

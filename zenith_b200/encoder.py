@@ -81,6 +81,10 @@ def init_params(cfg: EncoderConfig, seed: int = 1234, random_affine: bool = Fals
     return p
 
 
+def _plain_i32(t, like) -> bool:
+    return t.dtype == torch.int32 and t.device == like.device and t.is_contiguous()
+
+
 def _row_ptr(t: torch.Tensor, row0: int) -> int:
     """Device address of row ``row0`` of a contiguous 1-D / 2-D tensor."""
     return t.data_ptr() + row0 * (t.stride(0) if t.dim() > 1 else 1) * t.element_size()
@@ -225,6 +229,12 @@ class _EncoderBase:
         B, S = ids.shape
         same = self._shape is not None and self._shape[:2] == (B, S)
         self._prepare(B, S, self._packed_rows if same else None)
+        # what a caller usually has on the device goes in with one launch
+        if _plain_i32(ids, self.inputs) and (kv_lens is None or (_plain_i32(kv_lens, self.inputs) and kv_lens.shape == (B,))):
+            _capi.check("zen_set_inputs_i32", _capi.lib().zen_set_inputs_i32(
+                ids.data_ptr(), None if kv_lens is None else kv_lens.data_ptr(), B, S, self.inputs.data_ptr(),
+                torch.cuda.current_stream().cuda_stream))
+            return
         self.ids.copy_(ids.reshape(-1), non_blocking=True)
         if kv_lens is not None:
             self.kv_lens.copy_(kv_lens, non_blocking=True)
