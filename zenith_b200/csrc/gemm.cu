@@ -159,15 +159,21 @@ static int run_gemm(const void* A, int64_t lda, const void* B, int64_t ldb, Gemm
 // moves a third fewer operand bytes per operation but starts and ends more slowly (cluster scheduling, two
 // cluster-wide rendezvous), and it does nothing for the epilogue: it pays when the main loop dominates, i.e. for
 // large products, and for the GELU + requantisation epilogue only with a deep K (measured on 11 shapes: wins of
-// 8 - 17 % above the thresholds, losses of 3 - 9 % below them).
-static bool use_pair(int M, int N, int K, bool heavy_epilogue, unsigned flags) {
+// 8 - 17 % above the thresholds, losses of 3 - 9 % below them).  fp16 operands are twice the bytes and twice the
+// tensor work per element while the epilogue stays the same, and its threshold is lower: of 18 shapes of 2048 - 16384 rows
+// those from 2^33 multiply-adds on gained 2 - 14 % (4096 x 3072 x 768: 21.6 -> 20.2 us, 12288 x 1024 x 1024: 24.4 -> 22.5,
+// 3000 x 4096 x 1024: 28.3 -> 24.5), those below lost 1 - 8 %.
+static bool use_pair(int kind, int M, int N, int K, bool heavy_epilogue, unsigned flags) {
   if (flags & ZEN_GEMM_NO_PAIR) return false;
   if (flags & ZEN_GEMM_PAIR) return true;
   const double work = double(M) * double(N) * double(K);
-  return M >= 1024 && work >= 34359738368.0 /* 2^35 */ && (!heavy_epilogue || K >= 4096);
+  const double from = kind == KIND_F16 ? 8589934592.0 /* 2^33 */ : 34359738368.0 /* 2^35 */;
+  return M >= 1024 && work >= from && (!heavy_epilogue || K >= 4096);
 }
 
-// Pair tile width: fewest rounds of the resident pairs, wider tiles preferred on a tie (less traffic per operation).
+// Pair tile width: fewest rounds of the resident pairs, wider tiles preferred on a tie (less traffic per operation).  A tile
+// of 128 columns reads as much of A as one of 256 and is dearer than its columns (fp16 3700 x 3072 x 768: five rounds of 128
+// 21.2 us, three of 256 19.8).
 static int pick_bn_pair(int M, int N, unsigned flags) {
   static const int allowed[] = {256, 192, 128};
   const int forced = int((flags >> 8) & 0x3ffu);
@@ -180,7 +186,7 @@ static int pick_bn_pair(int M, int N, unsigned flags) {
   for (int bn : allowed) {
     const long tiles = long(tiles_m) * ((N + bn - 1) / bn);
     const long rounds = (tiles + pairs - 1) / pairs;
-    const long cost = rounds * (bn + 24);
+    const long cost = rounds * (bn + (bn == 128 ? 40 : 24));
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = bn;
@@ -228,7 +234,7 @@ int run_gemm_auto(int kind, const void* A, int64_t lda, const void* B, int64_t l
   static const int allowed[] = {64, 128, 192, 256};
   if (const SmallChoice c = use_small(kind, p.M, p.N, p.K, flags); c.ks > 0) return launch_gemm_small(kind, c.bn, c.ks, false, A, lda, B, ldb, p, s);
   if (kind == KIND_I8) {
-    if (use_pair(p.M, p.N, p.K, p.out_dtype == ZEN_DT_S8 && p.act == ZEN_ACT_GELU, flags)) {
+    if (use_pair(kind, p.M, p.N, p.K, p.out_dtype == ZEN_DT_S8 && p.act == ZEN_ACT_GELU, flags)) {
       switch (pick_bn_pair(p.M, p.N, flags)) {
         case 128: return run_gemm<KIND_I8, 128, 6, false, true>(A, lda, B, ldb, p, s);
         case 192: return run_gemm<KIND_I8, 192, 5, false, true>(A, lda, B, ldb, p, s);
@@ -242,7 +248,7 @@ int run_gemm_auto(int kind, const void* A, int64_t lda, const void* B, int64_t l
       default: return run_gemm<KIND_I8, 256, 3, false>(A, lda, B, ldb, p, s);
     }
   }
-  if (use_pair(p.M, p.N, 2 * p.K /* fp16 operands: twice the bytes per element */, false, flags)) {
+  if (use_pair(kind, p.M, p.N, p.K, false, flags)) {
     switch (pick_bn_pair(p.M, p.N, flags)) {
       case 128: return run_gemm<KIND_F16, 128, 6, false, true>(A, lda, B, ldb, p, s);
       case 192: return run_gemm<KIND_F16, 192, 5, false, true>(A, lda, B, ldb, p, s);
