@@ -162,12 +162,16 @@ static int run_gemm(const void* A, int64_t lda, const void* B, int64_t ldb, Gemm
 // 8 - 17 % above the thresholds, losses of 3 - 9 % below them).  fp16 operands are twice the bytes and twice the
 // tensor work per element while the epilogue stays the same, and its threshold is lower: of 18 shapes of 2048 - 16384 rows
 // those from 2^33 multiply-adds on gained 2 - 14 % (4096 x 3072 x 768: 21.6 -> 20.2 us, 12288 x 1024 x 1024: 24.4 -> 22.5,
-// 3000 x 4096 x 1024: 28.3 -> 24.5), those below lost 1 - 8 %.
+// 3000 x 4096 x 1024: 28.3 -> 24.5), those below lost 1 - 8 %.  Deep int8 products
+// with a light epilogue gain from 2^34.5 on (12288 x 768 x 3072: 27.8 -> 25.2 us, 6000 x 1024 x 4096: 22.1 -> 20.4), shallower
+// ones gain alone but not between other kernels (8192 x 3072 x 1024: 24.4 -> 23.7, its encoder 4286 -> 4304 us).
 static bool use_pair(int kind, int M, int N, int K, bool heavy_epilogue, unsigned flags) {
   if (flags & ZEN_GEMM_NO_PAIR) return false;
   if (flags & ZEN_GEMM_PAIR) return true;
   const double work = double(M) * double(N) * double(K);
-  const double from = kind == KIND_F16 ? 8589934592.0 /* 2^33 */ : 34359738368.0 /* 2^35 */;
+  const double from = kind == KIND_F16                 ? 8589934592.0    // 2^33
+                      : !heavy_epilogue && K >= 2048 ? 24296004000.0   // 2^34.5
+                                                     : 34359738368.0;  // 2^35
   return M >= 1024 && work >= from && (!heavy_epilogue || K >= 4096);
 }
 
