@@ -5,7 +5,7 @@
 //
 //   acc[128, 192] = xq[b] . {Wq_h, Wk_h, Wv_h}^T                  int8 tcgen05, s32 in TMEM       (GEMM issuer)
 //   Q, K, V       = half((float(acc) * s_x) * s_w[n] + bias[n])    written to shared memory as MMA operands
-//   S = Q K^T  ->  P = exp2(scale * S - max)  ->  O = P V          as in flash_attn_kernel (same arithmetic)
+//   S = Q K^T  ->  P = exp2(scale * S - max)  ->  O = P V          as in flash_attn_short_kernel (same arithmetic)
 //   ctx[b, :, h]  = half(O / rowsum)  (+ int8 copy)                TMA stores
 //
 // so the fp16 QKV tensor never travels to L2 / HBM and back, one kernel boundary and the attention kernel's load
@@ -363,7 +363,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       fence_proxy_async_smem();
       mbar_arrive(&qkv_ready[set]);
 
-      // ---- softmax (the arithmetic of flash_attn_kernel): this thread's 64 of the row's 128 keys
+      // ---- softmax (the arithmetic of flash_attn_short_kernel): this thread's 64 of the row's 128 keys
       if (!mbar_wait(&s_full[set], it & 1u, abort_flag)) break;
       tc_fence_after_sync();
       const int lim = kv_len;
