@@ -322,7 +322,8 @@ int zen_qkv_attention_i8(const int8_t* xq, int64_t ldx, const int8_t* wqkv, int6
  * No counterpart in the reference (its roadmap lists variable-length batching as future work). */
 /* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
  * computed in fp16 with fp32 softmax and accumulation.  Two launches: the operands to fp16 in `workspace`
- * (zen_flash_attention_f32_workspace_bytes, 16-byte aligned), attention with fp32 stores. */
+ * (zen_flash_attention_f32_workspace_bytes), attention with fp32 stores.  o and workspace 16-byte aligned; q, k and v may
+ * lie on any 4-byte boundary. */
 size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D);
 int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
                             const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,

@@ -154,6 +154,22 @@ def test_fp32_binding_rounds_like_the_fp16_call(cuda, S, D, causal):
         assert (got - want).abs().max().item() < 2e-3
 
 
+@pytest.mark.parametrize("which", [(0,), (1,), (2,), (0, 1, 2)])
+@pytest.mark.parametrize("S,D,offset", [(1, 64, 1), (33, 64, 2), (128, 128, 3), (197, 64, 1), (300, 128, 5)])
+def test_fp32_binding_takes_views_off_a_16_byte_boundary(cuda, S, D, offset, which):
+    """Contiguous operands that start at an odd element of a larger tensor: the bits of the aligned call."""
+    q, k, v = (torch.from_numpy(rng(S + i).standard_normal((2, 3, S, D)).astype(np.float32)).to(cuda) for i in range(3))
+
+    def shifted(t):
+        big = torch.full((t.numel() + offset,), float("nan"), device=cuda)
+        big[offset:] = t.flatten()
+        return big[offset:].view(t.shape)
+
+    args = [shifted(t) if i in which else t for i, t in enumerate((q, k, v))]
+    assert any(t.data_ptr() % 16 for t in args) and all(t.is_contiguous() for t in args)
+    assert torch.equal(ops.flash_attention(*args), ops.flash_attention(q, k, v))
+
+
 @pytest.mark.parametrize("B,H,S,D,causal", [(110, 9, 33, 64, False), (50, 9, 128, 64, True), (37, 9, 100, 128, False)])
 def test_single_block_kernel_many_items(cuda, B, H, S, D, causal):
     """More (head, batch) items than the SMs take at a time: tiles, columns and barriers are used again, empty sequences

@@ -506,13 +506,21 @@ static int launch_quantize(const EwParams& p, cudaStream_t s) {
 }
 
 // Three fp32 tensors of n values to fp16, back to back in y (the operands of the fp32 attention binding): one launch.
+// VEC: 32 bytes in, 16 out per thread and step; else element by element, for tensors off a 16-byte boundary (a view of an
+// odd offset).
+template <bool VEC>
 __global__ void __launch_bounds__(256) convert3_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
                                                        __half* __restrict__ y, int64_t n) {
   grid_launch_dependents();
   const float* x = blockIdx.y == 0 ? a : blockIdx.y == 1 ? b : c;
   __half* o = y + int64_t(blockIdx.y) * n;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) {
+  const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if constexpr (!VEC) {
+    for (int64_t i = first; i < n; i += stride) o[i] = __float2half_rn(x[i]);
+    return;
+  }
+  for (int64_t i = first; i < n / 8; i += stride) {
     float v[8];
     Vec16<float>::load(x + 8 * i, reinterpret_cast<float(&)[4]>(v[0]));
     Vec16<float>::load(x + 8 * i + 4, reinterpret_cast<float(&)[4]>(v[4]));
@@ -658,10 +666,13 @@ int zen_convert_f32_to_f16(const float* x, void* y, int64_t n, void* stream) {
 }
 // (internal to the library: used by zen_flash_attention_f32)
 __attribute__((visibility("hidden"))) int zen_convert3_f32_to_f16(const float* a, const float* b, const float* c, void* y, int64_t n, void* stream) {
-  int64_t blocks = (n / 8 + 255) / 256;
+  const bool vec = (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 16 == 0;
+  int64_t blocks = ((vec ? n / 8 : n) + 255) / 256;
   const int64_t cap = int64_t(num_sms()) * 3;
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
-  convert3_kernel<<<dim3(unsigned(blocks), 3), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
+  const dim3 grid(unsigned(blocks), 3);
+  if (vec) convert3_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
+  else convert3_kernel<false><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
   return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
 }
 int zen_convert_f16_to_f32(const void* x, float* y, int64_t n, void* stream) {
