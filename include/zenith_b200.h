@@ -170,7 +170,8 @@ int zen_linear_f16_add_layernorm_ex(const void* x, int64_t ldx, const void* w, i
 
 /* The same with a caller-provided workspace of M * N floats (16-byte aligned, scratch; NULL = the forms above): where the
  * four-CTA clusters of the one-kernel form would leave the chip idle (few rows) or run in more than one round, the call
- * becomes two launches, the projection with bias in fp32 into the workspace, then residual add and LayerNorm of its rows.
+ * becomes two launches, the projection with bias in fp32 into the workspace, then residual add and LayerNorm of its rows
+ * (gamma and beta on 8-byte boundaries; elsewhere the call stays one kernel).
  * Same results bit for bit (with fp16 operands: for the same K split). */
 int zen_linear_i8_add_layernorm_ws(const int8_t* xq, int64_t ldx, const int8_t* wq, int64_t ldw, int M, int N, int K,
                                    float x_scale, const float* w_scale, const float* bias, const void* residual,

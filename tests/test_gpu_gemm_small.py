@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from zenith_b200 import _capi
+from zenith_b200 import _capi, ops
 from zenith_b200._capi import ACT_GELU, ACT_NONE, DT_F16, DT_F32, DT_S8, DT_S32, GEMM_NARROW, gemm_split_k
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +77,23 @@ def test_layernorm_forms(cuda, M, N, K, flags):
     assert np.max(np.abs(got - want)) < 4e-3
     assert np.array_equal(yq.cpu().numpy(), O.quantize(got, 0.03))
     assert _capi.device_status() == 0
+
+
+@pytest.mark.parametrize("offset", [(1, 0), (0, 2), (3, 3)])
+@pytest.mark.parametrize("elem,M,N,K", [(1, 1, 768, 768), (1, 300, 1024, 1024), (1, 1025, 768, 128), (2, 1025, 768, 128)])
+def test_layernorm_parameters_may_start_anywhere(cuda, elem, M, N, K, offset):
+    """gamma and beta as views at an odd element of a larger vector, in sizes that run as two launches when they are aligned:
+    the same bits."""
+    x, w = (torch.from_numpy(rng(s).integers(-100, 100, (n, K), dtype=np.int8)).to(cuda) for s, n in ((M, M), (K, N)))
+    res = torch.from_numpy(rng(3).standard_normal((M, N)).astype(np.float16)).to(cuda)
+    vectors = [torch.from_numpy(rng(s).standard_normal(N + 8).astype(np.float16)).to(cuda) for s in (4, 5)]
+    moved = [torch.cat((v.new_zeros(o), v[:N]))[o:] for v, o in zip(vectors, offset)]
+    assert any(v.data_ptr() % 8 for v in moved)
+
+    def run(g, b):
+        if elem == 2:
+            return (ops.linear_fp16_add_layernorm(x.half() * 0.02, w.half() * 0.001, None, res, g, b, 1e-12),)
+        return ops.linear_int8_add_layernorm(x, w, 0.02, None, None, res, g, b, 1e-12, out_scale=0.03)
+
+    for got, want in zip(run(*moved), run(*(v[:N] for v in vectors))):
+        assert torch.equal(got, want)

@@ -645,6 +645,8 @@ static int run_linear_add_layernorm(const void* x, int64_t ldx, const void* w, i
       narrow = c.bn == 32 ? ZEN_GEMM_NARROW : 0u;
     }
     if (form != 1 && form != 2 && form != 4 && form != 8 && form != 14 && form != 15) return ZEN_ERR_INVALID_ARG;
+    // the row kernel reads gamma and beta in 8-byte units, the one-kernel form value by value: it takes views that start anywhere
+    if ((reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) % 8) form = 15;
   }
   if (form != 15) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
