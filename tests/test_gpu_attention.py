@@ -154,6 +154,23 @@ def test_fp32_binding_rounds_like_the_fp16_call(cuda, S, D, causal):
         assert (got - want).abs().max().item() < 2e-3
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.125, -1.5, 0.5])
+@pytest.mark.parametrize("S,D,causal", [(40, 64, False), (128, 128, True), (100, 64, True), (200, 64, False), (300, 128, True), (2100, 64, False)])
+def test_any_scale_with_masked_keys(cuda, S, D, causal, scale):
+    """A scale of zero (the mean of the valid keys' values) and negative ones: masked keys stay without weight."""
+    q, k, v = (torch.from_numpy(rng(S + i).standard_normal((2, 2, S, D)).astype(np.float16)).to(cuda) for i in range(3))
+    lens = torch.tensor([S, max(1, S - 39)], dtype=torch.int32, device=cuda)
+    got = ops.flash_attention(q, k, v, causal=causal, kv_lens=lens, scale=scale).double()
+    s = scale * (q.double() @ k.double().transpose(2, 3))
+    pos = torch.arange(S, device=cuda)
+    keep = (pos[None, :] < lens[:, None])[:, None, None, :]
+    if causal:
+        keep = keep & (pos[None, :] <= pos[:, None])
+    want = torch.softmax(s.masked_fill(~keep, float("-inf")), -1) @ v.double()
+    assert not torch.isnan(got).any()
+    assert (got - want).abs().max().item() < 1e-2 * max(1.0, want.abs().max().item())
+
+
 @pytest.mark.parametrize("which", [(0,), (1,), (2,), (0, 1, 2)])
 @pytest.mark.parametrize("S,D,offset", [(1, 64, 1), (33, 64, 2), (128, 128, 3), (197, 64, 1), (300, 128, 5)])
 def test_fp32_binding_takes_views_off_a_16_byte_boundary(cuda, S, D, offset, which):

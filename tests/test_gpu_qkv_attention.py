@@ -88,3 +88,17 @@ def test_longer_sequences_are_refused(cuda):
     with pytest.raises(_capi.ZenithError) as e:
         ops.qkv_attention_int8(x, w, 1.0, None, None, 1, 256, 1)
     assert e.value.status == _capi.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_fused_takes_any_scale(cuda, scale):
+    B, S, heads, K = 3, 70, 2, 128
+    H = heads * 64
+    x, w = dev(rng(1).integers(-128, 128, (B * S, K), dtype=np.int8), cuda), dev(rng(2).integers(-128, 128, (3 * H, K), dtype=np.int8), cuda)
+    ws = dev(np.full(3 * H, 0.009 / np.sqrt(K), np.float32), cuda)
+    lens = dev(np.array([70, 33, 1], np.int32), cuda)
+    ctx, qkv = ops.qkv_attention_int8(x, w, 0.02, ws, None, B, S, heads, kv_lens=lens, scale=scale, emit_qkv=True)
+    split = lambda i: qkv[:, i * H:(i + 1) * H].reshape(B, S, heads, 64).transpose(1, 2).contiguous()
+    want = ops.flash_attention(split(0), split(1), split(2), kv_lens=lens, scale=scale)
+    assert not torch.isnan(ctx).any()
+    assert torch.equal(ctx, want.transpose(1, 2).reshape(B * S, H))

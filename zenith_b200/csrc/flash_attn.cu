@@ -26,7 +26,8 @@ struct FaParams {
   const int32_t* cu_seqlens;  // unpadded batches (long-sequence kernel only): [B + 1] row offsets, null otherwise
   int rows;                   // ... rows of the packed tensors
   int causal;
-  float scale_log2;  // softmax scale * log2(e)
+  float scale_log2;    // |softmax scale| * log2(e)
+  uint32_t qk_negate;  // added to the descriptor of Q K^T: the sign of the scale
   // position of the (seq, head, batch) coordinates in each rank-4 tensor map (dim 0 is d)
   int q_perm[3], k_perm[3], v_perm[3];
   int box_rows;  // rows of a loaded tile: 128, for shorter sequences what holds all of them
@@ -45,6 +46,18 @@ __device__ __forceinline__ void fa_tma_tile(uint8_t* dst, const CUtensorMap* map
   const int c2 = perm[0] == 2 ? s : (perm[1] == 2 ? h : b);
   const int c3 = perm[0] == 3 ? s : (perm[1] == 3 ? h : b);
   tma_load_4d(dst, map, bar, d0, c1, c2, c3);
+}
+
+// The softmax scale as the kernels take it.  A masked score is -inf, which is no maximum and no probability as long as the
+// factor is positive: so the sign of the scale goes into Q K^T (the maximum is then the maximum of the scaled scores too), and
+// zero becomes a factor that leaves the exponent of every finite score at zero.
+struct SoftmaxScale {
+  float log2;
+  uint32_t negate;
+};
+inline SoftmaxScale softmax_scale(float scale) {
+  const float f = fabsf(scale) * 1.4426950408889634f;
+  return {f < 1e-30f ? 1e-30f : f, scale < 0.0f ? uint32_t(IDESC_NEGATE_A) : 0u};
 }
 
 }  // namespace zen
@@ -149,7 +162,8 @@ extern "C" int zen_flash_attention_f16(const void* q, const void* k, const void*
   FaParams p{};
   p.o = o; p.oq = oq; p.o_scale = o_scale; p.inv_o_scale = oq ? 1.0f / o_scale : 1.0f; p.B = B; p.H = H; p.S = S;
   p.o_sb = o_sb; p.o_sh = o_sh; p.o_ss = o_ss; p.kv_lens = kv_lens; p.causal = causal ? 1 : 0;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  const SoftmaxScale sc = softmax_scale(scale);
+  p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   p.box_rows = fa_box_rows(S);
   CUtensorMap tq, tk, tv;
   int st = encode_qkv_map(&tq, q, B, H, S, D, q_sb, q_sh, q_ss, p.q_perm, uint32_t(p.box_rows));
@@ -182,7 +196,8 @@ extern "C" int zen_flash_attention_f32(const float* q, const float* k, const flo
   FaParams p{};
   p.o = o; p.o_f32 = 1; p.B = B; p.H = H; p.S = S;
   p.o_sb = int64_t(H) * S * D; p.o_sh = int64_t(S) * D; p.o_ss = D; p.kv_lens = kv_lens; p.causal = causal ? 1 : 0;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  const SoftmaxScale sc = softmax_scale(scale);
+  p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   p.box_rows = fa_box_rows(S);
   CUtensorMap tq, tk, tv;
   int st = encode_qkv_map(&tq, w, B, H, S, D, p.o_sb, p.o_sh, D, p.q_perm, uint32_t(p.box_rows));
@@ -207,7 +222,8 @@ extern "C" int zen_flash_attention_unpadded_f16(const void* q, const void* k, co
   p.o = o; p.oq = oq; p.o_scale = o_scale; p.inv_o_scale = oq ? 1.0f / o_scale : 1.0f; p.B = B; p.H = H; p.S = max_seqlen;
   p.o_sb = 0; p.o_sh = o_sh; p.o_ss = o_st; p.kv_lens = nullptr; p.cu_seqlens = cu_seqlens; p.rows = int(rows);
   p.causal = causal ? 1 : 0;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  const SoftmaxScale sc = softmax_scale(scale);
+  p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   // the packed tensors as ONE batch of `rows` tokens: a tile may start at any row
   CUtensorMap tq, tk, tv;
   const int R = int(rows);
@@ -243,7 +259,8 @@ static int qkv_attention_launch(bool packed, const int8_t* xq, int64_t ldx, cons
   p.num_k_blocks = (K + 127) / 128;
   p.x_scale = x_scale; p.w_scale = w_scale; p.bias = bias; p.kv_lens = kv_lens;
   p.cu_seqlens = cu_seqlens; p.ctx = static_cast<__half*>(ctx); p.rows = int(rows);
-  p.scale_log2 = scale * 1.4426950408889634f;
+  const SoftmaxScale sc = softmax_scale(scale);
+  p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   p.ctxq = ctxq; p.ctx_scale = ctxq ? ctx_scale : 1.0f;
   p.qkv_out = static_cast<__half*>(qkv_out);
   p.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;

@@ -298,12 +298,13 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       const uint32_t ts = tmem_base + (S_SHARED ? 0u : uint32_t(g * 128));
       const uint32_t tp = tmem_base + P_OFF + uint32_t(g * 64);
       const uint32_t to = tmem_base + O_OFF + uint32_t(g * D);
+      const uint32_t idesc_qk = IDESC_QK | p.qk_negate;
       auto issue_qk = [&](int st) {
         const uint32_t ka = smem_u32(sK + st * TILE_BYTES);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const uint32_t off = (ks / 4) * CHUNK_BYTES + (ks % 4) * 32;
-          mma_f16_ss(ts, make_smem_desc_sw128(qa + off, 1024, 16), make_smem_desc_sw128(ka + off, 1024, 16), IDESC_QK, ks != 0 ? 1u : 0u);
+          mma_f16_ss(ts, make_smem_desc_sw128(qa + off, 1024, 16), make_smem_desc_sw128(ka + off, 1024, 16), idesc_qk, ks != 0 ? 1u : 0u);
         }
         tc_commit(&s_full[g]);
         tc_commit(&k_empty[st]);  // this tile has used the K tile

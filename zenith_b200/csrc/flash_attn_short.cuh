@@ -144,7 +144,7 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       for (int item = int(blockIdx.x) + g * int(gridDim.x); item < items; item += stride) {
         const int kv_len = keys_of(item / p.H);
         const int steps = (kv_len + 15) / 16;
-        const uint32_t idesc_qk = make_idesc(IDESC_C_F32, IDESC_F16, IDESC_F16, 0, 0, 128, steps * 16);
+        const uint32_t idesc_qk = make_idesc(IDESC_C_F32, IDESC_F16, IDESC_F16, 0, 0, 128, steps * 16) | p.qk_negate;
         if (!mbar_wait(&qk_full[g], ph, abort_flag)) break;
         tc_fence_after_sync();
 #pragma unroll

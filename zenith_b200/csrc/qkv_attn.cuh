@@ -52,7 +52,8 @@ struct QkvAttnParams {
   const int32_t* cu_seqlens;  // PACKED: [B + 1] row offsets; the key length of sequence b is their difference
   int rows;                   // PACKED: rows of the packed tensors; offsets beyond it are cut (nothing is stored there)
   __half* ctx;                // PACKED: output rows are written with plain stores (ld = heads * 64)
-  float scale_log2;  // softmax scale * log2(e)
+  float scale_log2;    // |softmax scale| * log2(e)
+  uint32_t qk_negate;  // added to the descriptor of Q K^T: the sign of the scale
   int8_t* ctxq;      // int8 copy of the output (may be null)
   float ctx_scale;
   __half* qkv_out;  // optional fp16 [B * S, 3 * heads * 64] copy of the projection (tests / calibration), may be null
@@ -268,7 +269,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         tc_fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          mma_f16_ss(region, make_smem_desc_sw128(qa + ks * 32, 1024, 16), make_smem_desc_sw128(ka + ks * 32, 1024, 16), IDESC_QK,
+          mma_f16_ss(region, make_smem_desc_sw128(qa + ks * 32, 1024, 16), make_smem_desc_sw128(ka + ks * 32, 1024, 16), IDESC_QK | p.qk_negate,
                      ks != 0 ? 1u : 0u);
         tc_commit(&s_full[set]);
         if (!mbar_wait(&p_ready[set], it & 1u, abort_flag)) break;

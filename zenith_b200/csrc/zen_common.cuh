@@ -587,6 +587,7 @@ enum : uint32_t { IDESC_C_F16 = 0, IDESC_C_F32 = 1, IDESC_C_S32 = 2 };
 enum : uint32_t { IDESC_F16 = 0, IDESC_BF16 = 1, IDESC_TF32 = 2 };
 enum : uint32_t { IDESC_U8 = 0, IDESC_S8 = 1 };
 enum : uint32_t { IDESC_E4M3 = 0, IDESC_E5M2 = 1 };  // kind::f8f6f4
+enum : uint32_t { IDESC_NEGATE_A = 1u << 13 };  // floating-point kinds: the product of -A and B
 
 __host__ __device__ constexpr uint32_t make_idesc(uint32_t c_fmt, uint32_t a_fmt, uint32_t b_fmt, uint32_t a_mn_major,
                                                   uint32_t b_mn_major, uint32_t M, uint32_t N) {
