@@ -69,6 +69,70 @@ def test_operators_refuse_cpu_tensors():
             call()
 
 
+def test_operators_refuse_vectors_that_a_kernel_would_read_past(monkeypatch):
+    """Scales, biases, LayerNorm parameters, key lengths and packed positions that are too short or on another device raise
+    before anything is launched (fake CUDA tensors: no device is needed)."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from zenith_b200 import ops
+
+    def launched(*a):
+        raise AssertionError("launched")
+
+    monkeypatch.setattr(ops, "_call", launched)
+    monkeypatch.setattr(ops, "_layernorm_workspace", lambda *a: (None, 0))
+    i8, u8, i32, f16, f32 = torch.int8, torch.uint8, torch.int32, torch.float16, torch.float32
+    with FakeTensorMode():
+        T = lambda *shape, dt=f32, dev="cuda:0": torch.empty(shape, dtype=dt, device=dev)
+        M, K, N = 4, 64, 768
+        q = T(3, 2, 16, 64, dt=f16)
+        x8, w8, res, h = T(M, K, dt=i8), T(N, K, dt=i8), T(M, N, dt=f16), T(N, dt=f16)
+        ids, word, pos, typ = T(32, dt=i32), T(100, N, dt=f16), T(16, N, dt=f16), T(2, N, dt=f16)
+        calls = {
+            "kv_lens": [
+                lambda n, dev="cuda:0": ops.flash_attention(q, q, q, kv_lens=T(n, dt=i32, dev=dev)),
+                lambda n, dev="cuda:0": ops.flash_attention(q.float(), q.float(), q.float(), kv_lens=T(n, dt=i32, dev=dev)),
+                lambda n, dev="cuda:0": ops.flash_attention_strided(q, q, q, q, 3, 2, 16, 64, *[(1, 1, 1)] * 4, kv_lens=T(n, dt=i32, dev=dev)),
+                lambda n, dev="cuda:0": ops.qkv_attention_int8(T(48, K, dt=i8), T(384, K, dt=i8), 1.0, None, None, 3, 16, 2, kv_lens=T(n, dt=i32, dev=dev)),
+                lambda n, dev="cuda:0": ops.pack_tokens(T(3, 16, dt=i32), T(n, dt=i32, dev=dev), 48)],
+            "w_scale": [
+                lambda n, dev="cuda:0": ops.linear_int8_add_layernorm(x8, w8, 1.0, T(n, dev=dev), None, res, h, h, 1e-5),
+                lambda n, dev="cuda:0": ops.qkv_attention_int8(T(48, K, dt=i8), T(384, K, dt=i8), 1.0, T(n, dev=dev), None, 3, 16, 2),
+                lambda n, dev="cuda:0": ops.qkv_attention_unpadded_int8(T(48, K, dt=i8), T(384, K, dt=i8), 1.0, T(n, dev=dev), None, T(4, dt=i32), 2),
+                lambda n, dev="cuda:0": ops.linear_fp8(x8.view(u8), w8.view(u8), 1.0, T(n, dev=dev))],
+            "bias": [
+                lambda n, dev="cuda:0": ops.linear_fp16(T(M, K, dt=f16), T(N, K, dt=f16), T(n, dev=dev)),
+                lambda n, dev="cuda:0": ops.linear_fp32(T(M, K), T(N, K), T(n, dev=dev)),
+                lambda n, dev="cuda:0": ops.linear_fp8(x8.view(u8), w8.view(u8), 1.0, None, T(n, dev=dev)),
+                lambda n, dev="cuda:0": ops.linear_int8_add_layernorm(x8, w8, 1.0, None, T(n, dev=dev), res, h, h, 1e-5),
+                lambda n, dev="cuda:0": ops.linear_fp16_add_layernorm(T(M, K, dt=f16), T(N, K, dt=f16), T(n, dev=dev), res, h, h, 1e-5),
+                lambda n, dev="cuda:0": ops.bias_gelu(T(M, N), T(n, dev=dev))],
+            "gamma": [
+                lambda n, dev="cuda:0": ops.layernorm(T(M, N), T(n, dev=dev), T(N)),
+                lambda n, dev="cuda:0": ops.add_layernorm(res, res, T(n, dt=f16, dev=dev), h),
+                lambda n, dev="cuda:0": ops.linear_int8_add_layernorm(x8, w8, 1.0, None, None, res, T(n, dt=f16, dev=dev), h, 1e-5),
+                lambda n, dev="cuda:0": ops.embed_layernorm(ids, None, word, pos, typ, T(n, dt=f16, dev=dev), h, 1e-5, 16),
+                lambda n, dev="cuda:0": ops.embed_layernorm_unpadded(ids, ids, None, word, pos, typ, T(n, dt=f16, dev=dev), h, 1e-5)],
+            "beta": [lambda n, dev="cuda:0": ops.layernorm(T(M, N), T(N), T(n, dev=dev))],
+            "type_ids": [lambda n, dev="cuda:0": ops.embed_layernorm(ids, T(n, dt=i32, dev=dev), word, pos, typ, h, h, 1e-5, 16)],
+            "pos_packed": [lambda n, dev="cuda:0": ops.embed_layernorm_unpadded(ids, T(n, dt=i32, dev=dev), None, word, pos, typ, h, h, 1e-5)],
+        }
+        for name, fns in calls.items():
+            for i, fn in enumerate(fns):
+                with pytest.raises(RuntimeError, match=f"{name} must have (at least|one entry)"):
+                    fn(2)
+                with pytest.raises(RuntimeError, match=f"{name} must be on cuda:0"):
+                    fn(2000, "cuda:1")
+        for fn in (ops.linear_fp16, ops.linear_int8):
+            dt = f16 if fn is ops.linear_fp16 else i8
+            scale = () if fn is ops.linear_fp16 else (1.0,)
+            with pytest.raises(RuntimeError, match="out must hold 4 x 768"):
+                fn(T(M, K, dt=dt), T(N, K, dt=dt), *scale, out=T(M - 1, N, dt=f16), out_dtype=f16)
+        with pytest.raises(RuntimeError, match="type must have at least 1536"):
+            ops.embed_layernorm(ids, ids, word, pos, typ[:1], h, h, 1e-5, 16)
+
+
 def test_missing_extension_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_capi, "_lib", None)
     monkeypatch.setattr(_capi, "LIB_PATH", tmp_path / "absent.so")

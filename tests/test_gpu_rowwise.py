@@ -139,3 +139,23 @@ def test_quantize_vector_and_tail(cuda, n, dtype):
     for v in (t[:n].contiguous(), t[1:]):
         got = ops.quantize(v, 0.03125).cpu().numpy()
         assert np.array_equal(got, O.quantize(v.float().cpu().numpy(), 0.03125))
+
+
+def test_vectors_shorter_than_a_row_are_refused_and_longer_ones_taken(cuda):
+    """The native path and the one behind it: nothing is launched that would read past a vector."""
+    x = torch.randn(5, 768, device=cuda)
+    g, b = torch.randn(768, device=cuda), torch.randn(768, device=cuda)
+    q = torch.randn(3, 2, 16, 64, device=cuda).half()
+    for short in (767, 1):
+        with pytest.raises(RuntimeError, match="gamma must have at least 768"):
+            ops.layernorm(x, g[:short], b)
+        with pytest.raises(RuntimeError, match="beta must have at least 768"):
+            ops.add_layernorm(x.half(), x.half(), g.half(), b[:short].half())
+    with pytest.raises(RuntimeError, match="kv_lens must have at least 3"):
+        ops.flash_attention(q, q, q, kv_lens=torch.ones(2, dtype=torch.int32, device=cuda))
+    more = lambda t: torch.cat((t, t))
+    assert torch.equal(ops.layernorm(x, more(g), more(b)), ops.layernorm(x, g, b))
+    w = torch.randn(768, 768, device=cuda)
+    assert torch.equal(ops.linear_fp32(x, w, more(b)), ops.linear_fp32(x, w, b))
+    lens = torch.tensor([3, 16, 9], dtype=torch.int32, device=cuda)
+    assert torch.equal(ops.flash_attention(q, q, q, kv_lens=more(lens)), ops.flash_attention(q, q, q, kv_lens=lens))

@@ -47,6 +47,9 @@ inline bool plain_rows(const at::Tensor* t, int dev, ScalarType st) {
   return (t->size(1) <= 1 || t->stride(1) == 1) && t->stride(0) >= t->size(1);
 }
 
+// A contiguous vector of at least the n entries that a kernel reads.
+inline bool vector_of(const at::Tensor* t, int dev, ScalarType st, int64_t n) { return plain(t, dev, st, 1) && t->numel() >= n; }
+
 // None or a contiguous fp32 vector of n entries.
 inline bool vector_or_none(PyObject* o, int dev, int64_t n, const float** p) {
   *p = nullptr;
@@ -199,7 +202,7 @@ PyObject* layernorm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const bool f32 = plain(x, dev, at::kFloat, 2);
   if ((!f32 && !plain(x, dev, at::kHalf, 2)) || !number(a[3], &eps)) Py_RETURN_NONE;
   const int64_t rows = x->size(0), hidden = x->size(1);
-  if (!plain(g, dev, x->scalar_type(), 1) || !plain(b, dev, x->scalar_type(), 1) || !fits(rows) || !fits(hidden)) Py_RETURN_NONE;
+  if (!vector_of(g, dev, x->scalar_type(), hidden) || !vector_of(b, dev, x->scalar_type(), hidden) || !fits(rows) || !fits(hidden)) Py_RETURN_NONE;
   return serve<1>([&](at::Tensor* o) {
     o[0] = empty(x->sizes(), x->scalar_type(), dev);
     if (f32)
@@ -223,7 +226,8 @@ PyObject* add_layernorm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   const int64_t rows = x->size(0), hidden = x->size(1);
   const ScalarType st = x->scalar_type();
-  if (!plain(r, dev, st, 2) || r->sizes() != x->sizes() || !plain(g, dev, st, 1) || !plain(b, dev, st, 1) || !fits(rows) || !fits(hidden))
+  if (!plain(r, dev, st, 2) || r->sizes() != x->sizes() || !vector_of(g, dev, st, hidden) || !vector_of(b, dev, st, hidden) || !fits(rows) ||
+      !fits(hidden))
     Py_RETURN_NONE;
   return serve<2>([&](at::Tensor* o) {
     o[0] = empty(x->sizes(), st, dev);
@@ -353,7 +357,7 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int32_t* lens = nullptr;
   if (a[4] != Py_None) {
     const at::Tensor* t = tensor_of(a[4]);
-    if (!plain(t, dev, at::kInt, 1) || t->numel() < B) Py_RETURN_NONE;
+    if (!vector_of(t, dev, at::kInt, B)) Py_RETURN_NONE;
     lens = static_cast<const int32_t*>(t->const_data_ptr());
   }
   double scale;

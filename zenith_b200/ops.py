@@ -42,17 +42,30 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-def _require(t: torch.Tensor, name: str, dtype=None, ndim=None, rows_may_be_strided: bool = False) -> None:
+def _require(t: torch.Tensor, name: str, dtype=None, ndim=None, rows_may_be_strided: bool = False, *, like=None,
+             at_least: int | None = None) -> None:
+    """``like``: a tensor whose device this one must share; ``at_least``: entries that the kernel reads of it."""
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise RuntimeError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype != dtype:
         raise RuntimeError(f"{name} must be {dtype}, got {t.dtype}")
     if ndim is not None and t.dim() != ndim:
         raise RuntimeError(f"{name} must be {ndim}-D, got {t.dim()}-D")
+    if like is not None and t.device != like.device:
+        raise RuntimeError(f"{name} must be on {like.device}, got {t.device}")
+    if at_least is not None and t.numel() < at_least:
+        raise RuntimeError(f"{name} must have at least {at_least} entries, got {t.numel()}")
     if rows_may_be_strided and t.dim() == 2 and (t.shape[1] <= 1 or t.stride(1) == 1) and t.stride(0) >= t.shape[1]:
         return
     if not t.is_contiguous():
         raise RuntimeError(f"{name} must be contiguous")
+
+
+def _require_out(out: torch.Tensor, dtype, M: int, N: int, like, rows_may_be_strided: bool = True) -> None:
+    """A caller's result matrix: at least ``M`` rows of ``N`` entries."""
+    _require(out, "out", dtype, 2, rows_may_be_strided, like=like)
+    if out.shape[0] < M or out.shape[1] < N:
+        raise RuntimeError(f"out must hold {M} x {N} entries, got {tuple(out.shape)}")
 
 
 def _ptr(t) -> int | None:
@@ -102,7 +115,7 @@ def linear_int8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", 
             launch_count += 1
             return y
     _require(xq, "xq", torch.int8, 2)
-    _require(wq, "wq", torch.int8, 2)
+    _require(wq, "wq", torch.int8, 2, like=xq)
     M, K = xq.shape
     N, K2 = wq.shape
     if len(prefetch) > 2 or any(not t.is_cuda for t in prefetch):
@@ -110,11 +123,11 @@ def linear_int8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", 
     if K != K2:
         raise RuntimeError(f"inner dimensions differ: xq {tuple(xq.shape)} vs wq {tuple(wq.shape)}")
     if w_scale is not None:
-        _require(w_scale, "w_scale", torch.float32, 1)
+        _require(w_scale, "w_scale", torch.float32, 1, like=xq)
         if w_scale.numel() != N:
             raise RuntimeError("w_scale must have one entry per output channel")
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=xq)
         if bias.numel() != N:
             raise RuntimeError("bias must have one entry per output channel")
     if out_dtype not in _OUT:
@@ -124,7 +137,7 @@ def linear_int8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", 
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=xq.device)
     else:
-        _require(out, "out", out_dtype, 2)
+        _require_out(out, out_dtype, M, N, xq, rows_may_be_strided=False)
     if M == 0 or N == 0:
         return out
     hint = [v for t in prefetch for v in (t.data_ptr(), t.numel() * t.element_size())] + [None, 0] * (2 - len(prefetch))
@@ -150,18 +163,18 @@ def linear_int8_add_layernorm(xq, wq, x_scale: float, w_scale, bias, residual, g
     Returns fp16 ``y`` and, with ``out_scale``, also the int8 copy ``quantize(y, out_scale)``.
     """
     _require(xq, "xq", torch.int8, 2)
-    _require(wq, "wq", torch.int8, 2)
-    _require(residual, "residual", torch.float16, 2)
-    _require(gamma, "gamma", torch.float16, 1)
-    _require(beta, "beta", torch.float16, 1)
+    _require(wq, "wq", torch.int8, 2, like=xq)
+    _require(residual, "residual", torch.float16, 2, like=xq)
+    _require(gamma, "gamma", torch.float16, 1, like=xq, at_least=wq.shape[0])
+    _require(beta, "beta", torch.float16, 1, like=xq, at_least=wq.shape[0])
     M, K = xq.shape
     N = wq.shape[0]
     if wq.shape[1] != K or tuple(residual.shape) != (M, N):
         raise RuntimeError("shape mismatch")
     if w_scale is not None:
-        _require(w_scale, "w_scale", torch.float32, 1)
+        _require(w_scale, "w_scale", torch.float32, 1, like=xq, at_least=N)
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=xq, at_least=N)
     y = torch.empty((M, N), dtype=torch.float16, device=xq.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=xq.device) if out_scale is not None else None
     if M:
@@ -179,16 +192,16 @@ def linear_fp16_add_layernorm(x, w, bias, residual, gamma, beta, eps: float, *, 
     """``LayerNorm(x @ w.T + bias + residual) * gamma + beta`` with fp16 operands (hidden 768 or 1024), as
     ``linear_int8_add_layernorm``.  Returns fp16 ``y`` and, with ``out_scale``, also ``quantize(y, out_scale)``."""
     _require(x, "x", torch.float16, 2)
-    _require(w, "w", torch.float16, 2)
-    _require(residual, "residual", torch.float16, 2)
-    _require(gamma, "gamma", torch.float16, 1)
-    _require(beta, "beta", torch.float16, 1)
+    _require(w, "w", torch.float16, 2, like=x)
+    _require(residual, "residual", torch.float16, 2, like=x)
+    _require(gamma, "gamma", torch.float16, 1, like=x, at_least=w.shape[0])
+    _require(beta, "beta", torch.float16, 1, like=x, at_least=w.shape[0])
     M, K = x.shape
     N = w.shape[0]
     if w.shape[1] != K or tuple(residual.shape) != (M, N):
         raise RuntimeError("shape mismatch")
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=x, at_least=N)
     y = torch.empty((M, N), dtype=torch.float16, device=x.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=x.device) if out_scale is not None else None
     if M:
@@ -210,17 +223,19 @@ def linear_fp16(x, w, bias=None, *, act="none", out_dtype=torch.float16, out=Non
             launch_count += 1
             return y
     _require(x, "x", torch.float16, 2, rows_may_be_strided=True)
-    _require(w, "w", torch.float16, 2)
+    _require(w, "w", torch.float16, 2, like=x)
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:
         raise RuntimeError(f"inner dimensions differ: x {tuple(x.shape)} vs w {tuple(w.shape)}")
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=x, at_least=N)
     if out_dtype not in (torch.float16, torch.float32):
         raise RuntimeError(f"unsupported out_dtype {out_dtype}")
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+    else:
+        _require_out(out, out_dtype, M, N, x)
     if M == 0 or N == 0:
         return out
     _call("zen_linear_f16_ex", x.data_ptr(), x.stride(0) if M > 1 else K, w.data_ptr(), K, M, N, K, _ptr(bias), _ACT[act], _OUT[out_dtype],
@@ -236,13 +251,13 @@ def linear_fp32(x, w, bias=None, *, act="none"):
         launch_count += 1
         return y
     _require(x, "x", torch.float32, 2)
-    _require(w, "w", torch.float32, 2)
+    _require(w, "w", torch.float32, 2, like=x)
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:
         raise RuntimeError(f"inner dimensions differ: x {tuple(x.shape)} vs w {tuple(w.shape)}")
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=x, at_least=N)
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     if M and N:
         _call("zen_linear_f32", x.data_ptr(), K, w.data_ptr(), K, M, N, K, _ptr(bias), _ACT[act], out.data_ptr(), N,
@@ -265,6 +280,7 @@ def wmma_matmul(a, b):
         raise RuntimeError("Inputs must be FP16")
     if a.shape[1] != b.shape[0]:
         raise RuntimeError("Inner dimensions must match")
+    _require(b.contiguous(), "B", like=a)
     a = a.contiguous()
     b = b.contiguous()
     M, K = a.shape
@@ -291,7 +307,7 @@ def matmul_f32(a, b):
     _require(a.contiguous(), "A", torch.float32)
     a = a.contiguous()
     b = b.contiguous()
-    _require(b, "B", torch.float32)
+    _require(b, "B", torch.float32, like=a)
     M, K = a.shape
     N = b.shape[1]
     c = torch.empty((M, N), dtype=torch.float32, device=a.device)
@@ -354,7 +370,7 @@ def relu(x):
 def bias_gelu(x, bias):
     """``gelu(x + bias[col])`` over [rows, features] (core/src/fused_kernels.cu:47-62)."""
     _require(x, "input", torch.float32, 2)
-    _require(bias, "bias", torch.float32, 1)
+    _require(bias, "bias", torch.float32, 1, like=x, at_least=x.shape[1])
     y = torch.empty_like(x)
     if x.numel():
         _call("zen_bias_gelu_f32", x.data_ptr(), bias.data_ptr(), y.data_ptr(), x.shape[0], x.shape[1], _stream())
@@ -371,8 +387,8 @@ def layernorm(x, gamma, beta, eps: float = 1e-5):
     if x.dtype not in (torch.float32, torch.float16):
         raise RuntimeError("input must be fp32 or fp16")
     _require(x, "input", x.dtype, 2)
-    _require(gamma, "gamma", x.dtype, 1)
-    _require(beta, "beta", x.dtype, 1)
+    _require(gamma, "gamma", x.dtype, 1, like=x, at_least=x.shape[1])
+    _require(beta, "beta", x.dtype, 1, like=x, at_least=x.shape[1])
     y = torch.empty_like(x)
     fn = "zen_layernorm_f32" if x.dtype == torch.float32 else "zen_layernorm_f16"
     if x.numel():
@@ -395,9 +411,9 @@ def add_layernorm(x, residual, gamma, beta, eps: float = 1e-5, *, out_scale: flo
     if x.dtype not in (torch.float32, torch.float16):
         raise RuntimeError("input must be fp32 or fp16")
     _require(x, "input", x.dtype, 2)
-    _require(residual, "residual", x.dtype, 2)
-    _require(gamma, "gamma", x.dtype, 1)
-    _require(beta, "beta", x.dtype, 1)
+    _require(residual, "residual", x.dtype, 2, like=x)
+    _require(gamma, "gamma", x.dtype, 1, like=x, at_least=x.shape[1])
+    _require(beta, "beta", x.dtype, 1, like=x, at_least=x.shape[1])
     if residual.shape != x.shape:
         raise RuntimeError("residual must have the shape of the input")
     y = torch.empty_like(x)
@@ -507,7 +523,7 @@ def absmax_rows(w):
 def quantize_rows(w, scale, *, round="nearest_even"):
     """``clamp(round(w[r, c] / scale[r]), -128, 127)`` as int8: per-output-channel weight conversion."""
     _require(w, "w", torch.float32, 2, rows_may_be_strided=True)
-    _require(scale, "scale", torch.float32, 1)
+    _require(scale, "scale", torch.float32, 1, like=w)
     if scale.numel() != w.shape[0]:
         raise RuntimeError("scale must have one entry per row")
     q = torch.empty(w.shape, dtype=torch.int8, device=w.device)
@@ -540,7 +556,7 @@ def flash_attention_strided(q, k, v, out, B, H, S, D, q_strides, k_strides, v_st
                             causal=False, scale=None, out_q=None, out_scale=None):
     """Attention over strided fp16 views: strides are (batch, head, seq) in elements, d contiguous."""
     if kv_lens is not None:
-        _require(kv_lens, "kv_lens", torch.int32, 1)
+        _require(kv_lens, "kv_lens", torch.int32, 1, like=q, at_least=B)
     scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
     _call("zen_flash_attention_f16", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), _ptr(out_q),
           float(out_scale or 1.0), B, H, S, D, *q_strides, *k_strides, *v_strides, *o_strides, _ptr(kv_lens),
@@ -571,9 +587,9 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
     if q.dtype == torch.float32:
         q, k, v = (t.contiguous() for t in (q, k, v))
         for name, t in (("Q", q), ("K", k), ("V", v)):
-            _require(t, name, torch.float32, 4)
+            _require(t, name, torch.float32, 4, like=q)
         if kv_lens is not None:
-            _require(kv_lens, "kv_lens", torch.int32, 1)
+            _require(kv_lens, "kv_lens", torch.int32, 1, like=q, at_least=B)
         out = torch.empty_like(q)
         nbytes = _capi.lib().zen_flash_attention_f32_workspace_bytes(B, H, S, D)
         workspace = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
@@ -582,7 +598,7 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
         launch_count_add(1)
         return out
     for name, t in (("Q", q), ("K", k), ("V", v)):
-        _require(t, name, torch.float16, 4)
+        _require(t, name, torch.float16, 4, like=q)
     out = torch.empty_like(q)
     st = (H * S * D, S * D, D)
     flash_attention_strided(q, k, v, out, B, H, S, D, st, st, st, st, kv_lens=kv_lens, causal=causal, scale=scale)
@@ -597,17 +613,17 @@ def qkv_attention_int8(xq, wqkv, x_scale: float, w_scale, bias, B: int, S: int, 
     then (with ``out_scale``) its int8 copy, then (with ``emit_qkv``) the fp16 projection ``[B*S, 3*heads*64]``.
     Bit-identical to ``linear_int8(..., out_dtype=float16)`` followed by ``flash_attention_strided``."""
     _require(xq, "xq", torch.int8, 2)
-    _require(wqkv, "wqkv", torch.int8, 2)
+    _require(wqkv, "wqkv", torch.int8, 2, like=xq)
     hidden = heads * 64
     T, K = xq.shape
     if T != B * S or tuple(wqkv.shape) != (3 * hidden, K):
         raise RuntimeError("shape mismatch")
     if w_scale is not None:
-        _require(w_scale, "w_scale", torch.float32, 1)
+        _require(w_scale, "w_scale", torch.float32, 1, like=xq, at_least=3 * hidden)
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=xq, at_least=3 * hidden)
     if kv_lens is not None:
-        _require(kv_lens, "kv_lens", torch.int32, 1)
+        _require(kv_lens, "kv_lens", torch.int32, 1, like=xq, at_least=B)
     if len(prefetch) > 2:
         raise RuntimeError("prefetch takes at most two CUDA tensors")
     ctx = torch.empty((T, hidden), dtype=torch.float16, device=xq.device)
@@ -636,17 +652,19 @@ def embed_layernorm(ids, type_ids, word, pos, typ, gamma, beta, eps: float, seq:
     (core/src/transformer_kernels.cu:236-262); position / type tables and the LayerNorm are the
     BERT embedding block that precedes the encoder.
     """
-    _require(ids, "ids", torch.int32, 1)
+    _require(ids, "ids", torch.int32, 1, like=word)
     if type_ids is not None:
-        _require(type_ids, "type_ids", torch.int32, 1)
+        _require(type_ids, "type_ids", torch.int32, 1, like=word, at_least=ids.numel())
     for name, t in (("word", word), ("pos", pos), ("type", typ)):
-        _require(t, name, torch.float16, 2)
-    _require(gamma, "gamma", torch.float16, 1)
-    _require(beta, "beta", torch.float16, 1)
+        _require(t, name, torch.float16, 2, like=word)
+    _require(gamma, "gamma", torch.float16, 1, like=word, at_least=word.shape[1])
+    _require(beta, "beta", torch.float16, 1, like=word, at_least=word.shape[1])
     tokens = ids.numel()
     hidden = word.shape[1]
     if pos.shape[0] < seq:
         raise RuntimeError("position table shorter than the sequence")
+    _require(pos, "pos", at_least=seq * hidden)
+    _require(typ, "type", at_least=hidden * (1 if type_ids is None else 2))
     y = torch.empty((tokens, hidden), dtype=torch.float16, device=word.device)
     yq = torch.empty((tokens, hidden), dtype=torch.int8, device=word.device) if out_scale is not None else None
     if tokens:
@@ -664,9 +682,9 @@ def pack_tokens(ids, kv_lens, capacity: int, type_ids=None):
     pos_packed, type_packed or None)`` of ``capacity`` rows (``zen_pack_tokens_i32``); rows beyond the total
     carry id 0 / position 0."""
     _require(ids, "ids", torch.int32, 2)
-    _require(kv_lens, "kv_lens", torch.int32, 1)
+    _require(kv_lens, "kv_lens", torch.int32, 1, like=ids, at_least=ids.shape[0])
     if type_ids is not None:
-        _require(type_ids, "type_ids", torch.int32, 2)
+        _require(type_ids, "type_ids", torch.int32, 2, like=ids, at_least=ids.numel())
     B, S = ids.shape
     d = ids.device
     cu = torch.empty(B + 1, dtype=torch.int32, device=d)
@@ -681,7 +699,7 @@ def pack_tokens(ids, kv_lens, capacity: int, type_ids=None):
 def unpad_rows(packed, cu_seqlens, B: int, S: int):
     """Padded ``[B*S, hidden]`` fp16 copy of packed rows: zeros at padding positions (``zen_unpad_rows_f16``)."""
     _require(packed, "packed", torch.float16, 2)
-    _require(cu_seqlens, "cu_seqlens", torch.int32, 1)
+    _require(cu_seqlens, "cu_seqlens", torch.int32, 1, like=packed)
     if cu_seqlens.numel() != B + 1:
         raise RuntimeError("cu_seqlens must hold B + 1 offsets")
     out = torch.empty((B * S, packed.shape[1]), dtype=torch.float16, device=packed.device)
@@ -693,16 +711,18 @@ def unpad_rows(packed, cu_seqlens, B: int, S: int):
 def embed_layernorm_unpadded(ids_packed, pos_packed, type_packed, word, pos, typ, gamma, beta, eps: float, *,
                              out_scale=None, round="nearest_even"):
     """``embed_layernorm`` on packed rows: the position of each row comes from ``pos_packed``."""
-    _require(ids_packed, "ids_packed", torch.int32, 1)
-    _require(pos_packed, "pos_packed", torch.int32, 1)
+    _require(ids_packed, "ids_packed", torch.int32, 1, like=word)
+    _require(pos_packed, "pos_packed", torch.int32, 1, like=word, at_least=ids_packed.numel())
     if type_packed is not None:
-        _require(type_packed, "type_packed", torch.int32, 1)
+        _require(type_packed, "type_packed", torch.int32, 1, like=word, at_least=ids_packed.numel())
     for name, t in (("word", word), ("pos", pos), ("type", typ)):
-        _require(t, name, torch.float16, 2)
-    _require(gamma, "gamma", torch.float16, 1)
-    _require(beta, "beta", torch.float16, 1)
+        _require(t, name, torch.float16, 2, like=word)
+    _require(gamma, "gamma", torch.float16, 1, like=word, at_least=word.shape[1])
+    _require(beta, "beta", torch.float16, 1, like=word, at_least=word.shape[1])
     rows = ids_packed.numel()
     hidden = word.shape[1]
+    _require(pos, "pos", at_least=pos.shape[0] * hidden)
+    _require(typ, "type", at_least=hidden * (1 if type_packed is None else 2))
     y = torch.empty((rows, hidden), dtype=torch.float16, device=word.device)
     yq = torch.empty((rows, hidden), dtype=torch.int8, device=word.device) if out_scale is not None else None
     if rows:
@@ -719,16 +739,16 @@ def qkv_attention_unpadded_int8(xq, wqkv, x_scale: float, w_scale, bias, cu_seql
     in rows ``cu_seqlens[b] .. cu_seqlens[b+1]-1`` (at most 128 each).  Rows that belong to no sequence are left
     unwritten in the outputs (which start as zeros here)."""
     _require(xq, "xq", torch.int8, 2)
-    _require(wqkv, "wqkv", torch.int8, 2)
-    _require(cu_seqlens, "cu_seqlens", torch.int32, 1)
+    _require(wqkv, "wqkv", torch.int8, 2, like=xq)
+    _require(cu_seqlens, "cu_seqlens", torch.int32, 1, like=xq)
     hidden = heads * 64
     T, K = xq.shape
     if tuple(wqkv.shape) != (3 * hidden, K):
         raise RuntimeError("shape mismatch")
     if w_scale is not None:
-        _require(w_scale, "w_scale", torch.float32, 1)
+        _require(w_scale, "w_scale", torch.float32, 1, like=xq, at_least=3 * hidden)
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=xq, at_least=3 * hidden)
     B = cu_seqlens.numel() - 1
     ctx = torch.zeros((T, hidden), dtype=torch.float16, device=xq.device)
     ctxq = torch.zeros((T, hidden), dtype=torch.int8, device=xq.device) if out_scale is not None else None
@@ -765,19 +785,21 @@ def linear_fp8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", o
     """``act((xq @ wq.T) * x_scale * w_scale + bias)`` with e4m3 operands (uint8 bit patterns) and fp32 accumulation on
     the tensor cores (``zen_linear_f8``); a tolerance path like ``linear_fp16``."""
     _require(xq, "xq", torch.uint8, 2, rows_may_be_strided=True)
-    _require(wq, "wq", torch.uint8, 2)
+    _require(wq, "wq", torch.uint8, 2, like=xq)
     M, K = xq.shape
     N, K2 = wq.shape
     if K != K2:
         raise RuntimeError(f"inner dimensions differ: xq {tuple(xq.shape)} vs wq {tuple(wq.shape)}")
     if w_scale is not None:
-        _require(w_scale, "w_scale", torch.float32, 1)
+        _require(w_scale, "w_scale", torch.float32, 1, like=xq, at_least=N)
     if bias is not None:
-        _require(bias, "bias", torch.float32, 1)
+        _require(bias, "bias", torch.float32, 1, like=xq, at_least=N)
     if out_dtype not in (torch.float16, torch.float32):
         raise RuntimeError(f"unsupported out_dtype {out_dtype}")
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=xq.device)
+    else:
+        _require_out(out, out_dtype, M, N, xq)
     if M == 0 or N == 0:
         return out
     _call("zen_linear_f8", xq.data_ptr(), xq.stride(0) if M > 1 else K, wq.data_ptr(), K, M, N, K, float(x_scale), _ptr(w_scale),
@@ -793,7 +815,7 @@ def flash_attention_unpadded(qkv, cu_seqlens, heads: int, head_dim: int, max_seq
     length up to ``max_seqlen``).  Returns the context ``[rows, heads * head_dim]`` (rows of no sequence stay zero),
     and with ``out_scale`` its int8 copy."""
     _require(qkv, "qkv", torch.float16, 2)
-    _require(cu_seqlens, "cu_seqlens", torch.int32, 1)
+    _require(cu_seqlens, "cu_seqlens", torch.int32, 1, like=qkv)
     hidden = heads * head_dim
     rows = qkv.shape[0]
     if qkv.shape[1] != 3 * hidden:
