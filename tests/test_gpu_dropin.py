@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import zenith_b200
-from zenith_b200 import _capi, registry
+from zenith_b200 import _capi, ops, registry
 
 pytestmark = pytest.mark.gpu
 
@@ -165,3 +165,23 @@ def test_torch_compile_of_a_huggingface_bert_runs_on_the_kernels(cuda):
     err = (got - want).abs()
     assert err.max().item() < 3e-2 and err.mean().item() < 2e-3
     assert _capi.device_status() == 0
+
+
+def test_wrapped_tensors_raise_and_do_not_end_the_process(cuda):
+    """Tensors without storage or sizes of their own (vmap, forward-mode and nested tensors) raise from the operators."""
+    x, w, b = torch.randn(4, 64, device=cuda), torch.randn(32, 64, device=cuda), torch.randn(3, 32, device=cuda)
+    q, lens = torch.randn(3, 1, 2, 16, 64, device=cuda).half(), torch.ones(3, 1, dtype=torch.int32, device=cuda)
+    g = torch.ones(64, device=cuda)
+    nested = torch.nested.nested_tensor([torch.randn(3, device=cuda), torch.randn(5, device=cuda)])
+    calls = [
+        lambda: torch.vmap(lambda v: ops.linear_fp32(x, w, v))(b),
+        lambda: torch.vmap(lambda v: ops.linear_fp16(x.half(), w.half(), v))(b),
+        lambda: torch.vmap(lambda n: ops.flash_attention(q[0], q[0], q[0], kv_lens=n))(lens),
+        lambda: torch.vmap(ops.gelu)(b),
+        lambda: torch.func.jvp(lambda v: ops.linear_fp32(x, w, v), (b[0],), (b[1],)),
+        lambda: ops.layernorm(nested, g, g),
+    ]
+    for call in calls:
+        with pytest.raises(RuntimeError):
+            call()
+    assert torch.equal(ops.linear_fp32(x, w, b[0]), ops.linear_fp32(x, w, b[0].clone()))

@@ -380,7 +380,19 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   });
 }
 
-#define FN(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+// No C++ exception leaves a function that Python calls.  Sizes and data pointers throw for tensors that have none of their
+// own (inside vmap or forward-mode transforms, nested tensors): such a call is not served either.
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t nargs) {
+  try {
+    return F(self, a, nargs);
+  } catch (...) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+}
+
+#define FN(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FN(gelu),        FN(relu),        FN(quantize),    FN(dequantize),  FN(layernorm),  FN(add_layernorm),
                          FN(linear_int8), FN(linear_fp16), FN(linear_fp32), FN(wmma_matmul), FN(matmul_f32), FN(flash_attention),
                          {nullptr, nullptr, 0, nullptr}};
