@@ -64,6 +64,20 @@ int zen_device_status_clear(void);
  * (benchmarks/mlperf_suite.py:750-850 runs independent replicas). */
 int zen_memcpy_async(void* dst, const void* src, size_t bytes, void* stream);
 
+/* A sequence of calls recorded once and launched as one graph.  Between zen_record_begin and zen_record_end the calling
+ * thread's entry points launch nothing: each of their kernels becomes a node of a graph, ordered as in one stream (the stream
+ * argument is not used); zen_record_branch starts a branch that does not wait for what was recorded before it.  zen_record_end
+ * always ends the recording; it leaves the executable graph in *graph_host (NULL on failure), or drops it if graph_host is NULL.
+ * The graph keeps the pointers that the calls were given.  No stream is captured: other threads may synchronise the device,
+ * allocate and launch meanwhile.  Every kernel has to have been launched once before (its attributes are set then).  Copies
+ * and graph launches return ZEN_ERR_UNSUPPORTED while the thread records.  A graph may be destroyed while it runs.
+ * The reference replays whole passes with torch's graphs (zenith/runtime/cuda_graphs.py). */
+int zen_record_begin(void);
+int zen_record_branch(void);
+int zen_record_end(void** graph_host);
+int zen_graph_launch(void* graph, void* stream);
+int zen_graph_destroy(void* graph);
+
 /* Self-test of the wait limit: one small CTA waits on a barrier that nothing signals, in a build of the wait
  * loop whose limit is 1 ms.  The wait gives up by itself, the kernel returns normally and leaves
  * ZEN_ERR_TIMEOUT in the device status word (read it with zen_device_status_read, reset it with

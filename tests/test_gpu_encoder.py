@@ -6,6 +6,8 @@ int8 encoder  : every int8 GEMM of every layer is checked BIT-EXACTLY against th
                 quantization of the fp16 tensors beside them, and the final hidden states track the
                 oracle's int8 encoder and the fp32 encoder.
 """
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -265,6 +267,94 @@ def test_repeated_plain_calls_equal_the_first(cuda, params, micro_batches):
     out.zero_()
     g.replay()
     assert torch.equal(out, want)
+
+
+def third_call(enc, ids, lens, during):
+    """The call that records, with ``during()`` run between two of the recorded launches."""
+    issue, calls = enc._issue, []
+
+    def patched(launches, stream):
+        issue(launches[:3], stream)
+        calls.append(stream)
+        if len(calls) == 1:
+            during()
+        issue(launches[3:], stream)
+
+    enc._issue = patched
+    try:
+        return enc.forward(ids, lens)
+    finally:
+        del enc._issue
+
+
+@pytest.mark.parametrize("error", [RuntimeError, KeyboardInterrupt, _capi.ZenithError])
+def test_a_recording_that_fails_is_closed(cuda, params, error):
+    enc = Fp16Encoder(CFG, params, cuda)
+    ids, lens = tdev(rng(5).integers(0, CFG.vocab, (2, 40)), np.array([40, 17], np.int32), cuda)
+    want = enc.forward(ids, lens).clone()
+    enc.forward(ids, lens)
+
+    def fail():
+        raise error("zen_x", 2, "refused") if error is _capi.ZenithError else error("stopped")
+
+    enc.out.zero_()
+    if error is _capi.ZenithError:  # the library refused: the call runs as plain launches
+        assert torch.equal(third_call(enc, ids, lens, fail), want)
+    else:
+        with pytest.raises(error, match="stopped"):
+            third_call(enc, ids, lens, fail)
+    assert enc._pass_graph is None and not torch.cuda.is_current_stream_capturing()
+    for _ in range(4):
+        enc.out.zero_()
+        assert torch.equal(enc.forward(ids, lens), want)
+    enc.forward(ids[:1], lens[:1])
+    for _ in range(4):
+        assert torch.equal(enc.forward(ids, lens), want)
+    assert enc._pass_graph is not None  # another shape in between: recorded anew
+
+
+def other_threads_work():
+    """What another thread of a program does at any time: random numbers, allocations, pooled streams, synchronisation."""
+    torch.randn(8, device="cuda")
+    torch.empty(1 << 28, device="cuda")
+    filled = []
+    for i in range(64):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            filled.append((s, torch.full((64,), i, device="cuda")))
+    for i, (s, t) in enumerate(filled):
+        s.synchronize()
+        assert bool((t == i).all())
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("micro_batches", [1, 2])
+def test_recording_leaves_other_threads_alone(cuda, params, micro_batches):
+    enc = Fp16Encoder(CFG, params, cuda, micro_batches=micro_batches)
+    ids, lens = tdev(rng(6).integers(0, CFG.vocab, (3, 40)), np.array([40, 17, 9], np.int32), cuda)
+    want = enc.forward(ids, lens).clone()
+    enc.forward(ids, lens)
+    errors = []
+
+    def body():
+        try:
+            other_threads_work()
+        except BaseException as e:
+            errors.append(e)
+
+    def during():
+        t = threading.Thread(target=body)
+        t.start()
+        t.join()
+
+    enc.out.zero_()
+    assert torch.equal(third_call(enc, ids, lens, during), want)
+    assert not errors and enc._pass_graph is not None
+    enc.out.zero_()
+    assert torch.equal(enc.forward(ids, lens), want)
+    del enc  # the graph and its buffers go while it may still run
+    torch.cuda.synchronize()
+    assert _capi.device_status() == 0
 
 
 @pytest.mark.parametrize("B,S,launches", [(1, 48, 5), (1, 49, 4), (112, 6, 5), (112, 16, 4), (150, 8, 5)])

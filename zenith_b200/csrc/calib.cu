@@ -118,9 +118,8 @@ static int run_minmax(const T* x, int64_t n, float* minmax, void* workspace, siz
   const int cap = min(MM_MAX_CTAS, num_sms() * 4);
   const int ctas = int(want < 1 ? 1 : (want > cap ? cap : want));
   float2* partial = static_cast<float2*>(workspace);
-  minmax_partial_kernel<T><<<ctas, MM_THREADS, 0, s>>>(x, n, partial);
-  minmax_merge_kernel<<<1, MM_THREADS, 0, s>>>(partial, ctas, minmax);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  if (int st = launch_kernel(minmax_partial_kernel<T>, LaunchShape{dim3(unsigned(ctas)), dim3(MM_THREADS)}, s, x, n, partial); st != ZEN_OK) return st;
+  return launch_kernel(minmax_merge_kernel, LaunchShape{dim3(1), dim3(MM_THREADS)}, s, partial, ctas, minmax);
 }
 
 // one warp per row: absmax over the row's columns
@@ -218,8 +217,8 @@ static int run_histogram(const T* x, int64_t n, const float* minmax, int bins, l
   const int cap = num_sms() * 4;
   const int ctas = int(want < 1 ? 1 : (want > cap ? cap : want));
   const size_t smem = size_t(2 * bins + 1) * 4;
-  histogram_kernel<T><<<ctas, HIST_THREADS, smem, s>>>(x, n, minmax, bins, reinterpret_cast<unsigned long long*>(hist));
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(histogram_kernel<T>, LaunchShape{dim3(unsigned(ctas)), dim3(HIST_THREADS), smem}, s, x, n, minmax, bins,
+                       reinterpret_cast<unsigned long long*>(hist));
 }
 
 }  // namespace zen
@@ -248,8 +247,8 @@ extern "C" int zen_absmax_rows_f32(const float* w, int rows, int cols, int64_t l
   if (rows < 0 || cols < 0 || ld < cols) return ZEN_ERR_INVALID_ARG;
   if (rows == 0) return ZEN_OK;
   if (!w || !out) return ZEN_ERR_INVALID_ARG;
-  absmax_rows_kernel<<<(rows + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(w, rows, cols, ld, out);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(absmax_rows_kernel, LaunchShape{dim3(unsigned((rows + 7) / 8)), dim3(256)}, static_cast<cudaStream_t>(stream), w, rows, cols, ld,
+                       out);
 }
 
 extern "C" int zen_quantize_rows_f32(const float* w, const float* scale, int rows, int cols, int64_t ldw, int8_t* q, int64_t ldq,
@@ -260,6 +259,6 @@ extern "C" int zen_quantize_rows_f32(const float* w, const float* scale, int row
   if (!w || !scale || !q) return ZEN_ERR_INVALID_ARG;
   if (rows > 65535) return ZEN_ERR_UNSUPPORTED;
   dim3 grid(min((cols + 255) / 256, 64), rows);
-  quantize_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(w, scale, rows, cols, ldw, q, ldq, round_mode);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(quantize_rows_kernel, LaunchShape{grid, dim3(256)}, static_cast<cudaStream_t>(stream), w, scale, rows, cols, ldw, q, ldq,
+                       round_mode);
 }

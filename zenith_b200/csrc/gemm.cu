@@ -90,25 +90,8 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   const int tiles = p.tiles_m * p.tiles_n;
   const int resident = max_resident_pairs(reinterpret_cast<const void*>(kernel), smem);
   const int pairs = tiles < resident ? tiles : resident;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(2 * pairs));
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (pdl_mask() & PDL_GEMM) ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, ta, tb, tc, p) != cudaSuccess) {
-    cudaGetLastError();
-    return ZEN_ERR_LAUNCH;
-  }
-  return ZEN_OK;
+  return launch_kernel(kernel, LaunchShape{dim3(unsigned(2 * pairs)), dim3(GEMM_THREADS), smem, (pdl_mask() & PDL_GEMM) != 0, 2}, stream,
+                       ta, tb, tc, p);
 }
 
 template <int KIND>
@@ -229,8 +212,7 @@ __global__ void __launch_bounds__(256) transpose_f32_kernel(const float* __restr
 static int launch_transpose_f32(const float* in, float* out, int rows, int cols, cudaStream_t s) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32);
   if (grid.y > 65535) return ZEN_ERR_UNSUPPORTED;
-  transpose_f32_kernel<<<grid, 256, 0, s>>>(in, out, rows, cols);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(transpose_f32_kernel, LaunchShape{grid, dim3(256)}, s, in, out, rows, cols);
 }
 
 // int8 or fp16 operands, B K-major: the small-product kernel, CTA pairs or the one-CTA kernel by shape (or by `flags`).

@@ -590,25 +590,8 @@ static int launch_gemm_ln(const CUtensorMap& ta, const CUtensorMap& tb, const CU
   if (int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); st != ZEN_OK) return st;
   int clusters = num_sms() / LN_CLUSTER;
   if (clusters > p.tiles_m) clusters = p.tiles_m;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(clusters * LN_CLUSTER);
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = LN_CLUSTER;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (pdl_mask() & PDL_GEMM) ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, ta, tb, ty, tq, tr, p) != cudaSuccess) {
-    cudaGetLastError();
-    return ZEN_ERR_LAUNCH;
-  }
-  return ZEN_OK;
+  return launch_kernel(kernel, LaunchShape{dim3(unsigned(clusters * LN_CLUSTER)), dim3(GEMM_THREADS), smem, (pdl_mask() & PDL_GEMM) != 0, LN_CLUSTER},
+                       stream, ta, tb, ty, tq, tr, p);
 }
 
 }  // namespace zen

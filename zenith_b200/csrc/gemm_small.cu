@@ -11,25 +11,8 @@ static int launch_ks(const CUtensorMap& ta, const CUtensorMap& tb, const GemmSma
   auto kernel = gemm_small_kernel<KIND, BN, KS, B_MN>;
   constexpr size_t smem = gs_smem_bytes<BN, KS>();
   if (int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); st != ZEN_OK) return st;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned((sp.g.N + BN - 1) / BN * KS), unsigned((sp.g.M + GEMM_BM - 1) / GEMM_BM));
-  cfg.blockDim = dim3(GS_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = KS;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = KS > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, ta, tb, sp) != cudaSuccess) {
-    cudaGetLastError();
-    return ZEN_ERR_LAUNCH;
-  }
-  return ZEN_OK;
+  const dim3 grid(unsigned((sp.g.N + BN - 1) / BN * KS), unsigned((sp.g.M + GEMM_BM - 1) / GEMM_BM));
+  return launch_kernel(kernel, LaunchShape{grid, dim3(GS_THREADS), smem, (pdl_mask() & PDL_GEMM) != 0, KS}, stream, ta, tb, sp);
 }
 
 template <int KIND, bool B_MN>

@@ -368,9 +368,8 @@ static int launch_ln(const RowParams& p, cudaStream_t s) {
       default: return launch_pdl(PDL_ROW, ln_warp_kernel<T, 8, SRC>, dim3(grid), dim3(ROW_WARPS * 32), 0, s, p);
     }
   } else {
-    ln_block_kernel<T, SRC><<<p.rows, 256, 0, s>>>(p);
+    return launch_kernel(ln_block_kernel<T, SRC>, LaunchShape{dim3(unsigned(p.rows)), dim3(256)}, s, p);
   }
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -488,9 +487,7 @@ static int launch_ew(const EwParams& p, cudaStream_t s) {
   const int64_t cap = int64_t(num_sms()) * 8;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  if (aligned) ew_kernel<OP, TI, TO, VEC><<<int(blocks), 256, 0, s>>>(p);
-  else ew_kernel<OP, TI, TO, 1><<<int(blocks), 256, 0, s>>>(p);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(aligned ? ew_kernel<OP, TI, TO, VEC> : ew_kernel<OP, TI, TO, 1>, LaunchShape{dim3(unsigned(blocks)), dim3(256)}, s, p);
 }
 
 template <typename TI>
@@ -501,8 +498,7 @@ static int launch_quantize(const EwParams& p, cudaStream_t s) {
   int64_t blocks = (p.n / 16 + 255) / 256;
   const int64_t cap = int64_t(num_sms()) * 8;
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
-  quantize_kernel<TI><<<int(blocks), 256, 0, s>>>(p);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(quantize_kernel<TI>, LaunchShape{dim3(unsigned(blocks)), dim3(256)}, s, p);
 }
 
 // Three fp32 tensors of n values to fp16, back to back in y (the operands of the fp32 attention binding): one launch.
@@ -670,10 +666,8 @@ __attribute__((visibility("hidden"))) int zen_convert3_f32_to_f16(const float* a
   int64_t blocks = ((vec ? n / 8 : n) + 255) / 256;
   const int64_t cap = int64_t(num_sms()) * 3;
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
-  const dim3 grid(unsigned(blocks), 3);
-  if (vec) convert3_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
-  else convert3_kernel<false><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, c, static_cast<__half*>(y), n);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(vec ? convert3_kernel<true> : convert3_kernel<false>, LaunchShape{dim3(unsigned(blocks), 3), dim3(256)},
+                       static_cast<cudaStream_t>(stream), a, b, c, static_cast<__half*>(y), n);
 }
 int zen_convert_f16_to_f32(const void* x, float* y, int64_t n, void* stream) {
   if (n < 0 || (n > 0 && (!x || !y))) return ZEN_ERR_INVALID_ARG;
@@ -745,9 +739,8 @@ int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S,
   const int64_t total = int64_t(B) * S + B;
   if (total >= (int64_t(1) << 31)) return ZEN_ERR_UNSUPPORTED;
   const int64_t blocks = (total + 255) / 256;
-  set_inputs_kernel<<<unsigned(blocks < 4 * num_sms() ? blocks : 4 * num_sms()), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      ids, kv_lens, B * S, B, S, inputs);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  const unsigned grid = unsigned(blocks < 4 * num_sms() ? blocks : 4 * num_sms());
+  return launch_kernel(set_inputs_kernel, LaunchShape{dim3(grid), dim3(256)}, static_cast<cudaStream_t>(stream), ids, kv_lens, B * S, B, S, inputs);
 }
 
 int zen_pack_tokens_i32(const int32_t* ids, const int32_t* type_ids, const int32_t* kv_lens, int B, int S, int capacity,
@@ -756,9 +749,8 @@ int zen_pack_tokens_i32(const int32_t* ids, const int32_t* type_ids, const int32
   if (B == 0) return ZEN_OK;
   if (!ids || !kv_lens || !cu_seqlens || !ids_packed || !pos_packed) return ZEN_ERR_INVALID_ARG;
   if (int64_t(B) * S >= (int64_t(1) << 31) || B > 65535) return ZEN_ERR_UNSUPPORTED;
-  pack_tokens_kernel<<<B + 1, 128, 0, static_cast<cudaStream_t>(stream)>>>(ids, type_ids, kv_lens, B, S, capacity, cu_seqlens,
-                                                                            ids_packed, pos_packed, type_packed);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return launch_kernel(pack_tokens_kernel, LaunchShape{dim3(unsigned(B + 1)), dim3(128)}, static_cast<cudaStream_t>(stream), ids, type_ids, kv_lens, B,
+                       S, capacity, cu_seqlens, ids_packed, pos_packed, type_packed);
 }
 
 int zen_unpad_rows_f16(const void* packed, const int32_t* cu_seqlens, int B, int S, int hidden, int capacity, void* padded,

@@ -8,6 +8,7 @@
 // usable.  The host then finds ZEN_ERR_TIMEOUT with zen_device_status_read and resets it with
 // zen_device_status_clear — the path a timed-out production kernel would take.
 #define ZEN_WAIT_LIMIT_NS 1000000ull
+#include "launch.cuh"
 #include "zen_common.cuh"
 
 namespace zen {
@@ -45,6 +46,5 @@ __global__ void __launch_bounds__(64) wait_limit_kernel(unsigned long long* out)
 ZEN_DEFINE_TU_STATUS(selftest)
 
 extern "C" int zen_selftest_wait_limit(unsigned long long* result3, void* stream) {
-  zen::wait_limit_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(result3);
-  return cudaGetLastError() == cudaSuccess ? ZEN_OK : ZEN_ERR_LAUNCH;
+  return zen::launch_kernel(zen::wait_limit_kernel, zen::LaunchShape{dim3(1), dim3(64)}, static_cast<cudaStream_t>(stream), result3);
 }

@@ -1,4 +1,5 @@
 // Device status word: folds the per-translation-unit words together for the host.
+#include "launch.cuh"
 #include "zen_common.cuh"
 
 extern "C" {
@@ -42,6 +43,7 @@ extern "C" int zen_device_status_clear(void) { return fold_status(nullptr, 1); }
 extern "C" int zen_memcpy_async(void* dst, const void* src, size_t bytes, void* stream) {
   if (bytes == 0) return ZEN_OK;
   if (!dst || !src) return ZEN_ERR_INVALID_ARG;
+  if (zen::recording()) return ZEN_ERR_UNSUPPORTED;
   if (cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
     cudaGetLastError();
     return ZEN_ERR_LAUNCH;

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <set>
 #include "../../include/zenith_b200.h"
+#include "launch.cuh"
 #include "zen_common.cuh"
 
 namespace zen {
@@ -77,21 +78,7 @@ constexpr int pdl_mask() { return ZEN_PDL_FAMILIES; }
 template <typename... KArgs, typename... Args>
 inline int launch_pdl(int family, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                       Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (pdl_mask() & family) ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...) != cudaSuccess) {
-    cudaGetLastError();
-    return ZEN_ERR_LAUNCH;
-  }
-  return ZEN_OK;
+  return launch_kernel(kernel, LaunchShape{grid, block, smem, (pdl_mask() & family) != 0}, stream, std::forward<Args>(args)...);
 }
 
 // Opt a kernel in to more than 48 KB of dynamic shared memory, once per (kernel, device).

@@ -20,6 +20,7 @@ With hidden size 768 the two "GEMM, +residual, LayerNorm" pairs each run as ONE 
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass
 
@@ -94,6 +95,20 @@ def _dev(a, dtype, device):
     return torch.from_numpy(np.ascontiguousarray(a)).to(device=device, dtype=dtype)
 
 
+class _RecordedPass:
+    """An executable graph of a pass; reads and writes the buffers of the encoder that recorded it."""
+
+    def __init__(self, handle: int):
+        self._handle = handle
+        self._destroy = _capi.lib().zen_graph_destroy
+
+    def launch(self, stream: int) -> None:
+        _capi.check("zen_graph_launch", _capi.lib().zen_graph_launch(self._handle, stream))
+
+    def __del__(self):
+        self._destroy(self._handle)
+
+
 class _EncoderBase:
     """Shared plumbing: embedding tables, per-shape buffers, the launch list, CUDA-graph capture."""
 
@@ -135,7 +150,7 @@ class _EncoderBase:
         self._shape = (B, S, packed_rows)
         self._packed_rows = packed_rows
         self._graph = None
-        self._pass_graph = None  # graph of the plain call, recorded once a shape has come a third time
+        self._pass_graph = None  # graph of the plain call, recorded at a shape's third consecutive call
         self._plain_calls = 0
         d = self.device
         # token ids and key lengths share one allocation, so that a host can feed both with one copy
@@ -199,29 +214,40 @@ class _EncoderBase:
         ops.launch_count += len(self._launches)
 
     def _run_plain(self) -> None:
-        """One pass for ``forward`` / ``forward_unpadded``.  Issuing 49 and more launches one by one costs the host 340 us,
-        more than a short batch takes on the device (BERT-base W8A8, one 24-token sequence: 300 us), so from the third call
-        for a shape on the pass is one graph of the same launches (recorded without running anything or waiting for the
-        device).  Inside a caller's own stream capture the launches are issued as they are."""
+        """One pass for ``forward`` / ``forward_unpadded``.  Issuing 49 and more calls one by one costs the host 340 us,
+        more than a short batch takes on the device (BERT-base W8A8, one 24-token sequence: 300 us), so from the third
+        consecutive call for a shape on the pass is one graph of the same launches.  That third call also pays for the
+        recording.  Inside a caller's own stream capture the launches are issued as they are."""
         if torch.cuda.is_current_stream_capturing():
             self._run()
             return
         if self._pass_graph is None:
             self._plain_calls += 1
-            if self._plain_calls < 3:
-                self._run()
-                return
-            side = torch.cuda.Stream(device=self.device)
-            side.wait_stream(torch.cuda.current_stream())
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.stream(side):
-                graph.capture_begin(capture_error_mode="thread_local")
-                self._run()
-                graph.capture_end()
-            ops.launch_count -= len(self._launches)  # recorded, not launched
-            self._pass_graph = graph
-        self._pass_graph.replay()
+            if self._plain_calls == 3:
+                self._pass_graph = self._record()
+        if self._pass_graph is None:
+            self._run()
+            return
+        self._pass_graph.launch(torch.cuda.current_stream().cuda_stream)
         ops.launch_count += len(self._launches)
+
+    def _record(self) -> "_RecordedPass | None":
+        """The pass as a graph; None where a launch refuses to be recorded (issued as it is, it then says why)."""
+        lib = _capi.lib()
+        _capi.check("zen_record_begin", lib.zen_record_begin())
+        graph = ctypes.c_void_p()
+        keep = None
+        try:
+            for i, launches in enumerate(self._micro):
+                if i:
+                    _capi.check("zen_record_branch", lib.zen_record_branch())
+                self._issue(launches, None)
+            keep = ctypes.byref(graph)
+        except _capi.ZenithError:
+            pass
+        finally:
+            status = lib.zen_record_end(keep)
+        return _RecordedPass(graph.value) if keep is not None and status == _capi.OK else None
 
     # -- public ------------------------------------------------------------------------------
     def set_inputs(self, ids, kv_lens=None) -> None:
