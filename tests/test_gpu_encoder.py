@@ -357,6 +357,22 @@ def test_recording_leaves_other_threads_alone(cuda, params, micro_batches):
     assert _capi.device_status() == 0
 
 
+@pytest.mark.parametrize("B,S,packed,workspace", [(1, 24, None, True), (16, 128, None, False), (3, 60, 128, True), (20, 100, 1920, False)])
+def test_a_new_shape_prepares_only_what_its_pass_uses(cuda, monkeypatch, B, S, packed, workspace):
+    """Kernel choices once per GEMM and not once per layer, LayerNorm scratch only where a choice is two launches, zeros only
+    where rows of no sequence exist."""
+    cfg = EncoderConfig(layers=3, hidden=768, heads=12, ffn=896, vocab=500, max_pos=128)
+    enc = Fp16Encoder(cfg, init_params(cfg, 3), cuda)
+    plans, zeros = [], []
+    plan, make = _capi.lib().zen_gemm_plan, torch.zeros
+    monkeypatch.setattr(_capi.lib(), "zen_gemm_plan", lambda *a: plans.append(a) or plan(*a))
+    monkeypatch.setattr(torch, "zeros", lambda *a, **k: zeros.append(a[0]) or make(*a, **k))
+    enc._prepare(B, S, packed)
+    assert len(plans) == len(set(plans)) and len(plans) <= 6
+    assert (enc.ln_ws is not None) == workspace
+    assert ((packed or B * S, 768) in zeros) == (packed is not None)
+
+
 @pytest.mark.parametrize("B,S,launches", [(1, 48, 5), (1, 49, 4), (112, 6, 5), (112, 16, 4), (150, 8, 5)])
 def test_int8_encoder_attention_form_by_size(cuda, params, B, S, launches):
     """Few rows, or many rounds of mostly empty tiles: projection and attention as two launches, with the same bits."""

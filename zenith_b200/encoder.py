@@ -163,7 +163,8 @@ class _EncoderBase:
             self.cu_seqlens = torch.zeros(B + 1, dtype=torch.int32, device=d)
             self.ids_packed = torch.zeros(packed_rows, dtype=torch.int32, device=d)
             self.pos_packed = torch.zeros(packed_rows, dtype=torch.int32, device=d)
-        self._alloc(B, S)
+        self._plan_gemms()
+        self._alloc(self._packed_rows or B * S)
         # Sequences are independent through the whole encoder, so the batch may be cut into micro-batches
         # whose launch sequences run side by side (separate streams / graph branches): the fill and
         # drain latency of one micro-batch's kernels then hides behind the other's work.  Every
@@ -179,14 +180,49 @@ class _EncoderBase:
         self.launches_per_forward = len(self._launches)
         self._streams = [torch.cuda.Stream(device=d) for _ in range(len(self._micro) - 1)]
 
-    def _plan(self, elem_bytes: int, N: int, K: int, layernorm: bool = False) -> int:
-        """Kernel-choice flags of a GEMM of this pass, chosen for the rows of the whole padded batch: the packed form and
-        micro-batches then run every row on the same kernels and keep its bits."""
-        return _capi.lib().zen_gemm_plan(elem_bytes, self._shape[0] * self._shape[1], N, K, int(layernorm))
+    def _plan_gemms(self) -> None:
+        """Kernel-choice flags of the pass's GEMMs (every layer's are the same), chosen for the rows of the whole padded
+        batch: the packed form and micro-batches then run every row on the same kernels and keep its bits."""
+        H, F = self.cfg.hidden, self.cfg.ffn
+        plan = lambda n, k, layernorm: _capi.lib().zen_gemm_plan(self.ELEM_BYTES, self._shape[0] * self._shape[1], n, k, layernorm)
+        forced = self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR)
+        self._gemm = {(n, k): self.gemm_flags | (0 if forced else plan(n, k, 0)) for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
+        # the weights of an encoder are written once, in __init__: every GEMM of the launch list carries the
+        # constant-weights promise for its own call (nothing process-wide is switched)
+        self._gemm_ln = {(n, k): GEMM_CONST_WEIGHTS | plan(n, k, 1) for n, k in ((H, H), (H, F))} if self.fuse_layernorm else {}
 
-    def _workspace(self, T: int) -> torch.Tensor:
-        """fp32 rows of a projection on its way to a LayerNorm (scratch of one launch pair)."""
-        return torch.empty((T, self.cfg.hidden), dtype=torch.float32, device=self.device)
+    @staticmethod
+    def _two_launches(flags: int) -> bool:
+        """Whether a projection + LayerNorm with these flags is two launches (with fp32 rows in a workspace between them)."""
+        return flags & _capi.gemm_split_k(15) != _capi.gemm_split_k(15)
+
+    def _alloc_shared(self, T: int) -> None:
+        """The buffers that both encoders have beside their own."""
+        H = self.cfg.hidden
+        f16 = dict(dtype=torch.float16, device=self.device)
+        if self._packed_rows is not None:
+            self.out_padded = torch.empty((self._shape[0] * self._shape[1], H), **f16)
+        self.x = [torch.empty((T, H), **f16) for _ in range(2)]
+        self.qkv = torch.empty((T, 3 * H), **f16)
+        self.ctx = self._attention_rows(T, torch.float16)
+        self.ao, self.h1, self.o = (torch.empty((T, H), **f16) for _ in range(3))
+        self.ln_ws = None  # scratch of one launch pair
+        if any(map(self._two_launches, self._gemm_ln.values())):
+            self.ln_ws = torch.empty((T, H), dtype=torch.float32, device=self.device)
+        self.out = self.x[len(self.layers) & 1]
+
+    def _attention_rows(self, T: int, dtype) -> torch.Tensor:
+        """An attention result.  Rows of no sequence (beyond a packed batch's total) are never written: zeros, so that
+        nothing non-finite can reach the values of the last sequence's key tile."""
+        make = torch.empty if self._packed_rows is None else torch.zeros
+        return make((T, self.cfg.hidden), dtype=dtype, device=self.device)
+
+    def _ln_args(self, K: int, row0: int, rows: int) -> tuple:
+        """(workspace, its bytes, flags) of a projection + LayerNorm of ``rows`` rows from ``row0`` on."""
+        flags = self._gemm_ln[self.cfg.hidden, K]
+        if not self._two_launches(flags):
+            return None, 0, flags
+        return _row_ptr(self.ln_ws, row0), rows * self.cfg.hidden * 4, flags
 
     def _add(self, fn: str, *args) -> None:
         self._launches.append((getattr(_capi.lib(), fn), fn, args))
@@ -374,6 +410,8 @@ class _EncoderBase:
 class Fp16Encoder(_EncoderBase):
     """fp16 weights and activations, fp32 accumulation and statistics."""
 
+    ELEM_BYTES = 2  # of a GEMM operand
+
     def __init__(self, cfg: EncoderConfig, params: dict, device="cuda:0", micro_batches: int = 1,
                  fuse_layernorm: bool | None = None, gemm_pair: bool | None = None):
         """``fuse_layernorm``: attention-output and FFN2 as one GEMM + residual + LayerNorm kernel each (5 launches
@@ -392,23 +430,9 @@ class Fp16Encoder(_EncoderBase):
             self.layers.append(L)
         self.taps: dict | None = None  # filled by forward_with_taps
 
-    def _alloc(self, B: int, S: int) -> None:
-        cfg, d = self.cfg, self.device
-        T, H, F = self._packed_rows or B * S, cfg.hidden, cfg.ffn
-        f16 = dict(dtype=torch.float16, device=d)
-        if self._packed_rows is not None:
-            self.out_padded = torch.empty((B * S, H), **f16)
-        self.x = [torch.empty((T, H), **f16) for _ in range(2)]
-        self.qkv = torch.empty((T, 3 * H), **f16)
-        # rows of no sequence (beyond a packed batch's total) are never written: zeros, so that nothing non-finite can reach
-        # the values of the last sequence's key tile
-        self.ctx = torch.zeros((T, H), **f16)
-        self.ao = torch.empty((T, H), **f16)
-        self.h1 = torch.empty((T, H), **f16)
-        self.g = torch.empty((T, F), **f16)
-        self.o = torch.empty((T, H), **f16)
-        self.ln_ws = self._workspace(T) if self.fuse_layernorm else None
-        self.out = self.x[len(self.layers) & 1]
+    def _alloc(self, T: int) -> None:
+        self._alloc_shared(T)
+        self.g = torch.empty((T, self.cfg.ffn), dtype=torch.float16, device=self.device)
 
     def _build(self, b0: int, B: int, S: int) -> None:
         """Launch list for sequences [b0, b0 + B) of the batch (rows b0*S .. of every buffer)."""
@@ -417,15 +441,10 @@ class Fp16Encoder(_EncoderBase):
         T, H, F, nh, hd = self._packed_rows or B * S, cfg.hidden, cfg.ffn, cfg.heads, cfg.head_dim
         r0 = b0 * S
         P = lambda t: _row_ptr(t, r0)
-        # the weights of this object are written once, in __init__: every GEMM of the launch list carries the
-        # constant-weights promise for its own call (nothing process-wide is switched)
-        CW = GEMM_CONST_WEIGHTS
-        # the plain GEMMs also carry the kernel choice
-        GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(2, n, k))
-              for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
+        GF = self._gemm
         fused_ln = self.fuse_layernorm
         self.launches_per_layer = 5 if fused_ln else 7
-        ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
+        ln_o, ln_2 = (self._ln_args(k, r0, T) for k in (H, F)) if fused_ln else (None, None)
         self.lead_launches = 2 if packed else 1
         if packed:
             self._add("zen_pack_tokens_i32", self.ids.data_ptr(), None, self.kv_lens.data_ptr(), B, S, T,
@@ -455,7 +474,7 @@ class Fp16Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_f16_add_layernorm_ws", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H,
                           L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(), cfg.eps, P(self.h1),
-                          None, 1.0, ROUND_NEAREST_EVEN, *ws, CW | self._plan(2, H, H, True))
+                          None, 1.0, ROUND_NEAREST_EVEN, *ln_o)
             else:
                 self._add("zen_linear_f16_ex", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H, L["bo"].data_ptr(),
                           ACT_NONE, DT_F16, P(self.ao), H, GF[H, H])
@@ -466,7 +485,7 @@ class Fp16Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_f16_add_layernorm_ws", P(self.g), F, L["w2"].data_ptr(), F, T, H, F,
                           L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(), L["ln2_b"].data_ptr(), cfg.eps, P(xn),
-                          None, 1.0, ROUND_NEAREST_EVEN, *ws, CW | self._plan(2, H, F, True))
+                          None, 1.0, ROUND_NEAREST_EVEN, *ln_2)
             else:
                 self._add("zen_linear_f16_ex", P(self.g), F, L["w2"].data_ptr(), F, T, H, F, L["b2"].data_ptr(),
                           ACT_NONE, DT_F16, P(self.o), H, GF[H, F])
@@ -548,6 +567,7 @@ class Int8Scales:
 class Int8Encoder(_EncoderBase):
     """W8A8 encoder: int8 GEMM operands, int32 accumulation, fp16 residual stream / LayerNorm / softmax."""
 
+    ELEM_BYTES = 1  # of a GEMM operand
 
     def __init__(self, cfg: EncoderConfig, params: dict, scales: Int8Scales, device="cuda:0", micro_batches: int = 1,
                  fuse_layernorm: bool | None = None, prefetch_weights: bool = True, gemm_pair: bool | None = None,
@@ -583,27 +603,13 @@ class Int8Encoder(_EncoderBase):
             L.update({k: _dev(lp[k], torch.float16, d) for k in ("ln1_g", "ln1_b", "ln2_g", "ln2_b")})
             self.layers.append(L)
 
-    def _alloc(self, B: int, S: int) -> None:
-        cfg, d = self.cfg, self.device
-        T, H, F = self._packed_rows or B * S, cfg.hidden, cfg.ffn
-        f16 = dict(dtype=torch.float16, device=d)
-        s8 = dict(dtype=torch.int8, device=d)
-        if self._packed_rows is not None:
-            self.out_padded = torch.empty((B * S, H), **f16)
-        self.x = [torch.empty((T, H), **f16) for _ in range(2)]
+    def _alloc(self, T: int) -> None:
+        self._alloc_shared(T)
+        H, s8 = self.cfg.hidden, dict(dtype=torch.int8, device=self.device)
         self.xq = [torch.empty((T, H), **s8) for _ in range(2)]
-        self.qkv = torch.empty((T, 3 * H), **f16)
-        # rows of no sequence (beyond a packed batch's total) are never written: zeros, so that nothing non-finite can reach
-        # the values of the last sequence's key tile
-        self.ctx = torch.zeros((T, H), **f16)
-        self.ctxq = torch.zeros((T, H), **s8)
-        self.ao = torch.empty((T, H), **f16)
-        self.h1 = torch.empty((T, H), **f16)
+        self.ctxq = self._attention_rows(T, torch.int8)
         self.h1q = torch.empty((T, H), **s8)
-        self.gq = torch.empty((T, F), **s8)
-        self.o = torch.empty((T, H), **f16)
-        self.ln_ws = self._workspace(T) if self.fuse_layernorm else None
-        self.out = self.x[len(self.layers) & 1]
+        self.gq = torch.empty((T, self.cfg.ffn), **s8)
 
     def _build(self, b0: int, B: int, S: int) -> None:
         """Launch list for sequences [b0, b0 + B) of the batch (rows b0*S .. of every buffer)."""
@@ -612,14 +618,9 @@ class Int8Encoder(_EncoderBase):
         T, H, F, nh, hd = self._packed_rows or B * S, cfg.hidden, cfg.ffn, cfg.heads, cfg.head_dim
         r0 = b0 * S
         P = lambda t: _row_ptr(t, r0)
-        # the weights of this object are written once, in __init__: every GEMM of the launch list carries the
-        # constant-weights promise for its own call (nothing process-wide is switched)
-        CW = GEMM_CONST_WEIGHTS
-        # the plain GEMMs also carry the kernel choice
-        GF = {(n, k): self.gemm_flags | (0 if self.gemm_flags & (GEMM_PAIR | GEMM_NO_PAIR) else self._plan(1, n, k))
-              for n, k in ((3 * H, H), (H, H), (F, H), (H, F))}
+        GF = self._gemm
         fused_ln = self.fuse_layernorm
-        ws = (P(self.ln_ws), T * H * 4) if fused_ln else None
+        ln_o, ln_2 = (self._ln_args(k, r0, T) for k in (H, F)) if fused_ln else (None, None)
         sc = self.act_scales
         can_fuse = S <= 128 and hd == 64
         if self.fuse_attention and not can_fuse:
@@ -662,11 +663,11 @@ class Int8Encoder(_EncoderBase):
                 self._add("zen_qkv_attention_unpadded_i8", P(xq), H, L["wqkv"].data_ptr(), H, B, T,
                           self.cu_seqlens.data_ptr(), nh, H, a["x"], L["wqkv_s"].data_ptr(), L["bqkv"].data_ptr(),
                           1.0 / math.sqrt(hd), P(self.ctx), P(self.ctxq), a["ctx"], P(self.qkv) if self.keep_qkv else None,
-                          *pf(L["wo"], L["w1"]), CW)
+                          *pf(L["wo"], L["w1"]), GEMM_CONST_WEIGHTS)
             elif fused_attn:
                 self._add("zen_qkv_attention_i8", P(xq), H, L["wqkv"].data_ptr(), H, B, S, nh, H, a["x"],
                           L["wqkv_s"].data_ptr(), L["bqkv"].data_ptr(), kv, 1.0 / math.sqrt(hd), P(self.ctx), P(self.ctxq),
-                          a["ctx"], P(self.qkv) if self.keep_qkv else None, *pf(L["wo"], L["w1"]), CW)
+                          a["ctx"], P(self.qkv) if self.keep_qkv else None, *pf(L["wo"], L["w1"]), GEMM_CONST_WEIGHTS)
             else:
                 self._add("zen_linear_i8_ex", P(xq), H, L["wqkv"].data_ptr(), H, T, 3 * H, H, a["x"],
                           L["wqkv_s"].data_ptr(), L["bqkv"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
@@ -676,7 +677,7 @@ class Int8Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_i8_add_layernorm_ws", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(),
-                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, *ws, CW | self._plan(1, H, H, True))
+                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, *ln_o)
             else:
                 self._add("zen_linear_i8_ex", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
@@ -690,7 +691,7 @@ class Int8Encoder(_EncoderBase):
                 self._add("zen_linear_i8_add_layernorm_ws", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(),
                           L["ln2_b"].data_ptr(), cfg.eps, P(xn), None if last else P(xqn),
-                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, *ws, CW | self._plan(1, H, F, True))
+                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, *ln_2)
             else:
                 self._add("zen_linear_i8_ex", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
