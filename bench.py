@@ -388,7 +388,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
         enc.replay()
     us = _event_us(torch, enc.replay, 15, flush)
     out["bert_base_fp16_seq128"] = {"sequences_per_s": round(BATCH / us * 1e6, 1), "ms_per_step": round(us / 1e3, 4),
-                                    "launches": enc.launches_per_forward, "workload": "BASELINE.json configs[1]"}
+                                    "launches": enc.kernels_per_forward, "workload": "BASELINE.json configs[1]"}
     del enc
     done("fp16 encoder")
     # attention forward sweep, B = 8, H = 16
@@ -479,7 +479,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
         enc.replay()
     us = _event_us(torch, enc.replay, 9, flush)
     out["bert_large_int8_seq384_shard32"] = {"ms_per_step": round(us / 1e3, 3), "sequences_per_s": round(32 / us * 1e6, 1),
-                                             "launches": enc.launches_per_forward,
+                                             "launches": enc.kernels_per_forward,
                                              "workload": "BASELINE.json configs[4], the 32-sequence shard one of 8 GPUs holds"}
     try:  # the same shard unpadded (projection GEMM on the packed rows, attention from the offsets)
         enc.capture_unpadded(32, LARGE_SEQ, Int8Encoder.unpadded_capacity(lens.tolist(), LARGE_SEQ))
@@ -511,7 +511,7 @@ def unpadded_metric(torch, cfg, params, scales, ids_np, lens_np, dev, flush, pad
     same = bool(torch.equal(out[rows], padded_out[rows]))
     us = _event_us(torch, enc.replay, 15, flush)
     return {"sequences_per_s": round(B / us * 1e6, 1), "ms_per_step": round(us / 1e3, 4), "packed_rows": cap,
-            "padded_rows": B * S, "valid_tokens": int(lens_np.sum()), "launches": enc.launches_per_forward,
+            "padded_rows": B * S, "valid_tokens": int(lens_np.sum()), "launches": enc.kernels_per_forward,
             "valid_tokens_equal_padded_pass": same,
             "note": "not the headline: the reference computes the padding positions too; their hidden states are zeros here"}
 
@@ -704,7 +704,7 @@ def run_ours(args) -> None:
     launches = ops.launch_count - launches0
     timed_e2e(W)
     e2e_ms = timed_e2e(K)
-    e2e_launches = enc.launches_per_forward  # the copies to and from the host run on the copy engines
+    e2e_launches = enc.kernels_per_forward  # the copies to and from the host run on the copy engines
     clocks = sampler.stop() if sampler else None
     sus = sustained(args.sustain_seconds) if args.sustain_seconds > 0 else None
     gather_check = None
@@ -743,7 +743,7 @@ def run_ours(args) -> None:
                                                              ", hidden states pushed onto rank 0 by the copy engines over NVLink every step "
                                                              "(peer-to-peer copies, the push of step i under the kernels of step i + 1)"),
                    "l2": "256 MB buffer written between timed steps",
-                   "launch": f"CUDA-graph replay of {enc.launches_per_forward} kernels in {args.micro_batches} concurrent micro-batch(es)"},
+                   "launch": f"CUDA-graph replay of {enc.kernels_per_forward} kernels in {args.micro_batches} concurrent micro-batch(es)"},
         "e2e": {"value": e2e_value, "unit": "sequences/s", "ms_per_step": e2e_ms / K,
                 "h2d_bytes_per_step": int(ids_h.numel() * ids_h.element_size() + lens_h.numel() * lens_h.element_size()),
                 "d2h_bytes_per_step": int(pipe.host_out[0].numel() * 2),

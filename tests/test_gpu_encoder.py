@@ -14,7 +14,7 @@ import torch
 
 from oracle import encoder_ref as ER
 from oracle import oracle as O
-from zenith_b200 import _capi
+from zenith_b200 import _capi, ops
 from zenith_b200.calibrate import activation_scales_from_ranges, calibrate, quantize_weights
 from zenith_b200.encoder import EncoderConfig, Fp16Encoder, Int8Encoder, Int8Scales, init_params
 
@@ -371,6 +371,23 @@ def test_a_new_shape_prepares_only_what_its_pass_uses(cuda, monkeypatch, B, S, p
     assert len(plans) == len(set(plans)) and len(plans) <= 6
     assert (enc.ln_ws is not None) == workspace
     assert ((packed or B * S, 768) in zeros) == (packed is not None)
+
+
+@pytest.mark.parametrize("B,S,fused,calls,kernels", [(1, 24, True, 5, 7), (16, 128, True, 5, 5), (1, 24, False, 7, 7)])
+def test_launch_counts_count_kernels(cuda, B, S, fused, calls, kernels):
+    """A projection + LayerNorm of few rows is one call and two kernels; plain calls, recorded ones and replays count alike."""
+    cfg = EncoderConfig(layers=3, hidden=768, heads=12, ffn=896, vocab=500, max_pos=128)
+    enc = Fp16Encoder(cfg, init_params(cfg, 3), cuda, fuse_layernorm=fused)
+    ids, lens = tdev(rng(5).integers(0, cfg.vocab, (B, S)).astype(np.int32), np.full(B, S, np.int32), cuda)
+    for _ in range(4):
+        before = ops.launch_count
+        enc.forward(ids, lens)
+        assert ops.launch_count - before == 1 + enc.kernels_per_forward  # and the one that takes the inputs
+    assert enc.launches_per_forward == 1 + 3 * calls and enc.kernels_per_forward == 1 + 3 * kernels
+    enc.capture(B, S)
+    before = ops.launch_count
+    enc.replay()
+    assert ops.launch_count - before == enc.kernels_per_forward
 
 
 @pytest.mark.parametrize("B,S,launches", [(1, 48, 5), (1, 49, 4), (112, 6, 5), (112, 16, 4), (150, 8, 5)])

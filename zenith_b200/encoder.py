@@ -134,7 +134,8 @@ class _EncoderBase:
         self._graph = None
         self._pass_graph = None
         self._plain_calls = 0
-        self.launches_per_forward = 0
+        self.launches_per_forward = 0  # library calls of a pass
+        self.kernels_per_forward = 0   # kernels that they launch: two for a projection + LayerNorm in its two-launch form
 
     # -- per-shape state --------------------------------------------------------------------
     def _prepare(self, B: int, S: int, packed_rows: int | None = None) -> None:
@@ -178,6 +179,7 @@ class _EncoderBase:
             self._micro.append(self._launches)
         self._launches = [l for m in self._micro for l in m]
         self.launches_per_forward = len(self._launches)
+        self.kernels_per_forward = sum(k for *_, k in self._launches)
         self._streams = [torch.cuda.Stream(device=d) for _ in range(len(self._micro) - 1)]
 
     def _plan_gemms(self) -> None:
@@ -224,12 +226,12 @@ class _EncoderBase:
             return None, 0, flags
         return _row_ptr(self.ln_ws, row0), rows * self.cfg.hidden * 4, flags
 
-    def _add(self, fn: str, *args) -> None:
-        self._launches.append((getattr(_capi.lib(), fn), fn, args))
+    def _add(self, fn: str, *args, kernels: int = 1) -> None:
+        self._launches.append((getattr(_capi.lib(), fn), fn, args, kernels))
 
     @staticmethod
     def _issue(launches, stream) -> None:
-        for f, name, args in launches:
+        for f, name, args, _ in launches:
             st = f(*args, stream)
             if st != 0:
                 _capi.check(name, st)
@@ -247,7 +249,7 @@ class _EncoderBase:
                     self._issue(launches, s.cuda_stream)
             for s in self._streams:
                 main.wait_stream(s)
-        ops.launch_count += len(self._launches)
+        ops.launch_count += self.kernels_per_forward
 
     def _run_plain(self) -> None:
         """One pass for ``forward`` / ``forward_unpadded``.  Issuing 49 and more calls one by one costs the host 340 us,
@@ -265,7 +267,7 @@ class _EncoderBase:
             self._run()
             return
         self._pass_graph.launch(torch.cuda.current_stream().cuda_stream)
-        ops.launch_count += len(self._launches)
+        ops.launch_count += self.kernels_per_forward
 
     def _record(self) -> "_RecordedPass | None":
         """The pass as a graph; None where a launch refuses to be recorded (issued as it is, it then says why)."""
@@ -296,6 +298,7 @@ class _EncoderBase:
             _capi.check("zen_set_inputs_i32", _capi.lib().zen_set_inputs_i32(
                 ids.data_ptr(), None if kv_lens is None else kv_lens.data_ptr(), B, S, self.inputs.data_ptr(),
                 torch.cuda.current_stream().cuda_stream))
+            ops.launch_count += 1
             return
         self.ids.copy_(ids.reshape(-1), non_blocking=True)
         if kv_lens is not None:
@@ -383,7 +386,7 @@ class _EncoderBase:
                                 return a - lo + new
                     return a
 
-                self._micro = [[(f, name, tuple(move(a) for a in args)) for f, name, args in m] for m in base_micro]
+                self._micro = [[(f, name, tuple(move(a) for a in args), n) for f, name, args, n in m] for m in base_micro]
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
                 self._run()
@@ -403,7 +406,7 @@ class _EncoderBase:
         if self._graph is None:
             raise RuntimeError("capture() first")
         self._graphs[slot].replay()
-        ops.launch_count += len(self._launches)
+        ops.launch_count += self.kernels_per_forward
         return self._slot_results[slot]
 
 
@@ -474,7 +477,7 @@ class Fp16Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_f16_add_layernorm_ws", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H,
                           L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(), cfg.eps, P(self.h1),
-                          None, 1.0, ROUND_NEAREST_EVEN, *ln_o)
+                          None, 1.0, ROUND_NEAREST_EVEN, *ln_o, kernels=1 if ln_o[0] is None else 2)
             else:
                 self._add("zen_linear_f16_ex", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H, L["bo"].data_ptr(),
                           ACT_NONE, DT_F16, P(self.ao), H, GF[H, H])
@@ -485,7 +488,7 @@ class Fp16Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_f16_add_layernorm_ws", P(self.g), F, L["w2"].data_ptr(), F, T, H, F,
                           L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(), L["ln2_b"].data_ptr(), cfg.eps, P(xn),
-                          None, 1.0, ROUND_NEAREST_EVEN, *ln_2)
+                          None, 1.0, ROUND_NEAREST_EVEN, *ln_2, kernels=1 if ln_2[0] is None else 2)
             else:
                 self._add("zen_linear_f16_ex", P(self.g), F, L["w2"].data_ptr(), F, T, H, F, L["b2"].data_ptr(),
                           ACT_NONE, DT_F16, P(self.o), H, GF[H, F])
@@ -513,18 +516,16 @@ class Fp16Encoder(_EncoderBase):
             observers = self.make_observers()
         stream = torch.cuda.current_stream().cuda_stream
         per_layer = self.launches_per_layer
-        f, name, args = self._launches[0]
-        _capi.check(name, f(*args, stream))
+        self._issue(self._launches[:1], stream)
         cur = 0
         for li in range(len(self.layers)):
             observers["x"][li].observe(self.x[cur])
-            for f, name, args in self._launches[1 + li * per_layer: 1 + (li + 1) * per_layer]:
-                _capi.check(name, f(*args, stream))
+            self._issue(self._launches[1 + li * per_layer: 1 + (li + 1) * per_layer], stream)
             observers["ctx"][li].observe(self.ctx)
             observers["h1"][li].observe(self.h1)
             observers["gelu"][li].observe(self.g)
             cur ^= 1
-        ops.launch_count += len(self._launches)
+        ops.launch_count += self.kernels_per_forward
         if not own:
             return None
         return {p: [o.range() for o in v] for p, v in observers.items()}
@@ -677,7 +678,7 @@ class Int8Encoder(_EncoderBase):
             if fused_ln:
                 self._add("zen_linear_i8_add_layernorm_ws", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(),
-                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, *ln_o)
+                          cfg.eps, P(self.h1), P(self.h1q), a["h1"], ROUND_NEAREST_EVEN, *ln_o, kernels=1 if ln_o[0] is None else 2)
             else:
                 self._add("zen_linear_i8_ex", P(self.ctxq), H, L["wo"].data_ptr(), H, T, H, H, a["ctx"],
                           L["wo_s"].data_ptr(), L["bo"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
@@ -691,7 +692,7 @@ class Int8Encoder(_EncoderBase):
                 self._add("zen_linear_i8_add_layernorm_ws", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), P(self.h1), H, L["ln2_g"].data_ptr(),
                           L["ln2_b"].data_ptr(), cfg.eps, P(xn), None if last else P(xqn),
-                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, *ln_2)
+                          1.0 if last else sc[li + 1]["x"], ROUND_NEAREST_EVEN, *ln_2, kernels=1 if ln_2[0] is None else 2)
             else:
                 self._add("zen_linear_i8_ex", P(self.gq), F, L["w2"].data_ptr(), F, T, H, F, a["gelu"],
                           L["w2_s"].data_ptr(), L["b2"].data_ptr(), ACT_NONE, DT_F16, 1.0, ROUND_NEAREST_EVEN,
@@ -729,13 +730,11 @@ class Int8Encoder(_EncoderBase):
             raise RuntimeError("forward_layerwise needs micro_batches == 1")
         stream = torch.cuda.current_stream().cuda_stream
         lead = self.lead_launches
-        for f, name, args in self._launches[:lead]:
-            _capi.check(name, f(*args, stream))
+        self._issue(self._launches[:lead], stream)
         cur = 0
         for li in range(len(self.layers)):
             n = self.launches_per_layer
-            for f, name, args in self._launches[lead + li * n: lead + (li + 1) * n]:
-                _capi.check(name, f(*args, stream))
+            self._issue(self._launches[lead + li * n: lead + (li + 1) * n], stream)
             torch.cuda.synchronize()
             yield li, {"x": self.x[cur], "xq": self.xq[cur], "qkv": self.qkv, "ctx": self.ctx, "ctxq": self.ctxq,
                        "ao": self.ao, "h1": self.h1, "h1q": self.h1q, "gq": self.gq, "o": self.o,

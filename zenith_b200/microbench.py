@@ -140,7 +140,7 @@ def main() -> None:
         attn_flops = 4.0 * a.batch * cfg.heads * a.seq * a.seq * cfg.head_dim * cfg.layers
         out.update(config=a.config, dtype=a.dtype, batch=a.batch, seq=a.seq, pair=a.pair, us=med, us_min=best,
                    seq_per_s=a.batch / med * 1e6, gemm_tops=gemm_ops / med / 1e6, attn_tflops=attn_flops / med / 1e6,
-                   launches=enc.launches_per_forward)
+                   launches=enc.kernels_per_forward)
     else:
         q = torch.randn(a.b, a.h, a.s, a.d, device=dev, dtype=torch.float16)
         k = torch.randn_like(q)

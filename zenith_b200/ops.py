@@ -148,11 +148,11 @@ def linear_int8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", 
     return out
 
 
-def _layernorm_workspace(elem_bytes: int, M: int, N: int, K: int, device):
+def _layernorm_workspace(elem_bytes: int, M: int, N: int, K: int, gamma, beta):
     """fp32 scratch of a ``*_add_layernorm_ws`` call, or None where the call runs as one kernel; with its size in bytes."""
-    if N not in (768, 1024) or (_capi.lib().zen_gemm_plan(elem_bytes, M, N, K, 1) >> 20) & 0xf == 15:
+    if N not in (768, 1024) or (gamma.data_ptr() | beta.data_ptr()) % 8 or (_capi.lib().zen_gemm_plan(elem_bytes, M, N, K, 1) >> 20) & 0xf == 15:
         return None, 0
-    return torch.empty((M, N), dtype=torch.float32, device=device), M * N * 4
+    return torch.empty((M, N), dtype=torch.float32, device=gamma.device), M * N * 4
 
 
 def linear_int8_add_layernorm(xq, wq, x_scale: float, w_scale, bias, residual, gamma, beta, eps: float, *,
@@ -178,7 +178,7 @@ def linear_int8_add_layernorm(xq, wq, x_scale: float, w_scale, bias, residual, g
     y = torch.empty((M, N), dtype=torch.float16, device=xq.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=xq.device) if out_scale is not None else None
     if M:
-        ws, ws_bytes = _layernorm_workspace(1, M, N, K, xq.device)
+        ws, ws_bytes = _layernorm_workspace(1, M, N, K, gamma, beta)
         _call("zen_linear_i8_add_layernorm_ws", xq.data_ptr(), K, wq.data_ptr(), K, M, N, K, float(x_scale), _ptr(w_scale),
               _ptr(bias), residual.data_ptr(), N, gamma.data_ptr(), beta.data_ptr(), float(eps), y.data_ptr(), _ptr(yq),
               float(out_scale or 1.0), _ROUND[round], _ptr(ws), ws_bytes, _capi.GEMM_CONST_WEIGHTS if constant_weights else 0,
@@ -205,7 +205,7 @@ def linear_fp16_add_layernorm(x, w, bias, residual, gamma, beta, eps: float, *, 
     y = torch.empty((M, N), dtype=torch.float16, device=x.device)
     yq = torch.empty((M, N), dtype=torch.int8, device=x.device) if out_scale is not None else None
     if M:
-        ws, ws_bytes = _layernorm_workspace(2, M, N, K, x.device)
+        ws, ws_bytes = _layernorm_workspace(2, M, N, K, gamma, beta)
         _call("zen_linear_f16_add_layernorm_ws", x.data_ptr(), K, w.data_ptr(), K, M, N, K, _ptr(bias), residual.data_ptr(), N,
               gamma.data_ptr(), beta.data_ptr(), float(eps), y.data_ptr(), _ptr(yq), float(out_scale or 1.0), _ROUND[round],
               _ptr(ws), ws_bytes, _capi.GEMM_CONST_WEIGHTS if constant_weights else 0, _stream())
