@@ -97,3 +97,38 @@ def test_layernorm_parameters_may_start_anywhere(cuda, elem, M, N, K, offset):
 
     for got, want in zip(run(*moved), run(*(v[:N] for v in vectors))):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 768, 768), (129, 768, 3072), (300, 1024, 1024), (1025, 768, 768), (4300, 768, 128)])
+def test_layernorm_forms_give_the_same_bits(cuda, M, N, K):
+    """One kernel, two launches, two launches with K split: a batch that crosses a rule's line keeps its rows' bits (int8; fp16
+    where K is not split).  4300 rows are more than one round of the clusters."""
+    x, w = (torch.from_numpy(rng(s).integers(-128, 128, (n, K), dtype=np.int8)).to(cuda) for s, n in ((M, M), (K, N)))
+    ws, b = dev(((rng(1).random(N) + 0.5) * 2e-4).astype(np.float32), cuda), dev(rng(2).standard_normal(N).astype(np.float32), cuda)
+    res = dev((rng(3).standard_normal((M, N)) * 3).astype(np.float16), cuda)
+    g, be = (dev(rng(s).standard_normal(N).astype(np.float16), cuda) for s in (4, 5))
+    scratch = torch.empty((M, N), dtype=torch.float32, device=cuda)
+
+    def run(flags, elem):
+        y, yq = torch.zeros((M, N), dtype=torch.float16, device=cuda), torch.zeros((M, N), dtype=torch.int8, device=cuda)
+        tail = (b, res, N, g, be, 1e-12, y, yq, 0.03, 0, scratch, scratch.numel() * 4, flags)
+        if elem == 1:
+            call("zen_linear_i8_add_layernorm_ws", x, K, w, K, M, N, K, 0.02, ws, *tail)
+        else:
+            call("zen_linear_f16_add_layernorm_ws", x.half() * 0.02, K, w.half() * 0.001, K, M, N, K, *tail)
+        return y, yq
+
+    for elem, flags in ((1, [14, 2, 4]), (2, [14])):
+        want = run(gemm_split_k(15), elem)
+        for f in flags:
+            got = run(gemm_split_k(f) | (GEMM_NARROW if f < 14 else 0), elem)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (elem, f)
+
+
+def test_layernorm_form_follows_the_resident_clusters(cuda):
+    """A row block more than the clusters that are resident at once (fewer than SMs / 4) is a second round."""
+    form = lambda blocks, K: (_capi.lib().zen_gemm_plan(1, blocks * 128, 768, K, 1) >> 20) & 0xf
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for K in (768, 3072):
+        line = next(n for n in range(26, sms // 4 + 2) if form(n, K) != 15)
+        assert line <= sms // 4 and all(form(n, K) == 14 for n in range(line, sms // 4 + 2))

@@ -3,7 +3,6 @@
 #include "gemm_pair.cuh"
 #include "gemm_small.h"
 #include "tma_host.cuh"
-#include <map>
 #include <mutex>
 
 namespace zen {
@@ -46,39 +45,6 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   return launch_pdl(PDL_GEMM, kernel, dim3(grid), dim3(GEMM_THREADS), smem, stream, ta, tb, tc, p);
 }
 
-// Pairs of CTAs that can be resident at once for a pair kernel (SMs of a GPC come in odd numbers on some
-// parts, so this may be below half the SM count); asked of the runtime once per (kernel, device).
-static int max_resident_pairs(const void* kernel, size_t smem) {
-  static std::mutex mu;
-  static std::map<std::pair<const void*, int>, int> cache;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) {
-    cudaGetLastError();
-    return num_sms() / 2;
-  }
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find({kernel, dev});
-  if (it != cache.end()) return it->second;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(num_sms() / 2 * 2));
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = num_sms() / 2;
-  }
-  cache[{kernel, dev}] = n;
-  return n;
-}
-
 template <int KIND, int BN, int STAGES>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, GemmParams p,
                             cudaStream_t stream) {
@@ -88,7 +54,7 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   p.tiles_m = (p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);  // 256-row blocks
   p.tiles_n = (p.N + BN - 1) / BN;
   const int tiles = p.tiles_m * p.tiles_n;
-  const int resident = max_resident_pairs(reinterpret_cast<const void*>(kernel), smem);
+  const int resident = max_resident_clusters(reinterpret_cast<const void*>(kernel), smem, GEMM_THREADS, 2);
   const int pairs = tiles < resident ? tiles : resident;
   return launch_kernel(kernel, LaunchShape{dim3(unsigned(2 * pairs)), dim3(GEMM_THREADS), smem, (pdl_mask() & PDL_GEMM) != 0, 2}, stream,
                        ta, tb, tc, p);

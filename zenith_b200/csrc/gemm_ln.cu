@@ -594,6 +594,19 @@ static int launch_gemm_ln(const CUtensorMap& ta, const CUtensorMap& tb, const CU
                        stream, ta, tb, ty, tq, tr, p);
 }
 
+template <int BN, int STAGES>
+static int resident_clusters(int elem_bytes) {
+  const void* kernel = elem_bytes == 2 ? reinterpret_cast<const void*>(gemm_f16_ln_kernel<BN, STAGES>)
+                                       : reinterpret_cast<const void*>(gemm_i8_ln_kernel<BN, STAGES>);
+  constexpr size_t smem = gemm_ln_smem_bytes<BN, STAGES>();
+  if (ensure_dynamic_smem(kernel, smem) != ZEN_OK) return num_sms() / LN_CLUSTER;
+  return max_resident_clusters(kernel, smem, GEMM_THREADS, LN_CLUSTER);
+}
+
+int ln_resident_clusters(int elem_bytes, int N) {
+  return N == 768 ? resident_clusters<192, 3>(elem_bytes) : resident_clusters<256, 2>(elem_bytes);
+}
+
 }  // namespace zen
 
 using namespace zen;

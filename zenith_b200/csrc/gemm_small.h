@@ -1,6 +1,7 @@
 // Host entry of the small-product GEMM (gemm_small.cu) and of the dispatch among all GEMM kernels (gemm.cu).
 #pragma once
 #include "gemm_small.cuh"
+#include "tma_host.cuh"
 
 namespace zen {
 
@@ -16,32 +17,62 @@ struct SmallChoice {
 // When a product runs on the small-product kernel (measured per launch in a graph, N = 768 .. 4096, K = 768 .. 4096).
 // 32-column tiles beat 64-column ones throughout (one exchange-and-epilogue step instead of two).  K is split while
 // every CTA keeps three k-blocks (below that the exchange costs more than the blocks; before a LayerNorm one and a half,
-// because the fp32 rows then also leave in narrower pieces), and while the CTAs fit the chip: 192 is where a second CTA
-// on some SMs still pays, with a deep K two per SM everywhere.  Beyond, the persistent kernels win (3072 x 768 at 385
+// because the fp32 rows then also leave in narrower pieces), and while the CTAs fit the chip: 1.3 per SM (192) is where a
+// second CTA on some SMs still pays, with a deep K two per SM everywhere.  Beyond, the persistent kernels win (3072 x 768 at 385
 // rows: 6.1 us against 7.9).  Without a split they are within 5 % of each other.
 //   2.4 MB of weights, 24 rows: K 3072 -> 768 9.5 -> 3.6 us; 128 rows: 9.7 -> 3.9; 512 rows 9.7 -> 5.2; 768 rows 9.8 -> 6.1.
 inline SmallChoice small_rule(int elem_bytes, int M, int N, int K, bool layernorm) {
   const long kb = (long(K) * elem_bytes + 127) / 128;
   const long tiles = long((M + GEMM_BM - 1) / GEMM_BM) * ((N + 31) / 32);
-  if (tiles * 4 <= 192 && kb >= (layernorm ? 6 : 12)) return {32, 4};
-  if (tiles * 2 <= (kb >= 16 ? 296 : 192) && kb >= 4) return {32, 2};
+  const long some_twice = num_sms() * 13 / 10, all_twice = num_sms() * 2;
+  if (tiles * 4 <= some_twice && kb >= (layernorm ? 6 : 12)) return {32, 4};
+  if (tiles * 2 <= (kb >= 16 ? all_twice : some_twice) && kb >= 4) return {32, 2};
   return {64, 0};
 }
 
+// Clusters of the one-kernel projection + LayerNorm (gemm_ln.cu) that are resident at once.
+__attribute__((visibility("hidden"))) int ln_resident_clusters(int elem_bytes, int N);
+
+// Rounds of row blocks until the one-kernel form is through: cluster c of `clusters` takes blocks c, c + clusters, ..; those
+// beyond the resident ones start when one of these has ended.
+inline int ln_cluster_rounds(int blocks, int resident, int clusters) {
+  if (clusters > blocks) clusters = blocks;
+  const int each = blocks / clusters, more = blocks % clusters;  // clusters below `more` have one block more
+  int last = each + (more > 0 ? 1 : 0);
+  for (int c = resident; c < clusters; ++c) {
+    const int start = c - resident < resident - more ? each : each + 1;
+    const int end = start + each + (c < more ? 1 : 0);
+    last = end > last ? end : last;
+  }
+  return last;
+}
+
 // Form of a projection + residual + LayerNorm: the value of the ZEN_GEMM_SPLIT_K field, 15 = one kernel (four-CTA clusters),
-// 14 = large-tile GEMM with fp32 output and a LayerNorm of its rows, else the small-product kernel and that LayerNorm.  A
-// round of the clusters (37 row blocks) takes 9.5 - 10.4 us (K 768) or 16.4 (K 3072) whatever it holds; the two launches
-// take 7.4 / 10.5 us at 1024 rows, 10.3 / 14.1 at 2048, 12 / 17 at 4096, 18 / 25 at 4864 against 19.6 / 30.9, 25 / 32 at
-// 7680 against 20 / 31: they win in a first round that is not full and where a further round would hold little.  At hidden
-// 1024 a cluster CTA holds 256 columns in a two-stage ring and never wins.
+// 14 = large-tile GEMM with fp32 output and a LayerNorm of its rows, else the small-product kernel and that LayerNorm.  The
+// one kernel's time follows its rounds, whatever they hold; that of the two launches follows the rows.  Measured per launch
+// in a graph, 148 SMs and 33 resident clusters, two launches against one kernel, us:
+//   blocks (rounds) 12 (1)     16 (1)     24 (1)     33 (1)     34 (2)     44 (2)     48 (2)     60 (2)     75 (4)     99 (4)     111 (6)
+//   int8  768 x 768   9.1/9.9    10.8/10.0  12.7/10.2  15.9/10.7  16.2/19.3  19.7/19.7  20.7/19.8  25.5/20.2  31.9/32.3  40.8/33.3  43.8/46.7
+//   int8  768 x 3072  11.8/14.8  14.0/15.3  16.5/16.1  21.1/16.8  21.4/30.0  27.2/31.2  28.3/31.4  35.4/31.8  46.4/51.8  54.5/56.8  63.6/77.7
+//   fp16  768 x 3072  15.3/23.6  18.7/23.7  20.5/23.8  25.7/24.2  26.6/43.5  33.7/44.2  35.2/45.4  46.3/47.7  60.9/82.3  78.9/87.7  92.0/122
+//   int8 1024 x 1024  11.7/12.9  12.8/12.8  16.7/12.9  21.2/13.4  21.8/25.0  26.9/25.7  28.5/26.0  35.2/26.4  45.5/42.9  55.1/45.3  59.4/64.1
+//   fp16 1024 x 4096  22.4/47.7  23.8/47.8  30.3/48.0  40.0/48.7  41.0/85.6  55.8/92.0  59.2/93.7  74.9/99.6  104/180    125/183    162/261
+// (fp16 768 x 768 is within 3 % of int8.)  So the first round is worth waiting for from 13 to 25 blocks on, the deeper the
+// product the later; further rounds are dearer than the rows they hold unless K is shallow, where the line moves up by 17
+// blocks a round.  At hidden 1024 and K 4096 in fp16 the two-stage ring of 256 columns never wins.  Over 7 .. 130 blocks,
+// hidden 768 and 1024, K = hidden and 4 x hidden, int8 and fp16, the rule loses 0.1 % on average to the better form, at most
+// 7 % (int8 1024 x 1024, 75 blocks).
 inline SmallChoice layernorm_rule(int elem_bytes, int M, int N, int K) {
   const SmallChoice c = small_rule(elem_bytes, M, N, K, true);
   if (c.ks > 0) return c;
-  const bool deep = (long(K) * elem_bytes + 127) / 128 >= 16;
+  const long kb = (long(K) * elem_bytes + 127) / 128;
   const int blocks = (M + GEMM_BM - 1) / GEMM_BM;
-  const int last = (blocks - 1) % 37 + 1;  // row blocks of the last round
-  const bool two = blocks <= 37 ? last <= (deep ? 24 : 12) : last <= (deep ? 18 : 5);
-  return {64, N != 768 || two ? 14 : 15};
+  const int rounds = ln_cluster_rounds(blocks, ln_resident_clusters(elem_bytes, N), num_sms() / 4);
+  bool two;
+  if (rounds == 1) two = blocks <= (kb >= 32 ? 24 : kb >= 16 ? 20 : N == 768 ? 12 : 16) || (N == 1024 && kb >= 64);
+  else if (kb < 16) two = blocks <= 10 + 17 * rounds;
+  else two = kb >= 32 || rounds > 2 || blocks <= 49;
+  return {64, two ? 14 : 15};
 }
 
 // kind: KIND_*; bn: 64 or 32; ks: 1, 2, 4 or (bn 64) 8; b_mn: B is [K, N] (fp16 only, bn 64).  num_k_blocks is filled in here.

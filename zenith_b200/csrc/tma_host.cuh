@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <utility>
+#include <map>
 #include <mutex>
 #include <set>
 #include "../../include/zenith_b200.h"
@@ -100,6 +101,10 @@ inline int ensure_dynamic_smem(const void* kernel, size_t smem) {
   return ZEN_OK;
 }
 
+// Clusters of `cluster` CTAs that can be resident at once for a kernel with its shared memory set: asked of the runtime once
+// per (kernel, device), because GPCs hold odd numbers of SMs (clusters of four: 33 on 148 SMs, not 37).
+inline int max_resident_clusters(const void* kernel, size_t smem, unsigned threads, unsigned cluster);
+
 inline int num_sms() {
   static int cached[64] = {};
   int dev = 0, v = 0;
@@ -108,6 +113,38 @@ inline int num_sms() {
   if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
   cached[dev] = v;
   return v;
+}
+
+inline int max_resident_clusters(const void* kernel, size_t smem, unsigned threads, unsigned cluster) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> cache;
+  const int guess = num_sms() / int(cluster);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return guess;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = cache.find({kernel, dev});
+  if (it != cache.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(guess) * cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = guess;
+  }
+  cache[{kernel, dev}] = n;
+  return n;
 }
 
 }  // namespace zen
