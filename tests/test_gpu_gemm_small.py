@@ -132,3 +132,14 @@ def test_layernorm_form_follows_the_resident_clusters(cuda):
     for K in (768, 3072):
         line = next(n for n in range(26, sms // 4 + 2) if form(n, K) != 15)
         assert line <= sms // 4 and all(form(n, K) == 14 for n in range(line, sms // 4 + 2))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 192), (3, 64, 200), (130, 72, 264), (256, 1024, 768), (257, 1024, 768), (64, 3072, 768), (65, 3072, 768),
+                                   (384, 1024, 1024), (385, 1024, 1024), (512, 1024, 2048), (513, 1024, 2048), (48, 4096, 1016)])
+def test_matmul_of_row_major_operands_at_the_lines_of_its_rule(cuda, M, N, K):
+    """wmma_matmul on both sides of every line between the K splits and the large tiles.  fp16 products are exact in fp32, and
+    sums of K of them in any order lie within K * 2^-24 of the sum of magnitudes; the bound leaves 2^-19 (K <= 2048: 2^-13)."""
+    a, b = (torch.from_numpy(rng(s).standard_normal(sh).astype(np.float16)).to(cuda) for s, sh in ((M, (M, K)), (N, (K, N))))
+    got = ops.wmma_matmul(a, b)
+    want, scale = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    assert bool(((got - want).abs() <= 2.0**-19 * scale).all())

@@ -369,7 +369,7 @@ int zen_wmma_matmul_f16(const void* A, const void* B, float* C, int M, int N, in
   p.x_scale = 1.0f; p.out_scale = 1.0f;
   static const int allowed[] = {64, 128, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const SmallChoice c = use_small(KIND_F16, M, N, K, 0u); c.ks > 0) return launch_gemm_small(KIND_F16, c.bn, c.ks, true, A, K, B, N, p, s);
+  if (const SmallChoice c = small_rule_mn(M, N, K); c.ks > 0) return launch_gemm_small(KIND_F16, c.bn, c.ks, true, A, K, B, N, p, s);
   switch (pick_bn(M, N, allowed, 3, 0u)) {
     case 64: return run_gemm<KIND_F16, 64, 7, true>(A, K, B, N, p, s);
     case 128: return run_gemm<KIND_F16, 128, 5, true>(A, K, B, N, p, s);

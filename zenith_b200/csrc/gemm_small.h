@@ -30,6 +30,21 @@ inline SmallChoice small_rule(int elem_bytes, int M, int N, int K, bool layernor
   return {64, 0};
 }
 
+// The same for B [K, N] (wmma_matmul, fp16), whose tiles are 64 columns wide: half the CTAs for the same product, twice the
+// exchange and epilogue.  From 12 k-blocks on K is split four ways while that fills the chip about once, 1.3 or 1.7 times the
+// deeper K is; two ways below, and where tiles with few rows of A to load go further.  us, two ways / four ways / large tile:
+//   30 x 1736 x 224 3.1/4.0/3.7    256 x 768 x 768 5.2/4.4/5.1    384 x 768 x 768 5.4/5.4/5.1    214 x 1176 x 912 6.2/5.8/6.8
+//   384 x 1024 x 1024 5.6/5.7/5.8    512 x 1024 x 1024 6.0/6.1/5.8    640 x 768 x 3072 11.7/9.1/11.1    640 x 1024 x 4096 15.1/17.2/14.3
+//   48 x 3072 x 768 4.4/5.0/4.9    128 x 3072 x 768 5.7/5.8/5.4    48 x 4096 x 1024 6.6/6.6/7.1    64 x 4096 x 1024 6.7/6.6/6.1
+inline SmallChoice small_rule_mn(int M, int N, int K) {
+  const long kb = (long(K) * 2 + 127) / 128;
+  const long tiles = long((M + GEMM_BM - 1) / GEMM_BM) * ((N + 63) / 64);
+  const long once = num_sms() * 7 / 32;  // 32: four CTAs each
+  if (kb >= 12 && tiles <= (kb >= 32 ? 2 * once : kb >= 15 ? once * 3 / 2 : once)) return {64, 4};
+  if (kb >= 4 && (tiles <= once || (tiles <= 2 * once && M * tiles <= 3072))) return {64, 2};
+  return {64, 0};
+}
+
 // Clusters of the one-kernel projection + LayerNorm (gemm_ln.cu) that are resident at once.
 __attribute__((visibility("hidden"))) int ln_resident_clusters(int elem_bytes, int N);
 
