@@ -37,10 +37,11 @@ def test_attention_fp16(cuda, B, H, S, D, causal, lens):
     assert np.mean(np.abs(got - want)) < 2e-4
 
 
-@pytest.mark.parametrize("S,D", [(129, 64), (255, 128), (257, 64), (383, 128), (385, 128), (640, 64), (2048, 64), (2049, 64)])
+@pytest.mark.parametrize("S,D", [(129, 64), (255, 128), (257, 64), (383, 128), (385, 128), (640, 64), (2048, 64), (2049, 64),
+                                 (3072, 64), (3073, 64)])
 @pytest.mark.parametrize("causal", [False, True])
 def test_attention_at_tile_edges(cuda, S, D, causal):
-    """Ends of query tiles and key blocks, a tile without keys of its own, both tile counts per CTA (the line lies at 2048
+    """Ends of query tiles and key blocks, a tile without keys of its own, both tile counts per CTA (the line lies at 3072
     tokens for head size 64), key lengths at and next to a block's end; the last query rows against the oracle."""
     lens = [S, max(1, S - 127), 128, 0] if S < 1000 else [S, S - 1, 1025, 128]
     r = rng(S + D)

@@ -128,9 +128,16 @@ static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CU
 
 static int launch_fa_long(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
   if (D == 128) return launch_fa_pipe<128, 2, 2>(tq, tk, tv, p, s);
-  // one tile per CTA, two CTAs per SM, as long as reading K and V once per 128 queries is hidden (batch 8, 16 heads: 49 us
-  // against 62 at 384 tokens, 115 / 123 us causal at 2048; 3107 against 2650 us at 8192)
-  return p.S <= 2048 ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
+  // Head size 64: one tile per CTA, two CTAs per SM, as long as reading K and V once per 128 queries is hidden; beyond, two
+  // tiles share K and V (the same bits).  us, one / two tiles, [batch x heads]:
+  //   384 tokens   [32 x 16] 49 / 62
+  //   2048         [1 x 8] 21 / 28   [2 x 12] 45 / 53   [8 x 16] 189 / 192, causal 112 / 121
+  //   3072         [1 x 8] 43 / 40, causal 32 / 38   [2 x 12] 80 / 76   [8 x 16] 465 / 473, causal 233 / 244   [16 x 16] 1028 / 1049
+  //   4096         [1 x 8] 55 / 50   [2 x 12] 153 / 145   [8 x 16] 923 / 894, causal 453 / 448   [16 x 16] 1844 / 1833
+  //   8192         [1 x 8] 202 / 184   [4 x 16] 1681 / 1589, causal 819 / 797
+  // Over 30 calls of 2304 .. 3072 tokens one tile is 5 % faster on average (the last wave decides single ones, -6 .. +31 %),
+  // over 22 of 4096 and more two are by 2 % (-13 .. +9 %).
+  return p.S <= 3072 ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
 }
 
 // One key block holds the sequence up to 128 tokens.
