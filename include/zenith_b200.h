@@ -148,11 +148,12 @@ int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const void* w, int6
  *                           a tuning hook for benchmarks.  Not accepted by the *_add_layernorm_ex forms.
  *   ZEN_GEMM_PAIR / _NO_PAIR force or forbid the CTA-pair kernel, which the library otherwise chooses by shape;
  *                           results are identical either way.  Tuning / test hook.
- *   ZEN_GEMM_SPLIT_K(n)     run the product on the small-product kernel with its K split n ways (1, 2, 4, 8), 15 = never on
- *                           that kernel; otherwise the library chooses by shape.  int8 results do not depend on it; with
+ *   ZEN_GEMM_SPLIT_K(n)     run the product on the small-product kernel with its K split n ways: 2 or 4 (1 and 8 are taken as
+ *                           the nearer of these; a K too short for a split runs on the large tiles), 15 = never on that
+ *                           kernel; otherwise the library chooses by shape.  int8 results do not depend on it; with
  *                           fp16 operands the fp32 partial sums are added in another order.
  *                           *_add_layernorm_ws forms: 15 = one kernel, 14 = two launches with the large-tile GEMM.
- *   ZEN_GEMM_NARROW         with ZEN_GEMM_SPLIT_K: its 32-column tile (K split at most 4 ways) instead of 64 columns.
+ *   ZEN_GEMM_NARROW         accepted, without effect (the small-product kernel has one tile width).
  * None of this has a counterpart in the reference. */
 #define ZEN_GEMM_CONST_WEIGHTS 0x1u
 #define ZEN_GEMM_NO_PAIR 0x2u /* never run this GEMM on CTA pairs (one CTA per 128-row tile) */
@@ -161,7 +162,7 @@ int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const void* w, int6
 #define ZEN_GEMM_SPLIT_K(n) ((unsigned)(n) << 20)
 #define ZEN_GEMM_NARROW 0x1000000u
 
-/* The ZEN_GEMM_SPLIT_K / ZEN_GEMM_NARROW flags the library would choose for a product of `rows` rows (elem_bytes 1, 2 or 4;
+/* The ZEN_GEMM_SPLIT_K flag the library would choose for a product of `rows` rows (elem_bytes 1, 2 or 4;
  * layernorm != 0: for the *_add_layernorm_ws forms).  A caller that runs the same rows in batches of another size (a packed
  * batch has fewer rows than its padded form) passes the flags of one size everywhere: every row then keeps its bits. */
 unsigned zen_gemm_plan(int elem_bytes, int rows, int N, int K, int layernorm);

@@ -1,5 +1,6 @@
-"""The small-product GEMM (32 / 64-column tiles, K split over a cluster) and the two-launch LayerNorm form, forced through the
-call flags at the edges of their tiles, against the CPU oracle."""
+"""The small-product GEMM (K split two or four ways over a cluster; other splits and the tile-width flag are taken as the
+nearest) and the two-launch LayerNorm form, forced through the call flags at the edges of their tiles, against the CPU
+oracle."""
 import numpy as np
 import pytest
 import torch

@@ -148,13 +148,13 @@ static int pick_bn_pair(int M, int N, unsigned flags) {
   return best;
 }
 
-// Whether (and with what tile and K split) a product runs on the small-product kernel: by shape, or as the flags say.  A
-// forced tile width or pair choice is about the large-tile kernels.
-static SmallChoice use_small(int kind, int M, int N, int K, unsigned flags) {
-  const int f = forced_split(flags);
-  if (f != 0) return {forced_small_bn(flags), f == 15 ? 0 : f};
-  if (flags & (ZEN_GEMM_PAIR | ZEN_GEMM_NO_PAIR | (0x3ffu << 8))) return {64, 0};
-  return small_rule(kind == KIND_F16 ? 2 : kind == KIND_TF32 ? 4 : 1, M, N, K, false);
+// K split of a product on the small-product kernel (0: not there), by shape or as the flags say.  A forced tile width or pair
+// choice is about the large-tile kernels.
+static int use_small(int kind, int M, int N, int K, unsigned flags) {
+  const int elem = kind == KIND_F16 ? 2 : kind == KIND_TF32 ? 4 : 1;
+  if (const int f = forced_split(flags); f != 0) return f == 15 ? 0 : nearest_split(f, (long(K) * elem + 127) / 128);
+  if (flags & (ZEN_GEMM_PAIR | ZEN_GEMM_NO_PAIR | (0x3ffu << 8))) return 0;
+  return small_rule(elem, M, N, K, false);
 }
 
 // out[c, r] = in[r, c] for a row-major [rows, cols] fp32 matrix, 32 x 32 tiles through shared memory.
@@ -184,7 +184,7 @@ static int launch_transpose_f32(const float* in, float* out, int rows, int cols,
 // int8 or fp16 operands, B K-major: the small-product kernel, CTA pairs or the one-CTA kernel by shape (or by `flags`).
 int run_gemm_auto(int kind, const void* A, int64_t lda, const void* B, int64_t ldb, const GemmParams& p, unsigned flags, cudaStream_t s) {
   static const int allowed[] = {64, 128, 192, 256};
-  if (const SmallChoice c = use_small(kind, p.M, p.N, p.K, flags); c.ks > 0) return launch_gemm_small(kind, c.bn, c.ks, false, A, lda, B, ldb, p, s);
+  if (const int ks = use_small(kind, p.M, p.N, p.K, flags); ks > 0) return launch_gemm_small(kind, ks, false, A, lda, B, ldb, p, s);
   if (kind == KIND_I8) {
     if (use_pair(kind, p.M, p.N, p.K, p.out_dtype == ZEN_DT_S8 && p.act == ZEN_ACT_GELU, flags)) {
       switch (pick_bn_pair(p.M, p.N, flags)) {
@@ -227,8 +227,8 @@ int zen_version(void) { return ZEN_VERSION; }
 
 unsigned zen_gemm_plan(int elem_bytes, int rows, int N, int K, int layernorm) {
   if ((elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4) || rows <= 0 || N <= 0 || K <= 0) return 0u;
-  const SmallChoice c = layernorm ? layernorm_rule(elem_bytes, rows, N, K) : small_rule(elem_bytes, rows, N, K, false);
-  return ZEN_GEMM_SPLIT_K(c.ks > 0 ? c.ks : 15) | (c.bn == 32 ? ZEN_GEMM_NARROW : 0u);
+  const int form = layernorm ? layernorm_rule(elem_bytes, rows, N, K) : small_rule(elem_bytes, rows, N, K, false);
+  return ZEN_GEMM_SPLIT_K(form > 0 ? form : 15);
 }
 
 const char* zen_status_string(int s) {
@@ -332,7 +332,7 @@ int zen_linear_f8(const uint8_t* xq, int64_t ldx, const uint8_t* wq, int64_t ldw
   p.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
   static const int allowed[] = {64, 128, 192, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const SmallChoice c = use_small(KIND_F8, M, N, K, flags); c.ks > 0) return launch_gemm_small(KIND_F8, c.bn, c.ks, false, xq, ldx, wq, ldw, p, s);
+  if (const int ks = use_small(KIND_F8, M, N, K, flags); ks > 0) return launch_gemm_small(KIND_F8, ks, false, xq, ldx, wq, ldw, p, s);
   switch (pick_bn(M, N, allowed, 4, flags)) {
     case 64: return run_gemm<KIND_F8, 64, 7, false>(xq, ldx, wq, ldw, p, s);
     case 128: return run_gemm<KIND_F8, 128, 5, false>(xq, ldx, wq, ldw, p, s);
@@ -352,7 +352,7 @@ int zen_linear_f32(const float* x, int64_t ldx, const float* w, int64_t ldw, int
   p.x_scale = 1.0f; p.out_scale = 1.0f; p.w_scale = nullptr; p.bias = bias;
   static const int allowed[] = {64, 128, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const SmallChoice c = use_small(KIND_TF32, M, N, K, 0u); c.ks > 0) return launch_gemm_small(KIND_TF32, c.bn, c.ks, false, x, ldx, w, ldw, p, s);
+  if (const int ks = use_small(KIND_TF32, M, N, K, 0u); ks > 0) return launch_gemm_small(KIND_TF32, ks, false, x, ldx, w, ldw, p, s);
   switch (pick_bn(M, N, allowed, 3, 0u)) {
     case 64: return run_gemm<KIND_TF32, 64, 7, false>(x, ldx, w, ldw, p, s);
     case 128: return run_gemm<KIND_TF32, 128, 5, false>(x, ldx, w, ldw, p, s);
@@ -369,7 +369,7 @@ int zen_wmma_matmul_f16(const void* A, const void* B, float* C, int M, int N, in
   p.x_scale = 1.0f; p.out_scale = 1.0f;
   static const int allowed[] = {64, 128, 256};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const SmallChoice c = small_rule_mn(M, N, K); c.ks > 0) return launch_gemm_small(KIND_F16, c.bn, c.ks, true, A, K, B, N, p, s);
+  if (const int ks = small_rule_mn(M, N, K); ks > 0) return launch_gemm_small(KIND_F16, ks, true, A, K, B, N, p, s);
   switch (pick_bn(M, N, allowed, 3, 0u)) {
     case 64: return run_gemm<KIND_F16, 64, 7, true>(A, K, B, N, p, s);
     case 128: return run_gemm<KIND_F16, 128, 5, true>(A, K, B, N, p, s);

@@ -630,16 +630,10 @@ static int run_linear_add_layernorm(const void* x, int64_t ldx, const void* w, i
       reinterpret_cast<uintptr_t>(residual) % 16)
     return ZEN_ERR_UNSUPPORTED;
   int form = 15;
-  unsigned narrow = 0;
   if (workspace != nullptr) {
     if (workspace_bytes < size_t(M) * size_t(N) * 4 || reinterpret_cast<uintptr_t>(workspace) % 16) return ZEN_ERR_INVALID_ARG;
     form = forced_split(flags);
-    narrow = flags & ZEN_GEMM_NARROW;
-    if (form == 0) {
-      const SmallChoice c = layernorm_rule(ELEM, M, N, K);
-      form = c.ks;
-      narrow = c.bn == 32 ? ZEN_GEMM_NARROW : 0u;
-    }
+    if (form == 0) form = layernorm_rule(ELEM, M, N, K);
     if (form != 1 && form != 2 && form != 4 && form != 8 && form != 14 && form != 15) return ZEN_ERR_INVALID_ARG;
     // the row kernel reads gamma and beta in 8-byte units, the one-kernel form value by value: it takes views that start anywhere
     if ((reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) % 8) form = 15;
@@ -651,7 +645,7 @@ static int run_linear_add_layernorm(const void* x, int64_t ldx, const void* w, i
     g.out = workspace; g.ldo = N; g.out_dtype = ZEN_DT_F32; g.act = ZEN_ACT_NONE; g.fold = 1;
     g.x_scale = x_scale; g.out_scale = 1.0f; g.w_scale = w_scale; g.bias = bias;
     g.early_b = (flags & ZEN_GEMM_CONST_WEIGHTS) ? 1 : 0;
-    if (int st = run_gemm_auto(KIND, x, ldx, w, ldw, g, ZEN_GEMM_SPLIT_K(form == 14 ? 15 : form) | narrow, s); st != ZEN_OK) return st;
+    if (int st = run_gemm_auto(KIND, x, ldx, w, ldw, g, ZEN_GEMM_SPLIT_K(form == 14 ? 15 : form), s); st != ZEN_OK) return st;
     const LnRowsParams lp{static_cast<const float*>(workspace), static_cast<const __half*>(residual), ldr, static_cast<const __half*>(gamma),
                           static_cast<const __half*>(beta), static_cast<__half*>(y), yq, yq ? out_scale : 1.0f, eps, round_mode};
     return N == 768 ? launch_ln_rows<768>(lp, M, s) : launch_ln_rows<1024>(lp, M, s);

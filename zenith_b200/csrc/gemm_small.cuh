@@ -1,5 +1,6 @@
 // GEMM for products that leave the chip idle under 128 x 128 .. 256 tiles: few rows, or narrow outputs with a deep K.
-//   D[M,N] = A[M,K] . B^T with the epilogues of gemm_tc.cuh, one 128 x BN tile (BN 64 or 32) per cluster of KS CTAs.
+//   D[M,N] = A[M,K] . B^T with the epilogues of gemm_tc.cuh, one 128 x BN tile (BN 32; 64 for B [K, N], whose box of 64 fp16
+//   columns is one swizzle span) per cluster of KS (2 or 4) CTAs.
 //
 // What bounds such a product is latency: with four to a few dozen CTAs each pulling its operands through a three-stage
 // ring, a K = 3072 projection of 24 rows took 9.5 us, 16 us with the fused LayerNorm (weights 2.4 MB: 0.4 us of HBM
@@ -22,10 +23,12 @@ namespace zen {
 constexpr int GS_EPI_WARPS = 8;
 constexpr int GS_THREADS = 64 + 32 * GS_EPI_WARPS;
 
+template <bool B_MN>
+__host__ __device__ constexpr int gs_bn() { return B_MN ? 64 : 32; }
 template <int BN>
 __host__ __device__ constexpr int gs_stage_bytes() { return GEMM_BM * 128 + BN * 128; }
 template <int BN, int KS>
-__host__ __device__ constexpr int gs_stages() { return BN == 32 ? (KS >= 4 ? 4 : 5) : KS == 1 ? 4 : 3; }
+__host__ __device__ constexpr int gs_stages() { return BN == 64 ? 3 : KS == 4 ? 4 : 5; }
 
 template <int BN, int KS>
 constexpr size_t gs_smem_bytes() {
@@ -174,7 +177,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       : KIND == KIND_F16 ? make_idesc(IDESC_C_F32, IDESC_F16, IDESC_F16, 0, B_MN ? 1 : 0, GEMM_BM, BN)
       : KIND == KIND_F8  ? make_idesc(IDESC_C_F32, IDESC_E4M3, IDESC_E4M3, 0, B_MN ? 1 : 0, GEMM_BM, BN)
                          : make_idesc(IDESC_C_F32, IDESC_TF32, IDESC_TF32, 0, B_MN ? 1 : 0, GEMM_BM, BN);
-  static_assert(!B_MN || (KIND == KIND_F16 && BN == 64), "MN-major B: one 128-byte wide box of 64 fp16 columns");
+  static_assert(BN == gs_bn<B_MN>() && (KS == 2 || KS == 4) && (!B_MN || KIND == KIND_F16), "forms of the kernel");
   static_assert(CH >= 4, "an epilogue warp finishes at least four columns");
   const GemmParams& p = sp.g;
 
@@ -192,7 +195,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = KS > 1 ? cluster_ctarank() : 0u;
+  const uint32_t rank = cluster_ctarank();
   const int n0 = (int(blockIdx.x) / KS) * BN;
   const int m0 = int(blockIdx.y) * GEMM_BM;
   const int kb0 = int(rank) * p.num_k_blocks / KS;
@@ -209,7 +212,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     mbar_init(xbar, 1);
     *abort_flag = 0;
     mbar_fence_init();
-    if (KS > 1) mbar_arrive_expect_tx(xbar, uint32_t(KS - 1) * 128 * CO * 4);
+    mbar_arrive_expect_tx(xbar, uint32_t(KS - 1) * 128 * CO * 4);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, BN);
@@ -217,7 +220,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
   tc_fence_before_sync();
   __syncthreads();
-  if constexpr (KS > 1) cluster_sync_all();  // every CTA's exchange barrier exists before a peer's bytes are counted on it
+  cluster_sync_all();  // every CTA's exchange barrier exists before a peer's bytes are counted on it
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   grid_launch_dependents();
@@ -316,7 +319,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     bool ok = mbar_wait(tfull_bar, 0, abort_flag);
     tc_fence_after_sync();
     const uint32_t tacc = tmem + (uint32_t(quad * 32) << 16);
-    if (KS > 1 && __all_sync(0xffffffffu, ok)) {
+    if (__all_sync(0xffffffffu, ok)) {
       // this CTA's partials of the columns that the peers finish
 #pragma unroll 1
       for (int i = 1; i < KS; ++i) {
@@ -347,18 +350,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         __syncwarp();
         gs_tmem_ld<CH>(tacc + uint32_t(c0 + s * CH), a);
         tmem_wait_ld();
-        if constexpr (KS > 1) {
 #pragma unroll
-          for (int src = 0; src < KS - 1; ++src)
+        for (int src = 0; src < KS - 1; ++src)
 #pragma unroll
-            for (int u = 0; u < CH / 4; ++u) {
-              const uint4 v = reinterpret_cast<const uint4*>(xbuf)[(src * (CO / 4) + (half * CWARP + s * CH) / 4 + u) * 128 + row];
-              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+          for (int u = 0; u < CH / 4; ++u) {
+            const uint4 v = reinterpret_cast<const uint4*>(xbuf)[(src * (CO / 4) + (half * CWARP + s * CH) / 4 + u) * 128 + row];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                a[4 * u + e] = KIND == KIND_I8 ? a[4 * u + e] + w[e] : __float_as_uint(__uint_as_float(a[4 * u + e]) + __uint_as_float(w[e]));
-            }
-        }
+            for (int e = 0; e < 4; ++e)
+              a[4 * u + e] = KIND == KIND_I8 ? a[4 * u + e] + w[e] : __float_as_uint(__uint_as_float(a[4 * u + e]) + __uint_as_float(w[e]));
+          }
         const int o = s * CH;
         const int col0 = n0 + c0 + o;
         if (p.act == ZEN_ACT_GELU)

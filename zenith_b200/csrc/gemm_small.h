@@ -5,29 +5,33 @@
 
 namespace zen {
 
-// ZEN_GEMM_SPLIT_K field of a call's flags: K split of the small-product kernel (1, 2, 4, 8), 15 = never that kernel,
-// 0 = chosen by shape; ZEN_GEMM_NARROW: its 32-column tile.
+// ZEN_GEMM_SPLIT_K field of a call's flags: K split of the small-product kernel, 15 = never that kernel, 0 = chosen by shape.
 inline int forced_split(unsigned flags) { return int((flags >> 20) & 0xfu); }
-inline int forced_small_bn(unsigned flags) { return (flags & ZEN_GEMM_NARROW) ? 32 : 64; }
 
-struct SmallChoice {
-  int bn, ks;  // ks 0: the product runs on the large-tile kernels
-};
+// The split that a forced one becomes: the kernel has two and four ways, and every CTA of a cluster needs a k-block.
+inline int nearest_split(int forced, long k_blocks) {
+  const int ks = forced >= 4 ? 4 : 2;
+  return k_blocks >= ks ? ks : k_blocks >= 2 ? 2 : 0;
+}
 
-// When a product runs on the small-product kernel (measured per launch in a graph, N = 768 .. 4096, K = 768 .. 4096).
-// 32-column tiles beat 64-column ones throughout (one exchange-and-epilogue step instead of two).  K is split while
-// every CTA keeps three k-blocks (below that the exchange costs more than the blocks; before a LayerNorm one and a half,
+// K split of a product on the small-product kernel, 0 = it runs on the large-tile kernels (measured per launch in a graph,
+// N = 768 .. 4096, K = 768 .. 4096).  A tile is 32 columns wide (64-column ones, with two exchange-and-epilogue steps, lost
+// throughout).  K is split while every CTA keeps three k-blocks (below that the exchange costs more than the blocks; before a LayerNorm one and a half,
 // because the fp32 rows then also leave in narrower pieces), and while the CTAs fit the chip: 1.3 per SM (192) is where a
 // second CTA on some SMs still pays, with a deep K two per SM everywhere.  Beyond, the persistent kernels win (3072 x 768 at 385
 // rows: 6.1 us against 7.9).  Without a split they are within 5 % of each other.
-//   2.4 MB of weights, 24 rows: K 3072 -> 768 9.5 -> 3.6 us; 128 rows: 9.7 -> 3.9; 512 rows 9.7 -> 5.2; 768 rows 9.8 -> 6.1.
-inline SmallChoice small_rule(int elem_bytes, int M, int N, int K, bool layernorm) {
+//   int8 3072 -> 768, 24 rows: 6.5 -> 3.6 us; 128 rows: 6.7 -> 3.9; 512: 6.7 -> 5.7; 768: 6.8 -> 6.3; 1024 (not split): 7.0, split 10.2
+//   fp16 9.9 -> 4.7, 10.2 -> 5.2, 10.6 -> 8.6, 10.9 -> 9.4, 11.2 (15.1);  TF32 18.9 -> 9.0, 19.5 -> 9.7, 19.1 -> 14.8, 19.0 -> 15.4,
+//   19.6 (25.2);  FP8 within 2 % of int8.
+// Of 48 products per type (24 .. 1024 rows) the choice is within 3 % of the best but where four ways would still fit two
+// CTAs per SM (200 x 1024 x 4096: fp16 9.7 us against 8.3, TF32 16.5 / 12.6) and at 200 x 768 x 768 in fp16 (4.1 / 3.7).
+inline int small_rule(int elem_bytes, int M, int N, int K, bool layernorm) {
   const long kb = (long(K) * elem_bytes + 127) / 128;
   const long tiles = long((M + GEMM_BM - 1) / GEMM_BM) * ((N + 31) / 32);
   const long some_twice = num_sms() * 13 / 10, all_twice = num_sms() * 2;
-  if (tiles * 4 <= some_twice && kb >= (layernorm ? 6 : 12)) return {32, 4};
-  if (tiles * 2 <= (kb >= 16 ? all_twice : some_twice) && kb >= 4) return {32, 2};
-  return {64, 0};
+  if (tiles * 4 <= some_twice && kb >= (layernorm ? 6 : 12)) return 4;
+  if (tiles * 2 <= (kb >= 16 ? all_twice : some_twice) && kb >= 4) return 2;
+  return 0;
 }
 
 // The same for B [K, N] (wmma_matmul, fp16), whose tiles are 64 columns wide: half the CTAs for the same product, twice the
@@ -36,13 +40,13 @@ inline SmallChoice small_rule(int elem_bytes, int M, int N, int K, bool layernor
 //   30 x 1736 x 224 3.1/4.0/3.7    256 x 768 x 768 5.2/4.4/5.1    384 x 768 x 768 5.4/5.4/5.1    214 x 1176 x 912 6.2/5.8/6.8
 //   384 x 1024 x 1024 5.6/5.7/5.8    512 x 1024 x 1024 6.0/6.1/5.8    640 x 768 x 3072 11.7/9.1/11.1    640 x 1024 x 4096 15.1/17.2/14.3
 //   48 x 3072 x 768 4.4/5.0/4.9    128 x 3072 x 768 5.7/5.8/5.4    48 x 4096 x 1024 6.6/6.6/7.1    64 x 4096 x 1024 6.7/6.6/6.1
-inline SmallChoice small_rule_mn(int M, int N, int K) {
+inline int small_rule_mn(int M, int N, int K) {
   const long kb = (long(K) * 2 + 127) / 128;
   const long tiles = long((M + GEMM_BM - 1) / GEMM_BM) * ((N + 63) / 64);
   const long once = num_sms() * 7 / 32;  // 32: four CTAs each
-  if (kb >= 12 && tiles <= (kb >= 32 ? 2 * once : kb >= 15 ? once * 3 / 2 : once)) return {64, 4};
-  if (kb >= 4 && (tiles <= once || (tiles <= 2 * once && M * tiles <= 3072))) return {64, 2};
-  return {64, 0};
+  if (kb >= 12 && tiles <= (kb >= 32 ? 2 * once : kb >= 15 ? once * 3 / 2 : once)) return 4;
+  if (kb >= 4 && (tiles <= once || (tiles <= 2 * once && M * tiles <= 3072))) return 2;
+  return 0;
 }
 
 // Clusters of the one-kernel projection + LayerNorm (gemm_ln.cu) that are resident at once.
@@ -77,9 +81,8 @@ inline int ln_cluster_rounds(int blocks, int resident, int clusters) {
 // blocks a round.  At hidden 1024 and K 4096 in fp16 the two-stage ring of 256 columns never wins.  Over 7 .. 130 blocks,
 // hidden 768 and 1024, K = hidden and 4 x hidden, int8 and fp16, the rule loses 0.1 % on average to the better form, at most
 // 7 % (int8 1024 x 1024, 75 blocks).
-inline SmallChoice layernorm_rule(int elem_bytes, int M, int N, int K) {
-  const SmallChoice c = small_rule(elem_bytes, M, N, K, true);
-  if (c.ks > 0) return c;
+inline int layernorm_rule(int elem_bytes, int M, int N, int K) {
+  if (const int ks = small_rule(elem_bytes, M, N, K, true); ks > 0) return ks;
   const long kb = (long(K) * elem_bytes + 127) / 128;
   const int blocks = (M + GEMM_BM - 1) / GEMM_BM;
   const int rounds = ln_cluster_rounds(blocks, ln_resident_clusters(elem_bytes, N), num_sms() / 4);
@@ -87,11 +90,11 @@ inline SmallChoice layernorm_rule(int elem_bytes, int M, int N, int K) {
   if (rounds == 1) two = blocks <= (kb >= 32 ? 24 : kb >= 16 ? 20 : N == 768 ? 12 : 16) || (N == 1024 && kb >= 64);
   else if (kb < 16) two = blocks <= 10 + 17 * rounds;
   else two = kb >= 32 || rounds > 2 || blocks <= 49;
-  return {64, two ? 14 : 15};
+  return two ? 14 : 15;
 }
 
-// kind: KIND_*; bn: 64 or 32; ks: 1, 2, 4 or (bn 64) 8; b_mn: B is [K, N] (fp16 only, bn 64).  num_k_blocks is filled in here.
-__attribute__((visibility("hidden"))) int launch_gemm_small(int kind, int bn, int ks, bool b_mn, const void* A, int64_t lda, const void* B,
+// kind: KIND_*; ks: 2 or 4, at most the k-blocks; b_mn: B is [K, N] (fp16 only).  num_k_blocks is filled in here.
+__attribute__((visibility("hidden"))) int launch_gemm_small(int kind, int ks, bool b_mn, const void* A, int64_t lda, const void* B,
                                                             int64_t ldb, const GemmParams& g, cudaStream_t stream);
 
 // int8 or fp16 operands, B [N, K]: picks among all GEMM kernels.
