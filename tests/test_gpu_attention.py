@@ -38,11 +38,11 @@ def test_attention_fp16(cuda, B, H, S, D, causal, lens):
 
 
 @pytest.mark.parametrize("S,D", [(129, 64), (255, 128), (257, 64), (383, 128), (385, 128), (640, 64), (2048, 64), (2049, 64),
-                                 (3072, 64), (3073, 64)])
+                                 (3072, 64), (3073, 64), (4097, 64)])
 @pytest.mark.parametrize("causal", [False, True])
 def test_attention_at_tile_edges(cuda, S, D, causal):
-    """Ends of query tiles and key blocks, a tile without keys of its own, both tile counts per CTA (the line lies at 3072
-    tokens for head size 64), key lengths at and next to a block's end; the last query rows against the oracle."""
+    """Ends of query tiles and key blocks, a tile without keys of its own, both tile counts per CTA (beyond 2048 tokens at
+    head size 64 the count follows the waves), key lengths at and next to a block's end; the last query rows against the oracle."""
     lens = [S, max(1, S - 127), 128, 0] if S < 1000 else [S, S - 1, 1025, 128]
     r = rng(S + D)
     q, k, v = (r.standard_normal((4, 2, S, D)).astype(np.float16) for _ in range(3))

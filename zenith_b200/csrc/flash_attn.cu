@@ -126,18 +126,27 @@ static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CU
   return launch_pdl(PDL_ATTENTION, kernel, dim3(unsigned(ctas)), dim3(fap_threads<GROUPS>()), smem, s, tq, tk, tv, p);
 }
 
+// Head size 64, one or two query tiles per CTA (the same bits): two tiles share K and V, one tile per CTA leaves room for two
+// CTAs on an SM.  Up to 2048 tokens one tile: reading K and V once per 128 queries is hidden (32 x 16 heads x 384: 49 us
+// against 62; 8 x 16 x 2048: 189 / 192, causal 112 / 121).  Beyond 4096 two (4 x 16 x 8192: 1681 / 1589 us, causal 819 / 797).
+// Between, with the last wave: an SM that holds one of its two CTAs runs it faster, one that holds a CTA of two tiles does not.
+// Measured at 14 lengths of 2049 .. 5120 for 12 batch x heads of 8 .. 192, two tiles / one tile, by waves of one-tile CTAs:
+//   full    0 .. 0.5: 1.32 - 1.35    0.5 .. 1: 0.91 - 0.94    1 .. 1.5: 1.03 - 1.19    1.5 .. 2: 0.92 - 0.96    2 .. 2.5: 1.02 - 1.13
+//           2.5 .. 3: 0.94 - 1.10, mean 0.97    3 .. 3.5: 1.01 - 1.10    3.5 .. 4: 0.95 - 0.99    more: 0.95 - 1.09, mean 1.02
+//   causal  (the heaviest tiles start first) 0 .. 0.8: 1.06 - 1.29    0.8 .. 2: 0.91 - 1.05, mean 0.97    more: 0.99 - 1.13, mean 1.07
+// The choice is 0.3 % from the better one on average.
+static bool one_tile_per_cta(const FaParams& p) {
+  if (p.S <= 2048 || p.S > 4096) return p.S <= 2048;
+  const double waves = double((p.S + 127) / 128) * p.H * p.B / (2.0 * num_sms());
+  if (p.causal) return waves <= 0.8 || waves >= 2.0;
+  if (waves >= 5.0) return p.S < 4096;
+  const double last = waves - double(int64_t(waves));
+  return last > 0.0 && last <= 0.5;
+}
+
 static int launch_fa_long(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
   if (D == 128) return launch_fa_pipe<128, 2, 2>(tq, tk, tv, p, s);
-  // Head size 64: one tile per CTA, two CTAs per SM, as long as reading K and V once per 128 queries is hidden; beyond, two
-  // tiles share K and V (the same bits).  us, one / two tiles, [batch x heads]:
-  //   384 tokens   [32 x 16] 49 / 62
-  //   2048         [1 x 8] 21 / 28   [2 x 12] 45 / 53   [8 x 16] 189 / 192, causal 112 / 121
-  //   3072         [1 x 8] 43 / 40, causal 32 / 38   [2 x 12] 80 / 76   [8 x 16] 465 / 473, causal 233 / 244   [16 x 16] 1028 / 1049
-  //   4096         [1 x 8] 55 / 50   [2 x 12] 153 / 145   [8 x 16] 923 / 894, causal 453 / 448   [16 x 16] 1844 / 1833
-  //   8192         [1 x 8] 202 / 184   [4 x 16] 1681 / 1589, causal 819 / 797
-  // Over 30 calls of 2304 .. 3072 tokens one tile is 5 % faster on average (the last wave decides single ones, -6 .. +31 %),
-  // over 22 of 4096 and more two are by 2 % (-13 .. +9 %).
-  return p.S <= 3072 ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
+  return one_tile_per_cta(p) ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
 }
 
 // One key block holds the sequence up to 128 tokens.
