@@ -193,3 +193,23 @@ def test_wmma_matmul_and_fp32_matmul(cuda, M, N, K):
 
 def test_no_device_timeout_recorded(cuda):
     assert _capi.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,ld,col", [(23, 39, 40, 0), (300, 19, 24, 0), (130, 319, 400, 16), (9, 3, 16, 8), (257, 1015, 1040, 0), (64, 64, 72, 8)])
+@pytest.mark.parametrize("pair", [None, True, False])
+def test_result_in_a_column_slice_leaves_the_columns_beside_it_alone(cuda, M, N, ld, col, pair):
+    """``out`` as columns of a wider matrix whose rows are 16-byte aligned, N not a multiple of 16 bytes."""
+    K = 64
+    x, w = (torch.from_numpy(np.random.default_rng(n).integers(-9, 9, (n, K)).astype(np.float16)).to(cuda) for n in (M, N))
+    want = ops.linear_fp16(x, w)
+    big = torch.full((M, ld), 7.0, dtype=torch.float16, device=cuda)
+    ops.linear_fp16(x, w, out=big[:, col:col + N], pair=pair)
+    assert torch.equal(big[:, col:col + N], want)
+    assert bool((big[:, :col] == 7).all()) and bool((big[:, col + N:] == 7).all())
+    out = torch.full((M, ld), 7, dtype=torch.int8, device=cuda)
+    xq, wq = x.to(torch.int8), w.to(torch.int8)
+    flags = 0 if pair is None else _capi.GEMM_PAIR if pair else _capi.GEMM_NO_PAIR
+    _capi.call("zen_linear_i8_ex", xq.data_ptr(), K, wq.data_ptr(), K, M, N, K, 0.01, None, None, 0, _capi.DT_S8, 0.1, 0,
+               out.data_ptr() + col, ld, None, 0, None, 0, flags, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(out[:, col:col + N], ops.linear_int8(xq, wq, 0.01, out_dtype=torch.int8, out_scale=0.1))
+    assert bool((out[:, :col] == 7).all()) and bool((out[:, col + N:] == 7).all())

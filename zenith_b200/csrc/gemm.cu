@@ -86,7 +86,8 @@ static int run_gemm(const void* A, int64_t lda, const void* B, int64_t ldb, Gemm
   CUtensorMap tc = ta;
   p.staged_store = 0;
   const int oelem = p.out_dtype == ZEN_DT_S8 ? 1 : p.out_dtype == ZEN_DT_F16 ? 2 : 4;
-  if (reinterpret_cast<uintptr_t>(p.out) % 16 == 0 && (p.ldo * oelem) % 16 == 0) {
+  // (a TMA store clips a row at N rounded up to 16 bytes: the rest of that unit may be the caller's next columns)
+  if (reinterpret_cast<uintptr_t>(p.out) % 16 == 0 && (p.ldo * oelem) % 16 == 0 && (oelem == 4 || (int64_t(p.N) * oelem) % 16 == 0)) {
     p.staged_store = 1;
     if (oelem < 4) {
       constexpr int SLAB = gemm_slab_cols<BN>();
