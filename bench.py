@@ -5,10 +5,10 @@
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N ... bench.py --gpus N ...
 
 ``--config bert_base`` (default, the headline): a step is one forward pass over one batch of 32 synthetic
-sequences of 128 tokens per GPU (BASELINE.json configs[2]: 12 layers, hidden 768, 12 heads, FFN 3072, post-LN,
+sequences of 128 tokens per GPU (12 layers, hidden 768, 12 heads, FFN 3072, post-LN,
 tanh-GELU, W8A8 with per-channel weight scales and min-max activation scales from 16 seeded batches; token ids
 uniform over 30522 words, the last 0..32 positions of each row masked).  Ranks are independent replicas (weak
-scaling, global batch 32 * N).  ``--config bert_large``: BASELINE.json configs[4], global batch 256 x 384 tokens
+scaling, global batch 32 * N).  ``--config bert_large``: global batch 256 x 384 tokens
 split over the ranks (strong scaling).  For N > 1 every step ends with the gather of the hidden states onto rank
 0.  Rank 0 prints ONE JSON line.
 
@@ -20,12 +20,12 @@ split over the ranks (strong scaling).  For N > 1 every step ends with the gathe
              rate of the short timed region.
 `roofline`   the launches of a layer that carry its int8 GEMM work: average launch durations measured with
              CUDA events inside a graph of 12 launches per shape, as the step runs them.
-`secondary`  the other configurations of BASELINE.json measured in the same run (fp16 encoder, attention
+`secondary`  the other configurations measured in the same run (fp16 encoder, attention
              sweep, a BERT-large shard), kernel yardsticks (int8 8192^3 against the library GEMM, add+LayerNorm
              against the copy bandwidth).
 `parity_check` one layer's FFN1 int8 output of the timed encoder against the CPU oracle, and replay == eager.
 `cpu_baseline` the CPU restatement of the reference's quantized executor (fake-quant + fp32 BLAS matmul) on a
-             bounded sample, plus the reference's two single-Linear CPU forms on BASELINE.json configs[0].
+             bounded sample, plus the reference's two single-Linear CPU forms at 128 x 3072 x 768.
 `--impl reference` times that CPU executor alone, on the same workload definition (32 sequences per step).
 """
 from __future__ import annotations
@@ -49,10 +49,10 @@ BATCH, SEQ = 32, 128
 MASTER_SEED = 1234
 CALIB_BATCHES = 16
 METRIC = "bert_base_int8_seq128_sequences_per_sec"
-WORKLOAD = "bert-base W8A8 encoder, batch 32 per GPU, seq 128 (BASELINE.json configs[2])"
+WORKLOAD = "bert-base W8A8 encoder, batch 32 per GPU, seq 128"
 LARGE_GLOBAL_BATCH, LARGE_SEQ = 256, 384
 LARGE_METRIC = "bert_large_int8_seq384_sequences_per_sec"
-LARGE_WORKLOAD = "bert-large W8A8 encoder, global batch 256 split over the GPUs, seq 384 (BASELINE.json configs[4])"
+LARGE_WORKLOAD = "bert-large W8A8 encoder, global batch 256 split over the GPUs, seq 384"
 
 
 def make_batch(seed: int, vocab: int, batch: int = BATCH, seq: int = SEQ):
@@ -170,7 +170,7 @@ def cpu_executor(sample_seqs: int, steps: int, warmup: int, large: bool = False)
 
 
 def cpu_single_linear_baselines() -> list:
-    """The reference's two other CPU forms of a quantized Linear, on BASELINE.json configs[0] (X [128, 768],
+    """The reference's two other CPU forms of a quantized Linear, at 128 x 3072 x 768 (X [128, 768],
     W [3072, 768]): the true-integer numpy product (benchmarks/int8_bench.py:42-45: int32 matmul, then dequant) and
     the reference's own AVX2 fp32 GEMM (core/src/cpu_kernels.cpp:129-165, compiled as it stands into oracle/_ref) on
     the dequantised operands.  Both are single-threaded by construction."""
@@ -195,7 +195,7 @@ def cpu_single_linear_baselines() -> list:
     out = []
     b32 = np.ascontiguousarray(wq.astype(np.int32).T)
     med, best = median_ms(lambda: (xq.astype(np.int32) @ b32).astype(np.float32) * s_x * s_w, reps=3, warm=1)
-    out.append({"name": "true-integer numpy GEMM + dequant (int8_bench.py:42-45)", "workload": "configs[0]: 128 x 3072 x 768",
+    out.append({"name": "true-integer numpy GEMM + dequant (int8_bench.py:42-45)", "workload": "quantized Linear, 128 x 3072 x 768",
                 "ms": round(med, 3), "ms_min": round(best, 3), "gops": round(2.0 * M * N * K / med / 1e6, 2), "cores": 1,
                 "kind": "reference formula in numpy"})
     if O.ref_lib() is not None:
@@ -203,7 +203,7 @@ def cpu_single_linear_baselines() -> list:
         wt = np.ascontiguousarray((wq.astype(np.float32) * s_w).T)  # [K, N]
         med, best = median_ms(lambda: O.ref_matmul_avx2(xf, wt))
         out.append({"name": "reference AVX2 fp32 GEMM on dequantised operands (cpu_kernels.cpp:129-165)",
-                    "workload": "configs[0]: 128 x 3072 x 768", "ms": round(med, 3), "ms_min": round(best, 3),
+                    "workload": "quantized Linear, 128 x 3072 x 768", "ms": round(med, 3), "ms_min": round(best, 3),
                     "gflops": round(2.0 * M * N * K / med / 1e6, 2), "cores": 1, "kind": "reference"})
     else:
         out.append({"name": "reference AVX2 fp32 GEMM", "ms": None, "kind": "reference",
@@ -369,7 +369,7 @@ def time_gemm_shapes(torch, ops, dev, flush) -> dict:
 
 
 def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> dict:
-    """The other BASELINE.json configurations and two kernel yardsticks, measured in this run (CUDA events, L2
+    """The other configurations and two kernel yardsticks, measured in this run (CUDA events, L2
     flushed between launches, medians)."""
     from zenith_b200.encoder import BERT_LARGE, Fp16Encoder, Int8Encoder, Int8Scales, init_params
 
@@ -379,7 +379,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
         torch.cuda.synchronize()
         print(f"[bench] secondary: {what} done", file=sys.stderr, flush=True)
 
-    # configs[1]: the fp16 encoder, batch 32 x 128
+    # the fp16 encoder, batch 32 x 128
     enc = Fp16Encoder(cfg_base, params_base, dev)
     ids, lens = make_batch(MASTER_SEED + 1000, cfg_base.vocab)
     enc.capture(BATCH, SEQ)
@@ -388,10 +388,10 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
         enc.replay()
     us = _event_us(torch, enc.replay, 15, flush)
     out["bert_base_fp16_seq128"] = {"sequences_per_s": round(BATCH / us * 1e6, 1), "ms_per_step": round(us / 1e3, 4),
-                                    "launches": enc.kernels_per_forward, "workload": "BASELINE.json configs[1]"}
+                                    "launches": enc.kernels_per_forward, "workload": "bert-base fp16 encoder, batch 32, seq 128"}
     del enc
     done("fp16 encoder")
-    # configs[3]: attention forward sweep, B = 8, H = 16
+    # attention forward sweep, B = 8, H = 16
     fp16_peak = peaks["bf16_tflops"]
     sweep = {}
     for D in (64, 128):
@@ -406,7 +406,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
                 sweep[f"d{D}_s{S}_{'causal' if causal else 'full'}"] = {"tflops": round(tf, 1), "frac_of_fp16_peak": round(tf / fp16_peak, 3)}
             del q, k, v
     out["attention_fwd_b8_h16"] = {"cases": sweep, "peak_tflops": fp16_peak,
-                                   "peak_source": f"{peaks['source']} bf16 GEMM burst", "workload": "BASELINE.json configs[3]"}
+                                   "peak_source": f"{peaks['source']} bf16 GEMM burst", "workload": "attention forward, batch 8, 16 heads"}
     done("attention sweep")
     # int8 GEMM yardstick: own kernel against the library GEMM on the same device in the same run
     n = 8192
@@ -465,7 +465,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
     except Exception as exc:
         out["bert_base_int8_batch128_unpadded"] = {"error": str(exc)}
     done("batch 128 padded / unpadded")
-    # configs[4]: one GPU's shard of the BERT-large run at 8 GPUs (32 sequences x 384 tokens)
+    # one GPU's shard of the BERT-large run at 8 GPUs (32 sequences x 384 tokens)
     cfg = BERT_LARGE
     params = init_params(cfg, MASTER_SEED)
     from zenith_b200.calibrate import calibrate
@@ -480,7 +480,7 @@ def secondary_metrics(torch, ops, dev, flush, peaks, cfg_base, params_base) -> d
     us = _event_us(torch, enc.replay, 9, flush)
     out["bert_large_int8_seq384_shard32"] = {"ms_per_step": round(us / 1e3, 3), "sequences_per_s": round(32 / us * 1e6, 1),
                                              "launches": enc.kernels_per_forward,
-                                             "workload": "BASELINE.json configs[4], the 32-sequence shard one of 8 GPUs holds"}
+                                             "workload": "bert-large W8A8, seq 384, the 32-sequence shard one of 8 GPUs holds"}
     try:  # the same shard unpadded (projection GEMM on the packed rows, attention from the offsets)
         enc.capture_unpadded(32, LARGE_SEQ, Int8Encoder.unpadded_capacity(lens.tolist(), LARGE_SEQ))
         enc.set_inputs(torch.from_numpy(ids).to(dev), torch.from_numpy(lens).to(dev))
@@ -817,7 +817,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--config", choices=["bert_base", "bert_large"], default="bert_base",
-                    help="bert_base: BASELINE.json configs[2] (the headline); bert_large: configs[4], global batch 256 x 384")
+                    help="bert_base: 32 x 128 tokens per GPU (the headline); bert_large: global batch 256 x 384")
     ap.add_argument("--micro-batches", type=int, default=1,
                     help="cut each GPU's batch into this many concurrently running micro-batches")
     ap.add_argument("--gather", choices=["peer", "nccl"], default="peer",

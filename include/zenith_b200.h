@@ -151,7 +151,9 @@ int zen_linear_f16_add_layernorm(const void* x, int64_t ldx, const void* w, int6
  *   ZEN_GEMM_SPLIT_K(n)     run the product on the small-product kernel with its K split n ways: 2 or 4 (1 and 8 are taken as
  *                           the nearer of these; a K too short for a split runs on the large tiles), 15 = never on that
  *                           kernel; otherwise the library chooses by shape.  int8 results do not depend on it; with
- *                           fp16 operands the fp32 partial sums are added in another order.
+ *                           fp16 operands the fp32 partial sums are added in another order.  Chosen by shape, the split
+ *                           depends on the rows: the last bits of an fp16, TF32 or FP8 result may differ between batches
+ *                           of different size (zen_gemm_plan pins the choice, 15 never splits).
  *                           *_add_layernorm_ws forms: 15 = one kernel, 14 = two launches with the large-tile GEMM.
  *   ZEN_GEMM_NARROW         accepted, without effect (the small-product kernel has one tile width).
  * None of this has a counterpart in the reference. */
@@ -305,6 +307,15 @@ int zen_flash_attention_f16(const void* q, const void* k, const void* v, void* o
                             int64_t k_ss, int64_t v_sb, int64_t v_sh, int64_t v_ss, int64_t o_sb, int64_t o_sh,
                             int64_t o_ss, const int32_t* kv_lens, int causal, float scale, void* stream);
 
+/* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
+ * computed in fp16 with fp32 softmax and accumulation.  Two launches: the operands to fp16 in `workspace`
+ * (zen_flash_attention_f32_workspace_bytes), attention with fp32 stores.  o and workspace 16-byte aligned; q, k and v may
+ * lie on any 4-byte boundary. */
+size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D);
+int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
+                            const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,
+                            void* stream);
+
 /* W8A8 QKV projection and attention of an encoder layer in ONE kernel, for sequences of at most 128 tokens and head
  * size 64:  [Q | K | V] = half((float(xq . wqkv^T) * x_scale) * w_scale[n] + bias[n]) per token, then per (sequence,
  * head)  ctx = softmax(scale * Q K^T [keys >= kv_lens[b] masked]) V.
@@ -321,6 +332,9 @@ int zen_qkv_attention_i8(const int8_t* xq, int64_t ldx, const int8_t* wqkv, int6
                          void* ctx, int8_t* ctxq, float ctx_scale, void* qkv_out, const void* next0, size_t next0_bytes,
                          const void* next1, size_t next1_bytes, unsigned flags, void* stream);
 
+/* inputs[0 .. B*S) = ids, inputs[B*S .. B*S + B) = kv_lens (NULL: S each): the two copies of a batch as one launch. */
+int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S, int32_t* inputs, void* stream);
+
 /* Unpadded batches.  The reference's encoder drivers pad every sequence to the batch's length and spend GEMM work
  * on the padding (benchmarks/bert_hybrid.py:88-120 reshapes [B, S, H] to [B * S, H] for every projection).  Here the
  * valid tokens are packed back to back, sequence b in rows cu_seqlens[b] .. cu_seqlens[b + 1] - 1, every row-wise
@@ -336,15 +350,6 @@ int zen_qkv_attention_i8(const int8_t* xq, int64_t ldx, const int8_t* wqkv, int6
  *   valid row's result equals, bit for bit, the padded call's result for that token.
  * zen_unpad_rows_f16: padded[b * S + s] = packed[cu_seqlens[b] + s] for valid positions, zeros for padding.
  * No counterpart in the reference (its roadmap lists variable-length batching as future work). */
-/* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
- * computed in fp16 with fp32 softmax and accumulation.  Two launches: the operands to fp16 in `workspace`
- * (zen_flash_attention_f32_workspace_bytes), attention with fp32 stores.  o and workspace 16-byte aligned; q, k and v may
- * lie on any 4-byte boundary. */
-size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D);
-int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
-                            const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,
-                            void* stream);
-
 /* zen_flash_attention_unpadded_f16: zen_flash_attention_f16 on packed tensors: token t of Q sits at q + t*q_st + h*q_sh + d
  * (likewise K, V, O), sequence b owns tokens cu_seqlens[b] .. cu_seqlens[b + 1] - 1 (cut at `rows`; at most max_seqlen
  * each: a longer one is cut to its first max_seqlen tokens), causal counts positions within the sequence.  Any
@@ -353,8 +358,6 @@ int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v
                                      int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh, int64_t k_st,
                                      int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st, int64_t o_sh,
                                      const int32_t* cu_seqlens, int causal, float scale, void* stream);
-/* inputs[0 .. B*S) = ids, inputs[B*S .. B*S + B) = kv_lens (NULL: S each): the two copies of a batch as one launch. */
-int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S, int32_t* inputs, void* stream);
 int zen_pack_tokens_i32(const int32_t* ids, const int32_t* type_ids, const int32_t* kv_lens, int B, int S, int capacity,
                         int32_t* cu_seqlens, int32_t* ids_packed, int32_t* pos_packed, int32_t* type_packed, void* stream);
 int zen_embed_layernorm_unpadded_f16(const int32_t* ids_packed, const int32_t* pos_packed, const int32_t* type_packed,

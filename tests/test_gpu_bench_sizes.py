@@ -1,4 +1,4 @@
-"""Parity with the CPU oracle AT THE BENCHMARK'S OWN SIZES (BASELINE.json configs 2-5), through the C ABI.
+"""Parity with the CPU oracle AT THE BENCHMARK'S OWN SIZES, through the C ABI.
 
 The small-shape tests elsewhere never give a persistent CTA more than one tile, a cluster more than one row
 block, or the attention kernel more than eight key blocks.  Here every kernel runs the code path the headline
@@ -196,7 +196,7 @@ def test_bert_base_int8_pass_every_kernel_against_the_oracle(cuda, bert_base):
 
 
 def test_bert_base_fp16_pass_tracks_the_fp32_reference_path(cuda, bert_base):
-    """the fp16 encoder against the oracle's fp32 encoder on the same weights and batch.
+    """The fp16 encoder against the oracle's fp32 encoder on the same weights and batch.
     The reference states < 0.1 (absolute) for its own 12-layer fp16 path against fp32
     (benchmarks/bert_fp16_full.py:210-229); LayerNorm outputs are O(1), so 1e-2 relative to the largest
     activation is the tighter of the two and is what is asserted, on four sequences."""
@@ -217,7 +217,7 @@ def test_bert_base_fp16_pass_tracks_the_fp32_reference_path(cuda, bert_base):
 
 
 # ------------------------------------------------------------------------------------------------------------
-# (d) attention at the sweep's long sequences (BASELINE config 4), on sampled query rows
+# (d) attention at the sweep's long sequences, on sampled query rows
 # ------------------------------------------------------------------------------------------------------------
 def _attention_case(cuda, S, D, causal, q, k, v, lens=None, tol=1e-2):
     B, H = q.shape[:2]

@@ -133,7 +133,7 @@ def test_int8_epilogue_trunc_rounding_and_no_scale_no_bias(cuda):
 
 
 def test_config1_on_device_matches_reference_digests(cuda):
-    """BASELINE config 1 end to end: quantize X on the device, int8 GEMM, dequant + bias + GELU."""
+    """A quantized Linear end to end: quantize X on the device, int8 GEMM, dequant + bias + GELU."""
     M = 1234
     X = rng(M).standard_normal((128, 768)).astype(np.float32)
     W = (rng(M + 100).standard_normal((3072, 768)) * 0.02).astype(np.float32)

@@ -17,7 +17,7 @@ constexpr int FA_BKV = 128;
 
 struct FaParams {
   void* o;
-  int o_f32;  // long-sequence kernel: the fp16 results are stored as fp32 (the fp32 binding)
+  int o_f32;  // the fp16 results are stored as fp32 (the fp32 binding)
   int8_t* oq;
   float o_scale, inv_o_scale;
   int B, H, S;

@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(256) convert3_kernel(const float* __restrict__
 }
 
 // ------------------------------------------------------------------------------------------
-// Unpadded batches: the valid tokens of a padded [B, S] batch packed back to back
+// Inputs of a recorded pass
 // ------------------------------------------------------------------------------------------
 // Token ids and key lengths of a batch into the static buffer that a recorded pass reads.  As two memory copies they took
 // 2.7 microseconds each in front of every pass, whatever their size.
@@ -535,6 +535,8 @@ __global__ void __launch_bounds__(256) set_inputs_kernel(const int32_t* __restri
     inputs[i] = i < n ? ids[i] : (kv_lens ? kv_lens[i - n] : S);
 }
 
+// ------------------------------------------------------------------------------------------
+// Unpadded batches: the valid tokens of a padded [B, S] batch packed back to back
 // ------------------------------------------------------------------------------------------
 // Block b < B: the offset of sequence b (sum of the clamped lengths before it), then its ids / positions / types.
 // Block B: the total, and defined values (id 0, position 0) for the rows between the total and the capacity.
