@@ -243,7 +243,7 @@ def test_fp16_encoder_with_fused_layernorm_kernels(cuda):
 
 @pytest.mark.parametrize("micro_batches", [1, 2])
 def test_repeated_plain_calls_equal_the_first(cuda, params, micro_batches):
-    """From its third call for a shape on ``forward`` replays a recorded graph: same bits as the launches it recorded, for
+    """From its third consecutive call for a shape on ``forward`` replays a recorded graph: same bits as the launches it recorded, for
     new inputs, after a change of shape, on another stream, and inside a caller's own capture."""
     enc, ref = (Fp16Encoder(CFG, params, cuda, micro_batches=micro_batches) for _ in range(2))
     mk = lambda s, B, S: tdev(rng(s).integers(0, CFG.vocab, (B, S)), (S - rng(s).integers(0, S // 2, B)).astype(np.int32), cuda)

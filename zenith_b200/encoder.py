@@ -336,7 +336,8 @@ class _EncoderBase:
     # Unpadded form: the valid tokens of the batch are packed back to back (sequence b in rows cu_seqlens[b] ..),
     # the row-wise kernels and GEMMs run on ``capacity`` rows instead of B * S, attention takes its sequences
     # from the offsets, and the last launch spreads the rows back out (zeros at padding positions).  Every
-    # valid token's result equals the padded pass's, bit for bit.
+    # valid token's result equals the padded pass's, bit for bit where both run the same attention kernel: sequences of
+    # more than 128 tokens, and shorter ones in the fused int8 form (elsewhere the last bits of fp16 sums differ).
     @staticmethod
     def unpadded_capacity(kv_lens, S: int) -> int:
         """Rows needed for these key lengths (host values), rounded up to a whole 128-row tile."""
