@@ -6,6 +6,7 @@ int8 encoder  : every int8 GEMM of every layer is checked BIT-EXACTLY against th
                 quantization of the fp16 tensors beside them, and the final hidden states track the
                 oracle's int8 encoder and the fp32 encoder.
 """
+import ctypes
 import threading
 
 import numpy as np
@@ -311,6 +312,24 @@ def test_a_recording_that_fails_is_closed(cuda, params, error):
     for _ in range(4):
         assert torch.equal(enc.forward(ids, lens), want)
     assert enc._pass_graph is not None  # another shape in between: recorded anew
+
+
+def test_a_pass_goes_into_the_callers_recording(cuda, params):
+    """Between zen_record_begin and zen_record_end of the caller, whatever call it is that would record itself."""
+    enc = Fp16Encoder(CFG, params, cuda)
+    ids, lens = tdev(rng(8).integers(0, CFG.vocab, (2, 40)).astype(np.int32), np.array([40, 17], np.int32), cuda)
+    want = enc.forward(ids, lens).clone()
+    enc.forward(ids, lens)
+    lib, graph = _capi.lib(), ctypes.c_void_p()
+    assert lib.zen_record_begin() == _capi.OK and lib.zen_record_begin() == _capi.ERR_INVALID_ARG
+    out = enc.forward(ids, lens)
+    assert lib.zen_memcpy_async(out.data_ptr(), want.data_ptr(), 16, None) == _capi.ERR_UNSUPPORTED
+    assert lib.zen_record_end(ctypes.byref(graph)) == _capi.OK and lib.zen_record_end(None) == _capi.ERR_INVALID_ARG
+    out.zero_()
+    enc.inputs.zero_()
+    _capi.call("zen_graph_launch", graph, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(out, want)
+    _capi.call("zen_graph_destroy", graph)
 
 
 def other_threads_work():

@@ -285,7 +285,8 @@ class _EncoderBase:
     def _record(self) -> "_RecordedPass | None":
         """The pass as a graph; None where a launch refuses to be recorded (issued as it is, it then says why)."""
         lib = _capi.lib()
-        _capi.check("zen_record_begin", lib.zen_record_begin())
+        if lib.zen_record_begin() != _capi.OK:  # e.g. the caller's own recording is open: the pass goes into it
+            return None
         graph = ctypes.c_void_p()
         keep = None
         try:
