@@ -1,0 +1,23 @@
+"""Every wait of a kernel is bounded: what the sources may and may not use to wait.
+
+A wait that has run out lets its warp leave the loop on its own, so nothing that waits without a limit may stand where such a
+warp is missed.  A kernel that hangs cannot be made to fail on purpose on a GPU, so this reads the sources."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "zenith_b200" / "csrc"
+SOURCES = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")])}
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_no_named_barriers(name):
+    """Warps of a group meet at an mbarrier (``mbar_wait`` has a limit), never at ``bar.sync`` / ``barrier.sync``."""
+    assert not re.search(r"\bbar(rier)?\.(cta\.)?(sync|arrive|red)\b", SOURCES[name])
+
+
+@pytest.mark.parametrize("name", [n for n in SOURCES if n != "zen_common.cuh"])
+def test_mbarriers_are_polled_with_a_limit(name):
+    """``mbarrier.try_wait`` / ``test_wait`` stand only in the helpers that ``mbar_wait`` and ``mbar_wait_cluster`` bound."""
+    assert not re.search(r"mbarrier\.(try|test)_wait|mbar_try_wait", SOURCES[name])

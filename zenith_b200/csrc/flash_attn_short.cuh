@@ -182,8 +182,9 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       const int kv_len = keys_of(b);
       float l_sum = 0.f;
       if constexpr (F32) {
-        // (the output of the item before is staged in its Q tile, by every warp)
-        if (item != int(blockIdx.x) + g * int(gridDim.x)) asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory");
+        // The output of the item before is staged in its Q tile, by every warp.  (A bounded wait, unlike bar.sync: a warp whose
+        // wait for S or O has run out never comes here.)
+        if (item != int(blockIdx.x) + g * int(gridDim.x) && !__all_sync(0xffffffffu, mbar_wait(&free_bar[g], ph ^ 1u, abort_flag))) break;
         uint8_t* tile = tiles + g * 3 * TILE_BYTES;
         const int t = int(threadIdx.x) - 128 - g * 128;
         const int64_t at = int64_t(item) * p.S * D;
@@ -261,7 +262,7 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       tc_fence_after_sync();
       fa_write_output<D>(p, tiles + g * 3 * TILE_BYTES + quad * 4096, tmem_o, kv_len > 0, l_sum, lane, quad * 32, p.S, b, h, 0);
       tc_fence_before_sync();
-      fence_proxy_async_smem();  // the next item's Q tile is loaded over the staged rows
+      fence_proxy_async_smem();  // the next item's Q tile is loaded (or converted) over the staged rows
       mbar_arrive(&free_bar[g]);
       ph ^= 1u;
     }
