@@ -21,3 +21,14 @@ def test_no_named_barriers(name):
 def test_mbarriers_are_polled_with_a_limit(name):
     """``mbarrier.try_wait`` / ``test_wait`` stand only in the helpers that ``mbar_wait`` and ``mbar_wait_cluster`` bound."""
     assert not re.search(r"mbarrier\.(try|test)_wait|mbar_try_wait", SOURCES[name])
+
+
+@pytest.mark.parametrize("name", ["gemm_small.cuh"])
+def test_a_cta_leaves_its_shared_memory_after_its_peers_are_through_with_it(name):
+    """A CTA whose waits have run out has not seen all that its peers write to it: the tear-down of a kernel with such writes
+    (behind its last ``__syncthreads``) holds a wait for every CTA of the cluster."""
+    text = SOURCES[name]
+    writes = [m.end() for m in re.finditer(r"map_to_cta\(", text)]
+    body = text[writes[-1]:]
+    tear_down = body[body.index("__syncthreads();"):]
+    assert re.search(r"cluster_(leave|sync_all)\(", tear_down[:tear_down.index("\n}\n")])

@@ -446,10 +446,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   }
 
-  // No cluster-wide rendezvous: a CTA has waited for everything its peers write here before it leaves.
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, BN);
+  // No rendezvous: a CTA has waited for everything its peers write here, unless a wait has run out.  (A pass of 24 tokens, 48 of
+  // these products: 288.7 us without the check, 290.4 with it, 302 against 293 with an arrival before the exchange and a wait here.)
+  if (warp == 1) {
+    tmem_dealloc(tmem, BN);
+    cluster_leave(abort_flag);
+  }
 }
 
 }  // namespace zen

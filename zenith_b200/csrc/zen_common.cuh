@@ -199,6 +199,18 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The end of a CTA whose peers write to its shared memory, for one of its warps behind the last __syncthreads(); the other warps
+// exit.  A CTA whose waits have all been met has seen everything that its peers send and leaves.  One with a wait that has run out
+// stays until its peers send no more: threads that have exited count as arrived, so nobody else need arrive, and every CTA ends
+// (its waits are bounded).  What a peer sent last is then given time to land.
+__device__ __forceinline__ void cluster_leave(volatile int* abort_flag) {
+  if (!*abort_flag) return;
+  asm volatile("barrier.cluster.arrive;" ::: "memory");
+  asm volatile("barrier.cluster.wait;" ::: "memory");
+#pragma unroll 1
+  for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
+
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, no multicast anywhere in this library)
 // ---------------------------------------------------------------------------
