@@ -23,7 +23,7 @@ def test_mbarriers_are_polled_with_a_limit(name):
     assert not re.search(r"mbarrier\.(try|test)_wait|mbar_try_wait", SOURCES[name])
 
 
-@pytest.mark.parametrize("name", ["gemm_small.cuh"])
+@pytest.mark.parametrize("name", ["gemm_small.cuh", "gemm_ln.cu", "gemm_pair.cuh"])
 def test_a_cta_leaves_its_shared_memory_after_its_peers_are_through_with_it(name):
     """A CTA whose waits have run out has not seen all that its peers write to it: the tear-down of a kernel with such writes
     (behind its last ``__syncthreads``) holds a wait for every CTA of the cluster."""

@@ -448,8 +448,11 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
   __syncthreads();
   // No cluster-wide rendezvous here: the only accesses a peer makes to this CTA's shared memory are the partial
   // statistics of a tile and the arrival that follows them, and this CTA has waited for all of them (stats_bar of
-  // its last tile) before it got here; a peer publishes nothing after its last tile.
-  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  // its last tile) before it got here, unless a wait has run out; a peer publishes nothing after its last tile.
+  if (warp == 1) {
+    tmem_dealloc(tmem_base, TMEM_COLS);
+    cluster_leave(abort_flag);
+  }
 }
 
 template <int BN, int STAGES>
