@@ -32,3 +32,19 @@ def test_a_cta_leaves_its_shared_memory_after_its_peers_are_through_with_it(name
     body = text[writes[-1]:]
     tear_down = body[body.index("__syncthreads();"):]
     assert re.search(r"cluster_(leave|sync_all)\(", tear_down[:tear_down.index("\n}\n")])
+
+
+@pytest.mark.parametrize("name", [n for n in SOURCES if n not in ("zen_common.cuh", "selftest.cu")])
+def test_the_lanes_of_a_warp_give_up_together(name):
+    """``mbar_wait`` is for single threads (inside ``if (.. elect_one()) {``); warps wait with the ``_warp`` forms, whose lanes all
+    get the same answer, as instructions of the whole warp follow."""
+    text = SOURCES[name]
+    elected = []
+    for m in re.finditer(r"elect_one\(\)\) \{", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        elected.append((m.end(), i))
+    for m in re.finditer(r"\bmbar_wait(_cluster)?\(", text):
+        assert any(lo <= m.start() < hi for lo, hi in elected), text[m.start():m.start() + 80]

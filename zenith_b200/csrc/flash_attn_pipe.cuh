@@ -452,10 +452,10 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     uint32_t ph = 1;
     for (int j = 0; j < n_blocks; ++j) {
       const int64_t at = base + int64_t(j) * 128 * D;
-      if (!__all_sync(0xffffffffu, mbar_wait(&k_empty[st], ph, abort_flag))) break;
+      if (!mbar_wait_warp(&k_empty[st], ph, abort_flag)) break;
       fa_convert_tile<D>(sK + st * TILE_BYTES, p.k32 + at, p.S - j * 128, 128, t);
       fa_tile_ready(&k_full[st], lane);
-      if (!__all_sync(0xffffffffu, mbar_wait(&v_empty[st], ph, abort_flag))) break;
+      if (!mbar_wait_warp(&v_empty[st], ph, abort_flag)) break;
       fa_convert_tile<D>(sV + st * TILE_BYTES, p.v32 + at, p.S - j * 128, 128, t);
       fa_tile_ready(&v_full[st], lane);
       if (++st == KV_STAGES) {
@@ -489,7 +489,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
 
     for (int j = 0; j < nb; ++j) {
-      if (!mbar_wait(&s_full[g], j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[g], j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t sv[4][32];
       __syncwarp();
@@ -528,7 +528,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.0f);
       // P V of the previous block has completed: P may be overwritten, O may be rescaled
       if (j > 0) {
-        if (!mbar_wait(&o_full[g], (j - 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&o_full[g], (j - 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
       }
       if (rescale) {
@@ -575,10 +575,10 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
 
     if (ok && nb > 0) {
-      if (!mbar_wait(&o_full[g], (nb - 1) & 1, abort_flag)) ok = false;
+      ok = mbar_wait_warp(&o_full[g], (nb - 1) & 1, abort_flag);
       tc_fence_after_sync();
     }
-    if (__all_sync(0xffffffffu, ok)) {
+    if (ok) {
       // the Q tile has been read for the last time by Q K^T of the last block
       fa_write_output<D>(p, sQ + g * TILE_BYTES + quad * 4096, tmem_o, nb > 0, l_run, lane, q0 + g * 128 + quad * 32, q_len, b, h, row_base);
     }

@@ -167,7 +167,7 @@ flash_attn_quad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
 
     for (int j = 0; j < nb; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, j & 1, abort_flag))) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       if (j * FAQ_KEYS < warp_end) {
         uint32_t sv[64];
@@ -241,10 +241,10 @@ flash_attn_quad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
 
     if (ok && nb > 0) {
-      if (!mbar_wait(o_full, 0, abort_flag)) ok = false;
+      ok = mbar_wait_warp(o_full, 0, abort_flag);
       tc_fence_after_sync();
     }
-    if (__all_sync(0xffffffffu, ok)) {
+    if (ok) {
       // the Q tile has been read for the last time by Q K^T of the last block
       fa_write_output<64>(p, sQ + quad * 4096, tmem_o, nb > 0, l_run, lane, qw, q_len, b, h, row_base);
     }

@@ -184,7 +184,7 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       if constexpr (F32) {
         // The output of the item before is staged in its Q tile, by every warp.  (A bounded wait, unlike bar.sync: a warp whose
         // wait for S or O has run out never comes here.)
-        if (item != int(blockIdx.x) + g * int(gridDim.x) && !__all_sync(0xffffffffu, mbar_wait(&free_bar[g], ph ^ 1u, abort_flag))) break;
+        if (item != int(blockIdx.x) + g * int(gridDim.x) && !mbar_wait_warp(&free_bar[g], ph ^ 1u, abort_flag)) break;
         uint8_t* tile = tiles + g * 3 * TILE_BYTES;
         const int t = int(threadIdx.x) - 128 - g * 128;
         const int64_t at = int64_t(item) * p.S * D;
@@ -202,7 +202,7 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         n_plain = min(n_plain, quad);
         lim = min(lim, q + 1);
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[g], ph, abort_flag))) break;
+      if (!mbar_wait_warp(&s_full[g], ph, abort_flag)) break;
       tc_fence_after_sync();
       // the row maximum, 64 columns a step
       float mx = -INFINITY;
@@ -258,7 +258,7 @@ flash_attn_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(&p_full[g]);
-      if (!__all_sync(0xffffffffu, mbar_wait(&o_full[g], ph, abort_flag))) break;
+      if (!mbar_wait_warp(&o_full[g], ph, abort_flag)) break;
       tc_fence_after_sync();
       fa_write_output<D>(p, tiles + g * 3 * TILE_BYTES + quad * 4096, tmem_o, kv_len > 0, l_sum, lane, quad * 32, p.S, b, h, 0);
       tc_fence_before_sync();

@@ -182,7 +182,7 @@ flash_attn_tri_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
       };
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, 0, abort_flag))) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, 0, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t sv[64];
       tmem_ld_32x64(tmem_s, sv);
@@ -192,7 +192,7 @@ flash_attn_tri_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       for (int c = 0; c < 2; ++c)
         if (lim_warp < 32 * (c + 1)) mask_scores(sv + 32 * c, lim - 32 * c);
       float mx = fmaxf(max32(sv), max32(sv + 32));
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, 1, abort_flag))) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -256,10 +256,10 @@ flash_attn_tri_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     }
 
     if (ok && nb > 0) {
-      if (!mbar_wait(o_full, 0, abort_flag)) ok = false;
+      ok = mbar_wait_warp(o_full, 0, abort_flag);
       tc_fence_after_sync();
     }
-    if (__all_sync(0xffffffffu, ok)) {
+    if (ok) {
       // the Q tile has been read for the last time by Q K^T of the last block
       fa_write_output<64>(p, sQ + quad * 4096, tmem_o, nb > 0, l_run, lane, qw, q_len, b, h, row_base);
     }

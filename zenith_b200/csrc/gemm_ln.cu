@@ -270,8 +270,8 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
           tma_load_2d(sty, &tmap_r, &res_bar[ew], n0, m0 + quad * 32);
         }
         __syncwarp();
-        if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
-        if (!mbar_wait(&res_bar[ew], uint32_t(it) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&res_bar[ew], uint32_t(it) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(acc * BN + sub * 64);
 
@@ -330,7 +330,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
         pstats[sub * 128 + r] = make_float2(mean, m2);
         mbar_arrive(slab_bar);
         if (sub == 0) {
-          if (!mbar_wait(slab_bar, uint32_t(it) & 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(slab_bar, uint32_t(it) & 1u, abort_flag)) { ok = false; break; }
           // one thread per row: this CTA's BN columns, published to all four CTAs of the cluster
           float c = 64.f, mu = mean, q2 = m2;
 #pragma unroll
@@ -352,7 +352,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
           }
         }
         // ---- all four partials of every row have arrived (phase of stats_bar[par] flips every 2 tiles)
-        if (!mbar_wait_cluster(&stats_bar[par], uint32_t(it >> 1) & 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_cluster_warp(&stats_bar[par], uint32_t(it >> 1) & 1u, abort_flag)) { ok = false; break; }
         float c = float(BN), mu, q2;
         {
           const float2 o0 = xstats[(par * LN_CLUSTER + 0) * 128 + r];
@@ -436,7 +436,7 @@ __device__ __forceinline__ void gemm_ln_body(const CUtensorMap& tmap_a, const CU
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int mt = cluster_id; mt < p.tiles_m; mt += num_clusters) {
-        if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, abort_flag)) break;
         mbar_arrive(&tempty_bar[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;

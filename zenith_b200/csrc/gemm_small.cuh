@@ -208,7 +208,7 @@ __device__ __forceinline__ void load_b_transposed(const GemmSmallParams& sp, uin
       for (int u = 0; u < 2; ++u) {
         bar[u] = &full_bar[st];
         if (first + i + u < nkb) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[st], phase, abort_flag))) return;
+          if (!mbar_wait_warp(&empty_bar[st], phase, abort_flag)) return;
           uint8_t* tile = smem + size_t(st) * STAGE_BYTES + A_BYTES;
 #pragma unroll
           for (int c = 0; c < COLS; ++c) {
@@ -390,10 +390,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const float risk_thr = 0.5f - 2e-6f - inv_scale * fmaf(4.2e-7f, bmax, 1.6e-7f);  // see requant_i8_step
     __syncwarp();
     if constexpr (LOAD_B) load_b_transposed<BN, STAGES, STAGE_BYTES, A_BYTES>(sp, smem, full_bar, empty_bar, kb0, nkb, n0, ew, lane, abort_flag);
-    bool ok = mbar_wait(tfull_bar, 0, abort_flag);
+    bool ok = mbar_wait_warp(tfull_bar, 0, abort_flag);
     tc_fence_after_sync();
     const uint32_t tacc = tmem + (uint32_t(quad * 32) << 16);
-    if (__all_sync(0xffffffffu, ok)) {
+    if (ok) {
       // this CTA's partials of the columns that the peers finish
 #pragma unroll 1
       for (int i = 1; i < KS; ++i) {
@@ -413,9 +413,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       }
-      ok = mbar_wait_cluster(xbar, 0, abort_flag);
+      ok = mbar_wait_cluster_warp(xbar, 0, abort_flag);
     }
-    if (__all_sync(0xffffffffu, ok)) {
+    if (ok) {
       const int elem = p.out_dtype == ZEN_DT_S8 ? 1 : p.out_dtype == ZEN_DT_F16 ? 2 : 4;
       const bool vec_ok = (reinterpret_cast<uintptr_t>(p.out) % 16 == 0) && ((p.ldo * elem) % 16 == 0);
 #pragma unroll
@@ -449,7 +449,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   // No rendezvous: a CTA has waited for everything its peers write here, unless a wait has run out.  (A pass of 24 tokens, 48 of
-  // these products: 288.7 us without the check, 290.4 with it, 302 against 293 with an arrival before the exchange and a wait here.)
+  // these products: 292.8 us without the check, 293.1 with it, 302 with an arrival before the exchange and a wait here.)
   if (warp == 1) {
     tmem_dealloc(tmem, BN);
     cluster_leave(abort_flag);

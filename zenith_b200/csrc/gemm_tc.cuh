@@ -579,7 +579,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
         if (lane == 0) tma_store_wait_read();  // the previous tile's store has finished reading the block
       }
       __syncwarp();
-      if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) break;
+      if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, abort_flag)) break;
       tc_fence_after_sync();
       const int row = m0 + quad * 32 + lane;
       const bool row_ok = row < p.M;
@@ -650,7 +650,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const CU
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = first_tile; tile < num_tiles; tile += tile_step) {
-      if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) break;
+      if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, abort_flag)) break;
       tc_fence_before_sync();
       release_accumulator<PAIR>(tempty, acc, lane);
       acc ^= 1;

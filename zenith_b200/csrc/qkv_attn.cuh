@@ -323,10 +323,10 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         // the staging rows of the Q / K tiles before any thread of the group writes Q / K / P rows again
         if (!PACKED && half == 0 && lane == 0) tma_store_wait_read();
         mbar_arrive(&wg_bar[set]);
-        if (!mbar_wait(&wg_bar[set], it & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(&wg_bar[set], it & 1u, abort_flag)) break;
       }
       // ---- projection epilogue: this thread's 96 of the row's 192 accumulators -> fp16 Q, K, V in shared memory
-      if (!mbar_wait(&acc_full[set], it & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&acc_full[set], it & 1u, abort_flag)) break;
       tc_fence_after_sync();
 #pragma unroll 1
       for (int k = 0; k < 6; ++k) {
@@ -365,7 +365,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       mbar_arrive(&qkv_ready[set]);
 
       // ---- softmax (the arithmetic of flash_attn_short_kernel): this thread's 64 of the row's 128 keys
-      if (!mbar_wait(&s_full[set], it & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&s_full[set], it & 1u, abort_flag)) break;
       tc_fence_after_sync();
       const int lim = kv_len;
       float mx = -INFINITY;
@@ -389,7 +389,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
       x_max[half * 128 + r] = mx;
       mbar_arrive(&my_pair[0]);
-      if (!mbar_wait(&my_pair[0], it & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&my_pair[0], it & 1u, abort_flag)) break;
       mx = fmaxf(mx, x_max[(half ^ 1) * 128 + r]);  // the row maximum over all valid keys, as one thread would find it
       const float m_use = mx == -INFINITY ? 0.f : mx * p.scale_log2;
       float csum[2] = {0.f, 0.f};  // this thread's two 32-key chunks
@@ -454,9 +454,9 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
       // ---- output: O / rowsum -> fp16 (+ int8 copy) for this thread's 32 of the 64 columns, staged in the rows of
       //      the Q / K tiles that belong to this pair of warps
-      if (!mbar_wait(&o_full[set], it & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&o_full[set], it & 1u, abort_flag)) break;
       tc_fence_after_sync();
-      if (!mbar_wait(&my_pair[1], it & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&my_pair[1], it & 1u, abort_flag)) break;
       const float l_sum = (x_sum[r] + x_sum[128 + r]) + x_sum[256 + r];
       const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
       uint8_t* sty = sQ + quad * 4096;  // 32 rows x 128 B, 128-byte swizzle
@@ -502,7 +502,7 @@ qkv_attn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       mbar_arrive(&my_pair[2]);
       if (half == 0) {
         // both warps of the pair have staged their halves of the 32 rows
-        if (!mbar_wait(&my_pair[2], it & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(&my_pair[2], it & 1u, abort_flag)) break;
         if (PACKED) {
           // Box-shaped stores would write the rows of the next sequence: the valid rows leave with plain stores,
           // consecutive lanes taking consecutive 16-byte pieces of a row (whole 128-byte lines per row).

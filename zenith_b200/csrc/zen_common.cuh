@@ -144,6 +144,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same for all lanes of a converged warp, which go on or give up together: what follows are instructions of the whole warp
+// (tensor-memory loads, __syncwarp), and a lane that left alone would be missed there without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // ---------------------------------------------------------------------------
 // thread-block clusters: rank, addresses of a peer CTA's shared memory, remote barrier arrivals
 // ---------------------------------------------------------------------------
@@ -191,6 +197,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
       }
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
 }
 // All threads of all CTAs of the cluster.  Hardware barrier: it cannot be given a time limit, so it is only
 // used where every CTA is certain to arrive (set-up and tear-down, outside any data-dependent wait).
