@@ -311,6 +311,20 @@ int zen_flash_attention_f16(const void* q, const void* k, const void* v, void* o
                             int64_t k_ss, int64_t v_sb, int64_t v_sh, int64_t v_ss, int64_t o_sb, int64_t o_sh,
                             int64_t o_ss, const int32_t* kv_lens, int causal, float scale, void* stream);
 
+/* zen_flash_attention_f16 with per-call options.  At head size 64, beyond 128 tokens and without an int8 copy the keys are taken
+ * 64 or 128 at a time, by the number of query tiles in the call (batch, heads, S): the two differ in the last bits.
+ *   ZEN_ATTN_KEYS_64 / _128  take them so whatever the number of tiles; no effect where there is one form (other head sizes,
+ *                            S <= 128, with an int8 copy).
+ * zen_attention_plan: the flag that the library would choose.  A caller that runs parts of a batch passes the flag of the
+ * whole everywhere: every sequence then keeps its bits.  No counterpart in the reference. */
+#define ZEN_ATTN_KEYS_64 0x1u
+#define ZEN_ATTN_KEYS_128 0x2u
+unsigned zen_attention_plan(int B, int H, int S, int D, int causal, int int8_copy);
+int zen_flash_attention_f16_ex(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale, int B,
+                               int H, int S, int D, int64_t q_sb, int64_t q_sh, int64_t q_ss, int64_t k_sb, int64_t k_sh,
+                               int64_t k_ss, int64_t v_sb, int64_t v_sh, int64_t v_ss, int64_t o_sb, int64_t o_sh,
+                               int64_t o_ss, const int32_t* kv_lens, int causal, float scale, unsigned flags, void* stream);
+
 /* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
  * computed in fp16 with fp32 softmax and accumulation.  The attention kernel converts the operands of few tiles itself
  * (zen_flash_attention_f32_direct); otherwise two launches: the operands to fp16 in `workspace`
@@ -363,11 +377,15 @@ int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S,
 /* zen_flash_attention_unpadded_f16: zen_flash_attention_f16 on packed tensors: token t of Q sits at q + t*q_st + h*q_sh + d
  * (likewise K, V, O), sequence b owns tokens cu_seqlens[b] .. cu_seqlens[b + 1] - 1 (cut at `rows`; at most max_seqlen
  * each: a longer one is cut to its first max_seqlen tokens), causal counts positions within the sequence.  Any
- * sequence length; rows that belong to no sequence are left unwritten. */
+ * sequence length; rows that belong to no sequence are left unwritten.  _ex: as zen_flash_attention_f16_ex. */
 int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale, int B,
                                      int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh, int64_t k_st,
                                      int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st, int64_t o_sh,
                                      const int32_t* cu_seqlens, int causal, float scale, void* stream);
+int zen_flash_attention_unpadded_f16_ex(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale, int B,
+                                        int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh, int64_t k_st,
+                                        int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st, int64_t o_sh,
+                                        const int32_t* cu_seqlens, int causal, float scale, unsigned flags, void* stream);
 int zen_pack_tokens_i32(const int32_t* ids, const int32_t* type_ids, const int32_t* kv_lens, int B, int S, int capacity,
                         int32_t* cu_seqlens, int32_t* ids_packed, int32_t* pos_packed, int32_t* type_packed, void* stream);
 int zen_embed_layernorm_unpadded_f16(const int32_t* ids_packed, const int32_t* pos_packed, const int32_t* type_packed,

@@ -270,6 +270,23 @@ def test_repeated_plain_calls_equal_the_first(cuda, params, micro_batches):
     assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("S,micro_batches", [(256, 2), (256, 5), (144, 3)])
+def test_fp16_micro_batches_keep_the_bits_of_the_batch(cuda, S, micro_batches):
+    """A batch of tiles enough for 64 keys at a time in attention, cut into parts that have too few by themselves."""
+    cfg = EncoderConfig(layers=2, hidden=768, heads=12, ffn=1024, vocab=2000, max_pos=256)
+    params = init_params(cfg, 3, random_affine=True)
+    B = 32
+    plan = _capi.lib().zen_attention_plan
+    assert plan(B, 12, S, 64, 0, 0) == _capi.ATTN_KEYS_64 and plan(B // micro_batches, 12, S, 64, 0, 0) == _capi.ATTN_KEYS_128
+    ids, lens = tdev(rng(1).integers(0, cfg.vocab, (B, S)), (S - rng(2).integers(0, S, B)).astype(np.int32), cuda)
+    want = Fp16Encoder(cfg, params, cuda).forward(ids, lens)
+    enc = Fp16Encoder(cfg, params, cuda, micro_batches=micro_batches)
+    assert torch.equal(enc.forward(ids, lens), want)
+    enc.capture(B, S)
+    enc.set_inputs(ids, lens)
+    assert torch.equal(enc.replay(), want)
+
+
 def third_call(enc, ids, lens, during):
     """The call that records, with ``during()`` run between two of the recorded launches."""
     issue, calls = enc._issue, []

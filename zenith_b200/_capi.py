@@ -18,6 +18,7 @@ DT_S32, DT_F32, DT_F16, DT_S8 = range(4)
 ACT_NONE, ACT_GELU, ACT_RELU = range(3)
 ROUND_NEAREST_EVEN, ROUND_TRUNC = range(2)
 GEMM_CONST_WEIGHTS, GEMM_NO_PAIR, GEMM_PAIR, GEMM_NARROW = 0x1, 0x2, 0x4, 0x1000000
+ATTN_KEYS_64, ATTN_KEYS_128 = 0x1, 0x2
 
 
 def gemm_tile_n(bn: int) -> int:
@@ -82,6 +83,8 @@ SIGNATURES = {
     "zen_quantize_f16": [_p, _p, _i64, _f, _i, _i, _p],
     "zen_dequantize_f32": [_p, _p, _i64, _f, _i, _p],
     "zen_flash_attention_f16": [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i] + [_i64] * 12 + [_p, _i, _f, _p],
+    "zen_attention_plan": [_i, _i, _i, _i, _i, _i],
+    "zen_flash_attention_f16_ex": [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i] + [_i64] * 12 + [_p, _i, _f, _u, _p],
     "zen_flash_attention_f32_workspace_bytes": [_i, _i, _i, _i],
     "zen_flash_attention_f32_direct": [_p, _p, _p, _p, _i, _i, _i, _i, _p, _i, _f, _p],
     "zen_flash_attention_f32": [_p, _p, _p, _p, _i, _i, _i, _i, _p, _i, _f, _p, C.c_size_t, _p],
@@ -102,6 +105,8 @@ SIGNATURES = {
     "zen_quantize_e4m3_f16": [_p, _p, _i64, _f, _p],
     "zen_flash_attention_unpadded_f16": [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                                          _i64, _i64, _p, _i, _f, _p],
+    "zen_flash_attention_unpadded_f16_ex": [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
+                                            _i64, _i64, _p, _i, _f, _u, _p],
     "zen_set_inputs_i32": [_p, _p, _i, _i, _p, _p],
     "zen_pack_tokens_i32": [_p, _p, _p, _i, _i, _i, _p, _p, _p, _p, _p],
     "zen_embed_layernorm_unpadded_f16": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _f, _i, _i, _i, _i, _i, _f, _p],
@@ -110,7 +115,7 @@ SIGNATURES = {
     "zen_unpad_rows_f16": [_p, _p, _i, _i, _i, _i, _p, _p],
 }
 _RESTYPES = {"zen_status_string": C.c_char_p, "zen_matmul_f32_workspace_bytes": C.c_size_t,
-             "zen_minmax_workspace_bytes": C.c_size_t, "zen_gemm_plan": C.c_uint,
+             "zen_minmax_workspace_bytes": C.c_size_t, "zen_gemm_plan": C.c_uint, "zen_attention_plan": C.c_uint,
              "zen_flash_attention_f32_workspace_bytes": C.c_size_t}
 
 _lib = None

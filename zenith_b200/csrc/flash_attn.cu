@@ -145,13 +145,16 @@ static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CU
 //           3 on: 0.77 - 0.87    1500 .. 4096: below 1 from 1.5, 2, 2.2, 2.2 on, 0.9 - 0.95 from 3 on; longer: 1.03 - 1.1
 // (32 x 16 x 384 full: 44.2 -> 37.6 us; 8 x 16 x 2048 causal: 113.5 -> 105.5 us.)  The two kernels differ in the last bits, which
 // a pass of int8 layers blows up to 3 % of its output (a value moved across a rounding boundary moves others): results with
-// an int8 copy stay with one kernel, whatever the batch.
-static bool four_tiles_per_sm(int D, const FaParams& p) {
-  if (p.oq != nullptr || D != 64 || p.S <= FA_BKV || p.S > (p.causal ? 4096 : 3072)) return false;
-  const double waves = double((p.S + 127) / 128) * p.H * p.B / (double(FAQ_CTAS) * num_sms());
-  if (p.causal) return waves >= (p.S <= 320 ? 0.8 : p.S <= 1100 ? 1.1 : p.S <= 2100 ? p.S / 1000.0 : 2.2);
-  return waves >= (p.S <= 768 ? 0.8 : p.S / 650.0);
+// an int8 copy stay with one kernel, whatever the batch.  `flags`: ZEN_ATTN_KEYS_64 / _128 of the call.
+static bool four_tiles_per_sm(int B, int H, int S, int D, bool causal, bool int8_copy, unsigned flags) {
+  if (int8_copy || D != 64 || S <= FA_BKV) return false;
+  if (flags != 0) return flags == ZEN_ATTN_KEYS_64;
+  if (S > (causal ? 4096 : 3072)) return false;
+  const double waves = double((S + 127) / 128) * H * B / (double(FAQ_CTAS) * num_sms());
+  if (causal) return waves >= (S <= 320 ? 0.8 : S <= 1100 ? 1.1 : S <= 2100 ? S / 1000.0 : 2.2);
+  return waves >= (S <= 768 ? 0.8 : S / 650.0);
 }
+static bool attn_flags_ok(unsigned flags) { return flags <= ZEN_ATTN_KEYS_128; }  // either of the two, or neither
 
 // Head size 64, with the bits of flash_attn_pipe_kernel: flash_attn_tri_kernel, where the other would need more than two rounds
 // of its two CTAs an SM.  Measured for 50 shapes with int8 copy, time against the other kernel:
@@ -211,23 +214,24 @@ static int launch_fa_tri(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
   return launch_pdl(PDL_ATTENTION, flash_attn_tri_kernel, dim3(unsigned(ctas)), dim3(FAT_THREADS), smem, s, tq, tk, tv, p);
 }
 
-static int launch_fa_long(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FaParams p, cudaStream_t s) {
+// `quad`: four_tiles_per_sm, for which the boxes of K and V were made.
+static int launch_fa_long(int D, bool quad, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FaParams p, cudaStream_t s) {
   p.order = tile_order(D, p);
   if (D == 128) return launch_fa_pipe<128, 2, 2>(tq, tk, tv, p, s);
-  if (four_tiles_per_sm(D, p)) return launch_fa_quad(tq, tk, tv, p, s);
+  if (quad) return launch_fa_quad(tq, tk, tv, p, s);
   if (three_tiles_per_sm(D, p)) return launch_fa_tri(tq, tk, tv, p, s);
   return one_tile_per_cta(p) ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
 }
 
 // One key block holds the sequence up to 128 tokens.
-static int launch_fa(int D, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
-  if (p.S > FA_BKV) return launch_fa_long(D, tq, tk, tv, p, s);
+static int launch_fa(int D, bool quad, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
+  if (p.S > FA_BKV) return launch_fa_long(D, quad, tq, tk, tv, p, s);
   return D == 64 ? launch_fa_short<64>(tq, tk, tv, p, s) : launch_fa_short<128>(tq, tk, tv, p, s);
 }
 
 // The load engine works through the rows of a box that lie beyond the sequence too: one of 24 tokens loads 32 rows.
 static int fa_box_rows(int S) { return S >= FA_BKV ? FA_BKV : (S + 15) / 16 * 16; }
-static uint32_t fa_key_box_rows(int D, const FaParams& p) { return four_tiles_per_sm(D, p) ? FAQ_KEYS : uint32_t(fa_box_rows(p.S)); }
+static uint32_t fa_key_box_rows(bool quad, int S) { return quad ? FAQ_KEYS : uint32_t(fa_box_rows(S)); }
 
 }  // namespace zen
 
@@ -235,12 +239,25 @@ using namespace zen;
 
 ZEN_DEFINE_TU_STATUS(flash_attn)
 
+extern "C" unsigned zen_attention_plan(int B, int H, int S, int D, int causal, int int8_copy) {
+  return four_tiles_per_sm(B, H, S, D, causal != 0, int8_copy != 0, 0u) ? ZEN_ATTN_KEYS_64 : ZEN_ATTN_KEYS_128;
+}
+
 extern "C" int zen_flash_attention_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale,
                                        int B, int H, int S, int D, int64_t q_sb, int64_t q_sh, int64_t q_ss,
                                        int64_t k_sb, int64_t k_sh, int64_t k_ss, int64_t v_sb, int64_t v_sh,
                                        int64_t v_ss, int64_t o_sb, int64_t o_sh, int64_t o_ss, const int32_t* kv_lens,
                                        int causal, float scale, void* stream) {
-  if (!q || !k || !v || !o || B <= 0 || H <= 0 || S <= 0) return ZEN_ERR_INVALID_ARG;
+  return zen_flash_attention_f16_ex(q, k, v, o, oq, o_scale, B, H, S, D, q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh,
+                                    o_ss, kv_lens, causal, scale, 0u, stream);
+}
+
+extern "C" int zen_flash_attention_f16_ex(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale,
+                                          int B, int H, int S, int D, int64_t q_sb, int64_t q_sh, int64_t q_ss,
+                                          int64_t k_sb, int64_t k_sh, int64_t k_ss, int64_t v_sb, int64_t v_sh,
+                                          int64_t v_ss, int64_t o_sb, int64_t o_sh, int64_t o_ss, const int32_t* kv_lens,
+                                          int causal, float scale, unsigned flags, void* stream) {
+  if (!q || !k || !v || !o || B <= 0 || H <= 0 || S <= 0 || !attn_flags_ok(flags)) return ZEN_ERR_INVALID_ARG;
   if (D != 64 && D != 128) return ZEN_ERR_UNSUPPORTED;
   if (H > 65535 || B > 65535) return ZEN_ERR_UNSUPPORTED;
   if (oq && !(o_scale > 0.f)) return ZEN_ERR_INVALID_ARG;
@@ -252,13 +269,14 @@ extern "C" int zen_flash_attention_f16(const void* q, const void* k, const void*
   const SoftmaxScale sc = softmax_scale(scale);
   p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   p.box_rows = fa_box_rows(S);
+  const bool quad = four_tiles_per_sm(B, H, S, D, causal != 0, oq != nullptr, flags);
   CUtensorMap tq, tk, tv;
   int st = encode_qkv_map(&tq, q, B, H, S, D, q_sb, q_sh, q_ss, p.q_perm, uint32_t(p.box_rows));
-  if (st == ZEN_OK) st = encode_qkv_map(&tk, k, B, H, S, D, k_sb, k_sh, k_ss, p.k_perm, fa_key_box_rows(D, p));
-  if (st == ZEN_OK) st = encode_qkv_map(&tv, v, B, H, S, D, v_sb, v_sh, v_ss, p.v_perm, fa_key_box_rows(D, p));
+  if (st == ZEN_OK) st = encode_qkv_map(&tk, k, B, H, S, D, k_sb, k_sh, k_ss, p.k_perm, fa_key_box_rows(quad, S));
+  if (st == ZEN_OK) st = encode_qkv_map(&tv, v, B, H, S, D, v_sb, v_sh, v_ss, p.v_perm, fa_key_box_rows(quad, S));
   if (st != ZEN_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return launch_fa(D, tq, tk, tv, p, s);
+  return launch_fa(D, quad, tq, tk, tv, p, s);
 }
 
 extern "C" int zen_convert3_f32_to_f16(const float* a, const float* b, const float* c, void* y, int64_t n, void* stream);
@@ -319,12 +337,13 @@ extern "C" int zen_flash_attention_f32(const float* q, const float* k, const flo
   const SoftmaxScale sc = softmax_scale(scale);
   p.scale_log2 = sc.log2; p.qk_negate = sc.negate;
   p.box_rows = fa_box_rows(S);
+  const bool quad = four_tiles_per_sm(B, H, S, D, causal != 0, false, 0u);
   CUtensorMap tq, tk, tv;
   int st = encode_qkv_map(&tq, w, B, H, S, D, p.o_sb, p.o_sh, D, p.q_perm, uint32_t(p.box_rows));
-  if (st == ZEN_OK) st = encode_qkv_map(&tk, w + n, B, H, S, D, p.o_sb, p.o_sh, D, p.k_perm, fa_key_box_rows(D, p));
-  if (st == ZEN_OK) st = encode_qkv_map(&tv, w + 2 * n, B, H, S, D, p.o_sb, p.o_sh, D, p.v_perm, fa_key_box_rows(D, p));
+  if (st == ZEN_OK) st = encode_qkv_map(&tk, w + n, B, H, S, D, p.o_sb, p.o_sh, D, p.k_perm, fa_key_box_rows(quad, S));
+  if (st == ZEN_OK) st = encode_qkv_map(&tv, w + 2 * n, B, H, S, D, p.o_sb, p.o_sh, D, p.v_perm, fa_key_box_rows(quad, S));
   if (st != ZEN_OK) return st;
-  return launch_fa(D, tq, tk, tv, p, static_cast<cudaStream_t>(stream));
+  return launch_fa(D, quad, tq, tk, tv, p, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale,
@@ -332,7 +351,16 @@ extern "C" int zen_flash_attention_unpadded_f16(const void* q, const void* k, co
                                                 int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st,
                                                 int64_t o_sh, const int32_t* cu_seqlens, int causal, float scale,
                                                 void* stream) {
-  if (!q || !k || !v || !o || !cu_seqlens || B <= 0 || H <= 0 || max_seqlen <= 0 || rows <= 0) return ZEN_ERR_INVALID_ARG;
+  return zen_flash_attention_unpadded_f16_ex(q, k, v, o, oq, o_scale, B, H, max_seqlen, D, rows, q_st, q_sh, k_st, k_sh, v_st, v_sh, o_st,
+                                             o_sh, cu_seqlens, causal, scale, 0u, stream);
+}
+
+extern "C" int zen_flash_attention_unpadded_f16_ex(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale,
+                                                   int B, int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh,
+                                                   int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st,
+                                                   int64_t o_sh, const int32_t* cu_seqlens, int causal, float scale,
+                                                   unsigned flags, void* stream) {
+  if (!q || !k || !v || !o || !cu_seqlens || B <= 0 || H <= 0 || max_seqlen <= 0 || rows <= 0 || !attn_flags_ok(flags)) return ZEN_ERR_INVALID_ARG;
   if (D != 64 && D != 128) return ZEN_ERR_UNSUPPORTED;
   if (H > 65535 || B > 65535 || rows >= (int64_t(1) << 31)) return ZEN_ERR_UNSUPPORTED;
   if (oq && !(o_scale > 0.f)) return ZEN_ERR_INVALID_ARG;
@@ -347,13 +375,14 @@ extern "C" int zen_flash_attention_unpadded_f16(const void* q, const void* k, co
   // the packed tensors as ONE batch of `rows` tokens: a tile may start at any row
   CUtensorMap tq, tk, tv;
   const int R = int(rows);
-  const uint32_t key_rows = four_tiles_per_sm(D, p) ? FAQ_KEYS : FA_BKV;
+  const bool quad = four_tiles_per_sm(B, H, max_seqlen, D, causal != 0, oq != nullptr, flags);
+  const uint32_t key_rows = quad ? FAQ_KEYS : FA_BKV;
   int st = encode_qkv_map(&tq, q, 1, H, R, D, int64_t(R) * q_st, q_sh, q_st, p.q_perm);
   if (st == ZEN_OK) st = encode_qkv_map(&tk, k, 1, H, R, D, int64_t(R) * k_st, k_sh, k_st, p.k_perm, key_rows);
   if (st == ZEN_OK) st = encode_qkv_map(&tv, v, 1, H, R, D, int64_t(R) * v_st, v_sh, v_st, p.v_perm, key_rows);
   if (st != ZEN_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return launch_fa_long(D, tq, tk, tv, p, s);
+  return launch_fa_long(D, quad, tq, tk, tv, p, s);
 }
 
 // Shared body of the padded and the packed entry points.  Padded: S tokens per sequence, kv_lens optional.

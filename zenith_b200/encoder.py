@@ -463,6 +463,8 @@ class Fp16Encoder(_EncoderBase):
         fused_ln = self.fuse_layernorm
         self.launches_per_layer = 5 if fused_ln else 7
         ln_o, ln_2 = (self._ln_args(k, r0, T) for k in (H, F)) if fused_ln else (None, None)
+        # fp16 results depend on how many keys attention takes at a time: a micro-batch does as the whole batch would
+        attn = _capi.lib().zen_attention_plan(self._shape[0], nh, S, hd, 0, 0)
         self.lead_launches = 2 if packed else 1
         if packed:
             self._add("zen_pack_tokens_i32", self.ids.data_ptr(), None, self.kv_lens.data_ptr(), B, S, T,
@@ -483,12 +485,12 @@ class Fp16Encoder(_EncoderBase):
             self._add("zen_linear_f16_ex", P(x), H, L["wqkv"].data_ptr(), H, T, 3 * H, H, L["bqkv"].data_ptr(),
                       ACT_NONE, DT_F16, P(self.qkv), 3 * H, GF[3 * H, H])
             if packed:
-                self._add("zen_flash_attention_unpadded_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H,
+                self._add("zen_flash_attention_unpadded_f16_ex", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H,
                           P(self.ctx), None, 1.0, B, nh, S, hd, T, 3 * H, hd, 3 * H, hd, 3 * H, hd, H, hd,
-                          self.cu_seqlens.data_ptr(), 0, 1.0 / math.sqrt(hd))
+                          self.cu_seqlens.data_ptr(), 0, 1.0 / math.sqrt(hd), attn)
             else:
-                self._add("zen_flash_attention_f16", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H, P(self.ctx), None,
-                          1.0, B, nh, S, hd, *qs, *qs, *qs, *os_, kv, 0, 1.0 / math.sqrt(hd))
+                self._add("zen_flash_attention_f16_ex", P(self.qkv), P(self.qkv) + 2 * H, P(self.qkv) + 4 * H, P(self.ctx), None,
+                          1.0, B, nh, S, hd, *qs, *qs, *qs, *os_, kv, 0, 1.0 / math.sqrt(hd), attn)
             if fused_ln:
                 self._add("zen_linear_f16_add_layernorm_ws", P(self.ctx), H, L["wo"].data_ptr(), H, T, H, H,
                           L["bo"].data_ptr(), P(x), H, L["ln1_g"].data_ptr(), L["ln1_b"].data_ptr(), cfg.eps, P(self.h1),
