@@ -304,6 +304,9 @@ int zen_quantize_e4m3_f16(const void* x, uint8_t* q, int64_t n, float scale, voi
  * masks keys >= kv_lens[b]; a row with no valid key yields zeros.  causal keeps key <= query.
  * If oq != NULL the int8 copy clamp(round(o / o_scale)) is written with the O strides as well.
  * head_dim 64 or 128.
+ * At head size 64 beyond 128 tokens the last bits of a sequence's fp16 result depend on the rest of the call: on the number of
+ * query tiles, hence on B, H and S, and on whether an int8 copy is asked for, with which o and oq are the same in every batch;
+ * zen_flash_attention_f16_ex pins them.  The int8 copy is always that of the o of the same call.
  * Replaces core/src/flash_attention.cu:55-355 (tiled_attention_kernel, fp16 twin),
  * core/src/flash_attention_v2.cu:121-462 (causal), core/src/fp16_kernels.cu:416-456 (cuBLAS path). */
 int zen_flash_attention_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale, int B,
@@ -328,7 +331,8 @@ int zen_flash_attention_f16_ex(const void* q, const void* k, const void* v, void
 /* The fp32 binding's attention (core/bindings/cuda_bindings.cpp:90-106): contiguous fp32 [B, H, S, D] operands and result,
  * computed in fp16 with fp32 softmax and accumulation.  The attention kernel converts the operands of few tiles itself
  * (zen_flash_attention_f32_direct); otherwise two launches: the operands to fp16 in `workspace`
- * (zen_flash_attention_f32_workspace_bytes), attention with fp32 stores.  The same bits either way.  o and workspace 16-byte
+ * (zen_flash_attention_f32_workspace_bytes), attention with fp32 stores: the bits of zen_flash_attention_f16 on converted
+ * operands either way, which follow the number of query tiles as there.  o and workspace 16-byte
  * aligned; q, k and v may lie on any 4-byte boundary. */
 size_t zen_flash_attention_f32_workspace_bytes(int B, int H, int S, int D);
 int zen_flash_attention_f32(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
@@ -377,7 +381,8 @@ int zen_set_inputs_i32(const int32_t* ids, const int32_t* kv_lens, int B, int S,
 /* zen_flash_attention_unpadded_f16: zen_flash_attention_f16 on packed tensors: token t of Q sits at q + t*q_st + h*q_sh + d
  * (likewise K, V, O), sequence b owns tokens cu_seqlens[b] .. cu_seqlens[b + 1] - 1 (cut at `rows`; at most max_seqlen
  * each: a longer one is cut to its first max_seqlen tokens), causal counts positions within the sequence.  Any
- * sequence length; rows that belong to no sequence are left unwritten.  _ex: as zen_flash_attention_f16_ex. */
+ * sequence length; rows that belong to no sequence are left unwritten.  Last bits as in zen_flash_attention_f16, with
+ * max_seqlen as S whatever the lengths in the offsets; _ex: as zen_flash_attention_f16_ex. */
 int zen_flash_attention_unpadded_f16(const void* q, const void* k, const void* v, void* o, int8_t* oq, float o_scale, int B,
                                      int H, int max_seqlen, int D, int64_t rows, int64_t q_st, int64_t q_sh, int64_t k_st,
                                      int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t o_st, int64_t o_sh,

@@ -98,6 +98,30 @@ def test_attention_with_int8_copy_does_not_depend_on_the_batch(cuda, S, causal):
     assert torch.equal(out[0], out[1]) and torch.equal(quant[0], quant[1]) and torch.isfinite(out[0]).all()
 
 
+@pytest.mark.parametrize("S,causal", [(129, False), (200, True), (300, False), (513, True)])
+def test_pinned_attention_does_not_depend_on_the_batch(cuda, S, causal):
+    """``keys``: the bits of a sequence alone, in a large batch, packed, and with another max_seqlen; 128 are the bits beside an
+    int8 copy, and the two differ.  No value of it changes what there is one form of (short sequences, head size 128)."""
+    B, H = 64, 12
+    assert _capi.lib().zen_attention_plan(B, H, S, 64, causal, 0) == _capi.ATTN_KEYS_64
+    qkv = torch.from_numpy(rng(S).standard_normal((B * S, 3 * H * 64)).astype(np.float16)).to(cuda)
+    q, k, v = (t.contiguous() for t in qkv.view(B, S, 3, H, 64).permute(2, 0, 3, 1, 4))
+    cu = torch.arange(0, B * S + 1, S, dtype=torch.int32, device=cuda)
+    rows = lambda o: o.transpose(1, 2).reshape(B * S, H * 64)
+    full = {keys: ops.flash_attention(q, k, v, causal=causal, keys=keys) for keys in (None, 64, 128)}
+    assert torch.equal(full[None], full[64]) and not torch.equal(full[64], full[128])
+    for keys in (64, 128):
+        for b in (0, B - 1):
+            part = [t[b:b + 1] for t in (q, k, v)]
+            assert torch.equal(ops.flash_attention(*part, causal=causal, keys=keys), full[keys][b:b + 1])
+        for max_seqlen in (S, 4 * S):
+            assert torch.equal(ops.flash_attention_unpadded(qkv, cu, H, 64, max_seqlen, causal=causal, keys=keys), rows(full[keys]))
+    assert torch.equal(ops.flash_attention_unpadded(qkv, cu, H, 64, S, causal=causal, out_scale=0.02, keys=64)[0], rows(full[128]))
+    for shape in ((2, 3, 128, 64), (2, 3, 300, 128)):
+        x, y, z = (torch.randn(shape, device=cuda, dtype=torch.float16) for _ in range(3))
+        assert torch.equal(ops.flash_attention(x, y, z, keys=64), ops.flash_attention(x, y, z, keys=128))
+
+
 @pytest.mark.parametrize("B,H,S,D,causal", [(3, 2, 700, 128, False), (2, 11, 18432, 64, False), (3, 16, 8320, 128, True)])
 def test_attention_does_not_depend_on_the_order_of_tiles(cuda, B, H, S, D, causal):
     """Every order of query tiles, heads and batches (tiles first: full, d = 128 or K and V beyond L2; tiles before batches:

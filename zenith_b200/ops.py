@@ -561,19 +561,27 @@ def to_fp32(x):
 # --------------------------------------------------------------------------------------------
 # attention
 # --------------------------------------------------------------------------------------------
+def _keys_flag(keys) -> int:
+    """``ZEN_ATTN_KEYS_*`` of the ``keys`` that an operator was given."""
+    if keys not in (None, 64, 128):
+        raise RuntimeError("keys must be 64, 128 or None")
+    return 0 if keys is None else (_capi.ATTN_KEYS_64 if keys == 64 else _capi.ATTN_KEYS_128)
+
+
 def flash_attention_strided(q, k, v, out, B, H, S, D, q_strides, k_strides, v_strides, o_strides, *, kv_lens=None,
-                            causal=False, scale=None, out_q=None, out_scale=None):
-    """Attention over strided fp16 views: strides are (batch, head, seq) in elements, d contiguous."""
+                            causal=False, scale=None, out_q=None, out_scale=None, keys: int | None = None):
+    """Attention over strided fp16 views: strides are (batch, head, seq) in elements, d contiguous.  ``keys``: see
+    ``flash_attention``."""
     if kv_lens is not None:
         _require(kv_lens, "kv_lens", torch.int32, 1, like=q, at_least=B)
     scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
-    _call("zen_flash_attention_f16", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), _ptr(out_q),
+    _call("zen_flash_attention_f16_ex", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), _ptr(out_q),
           float(out_scale or 1.0), B, H, S, D, *q_strides, *k_strides, *v_strides, *o_strides, _ptr(kv_lens),
-          1 if causal else 0, scale, _stream())
+          1 if causal else 0, scale, _keys_flag(keys), _stream())
     return out
 
 
-def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float | None = None):
+def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float | None = None, keys: int | None = None):
     """``softmax(scale * Q K^T) V`` for ``[batch, heads, seq, dim]`` tensors.
 
     fp16 inputs run directly; fp32 inputs (the reference binding's dtype,
@@ -581,9 +589,12 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
     where it has few tiles, else in one launch in front of it), run on the tensor cores with fp32 softmax and
     accumulation, and returned as fp32 (written by the kernel).
     ``kv_lens[b]`` masks keys at positions >= kv_lens[b]; a row with no valid key yields zeros.
+    ``keys`` (fp16): how many keys the kernel takes at a time at head size 64 beyond 128 tokens, 64 or 128.  They differ in
+    the last bits, and by default the number of query tiles in the call decides; with ``keys`` given a sequence's result
+    has the same bits in every batch.
     """
     global launch_count
-    out = native.flash_attention(q, k, v, causal, kv_lens, scale)
+    out = native.flash_attention(q, k, v, causal, kv_lens, scale) if keys is None else None
     if out is not None:
         if type(out) is tuple:
             out, kernels = out
@@ -599,6 +610,8 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
         raise RuntimeError("K and V must have the shape of Q")
     B, H, S, D = q.shape
     if q.dtype == torch.float32:
+        if keys is not None:
+            raise RuntimeError("keys is for fp16 operands")
         q, k, v = (t.contiguous() for t in (q, k, v))
         for name, t in (("Q", q), ("K", k), ("V", v)):
             _require(t, name, torch.float32, 4, like=q)
@@ -622,7 +635,7 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
         _require(t, name, torch.float16, 4, like=q)
     out = torch.empty_like(q)
     st = (H * S * D, S * D, D)
-    flash_attention_strided(q, k, v, out, B, H, S, D, st, st, st, st, kv_lens=kv_lens, causal=causal, scale=scale)
+    flash_attention_strided(q, k, v, out, B, H, S, D, st, st, st, st, kv_lens=kv_lens, causal=causal, scale=scale, keys=keys)
     return out
 
 
@@ -830,11 +843,12 @@ def linear_fp8(xq, wq, x_scale: float, w_scale=None, bias=None, *, act="none", o
 
 
 def flash_attention_unpadded(qkv, cu_seqlens, heads: int, head_dim: int, max_seqlen: int, *, causal: bool = False,
-                             scale: float | None = None, out_scale: float | None = None):
+                             scale: float | None = None, out_scale: float | None = None, keys: int | None = None):
     """Attention on packed rows (``zen_flash_attention_unpadded_f16``): ``qkv`` fp16 ``[rows, 3 * heads * head_dim]``
     (columns Q | K | V, each head's columns together), sequence b in rows ``cu_seqlens[b] .. cu_seqlens[b+1]-1`` (any
     length up to ``max_seqlen``).  Returns the context ``[rows, heads * head_dim]`` (rows of no sequence stay zero),
-    and with ``out_scale`` its int8 copy."""
+    and with ``out_scale`` its int8 copy.  ``keys``: see ``flash_attention``; by default ``max_seqlen`` counts for the tiles,
+    whatever the lengths."""
     _require(qkv, "qkv", torch.float16, 2)
     _require(cu_seqlens, "cu_seqlens", torch.int32, 1, like=qkv)
     hidden = heads * head_dim
@@ -845,8 +859,8 @@ def flash_attention_unpadded(qkv, cu_seqlens, heads: int, head_dim: int, max_seq
     ctxq = torch.zeros((rows, hidden), dtype=torch.int8, device=qkv.device) if out_scale is not None else None
     B = cu_seqlens.numel() - 1
     e = qkv.element_size()
-    _call("zen_flash_attention_unpadded_f16", qkv.data_ptr(), qkv.data_ptr() + hidden * e, qkv.data_ptr() + 2 * hidden * e,
+    _call("zen_flash_attention_unpadded_f16_ex", qkv.data_ptr(), qkv.data_ptr() + hidden * e, qkv.data_ptr() + 2 * hidden * e,
           ctx.data_ptr(), _ptr(ctxq), float(out_scale or 1.0), B, heads, int(max_seqlen), head_dim, rows, 3 * hidden, head_dim,
           3 * hidden, head_dim, 3 * hidden, head_dim, hidden, head_dim, cu_seqlens.data_ptr(), 1 if causal else 0,
-          float(1.0 / math.sqrt(head_dim) if scale is None else scale), _stream())
+          float(1.0 / math.sqrt(head_dim) if scale is None else scale), _keys_flag(keys), _stream())
     return ctx if ctxq is None else (ctx, ctxq)
