@@ -3,7 +3,7 @@
 //   * flash_attn_short_kernel (flash_attn_short.cuh): sequences of at most 128 keys, several (head, batch) items per SM;
 //   * flash_attn_pipe_kernel (flash_attn_pipe.cuh): longer sequences, one or two query tiles per CTA with an online softmax;
 //   * flash_attn_quad_kernel (flash_attn_quad.cuh): head size 64, tiles enough for four CTAs on every SM;
-//   * flash_attn_tri_kernel (flash_attn_tri.cuh): the same with an int8 copy, three CTAs.
+//   * flash_attn_tri_kernel (flash_attn_tri.cuh): the bits of flash_attn_pipe_kernel with three CTAs on every SM.
 //
 // Q, K, V, O are addressed through (batch, head, seq) strides with d contiguous, so both the
 // reference's [B, heads, S, d] tensors and column slices of a fused [tokens, 3*hidden] QKV
@@ -160,8 +160,13 @@ static bool attn_flags_ok(unsigned flags) { return flags <= ZEN_ATTN_KEYS_128; }
 // of its two CTAs an SM.  Measured for 50 shapes with int8 copy, time against the other kernel:
 //   full    up to 576 tiles 1.02 - 1.08; from 624 on S = 160 .. 384: 0.87 - 0.93, 512: 0.94 - 0.98, 700: 0.98 - 1.02, 1024: 0.99 - 1.06
 //   causal  up to 576 tiles 1.00 - 1.06; from 624 on S = 160 .. 512: 0.85 - 0.92, 700: 0.93 - 0.96, 1024: 0.95 - 0.98, 2048: 0.99
+// Without a copy the output, which the third CTA hides best, is shorter, and the line lies at shorter sequences (144 shapes of
+// 600 .. 2400 tiles; by default only the causal ones of 321 .. 1100 tokens and 593 .. 651 tiles come here, the others when
+// the call asks for 128 keys at a time):
+//   full    S = 160 .. 300: 0.88 - 0.97, 384: 0.95 - 0.98, 512: 0.97 - 1.02, 640: 0.99 - 1.04
+//   causal  S = 160 .. 640: 0.84 - 0.96, 700 .. 1024: 0.91 - 0.99, 1500: 0.98 - 1.04, 2048: 1.00 - 1.16
 static bool three_tiles_per_sm(int D, const FaParams& p) {
-  if (D != 64 || p.S > (p.causal ? 2048 : 640)) return false;
+  if (D != 64 || p.S > (p.oq != nullptr ? (p.causal ? 2048 : 640) : (p.causal ? 1100 : 512))) return false;
   return int64_t((p.S + 127) / 128) * p.H * p.B > 4 * num_sms();
 }
 
