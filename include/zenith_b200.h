@@ -33,6 +33,7 @@ extern "C" {
 #define ZEN_ERR_TIMEOUT 4       /* a bounded device-side wait ran out (device status word) */
 #define ZEN_ERR_DRIVER 5        /* tensor-map encoding entry point unavailable or failed */
 #define ZEN_ERR_TOO_LARGE 6     /* request exceeds a fixed capacity of the entry point */
+#define ZEN_ERR_NEEDS_WORKSPACE 7 /* a valid call that the one-launch (_direct) form does not take: call the form with a workspace */
 
 /* element types of GEMM outputs */
 #define ZEN_DT_S32 0
@@ -231,8 +232,10 @@ size_t zen_matmul_f32_workspace_bytes(int N, int K);
 int zen_matmul_f32(const float* A, const float* B, float* C, int M, int N, int K, void* workspace,
                    size_t workspace_bytes, void* stream);
 
-/* zen_matmul_f32 without a workspace, in one launch, for products whose B the kernel transposes on its way in (where that is
- * the faster form; zen_matmul_f32 takes it by itself): ZEN_ERR_TOO_LARGE for the others. */
+/* zen_matmul_f32 without a workspace, in one launch, for products whose B the kernel transposes on its way in.  Which these are is
+ * a rule of speed that may change with the library: a caller tries this form first and, on ZEN_ERR_NEEDS_WORKSPACE (nothing has
+ * been launched then), calls zen_matmul_f32 with a workspace; one that has a workspace in any case calls zen_matmul_f32, which
+ * tries by itself. */
 int zen_matmul_f32_direct(const float* A, const float* B, float* C, int M, int N, int K, void* stream);
 
 /* The same product as zen_matmul_f32 for callers that have no way to provide a workspace.  It has no
@@ -339,8 +342,9 @@ int zen_flash_attention_f32(const float* q, const float* k, const float* v, floa
                             const int32_t* kv_lens, int causal, float scale, void* workspace, size_t workspace_bytes,
                             void* stream);
 
-/* zen_flash_attention_f32 without a workspace, in one launch, where that is the faster form: ZEN_ERR_TOO_LARGE elsewhere, and for
- * q, k or v off a 16-byte boundary. */
+/* zen_flash_attention_f32 without a workspace, in one launch, where that is the faster form (a rule that may change with the
+ * library).  ZEN_ERR_NEEDS_WORKSPACE elsewhere, and for q, k or v off a 16-byte boundary: nothing has been launched, and
+ * zen_flash_attention_f32 with a workspace takes the call. */
 int zen_flash_attention_f32_direct(const float* q, const float* k, const float* v, float* o, int B, int H, int S, int D,
                                    const int32_t* kv_lens, int causal, float scale, void* stream);
 

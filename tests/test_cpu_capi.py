@@ -59,6 +59,19 @@ def test_argument_validation_needs_no_device():
     assert lib.zen_gelu_f32(z, z, 0, z) == 0 and lib.zen_layernorm_f16(z, z, z, z, 0, 8, 1e-5, z) == 0
 
 
+def test_one_launch_forms_name_what_they_do_not_take():
+    """A valid call that needs the form with a workspace has a status of its own, whether size or alignment is the reason, and
+    one that no form takes is refused as by the other form."""
+    lib, z, one, odd = _capi.lib(), None, ctypes.c_void_p(16), ctypes.c_void_p(20)  # never dereferenced: nothing is launched
+    needs = _capi.ERR_NEEDS_WORKSPACE
+    assert lib.zen_matmul_f32_direct(one, one, one, 4096, 4096, 64, z) == needs
+    assert lib.zen_matmul_f32_direct(one, one, one, 4096, 4096, 63, z) == _capi.ERR_UNSUPPORTED
+    attn = lambda q, k, o, S, D: lib.zen_flash_attention_f32_direct(q, k, one, o, 4, 64, S, D, z, 0, 1.0, z)
+    assert attn(one, one, one, 4096, 64) == attn(odd, one, one, 100, 64) == attn(one, odd, one, 100, 128) == needs
+    assert attn(one, one, odd, 100, 64) == attn(one, one, one, 100, 32) == _capi.ERR_UNSUPPORTED
+    assert "workspace" in _capi.status_string(needs) and _capi.status_string(needs) != _capi.status_string(_capi.ERR_TOO_LARGE)
+
+
 def test_operators_refuse_cpu_tensors():
     import torch
 

@@ -13,7 +13,7 @@ from pathlib import Path
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libzenith_b200.so"
 NATIVE_PATH = LIB_PATH.parent / "_native.so"
 
-OK, ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_LAUNCH, ERR_TIMEOUT, ERR_DRIVER, ERR_TOO_LARGE = range(7)
+OK, ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_LAUNCH, ERR_TIMEOUT, ERR_DRIVER, ERR_TOO_LARGE, ERR_NEEDS_WORKSPACE = range(8)
 DT_S32, DT_F32, DT_F16, DT_S8 = range(4)
 ACT_NONE, ACT_GELU, ACT_RELU = range(3)
 ROUND_NEAREST_EVEN, ROUND_TRUNC = range(2)

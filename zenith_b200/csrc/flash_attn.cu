@@ -309,7 +309,7 @@ extern "C" int zen_flash_attention_f32_direct(const float* q, const float* k, co
   if (H > 65535 || B > 65535) return ZEN_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(o) % 16) return ZEN_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) % 16 || !f32_in_one_launch(B, H, S, D))
-    return ZEN_ERR_TOO_LARGE;
+    return ZEN_ERR_NEEDS_WORKSPACE;
   FaParams p{};
   p.o = o; p.o_f32 = 1; p.q32 = q; p.k32 = k; p.v32 = v; p.B = B; p.H = H; p.S = S;
   p.o_sb = int64_t(H) * S * D; p.o_sh = int64_t(S) * D; p.o_ss = D; p.kv_lens = kv_lens; p.causal = causal ? 1 : 0;
@@ -332,7 +332,7 @@ extern "C" int zen_flash_attention_f32(const float* q, const float* k, const flo
   if (workspace_bytes < zen_flash_attention_f32_workspace_bytes(B, H, S, D)) return ZEN_ERR_INVALID_ARG;
   // (the operands may lie anywhere: the conversion has a form for them)
   if (reinterpret_cast<uintptr_t>(o) % 16 || reinterpret_cast<uintptr_t>(workspace) % 16) return ZEN_ERR_UNSUPPORTED;
-  if (const int st = zen_flash_attention_f32_direct(q, k, v, o, B, H, S, D, kv_lens, causal, scale, stream); st != ZEN_ERR_TOO_LARGE) return st;
+  if (const int st = zen_flash_attention_f32_direct(q, k, v, o, B, H, S, D, kv_lens, causal, scale, stream); st != ZEN_ERR_NEEDS_WORKSPACE) return st;
   const int64_t n = int64_t(B) * H * S * D;
   if (int st = zen_convert3_f32_to_f16(q, k, v, workspace, n, stream); st != ZEN_OK) return st;
   const __half* w = static_cast<const __half*>(workspace);

@@ -241,6 +241,7 @@ const char* zen_status_string(int s) {
     case ZEN_ERR_TIMEOUT: return "a bounded device-side wait ran out";
     case ZEN_ERR_DRIVER: return "tensor-map encoding unavailable or failed";
     case ZEN_ERR_TOO_LARGE: return "request exceeds a fixed capacity";
+    case ZEN_ERR_NEEDS_WORKSPACE: return "this call needs the form with a workspace";
     default: return "unknown status";
   }
 }
@@ -387,7 +388,7 @@ int zen_matmul_f32_direct(const float* A, const float* B, float* C, int M, int N
   if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return ZEN_ERR_INVALID_ARG;
   if (K % 4) return ZEN_ERR_UNSUPPORTED;
   const int ks = small_rule_f32_kn(M, N, K);
-  if (ks <= 0) return ZEN_ERR_TOO_LARGE;
+  if (ks <= 0) return ZEN_ERR_NEEDS_WORKSPACE;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.out = C; p.ldo = N; p.out_dtype = ZEN_DT_F32; p.act = ZEN_ACT_NONE;
@@ -402,7 +403,7 @@ int zen_matmul_f32(const float* A, const float* B, float* C, int M, int N, int K
   if (workspace_bytes < zen_matmul_f32_workspace_bytes(N, K) || reinterpret_cast<uintptr_t>(workspace) % 16)
     return ZEN_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const int st = zen_matmul_f32_direct(A, B, C, M, N, K, stream); st != ZEN_ERR_TOO_LARGE) return st;
+  if (const int st = zen_matmul_f32_direct(A, B, C, M, N, K, stream); st != ZEN_ERR_NEEDS_WORKSPACE) return st;
   float* Bt = static_cast<float*>(workspace);
   int st = launch_transpose_f32(B, Bt, K, N, s);
   if (st != ZEN_OK) return st;
@@ -445,7 +446,7 @@ int zen_matmul_f32_static(const float* A, const float* B, float* C, int M, int N
   if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return ZEN_ERR_INVALID_ARG;
   if (K % 4) return ZEN_ERR_UNSUPPORTED;
   if (size_t(N) * size_t(K) > size_t(ZEN_MATMUL_STATIC_MAX_ELEMS)) return ZEN_ERR_TOO_LARGE;
-  if (const int st = zen_matmul_f32_direct(A, B, C, M, N, K, stream); st != ZEN_ERR_TOO_LARGE) return st;
+  if (const int st = zen_matmul_f32_direct(A, B, C, M, N, K, stream); st != ZEN_ERR_NEEDS_WORKSPACE) return st;
   float* Bt = nullptr;
   int st = scratch_for_current_device(&Bt);
   if (st != ZEN_OK) return st;

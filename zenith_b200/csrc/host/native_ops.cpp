@@ -340,7 +340,7 @@ PyObject* matmul_f32(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const float *pa = static_cast<const float*>(x->const_data_ptr()), *pb = static_cast<const float*>(y->const_data_ptr());
     float* pc = static_cast<float*>(o[0].data_ptr());
     const int st = zen_matmul_f32_direct(pa, pb, pc, int(M), int(N), int(K), stream_of(dev));
-    if (st != ZEN_ERR_TOO_LARGE) return st == ZEN_OK;
+    if (st != ZEN_ERR_NEEDS_WORKSPACE) return st == ZEN_OK;
     kernels = 2;
     const size_t bytes = zen_matmul_f32_workspace_bytes(int(N), int(K));
     at::Tensor ws = empty({int64_t(bytes)}, at::kByte, dev);
@@ -385,7 +385,7 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                 *pv = static_cast<const float*>(v->const_data_ptr());
     float* po = static_cast<float*>(o[0].data_ptr());
     const int one = zen_flash_attention_f32_direct(pq, pk, pv, po, int(B), int(H), int(S), int(D), lens, causal, float(scale), s);
-    if (one != ZEN_ERR_TOO_LARGE) return one == ZEN_OK;
+    if (one != ZEN_ERR_NEEDS_WORKSPACE) return one == ZEN_OK;
     kernels = 2;
     const size_t bytes = zen_flash_attention_f32_workspace_bytes(int(B), int(H), int(S), int(D));
     at::Tensor ws = empty({int64_t(bytes)}, at::kByte, dev);

@@ -317,7 +317,7 @@ def matmul_f32(a, b):
     c = torch.empty((M, N), dtype=torch.float32, device=a.device)
     if M and N:
         st = _capi.lib().zen_matmul_f32_direct(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, _stream())
-        if st != _capi.ERR_TOO_LARGE:
+        if st != _capi.ERR_NEEDS_WORKSPACE:
             _capi.check("zen_matmul_f32_direct", st)
             launch_count_add(1)
             return c
@@ -621,7 +621,7 @@ def flash_attention(q, k, v, *, causal: bool = False, kv_lens=None, scale: float
         scale = float(1.0 / math.sqrt(D) if scale is None else scale)
         st = _capi.lib().zen_flash_attention_f32_direct(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, S, D, _ptr(kv_lens),
                                                         1 if causal else 0, scale, _stream())
-        if st != _capi.ERR_TOO_LARGE:
+        if st != _capi.ERR_NEEDS_WORKSPACE:
             _capi.check("zen_flash_attention_f32_direct", st)
             launch_count_add(1)
             return out
