@@ -331,12 +331,15 @@ def test_a_recording_that_fails_is_closed(cuda, params, error):
     assert enc._pass_graph is not None  # another shape in between: recorded anew
 
 
-def test_a_pass_goes_into_the_callers_recording(cuda, params):
-    """Between zen_record_begin and zen_record_end of the caller, whatever call it is that would record itself."""
+@pytest.mark.parametrize("calls_before", [2, 3, 6])
+def test_a_pass_goes_into_the_callers_recording(cuda, params, calls_before):
+    """Between zen_record_begin and zen_record_end of the caller, whatever call it is: one that would record itself (the third),
+    or that would launch what an earlier one has recorded."""
     enc = Fp16Encoder(CFG, params, cuda)
     ids, lens = tdev(rng(8).integers(0, CFG.vocab, (2, 40)).astype(np.int32), np.array([40, 17], np.int32), cuda)
     want = enc.forward(ids, lens).clone()
-    enc.forward(ids, lens)
+    for _ in range(calls_before - 1):
+        enc.forward(ids, lens)
     lib, graph = _capi.lib(), ctypes.c_void_p()
     assert lib.zen_record_begin() == _capi.OK and lib.zen_record_begin() == _capi.ERR_INVALID_ARG
     out = enc.forward(ids, lens)
@@ -347,6 +350,8 @@ def test_a_pass_goes_into_the_callers_recording(cuda, params):
     _capi.call("zen_graph_launch", graph, torch.cuda.current_stream().cuda_stream)
     assert torch.equal(out, want)
     _capi.call("zen_graph_destroy", graph)
+    for _ in range(4):  # and plain calls go on
+        assert torch.equal(enc.forward(ids, lens), want)
 
 
 def other_threads_work():

@@ -102,8 +102,13 @@ class _RecordedPass:
         self._handle = handle
         self._destroy = _capi.lib().zen_graph_destroy
 
-    def launch(self, stream: int) -> None:
-        _capi.check("zen_graph_launch", _capi.lib().zen_graph_launch(self._handle, stream))
+    def launch(self, stream: int) -> bool:
+        """False, with nothing launched, while the thread records: a graph is no node of a recording."""
+        status = _capi.lib().zen_graph_launch(self._handle, stream)
+        if status == _capi.ERR_UNSUPPORTED:
+            return False
+        _capi.check("zen_graph_launch", status)
+        return True
 
     def __del__(self):
         self._destroy(self._handle)
@@ -268,7 +273,7 @@ class _EncoderBase:
         """One pass for ``forward`` / ``forward_unpadded``.  Issuing 49 and more calls one by one costs the host 340 us,
         more than a short batch takes on the device (BERT-base W8A8, one 24-token sequence: 300 us), so from the third
         consecutive call for a shape on the pass is one graph of the same launches.  That third call also pays for the
-        recording.  Inside a caller's own stream capture the launches are issued as they are."""
+        recording.  Inside a caller's own stream capture or recording the launches are issued as they are."""
         if torch.cuda.is_current_stream_capturing():
             self._run()
             return
@@ -276,10 +281,9 @@ class _EncoderBase:
             self._plain_calls += 1
             if self._plain_calls == 3:
                 self._pass_graph = self._record()
-        if self._pass_graph is None:
+        if self._pass_graph is None or not self._pass_graph.launch(torch.cuda.current_stream().cuda_stream):
             self._run()
             return
-        self._pass_graph.launch(torch.cuda.current_stream().cuda_stream)
         ops.launch_count += self.kernels_per_forward
 
     def _record(self) -> "_RecordedPass | None":
