@@ -149,6 +149,33 @@ def test_operators_refuse_vectors_that_a_kernel_would_read_past(monkeypatch):
             ops.embed_layernorm(ids, ids, word, pos, typ[:1], h, h, 1e-5, 16)
 
 
+@pytest.mark.parametrize("name,dtype", [("wmma_matmul", "float16"), ("matmul_f32", "float32")])
+def test_products_copy_each_strided_operand_once(monkeypatch, name, dtype):
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from zenith_b200 import ops
+
+    copies = []
+
+    class Count(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func is torch.ops.aten.clone.default:
+                copies.append(tuple(args[0].shape))
+            return func(*args, **(kwargs or {}))
+
+    def no_device():
+        raise InterruptedError
+
+    monkeypatch.setattr(ops, "_stream", no_device)  # asked for after the copies, in front of the launch
+    with FakeTensorMode():
+        a, b = (torch.empty(s, dtype=getattr(torch, dtype), device="cuda:0").t() for s in ((64, 48), (32, 64)))
+        with Count(), pytest.raises(InterruptedError):
+            getattr(ops, name)(a, b)
+    assert sorted(copies) == [(48, 64), (64, 32)]
+
+
 def test_missing_extension_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_capi, "_lib", None)
     monkeypatch.setattr(_capi, "LIB_PATH", tmp_path / "absent.so")

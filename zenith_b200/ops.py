@@ -280,9 +280,9 @@ def wmma_matmul(a, b):
         raise RuntimeError("Inputs must be FP16")
     if a.shape[1] != b.shape[0]:
         raise RuntimeError("Inner dimensions must match")
-    _require(b.contiguous(), "B", like=a)
     a = a.contiguous()
     b = b.contiguous()
+    _require(b, "B", like=a)
     M, K = a.shape
     N = b.shape[1]
     c = torch.empty((M, N), dtype=torch.float32, device=a.device)
@@ -308,8 +308,8 @@ def matmul_f32(a, b):
         raise RuntimeError("Inputs must be 2D")
     if a.shape[1] != b.shape[0]:
         raise RuntimeError("Inner dimensions must match")
-    _require(a.contiguous(), "A", torch.float32)
     a = a.contiguous()
+    _require(a, "A", torch.float32)
     b = b.contiguous()
     _require(b, "B", torch.float32, like=a)
     M, K = a.shape
