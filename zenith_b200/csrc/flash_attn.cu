@@ -124,15 +124,20 @@ static int launch_fa_short(const CUtensorMap& tq, const CUtensorMap& tk, const C
   return launch_pdl(PDL_ATTENTION, kernel, dim3(grid), dim3(fas_threads<D>()), smem, s, tq, tk, tv, p);
 }
 
-template <int D, int GROUPS, int KV_STAGES, bool F32 = false>
-static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
-                          cudaStream_t s) {
-  auto kernel = flash_attn_pipe_kernel<D, GROUPS, KV_STAGES, F32>;
-  constexpr size_t smem = fap_smem_bytes<D, GROUPS, KV_STAGES>();
+// A kernel of `rows` query rows per CTA.
+using FaKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FaParams);
+static int launch_fa_tiles(FaKernel kernel, int rows, int threads, size_t smem, const CUtensorMap& tq, const CUtensorMap& tk,
+                           const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
   if (int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem); st != ZEN_OK) return st;
-  const int64_t ctas = int64_t((p.S + 128 * GROUPS - 1) / (128 * GROUPS)) * p.H * p.B;
+  const int64_t ctas = int64_t((p.S + rows - 1) / rows) * p.H * p.B;
   if (ctas >= (int64_t(1) << 31)) return ZEN_ERR_UNSUPPORTED;
-  return launch_pdl(PDL_ATTENTION, kernel, dim3(unsigned(ctas)), dim3(fap_threads<GROUPS, F32>()), smem, s, tq, tk, tv, p);
+  return launch_pdl(PDL_ATTENTION, kernel, dim3(unsigned(ctas)), dim3(unsigned(threads)), smem, s, tq, tk, tv, p);
+}
+
+template <int D, int GROUPS, int KV_STAGES, bool F32 = false>
+static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
+  return launch_fa_tiles(flash_attn_pipe_kernel<D, GROUPS, KV_STAGES, F32>, 128 * GROUPS, fap_threads<GROUPS, F32>(),
+                         fap_smem_bytes<D, GROUPS, KV_STAGES>(), tq, tk, tv, p, s);
 }
 
 // Head size 64: flash_attn_quad_kernel, where its tiles keep four CTAs on every SM.  With fewer its chains are longer than those
@@ -188,14 +193,6 @@ static bool one_tile_per_cta(const FaParams& p) {
   return last > 0.0 && last <= 0.5;
 }
 
-static int launch_fa_quad(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
-  constexpr size_t smem = faq_smem_bytes();
-  if (int st = ensure_dynamic_smem(reinterpret_cast<const void*>(flash_attn_quad_kernel), smem); st != ZEN_OK) return st;
-  const int64_t ctas = int64_t((p.S + 127) / 128) * p.H * p.B;
-  if (ctas >= (int64_t(1) << 31)) return ZEN_ERR_UNSUPPORTED;
-  return launch_pdl(PDL_ATTENTION, flash_attn_quad_kernel, dim3(unsigned(ctas)), dim3(FAQ_THREADS), smem, s, tq, tk, tv, p);
-}
-
 // The tiles that run at a time should share K and V while those are in L2: with heads and batches before tiles every CTA of a
 // wave streams another head's K and V, from HBM where all heads' do not fit L2 (8 x 16 x 8192 x 128: 537 MB, 32 times; the
 // power that this takes is what the chip's clock lacks then).  Measured with K and V of 39 .. 537 MB, time against heads, batches,
@@ -211,20 +208,12 @@ static int tile_order(int D, const FaParams& p) {
   return D == 128 || kv_mb > 100 ? FA_ORDER_TILES_HEADS : FA_ORDER_HEADS_BATCHES;
 }
 
-static int launch_fa_tri(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p, cudaStream_t s) {
-  constexpr size_t smem = fat_smem_bytes();
-  if (int st = ensure_dynamic_smem(reinterpret_cast<const void*>(flash_attn_tri_kernel), smem); st != ZEN_OK) return st;
-  const int64_t ctas = int64_t((p.S + 127) / 128) * p.H * p.B;
-  if (ctas >= (int64_t(1) << 31)) return ZEN_ERR_UNSUPPORTED;
-  return launch_pdl(PDL_ATTENTION, flash_attn_tri_kernel, dim3(unsigned(ctas)), dim3(FAT_THREADS), smem, s, tq, tk, tv, p);
-}
-
 // `quad`: four_tiles_per_sm, for which the boxes of K and V were made.
 static int launch_fa_long(int D, bool quad, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FaParams p, cudaStream_t s) {
   p.order = tile_order(D, p);
   if (D == 128) return launch_fa_pipe<128, 2, 2>(tq, tk, tv, p, s);
-  if (quad) return launch_fa_quad(tq, tk, tv, p, s);
-  if (three_tiles_per_sm(D, p)) return launch_fa_tri(tq, tk, tv, p, s);
+  if (quad) return launch_fa_tiles(flash_attn_quad_kernel, 128, FAQ_THREADS, faq_smem_bytes(), tq, tk, tv, p, s);
+  if (three_tiles_per_sm(D, p)) return launch_fa_tiles(flash_attn_tri_kernel, 128, FAT_THREADS, fat_smem_bytes(), tq, tk, tv, p, s);
   return one_tile_per_cta(p) ? launch_fa_pipe<64, 1, 2>(tq, tk, tv, p, s) : launch_fa_pipe<64, 2, 3>(tq, tk, tv, p, s);
 }
 

@@ -91,6 +91,46 @@ __device__ __forceinline__ void fa_tile(const FaParams& p, int q_tiles, int& b, 
   if (p.causal) qt = q_tiles - 1 - qt;
 }
 
+// The sequence of a tile: its keys and query rows, and where the tensor maps find them.
+// Unpadded batches: the sequences lie back to back in one [rows, ...] tensor, sequence b in rows cu_seqlens[b] ..
+// cu_seqlens[b + 1] - 1 (cut at the tensor's rows).  A tile then starts at the sequence's first row and may run on
+// into the next sequence's rows: as keys they lie beyond the key length and are masked like padding, as queries
+// their rows are not stored.  The tensor maps see one batch of `rows` tokens.
+struct FaSequence {
+  int kv_len;    // keys
+  int q_len;     // query rows
+  int row_base;  // first row in the packed tensors
+  int tma_b;     // batch coordinate
+};
+__device__ __forceinline__ FaSequence fa_sequence(const FaParams& p, int b) {
+  FaSequence s{p.kv_lens ? p.kv_lens[b] : p.S, p.S, 0, b};
+  if (p.cu_seqlens != nullptr) {
+    const int lo = p.cu_seqlens[b], hi = p.cu_seqlens[b + 1];
+    s.kv_len = lo < 0 ? 0 : (hi < p.rows ? hi : p.rows) - lo;
+    s.row_base = lo < 0 ? 0 : lo;
+    s.tma_b = 0;
+  }
+  s.kv_len = s.kv_len < 0 ? 0 : (s.kv_len > p.S ? p.S : s.kv_len);
+  if (p.cu_seqlens != nullptr) s.q_len = s.kv_len;
+  return s;
+}
+
+// The warp's rows of O scaled by each thread's alpha (16 columns at a time: the row of S occupies most of a thread's registers).
+// The stores are not waited for.
+template <int D>
+__device__ __forceinline__ void fa_rescale(uint32_t tmem_o, float alpha) {
+#pragma unroll 1
+  for (int c = 0; c < D; c += 16) {
+    uint32_t ov[16];
+    __syncwarp();
+    tmem_ld_32x16(tmem_o + c, ov);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+    tmem_st_32x16(tmem_o + c, ov);
+  }
+}
+
 // Output of one warp's 32 query rows (first row `qr0` of the sequence): O / l into the warp's part of the dead Q tile
 // (`stage`, + dc * 16 KB per 64 columns: 32 rows x 128 bytes, 16-byte units swizzled), then to global memory as whole
 // 128-byte lines, eight lanes per row piece, with the int8 copy beside it.  Only rows below q_len are stored.
@@ -296,21 +336,8 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   const uint32_t tmem_base = *tmem_slot;
   grid_dependency_wait();  // Q, K, V, the key lengths and the output buffers may belong to the previous kernel until here
   grid_launch_dependents();
-  int kv_len = p.kv_lens ? p.kv_lens[b] : p.S;
-  // Unpadded batches: the sequences lie back to back in one [rows, ...] tensor, sequence b in rows cu_seqlens[b] ..
-  // cu_seqlens[b + 1] - 1 (cut at the tensor's rows).  A tile then starts at the sequence's first row and may run on
-  // into the next sequence's rows: as keys they lie beyond the key length and are masked like padding, as queries
-  // their rows are not stored.  The tensor maps see one batch of `rows` tokens.
-  int row_base = 0;  // first row of this sequence in the packed tensors
-  int tma_b = b;
-  if (p.cu_seqlens != nullptr) {
-    const int lo = p.cu_seqlens[b], hi = p.cu_seqlens[b + 1];
-    kv_len = lo < 0 ? 0 : (hi < p.rows ? hi : p.rows) - lo;
-    row_base = lo < 0 ? 0 : lo;
-    tma_b = 0;
-  }
-  kv_len = kv_len < 0 ? 0 : (kv_len > p.S ? p.S : kv_len);
-  const int q_len = p.cu_seqlens != nullptr ? kv_len : p.S;  // query rows of this sequence
+  const FaSequence seq = fa_sequence(p, b);
+  const int kv_len = seq.kv_len, q_len = seq.q_len, row_base = seq.row_base, tma_b = seq.tma_b;
   // key blocks needed by each group (a group has none if the sequence ends before its tile)
   int nblk[GROUPS];
   int n_blocks = 0;
@@ -532,17 +559,7 @@ flash_attn_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         tc_fence_after_sync();
       }
       if (rescale) {
-        // (16 columns at a time: the row of S occupies most of the thread's registers)
-#pragma unroll 1
-        for (int c = 0; c < D / 16; ++c) {
-          uint32_t ov[16];
-          __syncwarp();
-          tmem_ld_32x16(tmem_o + c * 16, ov);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-          tmem_st_32x16(tmem_o + c * 16, ov);
-        }
+        fa_rescale<D>(tmem_o, alpha);
         tmem_wait_st();
         l_run *= alpha;
       }

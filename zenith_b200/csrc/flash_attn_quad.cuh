@@ -90,18 +90,8 @@ flash_attn_quad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   const uint32_t tmem_base = *tmem_slot;
   grid_dependency_wait();  // Q, K, V, the key lengths and the output buffers may belong to the previous kernel until here
   grid_launch_dependents();
-  int kv_len = p.kv_lens ? p.kv_lens[b] : p.S;
-  // Unpadded batches: as in flash_attn_pipe_kernel
-  int row_base = 0;
-  int tma_b = b;
-  if (p.cu_seqlens != nullptr) {
-    const int lo = p.cu_seqlens[b], hi = p.cu_seqlens[b + 1];
-    kv_len = lo < 0 ? 0 : (hi < p.rows ? hi : p.rows) - lo;
-    row_base = lo < 0 ? 0 : lo;
-    tma_b = 0;
-  }
-  kv_len = kv_len < 0 ? 0 : (kv_len > p.S ? p.S : kv_len);
-  const int q_len = p.cu_seqlens != nullptr ? kv_len : p.S;  // query rows of this sequence
+  const FaSequence seq = fa_sequence(p, b);
+  const int kv_len = seq.kv_len, q_len = seq.q_len, row_base = seq.row_base, tma_b = seq.tma_b;
   const int key_end = p.causal && q0 + 128 < kv_len ? q0 + 128 : kv_len;
   const int nb = q0 < q_len ? (key_end + FAQ_KEYS - 1) / FAQ_KEYS : 0;
 
@@ -199,17 +189,8 @@ flash_attn_quad_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         const float m_use = m_new == -INFINITY ? 0.f : m_new;
         m_ref = m_new;
         if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-          // (P V of the previous block completed before S did; 16 columns at a time: the row of S occupies the registers)
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t ov[16];
-            __syncwarp();
-            tmem_ld_32x16(tmem_o + c * 16, ov);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-            tmem_st_32x16(tmem_o + c * 16, ov);
-          }
+          // (P V of the previous block completed before S did)
+          fa_rescale<64>(tmem_o, alpha);
           l_run *= alpha;
         }
         // probabilities -> tensor memory (fp16 pairs), row sum
