@@ -227,6 +227,8 @@ int zen_wmma_matmul_f16(const void* A, const void* B, float* C, int M, int N, in
  * handle runs in TF32 math mode, core/include/zenith/cublas_ops.hpp:51).  B is transposed by the kernel
  * (zen_matmul_f32_direct), in the larger products first into `workspace` (at least zen_matmul_f32_workspace_bytes(N, K) bytes of device memory, 16-byte
  * aligned, caller-owned).  K a multiple of 4.
+ * K is split by M, N and K here and in zen_linear_f32, by different rules: the fp32 sums of one product are ordered differently
+ * in zen_matmul_f32(a, b), in zen_linear_f32(a, b^T) and in batches of another size (last bits; every order is as precise).
  * Replaces zenith::cuda_kernels::matmul_f32, core/src/cuda_kernels.cu:297-336 (zenith_cuda.matmul). */
 size_t zen_matmul_f32_workspace_bytes(int N, int K);
 int zen_matmul_f32(const float* A, const float* B, float* C, int M, int N, int K, void* workspace,

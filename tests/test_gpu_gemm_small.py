@@ -10,6 +10,7 @@ from zenith_b200 import _capi, ops
 from zenith_b200._capi import ACT_GELU, ACT_NONE, DT_F16, DT_F32, DT_S8, DT_S32, GEMM_NARROW, gemm_split_k
 
 pytestmark = pytest.mark.gpu
+# the kernel's two forms (K split two and four ways) under all the names that the flags have for them
 FORMS = [gemm_split_k(k) for k in (1, 2, 4, 8)] + [gemm_split_k(k) | GEMM_NARROW for k in (1, 2, 4)]
 
 

@@ -148,7 +148,8 @@ static int launch_fa_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CU
 //           S = 1024, 1500, 2048, 3000: below 1 from 1.5, 1.7, 2.2, 2.9 on, 0.94 - 0.98 at most; 4096 and longer: 1.02 - 1.2
 //   causal  S <= 300: 0.7: 0.89 - 1.11, 0.8 - 1: 0.76 - 0.99, 3 on: 0.70 - 0.77    384 .. 1024: 0.7 - 1: 1.01 - 1.3, 1.1: 0.84 - 1.07,
 //           3 on: 0.77 - 0.87    1500 .. 4096: below 1 from 1.5, 2, 2.2, 2.2 on, 0.9 - 0.95 from 3 on; longer: 1.03 - 1.1
-// (32 x 16 x 384 full: 44.2 -> 37.6 us; 8 x 16 x 2048 causal: 113.5 -> 105.5 us.)  The two kernels differ in the last bits, which
+// (In short runs 32 x 16 x 384 full 43.8 -> 38.0 us, 8 x 16 x 2048 causal 110.7 -> 99.8; in a stream of passes, where the chip is at
+// its power limit, 43.5 -> 39.7 and 118.5 -> 114.6 at 1965 and 1807, 1792 and 1702 MHz.)  The two kernels differ in the last bits, which
 // a pass of int8 layers blows up to 3 % of its output (a value moved across a rounding boundary moves others): results with
 // an int8 copy stay with one kernel, whatever the batch.  `flags`: ZEN_ATTN_KEYS_64 / _128 of the call.
 static bool four_tiles_per_sm(int B, int H, int S, int D, bool causal, bool int8_copy, unsigned flags) {
@@ -201,7 +202,8 @@ static bool one_tile_per_cta(const FaParams& p) {
 //           d = 64 0.89 - 0.94 at 268 MB (0.92 - 0.95), 0.97 at 134 MB (0.97), 0.98 - 1.04 below
 //   causal  heads, tiles, batches: d = 128 0.93 - 1.01 (32 x 16 x 384 0.93, 8 x 16 x 2048 0.95), d = 64 1.00 - 1.23 up to 134 MB, then
 //           0.95 - 1.00; tiles innermost 0.93 - 1.27: tiles start from the longest on, and the longest of the last heads start late
-// (8 x 16 x 8192 x 128: 4069 -> 3160 us.)
+// (In short runs 8 x 16 x 8192 x 128 3892 -> 3164 us, 4 x 16 x 4096 x 128 462 -> 415, 8 x 16 x 2048 x 128 causal 156 -> 145; in a
+// stream of passes, all at 985 W, 4695 -> 3600 at 1025 and 1440 MHz, 541 -> 476 at 1305 and 1470, 183 -> 169 at 1455 and 1567.)
 static int tile_order(int D, const FaParams& p) {
   const double kv_mb = 4e-6 * p.B * p.H * double(p.S) * D;
   if (p.causal) return D == 128 || kv_mb > 200 ? FA_ORDER_HEADS_TILES : FA_ORDER_HEADS_BATCHES;

@@ -11,10 +11,11 @@
 // of shared memory and 128 columns of tensor memory a CTA.  P lies over S (its thread has taken the row into registers), so
 // Q K^T of block j + 1 follows P V of block j; the other three tiles work meanwhile.
 //
-// Measured against flash_attn_pipe_kernel: 32 x 16 heads x 384 44.2 -> 37.6 us, 48 x 12 x 256 25.0 -> 21.0 (causal 23.0 ->
-// 18.4), 40 x 12 x 160 22.7 -> 16.0, 8 x 16 x 2048 causal 113.5 -> 105.5.  Slower were: three CTAs with P in columns of its own, so that Q K^T runs under the
-// softmax (39.4, 22.4 (28.8), 113 us); CTAs that take their next tile by cluster launch control and load ahead into it (39.8,
-// 23.9 (26.0), 123 us: longer code per block, spilled registers).
+// Measured against flash_attn_pipe_kernel in a stream of passes (short runs): 32 x 16 heads x 384 43.5 -> 39.7 us (43.8 -> 38.0),
+// 48 x 12 x 256 24.7 -> 20.8, causal 23.0 -> 18.2, 40 x 12 x 160 22.7 -> 15.8, 8 x 16 x 2048 causal 118.5 -> 114.6 (110.7 -> 99.8),
+// full 209 -> 210 (189 -> 186).  Slower were, where this took 37.6, 21.0 (causal 18.4) and 105.5 us: three CTAs with P in columns of its
+// own, so that Q K^T runs under the softmax (39.4, 22.4 (28.8), 113 us); CTAs that take their next tile by cluster launch
+// control and load ahead into it (39.8, 23.9 (26.0), 123 us: longer code per block, spilled registers).
 //
 // All of a tile's events form one cycle, so three kinds of barrier do: operands loaded, S complete (with it P V of the block
 // before), P complete (with it S read, hence the K tile and the V tile of the block before are free).

@@ -9,8 +9,8 @@
 // of 128 scores in registers allows (flash_attn_pipe_kernel); here a thread holds the first 64, passes over the second half
 // for its maximum, packs the first half's probabilities and reads the second half again: 124 registers.  P (64 columns) lies
 // over S (64), so that a CTA takes 128 columns of tensor memory, and 64 KB of shared memory, with one V tile.
-// Measured with int8 copy and key lengths against flash_attn_pipe_kernel: 48 x 12 x 256 36.0 -> 32.3 us, 32 x 16 x 384 58.7 ->
-// 54.0 (causal 52.3 -> 45.3), 40 x 12 x 160 29.6 -> 26.9.
+// Measured with int8 copy and key lengths against flash_attn_pipe_kernel in a stream of passes: 48 x 12 x 256 33.2 -> 29.5 us,
+// 32 x 16 x 384 53.5 -> 49.3 (causal 48.1 -> 40.9), 40 x 12 x 160 28.9 -> 26.0.
 //
 // The events of a tile form one cycle: S of the first half complete (with it P V of the block before, hence the V tile is
 // free), taken into registers, S of the second half complete, P complete (with it S read, hence the K tile is free).

@@ -19,8 +19,9 @@
 // 500 x 1000 x 768 took 9.2 us (6.5 now), 456 x 514 x 24 9.1 (5.2), 24 x 3072 x 768 10.7 (5.7).  What bounds the larger ones is the
 // operand traffic (288 KB an SM), the smaller ones one load's latency, the exchange and the launch.
 //
-// About 100 KB of shared memory and 64 TMEM columns per CTA, so that two CTAs fit on an SM and a kernel's CTAs become
-// resident (barriers, TMEM, constant weight tiles on their way) while the previous kernel in the stream still runs.
+// 92 to 112 KB of shared memory and 32 or 64 TMEM columns per CTA, so that two CTAs fit on an SM and a kernel's CTAs become
+// resident (barriers, TMEM, constant weight tiles on their way) while the previous kernel in the stream still runs.  The two
+// deeper rings for fp32 B [K, N] take 196 and 212 KB: one CTA per SM, which starts when the SM is free.
 #pragma once
 #include "gemm_tc.cuh"
 
