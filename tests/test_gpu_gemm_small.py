@@ -162,3 +162,25 @@ def test_fp32_matmul_transposes_b_on_its_way_in(cuda, M, N, K, offset):
     bound = (a.double().abs() @ b.double().abs()) * (2.0**-9 + 2.0**-15)
     assert bool(((c.double() - a.double() @ b.double()).abs() <= bound).all())
     assert _capi.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,direct", [(128, 1000, 4096, True), (860, 100, 2120, True), (385, 400, 96, True), (384, 352, 132, True),
+                                          (256, 544, 132, True), (384, 704, 264, True), (128, 2144, 264, True), (129, 2368, 512, True),
+                                          (129, 2369, 512, False), (128, 4736, 64, True), (128, 4737, 64, False), (1000, 1000, 68, False)])
+def test_fp32_matmul_at_the_lines_of_its_rule(cuda, M, N, K, direct):
+    """Which products are one launch, and their results: 32 and 28 tiles with more k-blocks than the deep ring has stages, 52 tiles of a
+    K that goes to 64 columns, 33 / 34 and 66 / 67 tiles of 128 x 32, 74 of 128 x 64 and one more.  The one launch's result is
+    zen_matmul_f32's, bit for bit; the bound against 64 bits as above."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines lie elsewhere")
+    a = torch.from_numpy(rng(M).standard_normal((M, K)).astype(np.float32)).to(cuda)
+    b = torch.from_numpy(rng(N).standard_normal((K, N)).astype(np.float32)).to(cuda)
+    one, c = (torch.full((M, N), float("nan"), device=cuda) for _ in range(2))
+    ws = torch.empty(4 * N * K, dtype=torch.uint8, device=cuda)
+    status = _capi.lib().zen_matmul_f32_direct(a.data_ptr(), b.data_ptr(), one.data_ptr(), M, N, K, torch.cuda.current_stream().cuda_stream)
+    assert status == (_capi.OK if direct else _capi.ERR_NEEDS_WORKSPACE)
+    call("zen_matmul_f32", a, b, c, M, N, K, ws, ws.numel())
+    bound = (a.double().abs() @ b.double().abs()) * (2.0**-9 + 2.0**-15)
+    assert bool(((c.double() - a.double() @ b.double()).abs() <= bound).all())
+    assert torch.equal(one, c) if direct else bool(one.isnan().all())
+    assert _capi.device_status() == 0
