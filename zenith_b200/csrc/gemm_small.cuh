@@ -15,7 +15,7 @@
 //
 // fp32 B [K, N] (TF32): the load engine cannot transpose, so the epilogue warps, idle until the accumulator is complete, bring
 // B in: a warp reads 32 columns of four rows (coalesced, at any alignment), each lane then holds four consecutive k of one
-// column and stores them as one 16-byte unit of the K-major tile, eight k-blocks ahead.  With a transposition launch in front
+// column and stores them as one 16-byte unit of the K-major tile, eight k-blocks ahead (four of 64 columns).  With a transposition launch in front
 // 500 x 1000 x 768 took 9.2 us (6.5 now), 456 x 514 x 24 9.1 (5.2), 24 x 3072 x 768 10.7 (5.7).  What bounds the larger ones is the
 // operand traffic (288 KB an SM), the smaller ones one load's latency, the exchange and the launch.
 //
